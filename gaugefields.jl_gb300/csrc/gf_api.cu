@@ -140,6 +140,7 @@ extern "C" int gf_ctx_destroy(gf_ctx* ctx) {
   for (int i = 0; i < 4; ++i) field_delete(ctx->w_mom[i]);
   field_delete(ctx->w_link32);
   field_delete(ctx->w_linkdf);
+  field_delete(ctx->w_linkfx);
   if (ctx->w_stout64) gf_stout_destroy(ctx->w_stout64);
   if (ctx->w_stout32) gf_stout_destroy(ctx->w_stout32);
   if (ctx->w_stoutdf) gf_stout_destroy(ctx->w_stoutdf);

@@ -2,6 +2,7 @@
 // hot starts, Gaussian momenta, field copies/conversions and the deterministic
 // two-stage reductions used by every global sum.
 #include "gf_internal.h"
+#include "fxlat.cuh"
 #include <vector>
 
 namespace gf {
@@ -16,6 +17,7 @@ size_t field_bytes(const Geom& g, int kind) {
     case GF_MAT64: return 4 * 9 * V * sizeof(double2);
     case GF_LINKDF:
     case GF_MATDF: return 4 * 9 * V * sizeof(float4);
+    case GF_LINKFX: return fx_field_bytes(V);
     case GF_LINK32: return 4 * 3 * V * sizeof(float4);
     case GF_MAT32: return 4 * 9 * V * sizeof(float2);
     case GF_MOM64: return 4 * 8 * V * sizeof(double);

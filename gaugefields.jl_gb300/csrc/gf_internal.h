@@ -43,6 +43,8 @@ void count_launch();
 // boundary.
 #define GF_LINKDF 101
 #define GF_MATDF 102
+// Fixed-point links and matrices (fxlat.cuh), internal too
+#define GF_LINKFX 103
 
 struct gf_field {
   gf_ctx* ctx;
@@ -70,6 +72,7 @@ struct gf_ctx {
   gf_field* w_mom[4];     // F0, F1, F2, Ftmp of the RK3 flow (fp64 coefficients)
   gf_field* w_link32;     // fp32 12-real shadow of the thin links (mixed form)
   gf_field* w_linkdf;     // double-float-native copy of the thin links (double-float rectangle force)
+  gf_field* w_linkfx;     // fixed-point copy of the links (fp64-class kernels)
   // Two scratch blocks of one fp64 link field each, shared by the mixed form's
   // internal stacks: the Hamiltonian's double-float level buffers and the
   // force adjoint's Z, Dp, D[0], D[1] (fp32). They are never live together:
@@ -172,6 +175,9 @@ void staple_up(gf_ctx* ctx, const gf_field* U, int mu, gf_field* V);  // constru
 // P <- keep * P + coef * TA-coefficients(U_mu * S_mu), S = sum of the six
 // staples (dS/dU order); keep = 0 overwrites P without reading it.
 void wilson_force_coef(gf_ctx* ctx, const gf_field* U, gf_field* P, double coef, double keep, bool df = false);
+
+// the same on fp64 links in fixed-point arithmetic (gf_fixed.cu)
+void wilson_force_fx(gf_ctx* ctx, const gf_field* U, gf_field* P, double coef, double keep);
 
 // ---- rectangle loops (gf_rect.cu) ----
 double rectangle_sum(gf_ctx* ctx, const gf_field* U);  // sum_x sum_{mu<nu} Re tr (R1x2 + R2x1)

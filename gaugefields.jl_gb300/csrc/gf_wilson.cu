@@ -145,8 +145,8 @@ void wilson_force_coef(gf_ctx* ctx, const gf_field* U, gf_field* P, double coef,
   } else if (df) {
     throw gf_error(GF_EINVAL, "force: the double-float force needs LINK64 links");
   } else if (U->kind == GF_LINK64) {
-    Src64 src{(const double2*)U->ptr};
-    k_force_ta<double><<<grid, 128, 0, ctx->stream>>>(src, (double*)P->ptr, ctx->geom, coef, keep);
+    wilson_force_fx(ctx, U, P, coef, keep);
+    return;
   } else if (U->kind == GF_LINK32) {
     Src32 src{(const float4*)U->ptr};
     k_force_ta<float><<<grid, 128, 0, ctx->stream>>>(src, (double*)P->ptr, ctx->geom, coef, keep);
