@@ -129,22 +129,211 @@ GF_HD fx_acc fx_row_mul(const fx_row& A, const MAT& B) {
 
 // acc (unit exponent ea) += v (unit exponent ev). Equal exponents, as for
 // unitary links, are plain adds; otherwise the smaller one is shifted down.
+GF_HD int fx_clamp_shift(int d) { return d < 0 ? 0 : (d > 63 ? 63 : d); }
 GF_HD void fx_add(fx_acc& acc, int& ea, fx_acc v, int ev) {
   if (ev != ea) {
-    const int d = ev > ea ? ev - ea : ea - ev;
-    const int s = d < 63 ? d : 63;
-    fx_acc& small = ev > ea ? acc : v;
+    const int da = fx_clamp_shift(ev - ea), dv = fx_clamp_shift(ea - ev);
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-      small.re[j] >>= s;
-      small.im[j] >>= s;
+      acc.re[j] >>= da;
+      acc.im[j] >>= da;
+      v.re[j] >>= dv;
+      v.im[j] >>= dv;
     }
-    if (ev > ea) ea = ev;
+    ea = ev > ea ? ev : ea;
   }
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
     acc.re[j] += v.re[j];
     acc.im[j] += v.im[j];
+  }
+}
+
+// ---------------------------------------------------------------------------
+// scalars in units of 2^-60 (|value| < 2), and sums of their products
+// ---------------------------------------------------------------------------
+struct fx_num {
+  int h, l;
+};
+GF_HD fx_num fx_pre(i64 R) {
+  fx_num n;
+  fx_split<0>(R, n.h, n.l);
+  return n;
+}
+GF_HD fx_num fx_neg(fx_num n) {
+  n.h = -n.h;
+  n.l = -n.l;
+  return n;
+}
+struct fx_sum {
+  i64 hh, x;
+};
+GF_HD fx_sum fx_zero_sum() { return fx_sum{0, 0}; }
+GF_HD void fx_mac(fx_sum& s, fx_num a, fx_num b) {
+  s.hh = fx_mad(a.h, b.h, s.hh);
+  s.x = fx_mad(a.h, b.l, s.x);
+  s.x = fx_mad(a.l, b.h, s.x);
+}
+GF_HD i64 fx_get(fx_sum s) { return s.hh + (s.x >> 30); }
+GF_HD i64 fx_mul(fx_num a, fx_num b) {
+  fx_sum s = fx_zero_sum();
+  fx_mac(s, a, b);
+  return fx_get(s);
+}
+// (re, im) += a b for complex a, b
+GF_HD void fx_cmac(fx_sum& re, fx_sum& im, fx_num ar, fx_num ai, fx_num br, fx_num bi) {
+  fx_mac(re, ar, br);
+  fx_mac(re, fx_neg(ai), bi);
+  fx_mac(im, ar, bi);
+  fx_mac(im, ai, br);
+}
+// R / 2^d, d of either sign, rounded
+GF_HD i64 fx_shift(i64 R, int d) {
+  if (d <= 0) return d > -63 ? (i64)((u64)R << -d) : 0;
+  return d < 62 ? (R + (1ll << (d - 1))) >> d : 0;
+}
+
+// A kernel parameter c = (h 2^30 + l) 2^(e - 60), |h 2^30 + l| < 2^60
+struct fx_scalar {
+  int h, l, e;
+};
+inline fx_scalar fx_scalar_of(double c) {
+  int e = 0;
+  const double m = frexp(c, &e);  // c = m 2^e, 1/2 <= |m| < 1
+  if (!(m == m) || m - m != 0.0) return fx_scalar{0, 0, GF_FX_BAD};
+  fx_scalar s;
+  fx_split<0>((i64)ldexp(m, 60), s.h, s.l);
+  s.e = m == 0.0 ? 0 : e;
+  return s;
+}
+GF_HD fx_num fx_num_of(const fx_scalar& s) { return fx_num{s.h, s.l}; }
+GF_HD void fx_scale_row(fx_acc& v, const fx_scalar& c) {
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    v.re[j] = fx_mul(fx_pre(v.re[j]), fx_num_of(c));
+    v.im[j] = fx_mul(fx_pre(v.im[j]), fx_num_of(c));
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Cayley-Hamilton exponential of iX, X = 2^s q, q traceless Hermitian with
+// |q| <= 1: exp(iX) = f0 + f1 q + f2 q^2, from the power series in Horner form
+// with q^3 = c1 q + c0. The coefficients are real series for their real and
+// imaginary parts, which two threads evaluate side by side. They are returned
+// in units of 2^(guard - 60), as are their derivatives in c1 and c0 (of q).
+// ---------------------------------------------------------------------------
+#define GF_FX_CH_TERMS 64
+#define GF_FX_CH_SCALES 5
+// guard bits: the sums reach cosh(2^s), their derivatives about 2^s times that
+GF_HD int fx_guard(int s) { return s == 0 ? 1 : (s == 1 ? 3 : (s == 2 ? 7 : (s == 3 ? 14 : 27))); }
+
+struct fx_kappa {
+  i64 k[GF_FX_CH_SCALES][GF_FX_CH_TERMS];
+};
+// 2^(s n) / n! in units of 2^(guard - 60), rounded
+constexpr fx_kappa fx_make_kappa() {
+  fx_kappa t{};
+  const int guard[GF_FX_CH_SCALES] = {1, 3, 7, 14, 27};
+  for (int s = 0; s < GF_FX_CH_SCALES; ++s) {
+    unsigned __int128 v = (unsigned __int128)1 << 100;
+    for (int n = 0; n < GF_FX_CH_TERMS; ++n) {
+      if (n > 0) v = (v << s) / (unsigned)n;
+      const int d = 40 + guard[s];
+      t.k[s][n] = (i64)((v + ((unsigned __int128)1 << (d - 1))) >> d);
+    }
+  }
+  return t;
+}
+
+// c1 = tr(q^2)/2 and c0 = det q; d the diagonal, o12 .. the upper entries
+struct fx_herm {
+  i64 d[3];
+  i64 re[3], im[3];  // entries (0,1), (0,2), (1,2)
+};
+GF_HD void fx_invariants(const fx_herm& q, i64& c0, i64& c1) {
+  fx_num d[3], re[3], im[3];
+  i64 n[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    d[k] = fx_pre(q.d[k]);
+    re[k] = fx_pre(q.re[k]);
+    im[k] = fx_pre(q.im[k]);
+    fx_sum t = fx_zero_sum();
+    fx_mac(t, re[k], re[k]);
+    fx_mac(t, im[k], im[k]);
+    n[k] = fx_get(t);
+  }
+  fx_sum sq = fx_zero_sum();
+#pragma unroll
+  for (int k = 0; k < 3; ++k) fx_mac(sq, d[k], d[k]);
+  c1 = (fx_get(sq) >> 1) + n[0] + n[1] + n[2];
+  // det = d0 d1 d2 + 2 Re(q01 q12 conj(q02)) - d0 |q12|^2 - d1 |q02|^2 - d2 |q01|^2
+  fx_sum tr = fx_zero_sum(), ti = fx_zero_sum();
+  fx_cmac(tr, ti, re[0], im[0], re[2], im[2]);
+  const fx_num t0 = fx_pre(fx_get(tr)), t1 = fx_pre(fx_get(ti));
+  fx_sum r = fx_zero_sum();
+  fx_mac(r, t0, re[1]);
+  fx_mac(r, t1, im[1]);
+  fx_sum det = fx_zero_sum();
+  fx_mac(det, fx_pre(fx_mul(d[0], d[1])), d[2]);
+  fx_mac(det, fx_neg(d[0]), fx_pre(n[2]));
+  fx_mac(det, fx_neg(d[1]), fx_pre(n[1]));
+  fx_mac(det, fx_neg(d[2]), fx_pre(n[0]));
+  c0 = fx_get(det) + 2 * fx_get(r);
+}
+
+// scale s and number of terms for a norm bound lam of X (real): lam <= 2^s,
+// lam^n / n! < 2^-62 from n = terms - extra on. The derivatives of the n-th
+// power's coefficients go as n lam^(n - 4), so they take four terms more.
+GF_HD void fx_series(float lam, int extra, int& s, int& terms) {
+  s = lam <= 1.f ? 0 : (lam <= 2.f ? 1 : (lam <= 4.f ? 2 : (lam <= 8.f ? 3 : 4)));
+  float t = 1.f;
+  int n = 1;
+  for (; n < GF_FX_CH_TERMS - 1; ++n) {
+    t *= lam / (float)n;
+    if (t < 2.2e-19f) break;
+  }
+  terms = n + extra < GF_FX_CH_TERMS - 1 ? n + extra : GF_FX_CH_TERMS - 1;
+}
+
+// Real (IM = 0) or imaginary (1) parts of f_j, and of df_j/dc1 (b1) and
+// df_j/dc0 (b2) when DERIV
+template <bool DERIV>
+GF_HD void fx_ch(const i64* kappa, int terms, int im, i64 c0, i64 c1, i64 f[3], i64 b1[3], i64 b2[3]) {
+  const fx_num n0 = fx_pre(c0), n1 = fx_pre(c1);
+  i64 a = 0, b = 0, c = 0;
+  i64 a0 = 0, b0 = 0, g0 = 0, a1 = 0, b1s = 0, g1 = 0;
+#pragma unroll 1
+  for (int n = terms; n >= 0; --n) {
+    const fx_num pc = fx_pre(c);
+    i64 k = ((n & 1) == im) ? kappa[n] : 0;
+    if (n & 2) k = -k;
+    const i64 na = fx_mul(pc, n0) + k, nb = a + fx_mul(pc, n1);
+    if (DERIV) {
+      const fx_num p0 = fx_pre(g0), p1 = fx_pre(g1);
+      const i64 na0 = c + fx_mul(p0, n0), nb0 = a0 + fx_mul(p0, n1);
+      const i64 na1 = fx_mul(p1, n0), nb1 = a1 + c + fx_mul(p1, n1);
+      g0 = b0;
+      a0 = na0;
+      b0 = nb0;
+      g1 = b1s;
+      a1 = na1;
+      b1s = nb1;
+    }
+    c = b;
+    a = na;
+    b = nb;
+  }
+  f[0] = a;
+  f[1] = b;
+  f[2] = c;
+  if (DERIV) {
+    b1[0] = a1;
+    b1[1] = b1s;
+    b1[2] = g1;
+    b2[0] = a0;
+    b2[1] = b0;
+    b2[2] = g0;
   }
 }
 

@@ -60,6 +60,109 @@ __device__ __forceinline__ fx_row fx_load_row(const FxMat& M, int r) {
   return a;
 }
 
+// writes element el of a field's matrix, and the matrix's exponent
+__device__ __forceinline__ void fx_store(char* p, size_t off, int el, i64 re, i64 im) {
+  int4 v;
+  fx_split<0>(re, v.x, v.y);
+  fx_split<0>(im, v.z, v.w);
+  *reinterpret_cast<int4*>(p + off + el * 512) = v;
+}
+__device__ __forceinline__ void fx_store_exp(char* p, size_t off, int s, int e) {
+  *reinterpret_cast<int*>(p + off + 9 * 512 - 12 * (s & 31)) = e > GF_FX_BAD / 2 ? GF_FX_BAD : e;
+}
+__device__ __forceinline__ void fx_store_row(char* p, size_t off, int r, const fx_acc& v) {
+#pragma unroll
+  for (int j = 0; j < 3; ++j) fx_store(p, off, 3 * r + j, v.re[j], v.im[j]);
+}
+
+// ---------------------------------------------------------------------------
+// exchange between the rows of a link through shared memory, component-major
+// over the block's links, so that a thread per link reads without conflicts
+// ---------------------------------------------------------------------------
+struct FxRaw {  // 64-bit matrix
+  i64 v[18][GF_FX_LINKS];
+};
+struct FxOperand {  // matrix as limbs, a right factor
+  int4 v[9][GF_FX_LINKS];
+};
+struct FxShMat {
+  const FxOperand* m;
+  int link;
+  __device__ __forceinline__ int4 operator()(int el) const { return m->v[el][link]; }
+};
+__device__ __forceinline__ void fx_share(FxRaw& sh, int link, int r, const fx_acc& m) {
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    sh.v[2 * (3 * r + j)][link] = m.re[j];
+    sh.v[2 * (3 * r + j) + 1][link] = m.im[j];
+  }
+}
+template <int K>
+__device__ __forceinline__ void fx_share(FxOperand& sh, int link, int r, const fx_acc& m) {
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    int4 v;
+    fx_split<K>(m.re[j], v.x, v.y);
+    fx_split<K>(m.im[j], v.z, v.w);
+    sh.v[3 * r + j][link] = v;
+  }
+}
+template <bool DAG>
+__device__ __forceinline__ fx_row fx_load_row(const FxShMat& M, int r) {
+  fx_row a;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int4 v = M(DAG ? 3 * k + r : 3 * r + k);
+    a.ah[k] = v.x;
+    a.al[k] = v.y;
+    a.bh[k] = DAG ? -v.z : v.z;
+    a.bl[k] = DAG ? -v.w : v.w;
+  }
+  return a;
+}
+
+// fp64 value of R (unit 1): the two words through exponent constants, no
+// integer-to-double conversion
+__device__ __forceinline__ double fx_value(i64 R) {
+  const int h = (int)(R >> 32);
+  const double dh = __hiloint2double(0x43300000, h ^ (int)0x80000000) - 4503601774854144.0;  // 2^52 + 2^31
+  const double dl = __hiloint2double(0x43300000, (int)(unsigned)R) - 4503599627370496.0;      // 2^52
+  return fma(dh, 4294967296.0, dl);
+}
+// c 2^(E - 60); NaN for GF_FX_BAD
+__device__ __forceinline__ double fx_unit(double c, int E) {
+  if (E > GF_FX_BAD / 2) return __longlong_as_double(0x7FF8000000000000ll);
+  const int k = E - 60;
+  if (k > -1000 && k < 1000) return c * __hiloint2double((k + 1023) << 20, 0);
+  return scalbn(c, k);
+}
+
+// P <- keep P + coef c(M), c the su(3) coefficients of TA(M) for the 32
+// matrices M of a block (raw, exponents se); thread t serves link t % 32 and,
+// by t / 32, the coefficients (0, 1, 2), (3, 4, 7) or (5, 6).
+__device__ __forceinline__ void fx_update_mom(const FxRaw& sh, const int* se, double* __restrict__ P, int mu, int s0,
+                                              int V, double coef, double keep) {
+  const int link = threadIdx.x & 31, part = threadIdx.x >> 5, s = s0 + link;
+  if (s >= V) return;
+  const int i = part == 2 ? 1 : 0, j = part == 0 ? 1 : 2;
+  const int ij = 2 * (3 * i + j), ji = 2 * (3 * j + i);
+  const i64 d1 = sh.v[1][link], d2 = sh.v[9][link], d3 = sh.v[17][link];
+  const i64 c[3] = {sh.v[ij + 1][link] + sh.v[ji + 1][link], sh.v[ij][link] - sh.v[ji][link],
+                    part == 0 ? d1 - d2 : d1 + d2 - 2 * d3};
+  const int a0 = part == 0 ? 0 : (part == 1 ? 3 : 5);
+  const int a[3] = {a0, a0 + 1, part == 0 ? 2 : 7};
+  const double sc = fx_unit(coef, se[link]);
+  double* p = P + (size_t)mu * 8 * V + s;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    if (q == 2 && part == 2) break;
+    const double f = (q == 2 && part == 1) ? sc * 0.57735026918962576451 : sc;
+    double* d = p + (size_t)a[q] * V;
+    const double old = keep != 0.0 ? keep * *d : 0.0;
+    *d = fma(f, fx_value(c[q]), old);
+  }
+}
+
 // lexicographic offset of a unit step from a site (periodic), along mu
 __device__ __forceinline__ int fx_up(const Geom& g, const Site& st, int mu) {
   const int str = g.stride[mu];
@@ -94,5 +197,41 @@ __device__ __forceinline__ void fx_add_staples(fx_acc& acc, int& ea, const FxFie
     fx_add(acc, ea, fx_row_mul<false>(fx_operand<0>(t), fx_mat(U, nu, xpm_mn, V)), e);
   }
 }
+
+// (R / 2^20)^2 in fp32
+__device__ __forceinline__ float fx_square(i64 R) {
+  const float v = fmaf((float)(int)(R >> 32), 4096.f, (float)(unsigned)R * 9.5367431640625e-7f);
+  return v * v;
+}
+__device__ __forceinline__ float fx_square(const fx_acc& v) {
+  float n = 0.f;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) n += fx_square(v.re[j]) + fx_square(v.im[j]);
+  return n;
+}
+// shift d for which a matrix of raw norm^2 n (units of fx_square) has
+// norm <= 2^60 after R >> d, and > 2^58 (0 for a zero or non-finite matrix)
+__device__ __forceinline__ int fx_norm_shift(float n, int e) {
+  if (n == 0.f || e > GF_FX_BAD / 2) return 0;
+  // n (1 + 2^-10) < 2^k4, norm < 2^(20 + k4 / 2)
+  const int k4 = (int)(__float_as_uint(n * 1.0009765625f) >> 23) - 126;
+  return ((k4 + 1) >> 1) - 40;
+}
+
+// fp64 view of a fixed-point field (fp64 kernels)
+struct LinkSrcFx64 {
+  FxField F;
+  __device__ __forceinline__ mat3<double> operator()(int mu, int s, int V) const {
+    mat3<double> m;
+    const FxMat M = fx_mat(F, mu, s, V);
+    const int e = fx_exp(F, mu, s, V);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      const int4 v = M(k);
+      m.e[k / 3][k % 3] = mk(fx_to_f64(fx_join(v.x, v.y), e), fx_to_f64(fx_join(v.z, v.w), e));
+    }
+    return m;
+  }
+};
 
 }  // namespace gf

@@ -2,6 +2,7 @@
 // drivers (MD trajectory, HMC update, RK3 flow) that sequence the kernels on
 // the context's stream.
 #include "gf_internal.h"
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <new>
@@ -108,7 +109,8 @@ extern "C" int gf_ctx_create(const int L[4], int device, gf_ctx** out) {
   ctx->geom.stride[3] = L[0] * L[1] * L[2];
   GF_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
   ctx->own_stream = 1;
-  ctx->partial_cap = blocks_for((int)V, 128) + 1;
+  // at least one partial per resident block of the grid-stride sums
+  ctx->partial_cap = std::max(blocks_for((int)V, 128) + 1, ctx->sm_count * 64);
   GF_CUDA(cudaMalloc(&ctx->d_partials, sizeof(double) * ctx->partial_cap));
   GF_CUDA(cudaMalloc(&ctx->d_result, sizeof(double) * 4));
   GF_CUDA(cudaMallocHost(&ctx->h_result, sizeof(double) * 4));
@@ -418,8 +420,8 @@ static gf_stout* stout_new(gf_ctx* ctx, int nlev, const double* rho, int precisi
   st->store = store ? 1 : 0;
   // double-float stacks keep their levels and adjoint fields as fp32 hi/lo
   // pairs (no conversion on the kernels' loads)
-  int lk = precision == GF_MIXED ? GF_LINK32 : (precision == GF_PREC_DF ? GF_LINKDF : GF_LINK64);
-  int mk = precision == GF_MIXED ? GF_MAT32 : (precision == GF_PREC_DF ? GF_MATDF : GF_MAT64);
+  int lk = precision == GF_MIXED ? GF_LINK32 : (precision == GF_PREC_DF ? GF_LINKDF : GF_LINKFX);
+  int mk = precision == GF_MIXED ? GF_MAT32 : (precision == GF_PREC_DF ? GF_MATDF : GF_MATFX);
   try {
     for (int l = 1; l <= nlev; ++l) {
       if (fwd_only && arena && l <= 2) {

@@ -2,7 +2,6 @@
 // hot starts, Gaussian momenta, field copies/conversions and the deterministic
 // two-stage reductions used by every global sum.
 #include "gf_internal.h"
-#include "fxlat.cuh"
 #include <vector>
 
 namespace gf {
@@ -17,7 +16,8 @@ size_t field_bytes(const Geom& g, int kind) {
     case GF_MAT64: return 4 * 9 * V * sizeof(double2);
     case GF_LINKDF:
     case GF_MATDF: return 4 * 9 * V * sizeof(float4);
-    case GF_LINKFX: return fx_field_bytes(V);
+    case GF_LINKFX:
+    case GF_MATFX: return fx_field_bytes(V);
     case GF_LINK32: return 4 * 3 * V * sizeof(float4);
     case GF_MAT32: return 4 * 9 * V * sizeof(float2);
     case GF_MOM64: return 4 * 8 * V * sizeof(double);
@@ -496,12 +496,14 @@ __global__ void k_dfn_to_f64(const float4* __restrict__ in, double2* __restrict_
 
 static bool is_f64_full(int k) { return k == GF_LINK64 || k == GF_MAT64; }
 static bool is_dfn(int k) { return k == GF_LINKDF || k == GF_MATDF; }
+static bool is_fx(int k) { return k == GF_LINKFX || k == GF_MATFX; }
 
 void copy_field(gf_ctx* ctx, gf_field* dst, const gf_field* src) {
   if (!dst || !src) throw gf_error(GF_EINVAL, "copy: null field");
   if (dst == src) return;
   int a = src->kind, b = dst->kind;
-  bool full64 = (is_f64_full(a) && is_f64_full(b)) || (is_dfn(a) && is_dfn(b));
+  bool full64 = (is_f64_full(a) && is_f64_full(b)) || (is_dfn(a) && is_dfn(b)) ||
+                (is_fx(a) && is_fx(b));
   if (a == b || full64) {
     GF_CUDA(cudaMemcpyAsync(dst->ptr, src->ptr, src->bytes, cudaMemcpyDeviceToDevice, ctx->stream));
     return;
@@ -521,6 +523,12 @@ void copy_field(gf_ctx* ctx, gf_field* dst, const gf_field* src) {
     k_f64_to_dfn<<<nb, 256, 0, ctx->stream>>>((const double2*)src->ptr, (float4*)dst->ptr, n);
   } else if (is_dfn(a) && is_f64_full(b)) {
     k_dfn_to_f64<<<nb, 256, 0, ctx->stream>>>((const float4*)src->ptr, (double2*)dst->ptr, n);
+  } else if (is_f64_full(a) && is_fx(b)) {
+    f64_to_fx(ctx, dst, src);
+    return;
+  } else if (is_fx(a) && is_f64_full(b)) {
+    fx_to_f64_field(ctx, dst, src);
+    return;
   } else {
     throw gf_error(GF_EINVAL, "copy: unsupported kind conversion " + std::to_string(a) + " -> " + std::to_string(b));
   }

@@ -1,7 +1,8 @@
 // Fixed-point (block floating, integer pipes) kernels of the fp64-class path:
-// conversions and the Wilson force.
+// conversions, the plaquette sum and the Wilson force.
 #include "gf_internal.h"
-#include "fxlat.cuh"
+#include <algorithm>
+#include "stencil.cuh"
 
 namespace gf {
 
@@ -25,8 +26,6 @@ __global__ void __launch_bounds__(128) k_f64_to_fx(const double2* __restrict__ i
   *reinterpret_cast<int*>(o + 9 * 512 - 12 * (s & 31)) = e;
 }
 
-FxField fx_view(const gf_field* f) { return FxField{(const char*)f->ptr}; }
-
 void f64_to_fx(gf_ctx* ctx, gf_field* dst, const gf_field* src) {
   const int V = ctx->geom.vol;
   dim3 grid(blocks_for(V, 128), 4);
@@ -34,32 +33,61 @@ void f64_to_fx(gf_ctx* ctx, gf_field* dst, const gf_field* src) {
   GF_CHECK_LAUNCH();
 }
 
-// the 18 reals of 32 rows-split matrices in shared memory: component-major
-// over the links, so a thread per link reads without bank conflicts
-struct FxShare {
-  i64 v[18][GF_FX_LINKS];
-};
-__device__ __forceinline__ void fx_share_row(FxShare& sh, int link, int r, const fx_acc& m) {
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    sh.v[2 * (3 * r + j)][link] = m.re[j];
-    sh.v[2 * (3 * r + j) + 1][link] = m.im[j];
-  }
+__global__ void __launch_bounds__(128) k_fx_to_f64(FxField F, double2* __restrict__ out, int V) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x, mu = blockIdx.y;
+  if (s >= V) return;
+  LinkFull<double>::store(out, mu, s, V, LinkSrcFx64{F}(mu, s, V));
 }
 
-// R 2^(E - 60) * scale, E folded into the scale by fx_scale
-__device__ __forceinline__ double fx_value(i64 R) {
-  const int h = (int)(R >> 32);
-  const unsigned int l = (unsigned int)R;
-  const double dh = __hiloint2double(0x43300000, h ^ (int)0x80000000) - 4503601774854144.0;  // 2^52 + 2^31
-  const double dl = __hiloint2double(0x43300000, (int)l) - 4503599627370496.0;               // 2^52
-  return fma(dh, 4294967296.0, dl);
+void fx_to_f64_field(gf_ctx* ctx, gf_field* dst, const gf_field* src) {
+  const int V = ctx->geom.vol;
+  dim3 grid(blocks_for(V, 128), 4);
+  k_fx_to_f64<<<grid, 128, 0, ctx->stream>>>(fx_view(src), (double2*)dst->ptr, V);
+  GF_CHECK_LAUNCH();
 }
-__device__ __forceinline__ double fx_scale(double c, int E) {
-  if (E > GF_FX_BAD / 2) return __longlong_as_double(0x7FF8000000000000ll);
-  const int k = E - 60;
-  if (k > -1000 && k < 1000) return c * __hiloint2double((k + 1023) << 20, 0);
-  return scalbn(c, k);
+
+// Sum over the sites and the planes mu < nu of Re tr P_munu, one partial per
+// block. A work item is one plane of 32 sites; a thread forms row r of
+// U_mu(x) U_nu(x+mu) U_mu(x+nu)^dag and its product with row r of U_nu(x).
+// Integer-issue-bound: 2M sites (32^3 x 64) 7.16 ms in fp64, 1.68 ms here with
+// the conversion (0.4 ms, bandwidth-bound); 8^4 89 -> 31 us, a launch and a
+// wait each for the conversion, the sum and its second stage.
+__global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_MINB)
+    k_plaquette_fx(FxField U, Geom g, int items, double* __restrict__ part) {
+  const int t = threadIdx.x, V = g.vol;
+  const int link = t / 3, r = t - 3 * link;
+  double v = 0.0;
+#pragma unroll 1
+  for (int it = blockIdx.x; it < items; it += gridDim.x) {
+    const int tile = it / 6, p = it - 6 * tile;
+    const int mu = p < 3 ? 0 : (p < 5 ? 1 : 2), nu = p < 3 ? p + 1 : (p < 5 ? p - 1 : 3);
+    const int s = tile * GF_FX_LINKS + link;
+    if (s >= V) continue;
+    const Site st = site_of(g, s);
+    const int xpm = eo_of_lex(g, st.lex + fx_up(g, st, mu), st.par ^ 1);
+    const int xpn = eo_of_lex(g, st.lex + fx_up(g, st, nu), st.par ^ 1);
+    const int e = fx_exp(U, mu, s, V) + fx_exp(U, nu, xpm, V) + fx_exp(U, mu, xpn, V) + fx_exp(U, nu, s, V);
+    fx_acc a = fx_row_mul<false>(fx_load_row<false>(fx_mat(U, mu, s, V), r), fx_mat(U, nu, xpm, V));
+    a = fx_row_mul<true>(fx_operand<0>(a), fx_mat(U, mu, xpn, V));
+    const fx_row b = fx_load_row<false>(fx_mat(U, nu, s, V), r);
+    fx_sum d = fx_zero_sum();
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      fx_mac(d, fx_pre(a.re[k]), fx_num{b.ah[k], b.al[k]});
+      fx_mac(d, fx_pre(a.im[k]), fx_num{b.bh[k], b.bl[k]});
+    }
+    v = fma(fx_value(fx_get(d)), fx_unit(1.0, e), v);
+  }
+  block_partial_sum(v, part);
+}
+
+double plaquette_sum_fx(gf_ctx* ctx, const gf_field* F) {
+  const int items = 6 * blocks_for(ctx->geom.vol, GF_FX_LINKS);
+  // a few waves of resident blocks, so that the second stage stays short
+  const int nb = std::min(std::min(items, ctx->sm_count * GF_FX_MINB * 8), ctx->partial_cap);
+  k_plaquette_fx<<<nb, GF_FX_THREADS, 0, ctx->stream>>>(fx_view(F), ctx->geom, items, ctx->d_partials);
+  GF_CHECK_LAUNCH();
+  return finish_reduction(ctx, nb);
 }
 
 // P_mu(x) <- keep * P_mu(x) + coef * c(U_mu(x) S_mu(x)) as k_force_ta. The
@@ -71,7 +99,7 @@ __device__ __forceinline__ double fx_scale(double c, int E) {
 // registers) measured 0.70 ms, six 0.73, five 0.74, eight (spills) 0.72.
 __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_MINB)
     k_force_fx(FxField U, double* __restrict__ P, Geom g, double coef, double keep) {
-  __shared__ FxShare sh;
+  __shared__ FxRaw sh;
   __shared__ int se[GF_FX_LINKS];
   const int t = threadIdx.x, mu = blockIdx.x & 3, V = g.vol;
   const int s0 = (blockIdx.x >> 2) * GF_FX_LINKS;
@@ -85,38 +113,14 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_MINB)
 #pragma unroll 1
     for (int k = 1; k < 4; ++k) fx_add_staples(acc, ea, U, g, st, s, mu, (mu + k) & 3, mu_up, r);
     // |V| <= 6: three bits down to serve as an operand
-    const fx_acc m = fx_row_mul<true>(fx_operand<3>(acc), fx_mat(U, mu, s, V));
-    fx_share_row(sh, link, r, m);
+    fx_share(sh, link, r, fx_row_mul<true>(fx_operand<3>(acc), fx_mat(U, mu, s, V)));
     if (r == 0) se[link] = ea + 3 + fx_exp(U, mu, s, V);
   }
   __syncthreads();
-  const int link = t & 31, part = t >> 5, s = s0 + link;
-  if (s >= V) return;
-  // c of TA(M^dag): x_ij(M^dag) = conj(M_ji) - M_ij
-  i64 c[3];
-  int a[3];
-  const int i = part == 2 ? 1 : 0, j = part == 0 ? 1 : 2;
-  const int ij = 2 * (3 * i + j), ji = 2 * (3 * j + i);
-  c[0] = -sh.v[ji + 1][link] - sh.v[ij + 1][link];
-  c[1] = sh.v[ji][link] - sh.v[ij][link];
-  a[0] = part == 0 ? 0 : (part == 1 ? 3 : 5);
-  const i64 d1 = -sh.v[1][link], d2 = -sh.v[9][link], d3 = -sh.v[17][link];
-  c[2] = part == 0 ? d1 - d2 : d1 + d2 - 2 * d3;
-  a[1] = a[0] + 1;
-  a[2] = part == 0 ? 2 : 7;
-  const double sc = fx_scale(coef, se[link]);
-  double* p = P + (size_t)mu * 8 * V + s;
-#pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    if (q == 2 && part == 2) break;
-    const double f = (q == 2 && part == 1) ? sc * 0.57735026918962576451 : sc;
-    double* d = p + (size_t)a[q] * V;
-    const double old = keep != 0.0 ? keep * *d : 0.0;
-    *d = fma(f, fx_value(c[q]), old);
-  }
+  fx_update_mom(sh, se, P, mu, s0, V, -coef, keep);
 }
 
-static gf_field* fx_links(gf_ctx* ctx, const gf_field* U) {
+const gf_field* fx_links(gf_ctx* ctx, const gf_field* U) {
   if (!ctx->w_linkfx) ctx->w_linkfx = field_new(ctx, GF_LINKFX);
   f64_to_fx(ctx, ctx->w_linkfx, U);
   return ctx->w_linkfx;

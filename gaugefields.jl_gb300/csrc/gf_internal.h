@@ -4,7 +4,7 @@
 #include <stdint.h>
 #include <string>
 #include <stdexcept>
-#include "lattice.cuh"
+#include "fxlat.cuh"
 #include "../../include/gaugefields_gb300.h"
 
 // Error carried from the CUDA layer to the C-ABI wrappers, which turn it into
@@ -45,6 +45,7 @@ void count_launch();
 #define GF_MATDF 102
 // Fixed-point links and matrices (fxlat.cuh), internal too
 #define GF_LINKFX 103
+#define GF_MATFX 104
 
 struct gf_field {
   gf_ctx* ctx;
@@ -179,6 +180,14 @@ void wilson_force_coef(gf_ctx* ctx, const gf_field* U, gf_field* P, double coef,
 // the same on fp64 links in fixed-point arithmetic (gf_fixed.cu)
 void wilson_force_fx(gf_ctx* ctx, const gf_field* U, gf_field* P, double coef, double keep);
 
+double plaquette_sum_fx(gf_ctx* ctx, const gf_field* F);  // of a fixed-point field
+inline FxField fx_view(const gf_field* f) { return FxField{(const char*)f->ptr}; }
+// the context's fixed-point copy of fp64 links
+const gf_field* fx_links(gf_ctx* ctx, const gf_field* U);
+// LINK64 / MAT64 <-> fixed-point fields
+void f64_to_fx(gf_ctx* ctx, gf_field* dst, const gf_field* src);
+void fx_to_f64_field(gf_ctx* ctx, gf_field* dst, const gf_field* src);
+
 // ---- rectangle loops (gf_rect.cu) ----
 double rectangle_sum(gf_ctx* ctx, const gf_field* U);  // sum_x sum_{mu<nu} Re tr (R1x2 + R2x1)
 // P <- keep * P + TA-coefficients(U_mu (cp S_mu + cr R_mu)), S the six
@@ -191,6 +200,11 @@ void loops_dsdu(gf_ctx* ctx, const gf_field* Ubar, gf_field* D, double cp, doubl
 // P <- keep P + coef c(U S), S the six plaquette staples, as a double-float
 // table loop of fixed-grid products on a double-float-native copy of U
 void plaquette_force_df(gf_ctx* ctx, const gf_field* U, gf_field* P, double coef, double keep);
+
+// the same on a fixed-point field (gf_fxrect.cu): the loop sum; the force into
+// P, or D = cp S + cr R into a fixed-point D
+double rectangle_sum_fx(gf_ctx* ctx, const gf_field* F);
+void loops_fx(gf_ctx* ctx, const gf_field* F, gf_field* P, gf_field* D, double cp, double cr, double keep);
 
 // ---- link update (gf_update.cu) ----
 // U <- exp(i eps P) U, optional re-unitarisation, optional fp32 shadow copy.
@@ -212,6 +226,12 @@ void stout_forward(gf_ctx* ctx, gf_stout* st, const gf_field* U, gf_field* Uout)
 void stout_backward(gf_ctx* ctx, gf_stout* st, const gf_field* dSdUbar, double beta, gf_field* dSdU,
                     gf_field* P, double eps, double* dsdrho = nullptr);
 const gf_field* stout_top(const gf_stout* st);
+// forward and backward of a fixed-point stack (gf_fxstout.cu)
+void stout_forward_fx(gf_ctx* ctx, gf_stout* st);
+void stout_backward_fx(gf_ctx* ctx, gf_stout* st, const gf_field* dSdUbar, double beta, gf_field* dSdU, gf_field* P,
+                       double eps, double* dsdrho);
+// dS/drho of level `l` from the stack's Z (after that level's local adjoint)
+double level_dsdrho(gf_ctx* ctx, gf_stout* st, int l);
 
 // ---- flow (gf_flow.cu) ----
 // F <- keep * F + factor * TA-coefficients(U_mu V_mu^dag), V = six-staple sum

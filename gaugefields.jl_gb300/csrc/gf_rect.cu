@@ -22,8 +22,6 @@
 
 namespace gf {
 
-typedef LinkSrc<double, false> SrcRect;
-
 // even/odd index of x + a e_mu + b e_nu (mu != nu, any a, b; periodic)
 __device__ __forceinline__ int site_off(const Geom& g, const Site& st, int mu, int a, int nu, int b) {
   int lex = st.lex;
@@ -295,7 +293,8 @@ static double rect_sum_of(gf_ctx* ctx, SRC src) {
 }
 
 double rectangle_sum(gf_ctx* ctx, const gf_field* U) {
-  if (U->kind == GF_LINK64 || U->kind == GF_MAT64) return rect_sum_of(ctx, SrcRect{(const double2*)U->ptr});
+  if (U->kind == GF_LINK64 || U->kind == GF_MAT64) return rectangle_sum_fx(ctx, fx_links(ctx, U));
+  if (U->kind == GF_LINKFX) return rectangle_sum_fx(ctx, U);
   // top level of a double-float stack: fp64 arithmetic on hi + lo
   if (U->kind == GF_LINKDF) return rect_sum_of(ctx, LinkSrcDfn64{(const float4*)U->ptr});
   throw gf_error(GF_EINVAL, "rectangle: links must be LINK64");
@@ -313,9 +312,9 @@ void loops_force_coef(gf_ctx* ctx, const gf_field* U, gf_field* P, double cp, do
     return;
   }
   if (U->kind == GF_LINK64 || U->kind == GF_MAT64) {
-    ProfScope prof(ctx, GF_K_RECT);
-    k_force_rect<double><<<grid, 128, 0, ctx->stream>>>(SrcRect{(const double2*)U->ptr}, (double*)P->ptr, ctx->geom,
-                                                        cp, cr, keep);
+    if (cr == 0.0) wilson_force_coef(ctx, U, P, cp, keep);
+    else loops_fx(ctx, fx_links(ctx, U), P, nullptr, cp, cr, keep);
+    return;
   } else if (U->kind == GF_LINK32) {
     ProfScope prof(ctx, GF_K_RECT);
     k_force_rect<float><<<grid, 128, 0, ctx->stream>>>(LinkSrc<float, true>{(const float4*)U->ptr}, (double*)P->ptr,
@@ -340,11 +339,12 @@ void loops_dsdu(gf_ctx* ctx, const gf_field* Ubar, gf_field* D, double cp, doubl
     rect_df(ctx, (const float4*)Ubar->ptr, nullptr, D, cp, cr, 0.0);
     return;
   }
+  if (Ubar->kind == GF_LINKFX && D->kind == GF_MATFX) {
+    loops_fx(ctx, Ubar, nullptr, D, cp, cr, 0.0);
+    return;
+  }
   ProfScope prof(ctx, GF_K_RECT);
-  if (Ubar->kind == GF_LINK64 && D->kind == GF_MAT64) {
-    k_dsdu_rect<double><<<grid, 128, 0, ctx->stream>>>(SrcRect{(const double2*)Ubar->ptr}, (double2*)D->ptr,
-                                                       ctx->geom, cp, cr);
-  } else if (Ubar->kind == GF_LINK32 && D->kind == GF_MAT32) {
+  if (Ubar->kind == GF_LINK32 && D->kind == GF_MAT32) {
     k_dsdu_rect<float><<<grid, 128, 0, ctx->stream>>>(LinkSrc<float, true>{(const float4*)Ubar->ptr},
                                                       (float2*)D->ptr, ctx->geom, (float)cp, (float)cr);
   } else {

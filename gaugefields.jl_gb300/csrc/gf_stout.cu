@@ -30,17 +30,6 @@ namespace gf {
 template <typename R>
 struct Prec;
 template <>
-struct Prec<double> {
-  typedef LinkSrc<double, false> Src;
-  typedef double2 LinkElem;
-  typedef double2 MatElem;
-  static constexpr int link_kind = GF_LINK64;
-  static constexpr int mat_kind = GF_MAT64;
-  static __device__ __forceinline__ void store_link(double2* p, int mu, int s, int V, const mat3<double>& m) {
-    LinkFull<double>::store(p, mu, s, V, m);
-  }
-};
-template <>
 struct Prec<float> {
   typedef LinkSrc<float, true> Src;
   typedef float4 LinkElem;
@@ -611,13 +600,11 @@ __global__ void __launch_bounds__(128) k_dsdrho(SRC U, ZL Z, Geom g, double* __r
   block_partial_sum(v, part);
 }
 
-// dS/drho of level `l` from the stack's Z (after that level's local adjoint)
-static double level_dsdrho(gf_ctx* ctx, gf_stout* st, int l) {
+double level_dsdrho(gf_ctx* ctx, gf_stout* st, int l) {
   const int nb = blocks_for(ctx->geom.vol, 128);
   const gf_field* u = st->lev_in[l];
   if (st->precision == GF_FP64) {
-    k_dsdrho<double><<<nb, 128, 0, ctx->stream>>>(LinkSrc<double, false>{(const double2*)u->ptr},
-                                                  LinkSrc<double, false>{(const double2*)st->Z->ptr}, ctx->geom,
+    k_dsdrho<double><<<nb, 128, 0, ctx->stream>>>(LinkSrcFx64{fx_view(u)}, LinkSrcFx64{fx_view(st->Z)}, ctx->geom,
                                                   ctx->d_partials);
   } else if (st->precision == GF_MIXED) {
     k_dsdrho<float><<<nb, 128, 0, ctx->stream>>>(LinkSrc<float, true>{(const float4*)u->ptr},
@@ -676,14 +663,14 @@ static void forward_impl(gf_ctx* ctx, gf_stout* st) {
   }
 }
 
-// Kind of a stack's level-0 input: fp32 12-real (mixed), double-float-native
-// (a double-float stack with an adjoint keeps its own copy of the thin
-// links), or the caller's fp64 links (plain form; forward-only double-float
-// stacks read them in place).
+// Kind of a stack's level-0 input: fp32 12-real (mixed), fixed point (plain
+// form) and double-float-native (a double-float stack with an adjoint), the
+// stack's own copies of the thin links, or the caller's fp64 links
+// (forward-only double-float stacks read them in place).
 static int level0_kind(const gf_stout* st) {
   if (st->precision == GF_MIXED) return GF_LINK32;
-  if (st->precision == GF_PREC_DF && !st->fwd_only) return GF_LINKDF;
-  return GF_LINK64;
+  if (st->precision == GF_FP64) return GF_LINKFX;
+  return st->fwd_only ? GF_LINK64 : GF_LINKDF;
 }
 
 void stout_forward(gf_ctx* ctx, gf_stout* st, const gf_field* U, gf_field* Uout) {
@@ -695,7 +682,7 @@ void stout_forward(gf_ctx* ctx, gf_stout* st, const gf_field* U, gf_field* Uout)
     a->owned = 0;
     st->lev_in[0] = a;
     field_delete(old);  // frees storage only if the old entry was owned
-  } else if ((lk == GF_LINK32 || lk == GF_LINKDF) && U->kind == GF_LINK64) {
+  } else if (lk != GF_LINK64 && U->kind == GF_LINK64) {
     // keep an owned copy of the fp64 thin links in the stack's storage
     if (!old || !old->owned) {
       st->lev_in[0] = field_new(ctx, lk);
@@ -705,7 +692,7 @@ void stout_forward(gf_ctx* ctx, gf_stout* st, const gf_field* U, gf_field* Uout)
   } else {
     throw gf_error(GF_EINVAL, "stout forward: link field kind does not match the stack precision");
   }
-  if (st->precision == GF_FP64) forward_impl<double>(ctx, st);
+  if (st->precision == GF_FP64) stout_forward_fx(ctx, st);
   else if (st->precision == GF_PREC_DF) forward_impl<dfl>(ctx, st);
   else forward_impl<float>(ctx, st);
   st->have_forward = 1;
@@ -818,7 +805,7 @@ void stout_backward(gf_ctx* ctx, gf_stout* st, const gf_field* dSdUbar, double b
   // dSdU == NULL without P: only dS/drho is wanted (the thin-link result stays internal)
   if (!P && dSdU && dSdU->kind != mk) throw gf_error(GF_EINVAL, "stout backward: dS/dU kind does not match the stack precision");
   if (!P && !dSdU && !dsdrho) throw gf_error(GF_EINVAL, "stout backward: no output");
-  if (st->precision == GF_FP64) backward_impl<double>(ctx, st, dSdUbar, beta, dSdU, P, eps, dsdrho);
+  if (st->precision == GF_FP64) stout_backward_fx(ctx, st, dSdUbar, beta, dSdU, P, eps, dsdrho);
   else if (st->precision == GF_PREC_DF) backward_df(ctx, st, dSdUbar, beta, dSdU, P, eps, dsdrho);
   else backward_impl<float>(ctx, st, dSdUbar, beta, dSdU, P, eps, dsdrho);
 }

@@ -31,8 +31,9 @@ double plaquette_sum(gf_ctx* ctx, const gf_field* U, bool df) {
     LinkSrc<dfl, false> src{(const double2*)U->ptr};
     k_plaquette<dfl><<<nb, 128, 0, ctx->stream>>>(src, ctx->geom, ctx->d_partials);
   } else if (U->kind == GF_LINK64 || U->kind == GF_MAT64) {
-    Src64 src{(const double2*)U->ptr};
-    k_plaquette<double><<<nb, 128, 0, ctx->stream>>>(src, ctx->geom, ctx->d_partials);
+    return plaquette_sum_fx(ctx, fx_links(ctx, U));
+  } else if (U->kind == GF_LINKFX) {
+    return plaquette_sum_fx(ctx, U);
   } else if (U->kind == GF_LINK32) {
     Src32 src{(const float4*)U->ptr};
     k_plaquette<float><<<nb, 128, 0, ctx->stream>>>(src, ctx->geom, ctx->d_partials);

@@ -9,6 +9,8 @@ sums involved (the oracle's own).
 import numpy as np
 import pytest
 
+from test_gpu_parity import exact_exp_oracle  # noqa: F401 (fixture)
+
 pytestmark = pytest.mark.gpu
 
 SIZES = [(2, 2, 2, 2), (2, 4, 2, 6), (6, 2, 10, 2), (4, 6, 10, 14), (34, 2, 2, 6)]
@@ -60,3 +62,98 @@ def test_wilson_force_with_a_nan(pkg, oracle):
     # the link itself and the 18 links that share a plaquette with it
     assert hit.sum() == 19 and hit[2, 37]
     close(got[~hit], ref[~hit])
+
+
+@pytest.mark.parametrize("kind", ["unitary", "scaled"])
+@pytest.mark.parametrize("L", SIZES)
+def test_plaquette_and_rectangles(pkg, oracle, L, kind):
+    U, Uh = start(pkg, oracle, L, kind)
+    for got, ref in ((pkg.calculate_Plaquette(U), oracle.plaquette(list(L), Uh)),
+                     (pkg.rectangle_sum(U), oracle.rectangle_sum(list(L), Uh))):
+        # of the sum of the loops' norms, which bounds what rounding sees
+        size = np.abs(Uh).max() ** 6 * 18 * np.prod(L)
+        assert abs(got - ref) <= TOL * size
+
+
+@pytest.mark.parametrize("kind", ["unitary", "scaled"])
+@pytest.mark.parametrize("coefficients", [(3.648, -0.1655), (-0.25, 4.0), (0.0, 1.0), (1.5, 0.0)])
+@pytest.mark.parametrize("L", SIZES)
+def test_rectangle_force(pkg, oracle, L, kind, coefficients):
+    U, Uh = start(pkg, oracle, L, kind)
+    action = pkg.GaugeAction(U)
+    pkg.push_(action, coefficients[0], "plaquette")
+    pkg.push_(action, coefficients[1], "rectangular")
+    F = pkg.gauge_momenta(U)
+    pkg.md_force_(F, action, U)
+    close(F.to_host(), oracle.force_loops(list(L), Uh, *coefficients))
+
+
+def general(pkg, U, L, spread):
+    """A dS/dUbar whose matrices differ in size by up to `spread` orders of magnitude."""
+    rng = np.random.RandomState(8)
+    V = int(np.prod(L))
+    D = rng.normal(size=(4, V, 3, 3)) + 1j * rng.normal(size=(4, V, 3, 3))
+    D *= 10.0 ** rng.uniform(-spread, 0, size=(4, V))[:, :, None, None]
+    d = pkg.Gaugefields4D(U.ctx, pkg._lib.GF_MAT64)
+    return d.from_host(D), D
+
+
+# |Q| from 0.3 to about 6: every scale of the exponential's series that a stack meets
+@pytest.mark.parametrize("rho", [0.0, 0.1, 0.45, 1.0])
+@pytest.mark.parametrize("L", SIZES)
+def test_stout_forward_and_backward(pkg, exact_exp_oracle, L, rho):
+    oracle = exact_exp_oracle
+    U, Uh = start(pkg, oracle, L, "unitary")
+    net = pkg.CovNeuralnet(U)
+    for _ in range(2):
+        pkg.push_(net, pkg.STOUT_Layer("plaquette", rho))
+    Ubar, history, _ = pkg.calc_smearedU(U, net)
+    close(Ubar.to_host(), oracle.stout_forward(list(L), Uh, [rho, rho]), 1e-12)
+    d, D = general(pkg, U, L, 2)
+    got = pkg.back_prop(d, net, history, U).to_host()
+    close(got, oracle.stout_backward(list(L), Uh, [rho, rho], D)[0], 1e-11)
+
+
+@pytest.mark.parametrize("recompute", [False, True])
+@pytest.mark.parametrize("c_rect", [0.0, -0.2])
+@pytest.mark.parametrize("L", SIZES)
+def test_stout_force(pkg, exact_exp_oracle, L, c_rect, recompute):
+    oracle = exact_exp_oracle
+    U, Uh = start(pkg, oracle, L, "unitary")
+    net = pkg.CovNeuralnet(U)
+    for rho in (0.1, 0.15, 0.05):
+        pkg.push_(net, pkg.STOUT_Layer("plaquette", rho))
+    action = pkg.GaugeAction(U)
+    pkg.push_(action, 3.0, "plaquette")
+    pkg.push_(action, c_rect, "rectangular")
+    drv = pkg.md_driver(U, action, steps=1, smearing=net, recompute=recompute)
+    P = pkg.update_momenta_(pkg.gauge_momenta(U), U, 1.0, drv)
+    close(P.to_host(), oracle.stout_force_loops(list(L), Uh, [0.1, 0.15, 0.05], 3.0, c_rect), 1e-11)
+
+
+def test_stout_with_links_of_different_exponents(pkg, exact_exp_oracle):
+    """Links off the group by factors 0.6 .. 1.7: exponents 0 and 1 side by side in every sum."""
+    oracle = exact_exp_oracle
+    L = (4, 6, 2, 8)
+    Uh = oracle.hot_start(list(L), 21)
+    Uh *= np.random.RandomState(2).uniform(0.6, 1.7, size=Uh.shape[:2])[:, :, None, None]
+    U = pkg.gauge_configuration(L, start="cold")
+    U.from_host(Uh)
+    net = pkg.CovNeuralnet(U)
+    pkg.push_(net, pkg.STOUT_Layer("plaquette", 0.05))
+    Ubar, history, _ = pkg.calc_smearedU(U, net)
+    close(Ubar.to_host(), oracle.stout_forward(list(L), Uh, [0.05]), 1e-12)
+    d, D = general(pkg, U, L, 6)
+    close(pkg.back_prop(d, net, history, U).to_host(), oracle.stout_backward(list(L), Uh, [0.05], D)[0], 1e-11)
+
+
+def test_stout_with_a_nan(pkg, oracle):
+    L = (4, 4, 4, 6)
+    U, Uh = start(pkg, oracle, L, "unitary")
+    ref = oracle.stout_forward(list(L), Uh, [0.1])
+    Uh[1, 50, 0, 2] = np.nan
+    U.from_host(Uh)
+    got = pkg.smear(U, pkg.stout_smearing(U)).to_host()
+    hit = np.isnan(got).any(axis=(-1, -2))
+    assert hit.sum() == 19 and hit[1, 50]
+    close(got[~hit], ref[~hit], 1e-11)
