@@ -193,6 +193,20 @@ GF_HD i64 fx_shift(i64 R, int d) {
   return d < 62 ? (R + (1ll << (d - 1))) >> d : 0;
 }
 
+// 1 / sqrt(m) for m in [1/2, 2), from a fp32 seed y by two Newton steps
+// y <- y + y (1 - m y^2) / 2, whose relative errors go 2^-23, 2^-45, 2^-59
+GF_HD i64 fx_rsqrt(i64 m, float y0) {
+  const fx_num n = fx_pre(m);
+  i64 y = (i64)(int)(y0 * 1073741824.f) << 30;
+#pragma unroll
+  for (int it = 0; it < 2; ++it) {
+    const fx_num py = fx_pre(y);
+    const i64 e = (1ll << 60) - fx_mul(n, fx_pre(fx_mul(py, py)));
+    y += fx_mul(py, fx_pre(e)) >> 1;
+  }
+  return y;
+}
+
 // A kernel parameter c = (h 2^30 + l) 2^(e - 60), |h 2^30 + l| < 2^60
 struct fx_scalar {
   int h, l, e;
@@ -224,21 +238,19 @@ GF_HD void fx_scale_row(fx_acc& v, const fx_scalar& c) {
 // ---------------------------------------------------------------------------
 #define GF_FX_CH_TERMS 64
 #define GF_FX_CH_SCALES 5
-// guard bits: the sums reach cosh(2^s), their derivatives about 2^s times that
-GF_HD int fx_guard(int s) { return s == 0 ? 1 : (s == 1 ? 3 : (s == 2 ? 7 : (s == 3 ? 14 : 27))); }
 
+// 2^(s n) / n! in units of 2^(base - 60), rounded
+GF_HD constexpr int fx_kappa_base(int s) { return s == 0 ? 0 : (s == 1 ? 1 : (s == 2 ? 3 : (s == 3 ? 8 : 19))); }
 struct fx_kappa {
   i64 k[GF_FX_CH_SCALES][GF_FX_CH_TERMS];
 };
-// 2^(s n) / n! in units of 2^(guard - 60), rounded
 constexpr fx_kappa fx_make_kappa() {
   fx_kappa t{};
-  const int guard[GF_FX_CH_SCALES] = {1, 3, 7, 14, 27};
   for (int s = 0; s < GF_FX_CH_SCALES; ++s) {
     unsigned __int128 v = (unsigned __int128)1 << 100;
     for (int n = 0; n < GF_FX_CH_TERMS; ++n) {
       if (n > 0) v = (v << s) / (unsigned)n;
-      const int d = 40 + guard[s];
+      const int d = 40 + fx_kappa_base(s);
       t.k[s][n] = (i64)((v + ((unsigned __int128)1 << (d - 1))) >> d);
     }
   }
@@ -282,31 +294,57 @@ GF_HD void fx_invariants(const fx_herm& q, i64& c0, i64& c1) {
   c0 = fx_get(det) + 2 * fx_get(r);
 }
 
-// scale s and number of terms for a norm bound lam of X (real): lam <= 2^s,
-// lam^n / n! < 2^-62 from n = terms - extra on. The derivatives of the n-th
-// power's coefficients go as n lam^(n - 4), so they take four terms more.
-GF_HD void fx_series(float lam, int extra, int& s, int& terms) {
-  s = lam <= 1.f ? 0 : (lam <= 2.f ? 1 : (lam <= 4.f ? 2 : (lam <= 8.f ? 3 : 4)));
+// How to sum the series for a norm bound lam of X (real).
+struct fx_plan {
+  int pow2;     // q = X / 2^pow2
+  int series;   // power of two of the series, <= pow2
+  int squares;  // squarings of the result, pow2 - series
+  int guard;
+  int terms;
+};
+// Terms: lam^n / n! < 2^-62 from n = terms - 4 on; the derivatives of the n-th
+// power's coefficients go as n lam^(n - 4), so they need the four more.
+// Without derivatives the series runs to |X| <= 2 and larger exponentials are
+// squared from it. With them it takes |X| <= 16 (larger ones are not summed to
+// the end) and the guard bits follow the largest coefficient, a derivative of
+// at most lam e^lam / 2 (1 / |q|)^4, half of it in each part.
+template <bool DERIV>
+GF_HD fx_plan fx_series(float lam) {
+  fx_plan p;
+  p.pow2 = 0;
+  for (float x = lam; x > 1.f && p.pow2 < 60; x *= 0.5f) ++p.pow2;
+  if (DERIV && p.pow2 > GF_FX_CH_SCALES - 1) p.pow2 = GF_FX_CH_SCALES - 1;
+  p.series = DERIV || p.pow2 < 1 ? p.pow2 : 1;
+  p.squares = p.pow2 - p.series;
+  for (int k = 0; k < p.squares; ++k) lam *= 0.5f;
+  p.guard = DERIV ? 1 : 0;
+  if (DERIV && p.series > 0) {
+    const float w = (float)(1 << p.series) / lam, b = 0.25f * lam * expf(lam) * (w * w) * (w * w);
+    for (float x = b; x > 1.f && p.guard < 40; x *= 0.5f) ++p.guard;
+  }
+  if (p.guard < fx_kappa_base(p.series)) p.guard = fx_kappa_base(p.series);
+  if (p.guard < 1) p.guard = 1;
   float t = 1.f;
   int n = 1;
-  for (; n < GF_FX_CH_TERMS - 1; ++n) {
+  for (; n < GF_FX_CH_TERMS - 5; ++n) {
     t *= lam / (float)n;
     if (t < 2.2e-19f) break;
   }
-  terms = n + extra < GF_FX_CH_TERMS - 1 ? n + extra : GF_FX_CH_TERMS - 1;
+  p.terms = DERIV ? n + 4 : n;
+  return p;
 }
 
-// Real (IM = 0) or imaginary (1) parts of f_j, and of df_j/dc1 (b1) and
+// Real (im = 0) or imaginary (1) parts of f_j, kappa taken `down` bits down, and of df_j/dc1 (b1) and
 // df_j/dc0 (b2) when DERIV
 template <bool DERIV>
-GF_HD void fx_ch(const i64* kappa, int terms, int im, i64 c0, i64 c1, i64 f[3], i64 b1[3], i64 b2[3]) {
+GF_HD void fx_ch(const i64* kappa, int down, int terms, int im, i64 c0, i64 c1, i64 f[3], i64 b1[3], i64 b2[3]) {
   const fx_num n0 = fx_pre(c0), n1 = fx_pre(c1);
   i64 a = 0, b = 0, c = 0;
   i64 a0 = 0, b0 = 0, g0 = 0, a1 = 0, b1s = 0, g1 = 0;
 #pragma unroll 1
   for (int n = terms; n >= 0; --n) {
     const fx_num pc = fx_pre(c);
-    i64 k = ((n & 1) == im) ? kappa[n] : 0;
+    i64 k = ((n & 1) == im) ? kappa[n] >> down : 0;
     if (n & 2) k = -k;
     const i64 na = fx_mul(pc, n0) + k, nb = a + fx_mul(pc, n1);
     if (DERIV) {
@@ -368,6 +406,28 @@ GF_HD float fx_float_bits(unsigned int u) {
 #endif
 }
 
+GF_HD int fx_exponent_field(double d) { return (int)((fx_bits(d) >> 52) & 0x7FF); }
+// d / 2^(emax - 1083 + up), rounded; emax at least d's exponent field, so that
+// |result| < 2^(61 - up)
+GF_HD i64 fx_mantissa(double d, int emax, int up) {
+  const u64 b = fx_bits(d);
+  int e = (int)((b >> 52) & 0x7FF);
+  i64 v = (i64)(b & 0xFFFFFFFFFFFFFull);
+  if (e) v |= 1ll << 52;
+  else e = 1;
+  const int s = 8 - up - (emax - e);
+  if (s >= 0) v <<= s;
+  else v = s > -55 ? (v + (1ll << (-s - 1))) >> -s : 0;
+  return (b >> 63) ? -v : v;
+}
+// d / 2^(emax - 1023) in fp32 from the leading bits (0 below 2^-126)
+GF_HD float fx_leading(double d, int emax) {
+  const u64 b = fx_bits(d);
+  const int e = (int)((b >> 52) & 0x7FF), ef = e - emax + 127;
+  const unsigned int man = (unsigned int)(b >> 29) & 0x7FFFFFu, sg = (unsigned int)(b >> 32) & 0x80000000u;
+  return (e == 0 || ef <= 0) ? 0.f : fx_float_bits(sg | ((unsigned int)ef << 23) | man);
+}
+
 // One matrix to fixed point; returns its exponent. A bound on the squared
 // spectral norm, max_i sum_j |(M^dag M)_ij|, is formed in fp32 from the
 // leading bits; it is 1 for a unitary matrix.
@@ -375,7 +435,7 @@ GF_HD int fx_from_f64(const double* m /* 18, row-major, re im */, int4 out[9]) {
   int emax = 1;
 #pragma unroll
   for (int i = 0; i < 18; ++i) {
-    const int e = (int)((fx_bits(m[i]) >> 52) & 0x7FF);
+    const int e = fx_exponent_field(m[i]);
     emax = e > emax ? e : emax;
   }
   if (emax == 0x7FF) {
@@ -383,17 +443,9 @@ GF_HD int fx_from_f64(const double* m /* 18, row-major, re im */, int4 out[9]) {
     for (int i = 0; i < 9; ++i) out[i] = make_int4(0, 0, 0, 0);
     return GF_FX_BAD;
   }
-  // leading bits relative to 2^emax: |f| < 2, entries below 2^-126 of it as 0
   float f[18];
 #pragma unroll
-  for (int i = 0; i < 18; ++i) {
-    const u64 b = fx_bits(m[i]);
-    const int e = (int)((b >> 52) & 0x7FF);
-    const int ef = e - emax + 127;
-    const unsigned int man = (unsigned int)(b >> 29) & 0x7FFFFFu;
-    const unsigned int sg = (unsigned int)(b >> 32) & 0x80000000u;
-    f[i] = (e == 0 || ef <= 0) ? 0.f : fx_float_bits(sg | ((unsigned int)ef << 23) | man);
-  }
+  for (int i = 0; i < 18; ++i) f[i] = fx_leading(m[i], emax);
   float bound = 0.f;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
@@ -416,24 +468,38 @@ GF_HD int fx_from_f64(const double* m /* 18, row-major, re im */, int4 out[9]) {
   const int E2 = (bound > 1.0009765625f) + (bound > 4.00390625f) + (bound > 16.015625f) + (bound > 64.0625f);
   i64 R[18];
 #pragma unroll
-  for (int i = 0; i < 18; ++i) {
-    const u64 b = fx_bits(m[i]);
-    int e = (int)((b >> 52) & 0x7FF);
-    i64 v = (i64)(b & 0xFFFFFFFFFFFFFull);
-    if (e) v |= 1ll << 52;
-    else e = 1;
-    // value = v 2^(e - 1075) = R 2^(emax - 1023 + E2 - 60)
-    const int s = 8 - E2 - (emax - e);
-    if (s >= 0) v <<= s;
-    else v = s > -55 ? (v + (1ll << (-s - 1))) >> -s : 0;
-    R[i] = (b >> 63) ? -v : v;
-  }
+  for (int i = 0; i < 18; ++i) R[i] = fx_mantissa(m[i], emax, E2);
 #pragma unroll
   for (int i = 0; i < 9; ++i) {
     fx_split<0>(R[2 * i], out[i].x, out[i].y);
     fx_split<0>(R[2 * i + 1], out[i].z, out[i].w);
   }
   return emax - 1023 + E2;
+}
+
+// real and imaginary parts of the f_j, side by side: f at [2 j + im]
+GF_HD void fx_ch_both(const i64* kappa, int down, int terms, i64 c0, i64 c1, i64 f[6]) {
+  const fx_num n0 = fx_pre(c0), n1 = fx_pre(c1);
+  i64 a[2] = {0, 0}, b[2] = {0, 0}, c[2] = {0, 0};
+#pragma unroll 1
+  for (int n = terms; n >= 0; --n) {
+    i64 k = kappa[n] >> down;
+    if (n & 2) k = -k;
+#pragma unroll
+    for (int im = 0; im < 2; ++im) {
+      const fx_num pc = fx_pre(c[im]);
+      const i64 na = fx_mul(pc, n0) + ((n & 1) == im ? k : 0), nb = a[im] + fx_mul(pc, n1);
+      c[im] = b[im];
+      a[im] = na;
+      b[im] = nb;
+    }
+  }
+#pragma unroll
+  for (int im = 0; im < 2; ++im) {
+    f[im] = a[im];
+    f[2 + im] = b[im];
+    f[4 + im] = c[im];
+  }
 }
 
 // R 2^(E - 60) as fp64, rounded once to nearest (ties up in magnitude; at

@@ -198,6 +198,151 @@ __device__ __forceinline__ void fx_add_staples(fx_acc& acc, int& ea, const FxFie
   }
 }
 
+// ---------------------------------------------------------------------------
+// exp(iX) of the block's links
+// ---------------------------------------------------------------------------
+static __constant__ fx_kappa c_fx_kappa = fx_make_kappa();
+
+struct FxExp {      // exp(iX) of the block's links
+  FxRaw m;          // in: the matrix whose TA gives q
+  FxOperand q;      // X / 2^scale as operand
+  i64 f[6][GF_FX_LINKS];   // f_j at [2 j + im], units 2^(guard - 60)
+  int e[GF_FX_LINKS];      // in: exponent of m
+  int s[GF_FX_LINKS];      // scale
+  int g[GF_FX_LINKS];      // guard
+  int sq[GF_FX_LINKS];     // squarings
+  int most;                // most squarings of a link of the block
+};
+
+// Plan of exp(iX), X = q 2^(e - 60) Hermitian and traceless; q becomes
+// X / 2^pow2 in units of 2^-60. q = 0 for a non-finite X.
+template <bool DERIV>
+__device__ __forceinline__ fx_plan fx_exp_plan(fx_herm& q, int e) {
+  // |X|^2 <= (2/3) tr X^2 for a traceless Hermitian X
+  float n2 = 0.f;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float u = (float)(int)(q.d[k] >> 32), v = (float)(int)(q.re[k] >> 32), w = (float)(int)(q.im[k] >> 32);
+    n2 = fmaf(u, u, fmaf(2.f * v, v, fmaf(2.f * w, w, n2)));
+  }
+  const bool bad = e > GF_FX_BAD / 2;
+  const int ee = e < -90 ? -90 : (e > 90 ? 90 : e);
+  const float lam = bad ? 0.f : sqrtf(0.66667f * n2) * 1.00001f * exp2f((float)(ee - 28));
+  const fx_plan plan = fx_series<DERIV>(lam);
+  const int d = plan.pow2 - e;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    q.d[k] = bad ? 0 : fx_shift(q.d[k], d);
+    q.re[k] = bad ? 0 : fx_shift(q.re[k], d);
+    q.im[k] = bad ? 0 : fx_shift(q.im[k], d);
+  }
+  q.d[2] = -q.d[0] - q.d[1];
+  return plan;
+}
+// element (i, j) of q as an operand
+__device__ __forceinline__ int4 fx_herm_element(const fx_herm& q, int i, int j) {
+  if (i == j) {
+    const fx_num x = fx_pre(q.d[i]);
+    return make_int4(x.h, x.l, 0, 0);
+  }
+  const int k = i + j - 1;
+  const fx_num u = fx_pre(q.re[k]), v = fx_pre(q.im[k]);
+  return i < j ? make_int4(u.h, u.l, v.h, v.l) : make_int4(u.h, u.l, -v.h, -v.l);
+}
+
+// Plan, operand and coefficients of exp(iX) for a block's links; thread per
+// link, im = 0 or 1. b: derivatives, df_j/dc1 at [2 j + im] and df_j/dc0 at
+// [6 + 2 j + im].
+template <bool DERIV>
+__device__ __forceinline__ void fx_exp_coefficients(FxExp& sh, i64 (*b)[GF_FX_LINKS], int link, int im, fx_herm q,
+                                                    int e) {
+  const fx_plan plan = fx_exp_plan<DERIV>(q, e);
+  i64 c0, c1, f[3], b1[3], b2[3];
+  fx_invariants(q, c0, c1);
+  const int terms = __reduce_max_sync(0xffffffffu, plan.terms);
+  fx_ch<DERIV>(c_fx_kappa.k[plan.series], plan.guard - fx_kappa_base(plan.series), terms, im, c0, c1, f, b1, b2);
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    sh.f[2 * j + im][link] = f[j];
+    if (DERIV) {
+      b[2 * j + im][link] = b1[j];
+      b[6 + 2 * j + im][link] = b2[j];
+    }
+  }
+  if (im == 0) {
+#pragma unroll
+    for (int el = 0; el < 9; ++el) sh.q.v[el][link] = fx_herm_element(q, el / 3, el % 3);
+    sh.s[link] = plan.pow2;
+    sh.g[link] = plan.guard;
+    sh.sq[link] = plan.squares;
+    const int most = __reduce_max_sync(0xffffffffu, plan.squares);
+    if (link == 0) sh.most = most;
+  }
+}
+// X = -i TA(rho m) of the block's matrices m as entries and exponent
+__device__ __forceinline__ fx_herm fx_ta_herm(const FxExp& sh, int link, const fx_scalar rho, const fx_scalar rho3,
+                                              int& e) {
+  e = sh.e[link] + rho.e + 1;  // of the entries below
+  fx_herm q;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int i = k == 2 ? 1 : 0, j = k == 0 ? 1 : 2, ij = 2 * (3 * i + j), ji = 2 * (3 * j + i);
+    const i64 xr = sh.m.v[ij][link] - sh.m.v[ji][link], xi = sh.m.v[ij + 1][link] + sh.m.v[ji + 1][link];
+    q.re[k] = fx_mul(fx_pre(xi >> 2), fx_num_of(rho));
+    q.im[k] = -fx_mul(fx_pre(xr >> 2), fx_num_of(rho));
+  }
+  const i64 d0 = sh.m.v[1][link], d1 = sh.m.v[9][link], d2 = sh.m.v[17][link];
+  q.d[0] = fx_mul(fx_pre((2 * d0 - d1 - d2) >> 1), fx_num_of(rho3));
+  q.d[1] = fx_mul(fx_pre((2 * d1 - d0 - d2) >> 1), fx_num_of(rho3));
+  q.d[2] = -q.d[0] - q.d[1];
+  return q;
+}
+
+// row r of exp(iX), exponent 0: f0 + (f1 + f2 q) q; qrow is row r of q, f the
+// coefficients (re, im) in units of 2^(g - 60)
+template <class MAT>
+__device__ __forceinline__ fx_acc fx_exp_row(const i64 f[6], int g, const fx_row& qrow, const MAT& q, int r) {
+  const fx_num f2r = fx_pre(f[4]), f2i = fx_pre(f[5]);
+  fx_acc G;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    fx_sum re = fx_zero_sum(), im = fx_zero_sum();
+    fx_cmac(re, im, f2r, f2i, fx_num{qrow.ah[j], qrow.al[j]}, fx_num{qrow.bh[j], qrow.bl[j]});
+    G.re[j] = fx_get(re) + (j == r ? f[2] : 0);
+    G.im[j] = fx_get(im) + (j == r ? f[3] : 0);
+  }
+  fx_acc E = fx_row_mul<false>(fx_operand<1>(G), q);
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    E.re[j] = (E.re[j] + (j == r ? f[0] >> 1 : 0)) << (g + 1);
+    E.im[j] = (E.im[j] + (j == r ? f[1] >> 1 : 0)) << (g + 1);
+  }
+  return E;
+}
+__device__ __forceinline__ fx_acc fx_exp_row(const FxExp& sh, int link, int r) {
+  i64 f[6];
+#pragma unroll
+  for (int j = 0; j < 6; ++j) f[j] = sh.f[j][link];
+  const FxShMat q{&sh.q, link};
+  return fx_exp_row(f, sh.g[link], fx_load_row<false>(q, r), q, r);
+}
+
+// the same after the squarings that |X| > 2 takes; every thread of the block
+// calls it. sh.m is overwritten by those.
+__device__ __forceinline__ fx_acc fx_exp_row_squared(FxExp& sh, int link, int r) {
+  fx_acc E = fx_exp_row(sh, link, r);
+  const int most = sh.most, mine = sh.sq[link];
+  FxOperand& em = reinterpret_cast<FxOperand&>(sh.m);
+#pragma unroll 1
+  for (int k = 0; k < most; ++k) {
+    fx_share<0>(em, link, r, E);
+    __syncthreads();
+    if (k < mine) E = fx_row_mul<false>(fx_operand<0>(E), FxShMat{&em, link});
+    __syncthreads();
+  }
+  return E;
+}
+
 // (R / 2^20)^2 in fp32
 __device__ __forceinline__ float fx_square(i64 R) {
   const float v = fmaf((float)(int)(R >> 32), 4096.f, (float)(unsigned)R * 9.5367431640625e-7f);

@@ -12,103 +12,6 @@
 
 namespace gf {
 
-__constant__ fx_kappa c_fx_kappa = fx_make_kappa();
-
-struct FxExp {      // exp(iX) of the block's links
-  FxRaw m;          // in: the matrix whose TA gives q
-  FxOperand q;      // X / 2^scale as operand
-  i64 f[6][GF_FX_LINKS];   // f_j at [2 j + im], units 2^(guard - 60)
-  int e[GF_FX_LINKS];      // in: exponent of m; out: GF_FX_BAD or 0
-  int s[GF_FX_LINKS];      // scale
-};
-
-// X = -i TA(rho m) (Hermitian, traceless), its scale, its operand and the
-// coefficients of exp(iX); thread per link, im = 0 or 1. b: derivatives,
-// df_j/dc1 at [2 j + im] and df_j/dc0 at [6 + 2 j + im].
-template <bool DERIV>
-__device__ __forceinline__ void fx_exp_coefficients(FxExp& sh, i64 (*b)[GF_FX_LINKS], int link, int im,
-                                                    const fx_scalar rho, const fx_scalar rho3) {
-  const int e = sh.e[link] + rho.e + 1;  // exponent of the entries below
-  fx_herm q;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const int i = k == 2 ? 1 : 0, j = k == 0 ? 1 : 2, ij = 2 * (3 * i + j), ji = 2 * (3 * j + i);
-    const i64 xr = sh.m.v[ij][link] - sh.m.v[ji][link], xi = sh.m.v[ij + 1][link] + sh.m.v[ji + 1][link];
-    q.re[k] = fx_mul(fx_pre(xi >> 2), fx_num_of(rho));
-    q.im[k] = -fx_mul(fx_pre(xr >> 2), fx_num_of(rho));
-  }
-  const i64 d0 = sh.m.v[1][link], d1 = sh.m.v[9][link], d2 = sh.m.v[17][link];
-  q.d[0] = fx_mul(fx_pre((2 * d0 - d1 - d2) >> 1), fx_num_of(rho3));
-  q.d[1] = fx_mul(fx_pre((2 * d1 - d0 - d2) >> 1), fx_num_of(rho3));
-  q.d[2] = -q.d[0] - q.d[1];
-  // |X|^2 <= (2/3) tr X^2 for a traceless Hermitian X
-  float n2 = 0.f;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const float u = (float)(int)(q.d[k] >> 32), v = (float)(int)(q.re[k] >> 32), w = (float)(int)(q.im[k] >> 32);
-    n2 = fmaf(u, u, fmaf(2.f * v, v, fmaf(2.f * w, w, n2)));
-  }
-  const bool bad = e > GF_FX_BAD / 2;
-  const int ee = e < -90 ? -90 : (e > 90 ? 90 : e);
-  const float lam = bad ? 0.f : sqrtf(0.66667f * n2) * 1.00001f * exp2f((float)(ee - 28));
-  int s, terms;
-  fx_series(lam, DERIV ? 4 : 0, s, terms);
-  const int d = s - e;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    q.d[k] = bad ? 0 : fx_shift(q.d[k], d);
-    q.re[k] = bad ? 0 : fx_shift(q.re[k], d);
-    q.im[k] = bad ? 0 : fx_shift(q.im[k], d);
-  }
-  q.d[2] = -q.d[0] - q.d[1];
-  i64 c0, c1, f[3], b1[3], b2[3];
-  fx_invariants(q, c0, c1);
-  terms = __reduce_max_sync(0xffffffffu, terms);
-  fx_ch<DERIV>(c_fx_kappa.k[s], terms, im, c0, c1, f, b1, b2);
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    sh.f[2 * j + im][link] = f[j];
-    if (DERIV) {
-      b[2 * j + im][link] = b1[j];
-      b[6 + 2 * j + im][link] = b2[j];
-    }
-  }
-  if (im == 0) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const fx_num x = fx_pre(q.d[k]);
-      sh.q.v[4 * k][link] = make_int4(x.h, x.l, 0, 0);
-      const int i = k == 2 ? 1 : 0, j = k == 0 ? 1 : 2;
-      const fx_num u = fx_pre(q.re[k]), v = fx_pre(q.im[k]);
-      sh.q.v[3 * i + j][link] = make_int4(u.h, u.l, v.h, v.l);
-      sh.q.v[3 * j + i][link] = make_int4(u.h, u.l, -v.h, -v.l);
-    }
-    sh.s[link] = s;
-  }
-}
-
-// row r of exp(iX), exponent 0: f0 + (f1 + f2 q) q
-__device__ __forceinline__ fx_acc fx_exp_row(const FxExp& sh, int link, int r) {
-  const int g = fx_guard(sh.s[link]);
-  const fx_num f2r = fx_pre(sh.f[4][link]), f2i = fx_pre(sh.f[5][link]);
-  fx_acc G;
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    const int4 v = sh.q.v[3 * r + j][link];
-    fx_sum re = fx_zero_sum(), im = fx_zero_sum();
-    fx_cmac(re, im, f2r, f2i, fx_num{v.x, v.y}, fx_num{v.z, v.w});
-    G.re[j] = fx_get(re) + (j == r ? sh.f[2][link] : 0);
-    G.im[j] = fx_get(im) + (j == r ? sh.f[3][link] : 0);
-  }
-  fx_acc E = fx_row_mul<false>(fx_operand<1>(G), FxShMat{&sh.q, link});
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    E.re[j] = (E.re[j] + (j == r ? sh.f[0][link] >> 1 : 0)) << (g + 1);
-    E.im[j] = (E.im[j] + (j == r ? sh.f[1][link] >> 1 : 0)) << (g + 1);
-  }
-  return E;
-}
-
 // rows of V = S^dag of a field at s: the staple sum, |V| <= 6 2^ea
 __device__ __forceinline__ fx_acc fx_staple_row(const FxField& U, const Geom& g, const Site& st, int s, int mu, int r,
                                                 int& ea) {
@@ -163,9 +66,13 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_MINB)
   }
   __syncthreads();
   const int E0 = sh.e[link];
-  if (t < 64) fx_exp_coefficients<false>(sh, nullptr, t & 31, t >> 5, rho, rho3);
+  if (t < 64) {
+    int e;
+    const fx_herm q = fx_ta_herm(sh, t & 31, rho, rho3, e);
+    fx_exp_coefficients<false>(sh, nullptr, t & 31, t >> 5, q, e);
+  }
   __syncthreads();
-  const fx_acc E = fx_exp_row(sh, link, r);
+  const fx_acc E = fx_exp_row_squared(sh, link, r);
   const fx_acc W = fx_row_mul<false>(fx_operand<0>(E), fx_mat(U, mu, s, V));
   if (sx >= V) return;
   fx_store_row(Uout, off, r, W);
@@ -233,7 +140,11 @@ __global__ void __launch_bounds__(GF_FX_THREADS, 5)
     fx_share<0>(sh.lam, link, r, lam);
   }
   const int el = eu + ed;
-  if (t < 64) fx_exp_coefficients<true>(sh.x, sh.b, t & 31, t >> 5, one, one3);
+  if (t < 64) {
+    int e;
+    const fx_herm q = fx_ta_herm(sh.x, t & 31, one, one3, e);
+    fx_exp_coefficients<true>(sh.x, sh.b, t & 31, t >> 5, q, e);
+  }
   __syncthreads();
   // Lambda Q, Q Lambda, Q^2, e^Q by rows; partial traces
   fx_acc W, X, Q2;
@@ -277,7 +188,7 @@ __global__ void __launch_bounds__(GF_FX_THREADS, 5)
   __syncthreads();
   // Gamma, in units of 2^(el + guard - scale). As a derivative of a unitary
   // exponential it is no larger than 2^scale Lambda; its parts wrap harmlessly.
-  const int eg = el + fx_guard(sh.x.s[link]) - sh.x.s[link] + (sh.x.e[link] > GF_FX_BAD / 2 ? GF_FX_BAD : 0);
+  const int eg = el + sh.x.g[link] - sh.x.s[link] + (sh.x.e[link] > GF_FX_BAD / 2 ? GF_FX_BAD : 0);
   {
     const fx_num b1r = fx_pre(sh.b[0][link]), b1i = fx_pre(sh.b[1][link]);
     const fx_num b2r = fx_pre(sh.b[6][link]), b2i = fx_pre(sh.b[7][link]);

@@ -157,3 +157,48 @@ def test_stout_with_a_nan(pkg, oracle):
     hit = np.isnan(got).any(axis=(-1, -2))
     assert hit.sum() == 19 and hit[1, 50]
     close(got[~hit], ref[~hit], 1e-11)
+
+
+@pytest.mark.parametrize("reunit", [False, True])
+@pytest.mark.parametrize("eps", [0.05, 1.0, -3.0])
+@pytest.mark.parametrize("L", SIZES)
+def test_link_update(pkg, exact_exp_oracle, L, eps, reunit):
+    """|eps P| up to 7 and links off the group by factors 0.5 .. 2."""
+    oracle = exact_exp_oracle
+    Uh = oracle.hot_start(list(L), 31)
+    Uh *= np.random.RandomState(6).uniform(0.5, 2.0, size=Uh.shape[:2])[:, :, None, None]
+    U = pkg.gauge_configuration(L, start="cold")
+    U.from_host(Uh)
+    P = pkg.gaussian_momenta(U, seed=5)
+    action = pkg.GaugeAction(U)
+    pkg.push_(action, 3.0, "plaquette")
+    drv = pkg.md_driver(U, action, steps=1, reunitarize=reunit)
+    pkg.update_gaugefields_(U, P, eps, drv)
+    oracle.link_update(list(L), Uh, P.to_host(), eps)
+    if reunit:
+        oracle.normalize(list(L), Uh)
+    close(U.to_host(), Uh, 1e-12)
+
+
+def test_link_update_keeps_bad_values_where_they_are(pkg, exact_exp_oracle):
+    """A NaN momentum, a NaN link and a zero link: those links only are not finite."""
+    oracle = exact_exp_oracle
+    L = (4, 4, 4, 6)
+    Uh = oracle.hot_start(list(L), 31)
+    Ph = np.random.RandomState(3).normal(size=(4, 384, 8))
+    ref = Uh.copy()
+    oracle.link_update(list(L), ref, Ph.copy(), 0.1)
+    oracle.normalize(list(L), ref)
+    Ph[0, 5, 3] = np.inf
+    Uh[1, 60, 2, 0] = np.nan
+    Uh[3, 100] = 0.0
+    U = pkg.gauge_configuration(L, start="cold")
+    U.from_host(Uh)
+    P = pkg.gauge_momenta(U).from_host(Ph)
+    action = pkg.GaugeAction(U)
+    pkg.push_(action, 3.0, "plaquette")
+    pkg.update_gaugefields_(U, P, 0.1, pkg.md_driver(U, action, steps=1))
+    got = U.to_host()
+    hit = ~np.isfinite(got).all(axis=(-1, -2))
+    assert sorted(zip(*np.nonzero(hit))) == [(0, 5), (1, 60), (3, 100)]
+    close(got[~hit], ref[~hit], 1e-12)
