@@ -334,13 +334,15 @@ GF_HD fx_plan fx_series(float lam) {
   return p;
 }
 
-// Real (im = 0) or imaginary (1) parts of f_j, kappa taken `down` bits down, and of df_j/dc1 (b1) and
-// df_j/dc0 (b2) when DERIV
+// Real (im = 0) or imaginary (1) parts of f_j, kappa taken `down` bits down,
+// and of df_j/dc1 (b1) and df_j/dc0 (b2) when DERIV. Only the c0 derivatives
+// are summed: with C_n the q^2 coefficient of q^n, dC_n/dc0 = dC_(n-1)/dc1, so
+// b1_0 = c0 b2_2, b1_1 = b2_0 + c1 b2_2 and b1_2 = b2_1, term by term.
 template <bool DERIV>
 GF_HD void fx_ch(const i64* kappa, int down, int terms, int im, i64 c0, i64 c1, i64 f[3], i64 b1[3], i64 b2[3]) {
   const fx_num n0 = fx_pre(c0), n1 = fx_pre(c1);
   i64 a = 0, b = 0, c = 0;
-  i64 a0 = 0, b0 = 0, g0 = 0, a1 = 0, b1s = 0, g1 = 0;
+  i64 a0 = 0, b0 = 0, g0 = 0;
 #pragma unroll 1
   for (int n = terms; n >= 0; --n) {
     const fx_num pc = fx_pre(c);
@@ -348,15 +350,11 @@ GF_HD void fx_ch(const i64* kappa, int down, int terms, int im, i64 c0, i64 c1, 
     if (n & 2) k = -k;
     const i64 na = fx_mul(pc, n0) + k, nb = a + fx_mul(pc, n1);
     if (DERIV) {
-      const fx_num p0 = fx_pre(g0), p1 = fx_pre(g1);
+      const fx_num p0 = fx_pre(g0);
       const i64 na0 = c + fx_mul(p0, n0), nb0 = a0 + fx_mul(p0, n1);
-      const i64 na1 = fx_mul(p1, n0), nb1 = a1 + c + fx_mul(p1, n1);
       g0 = b0;
       a0 = na0;
       b0 = nb0;
-      g1 = b1s;
-      a1 = na1;
-      b1s = nb1;
     }
     c = b;
     a = na;
@@ -366,12 +364,13 @@ GF_HD void fx_ch(const i64* kappa, int down, int terms, int im, i64 c0, i64 c1, 
   f[1] = b;
   f[2] = c;
   if (DERIV) {
-    b1[0] = a1;
-    b1[1] = b1s;
-    b1[2] = g1;
+    const fx_num g = fx_pre(g0);
     b2[0] = a0;
     b2[1] = b0;
     b2[2] = g0;
+    b1[0] = fx_mul(g, n0);
+    b1[1] = a0 + fx_mul(g, n1);
+    b1[2] = b0;
   }
 }
 

@@ -182,8 +182,11 @@ __device__ __forceinline__ fx_acc fx_loops_row(const FxField& U, const Geom& g, 
 }
 
 // P <- keep P + c(U (cp S + cr R)), or (DSDU) D = cp S + cr R
+#ifndef GF_FX_LOOPS_MINB
+#define GF_FX_LOOPS_MINB 5
+#endif
 template <bool DSDU>
-__global__ void __launch_bounds__(GF_FX_THREADS, 5)
+__global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_LOOPS_MINB)
     k_loops_fx(FxField U, double* __restrict__ P, char* __restrict__ D, Geom g, fx_scalar cp, fx_scalar cr,
                double keep) {
   __shared__ union {

@@ -4,8 +4,8 @@
 // two warps evaluate the Cayley-Hamilton series with a thread per link (real
 // and imaginary parts), exchanging through shared memory. All three kernels
 // are bound by integer multiply-add issue. A two-level smearing with its
-// adjoint at 16^4: 9.65 ms in fp64 arithmetic, 2.6 ms here (allocation of the
-// stack included), at no larger an error (gradient 4.3e-16 against 4.8e-16).
+// adjoint at 16^4: 9.65 ms in fp64 arithmetic, 1.74 ms here (1.5 ms of it in
+// these kernels), at no larger an error (gradient 4.3e-16 against 4.8e-16).
 #include "gf_internal.h"
 #include "fxlat.cuh"
 #include <cstddef>
@@ -42,7 +42,20 @@ __device__ __forceinline__ void fx_down_row(fx_acc& v) {
 }
 
 // Ubar = exp(TA(C U^dag)) U, C = rho V stored when Cout is given
-__global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_MINB)
+// Blocks per SM, by 32^4 launches: gather 5.72 ms with three or four (168
+// registers), 5.99 with five, 8.25 with six (spills); local adjoint 4.36 with
+// five, 4.46 with three, four or six; forward 2.85 with seven, 2.93 with eight,
+// 3.1 with five or six.
+#ifndef GF_FX_GATHER_MINB
+#define GF_FX_GATHER_MINB 4
+#endif
+#ifndef GF_FX_LOCAL_MINB
+#define GF_FX_LOCAL_MINB 5
+#endif
+#ifndef GF_FX_FWD_MINB
+#define GF_FX_FWD_MINB 7
+#endif
+__global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_FWD_MINB)
     k_stout_fwd_fx(FxField U, char* __restrict__ Uout, char* __restrict__ Cout, Geom g, fx_scalar rho,
                    fx_scalar rho3) {
   __shared__ FxExp sh;
@@ -95,7 +108,7 @@ static size_t fx_local_bytes(bool top, bool recompute) {
 }
 
 template <bool TOP>
-__global__ void __launch_bounds__(GF_FX_THREADS, 5)
+__global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_LOCAL_MINB)
     k_bwd_local_fx(FxField U, FxField F1, FxField Cst, char* __restrict__ Zout, char* __restrict__ Dpout, Geom g,
                    fx_scalar rho, fx_scalar one, fx_scalar one3, fx_scalar halfbeta) {
   extern __shared__ __align__(16) char smem[];
@@ -152,7 +165,22 @@ __global__ void __launch_bounds__(GF_FX_THREADS, 5)
   W = fx_row_mul<false>(fx_operand<0>(lam), FxShMat{&sh.x.q, link});
   X = fx_row_mul<false>(qr, FxShMat{&sh.lam, link});
   Q2 = fx_row_mul<false>(qr, FxShMat{&sh.x.q, link});
-  fx_share<0>(sh.em, link, r, fx_exp_row(sh.x, link, r));
+  {
+    // row r of e^Q = f0 + f1 q + f2 q^2, q^2 being at hand
+    const int g = sh.x.g[link];
+    const fx_num f1r = fx_pre(sh.x.f[2][link]), f1i = fx_pre(sh.x.f[3][link]);
+    const fx_num f2r = fx_pre(sh.x.f[4][link]), f2i = fx_pre(sh.x.f[5][link]);
+    fx_acc E;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      fx_sum re = fx_zero_sum(), im = fx_zero_sum();
+      fx_cmac(re, im, f1r, f1i, fx_num{qr.ah[j], qr.al[j]}, fx_num{qr.bh[j], qr.bl[j]});
+      fx_cmac(re, im, f2r, f2i, fx_pre(Q2.re[j]), fx_pre(Q2.im[j]));
+      E.re[j] = (fx_get(re) + (j == r ? sh.x.f[0][link] : 0)) << g;
+      E.im[j] = (fx_get(im) + (j == r ? sh.x.f[1][link] : 0)) << g;
+    }
+    fx_share<0>(sh.em, link, r, E);
+  }
   {
     fx_sum re = fx_zero_sum(), im = fx_zero_sum();
 #pragma unroll
@@ -311,12 +339,6 @@ __device__ __forceinline__ void fx_gather_axis(fx_acc& acc, int& ea, const FxFie
 
 // D = Dp + rho (pull-back). OUT 0: fixed-point Dout; 1: fp64 Dout (MAT64);
 // 2: the thin-link momentum update P += coef c(U D) instead.
-#ifndef GF_FX_GATHER_MINB
-#define GF_FX_GATHER_MINB 5
-#endif
-#ifndef GF_FX_LOCAL_MINB
-#define GF_FX_LOCAL_MINB 5
-#endif
 template <int OUT>
 __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_GATHER_MINB)
     k_bwd_gather_fx(FxField U, FxField Z, FxField Dp, char* __restrict__ Dout, double* __restrict__ P, Geom g,
