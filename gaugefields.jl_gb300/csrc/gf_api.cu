@@ -98,6 +98,7 @@ extern "C" int gf_ctx_create(const int L[4], int device, gf_ctx** out) {
   }
   GF_CUDA(cudaSetDevice(device));
   ctx = new gf_ctx();
+  ctx->pool = std::make_shared<gf_pool>();
   ctx->device = device;
   GF_CUDA(cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device));
   for (int i = 0; i < 4; ++i) ctx->geom.L[i] = L[i];
@@ -146,6 +147,7 @@ extern "C" int gf_ctx_destroy(gf_ctx* ctx) {
   if (ctx->w_stout64) gf_stout_destroy(ctx->w_stout64);
   if (ctx->w_stout32) gf_stout_destroy(ctx->w_stout32);
   if (ctx->w_stoutdf) gf_stout_destroy(ctx->w_stoutdf);
+  pool_trim(ctx->pool.get(), true);
   if (ctx->d_partials) cudaFree(ctx->d_partials);
   if (ctx->d_result) cudaFree(ctx->d_result);
   if (ctx->h_result) cudaFreeHost(ctx->h_result);
@@ -431,9 +433,10 @@ static gf_stout* stout_new(gf_ctx* ctx, int nlev, const double* rho, int precisi
         // level l writes where level l - 2 wrote (two buffers in turn)
         gf_field* a = new gf_field(*st->lev_in[l - 2]);
         a->owned = 0;
+        a->pool = nullptr;
         st->lev_in[l] = a;
       } else {
-        st->lev_in[l] = field_new(ctx, lk);
+        st->lev_in[l] = field_pooled(ctx, lk);
       }
     }
     if (fwd_only) {
@@ -442,7 +445,7 @@ static gf_stout* stout_new(gf_ctx* ctx, int nlev, const double* rho, int precisi
       return st;
     }
     if (st->store)
-      for (int l = 0; l < nlev; ++l) st->C[l] = field_new(ctx, mk);
+      for (int l = 0; l < nlev; ++l) st->C[l] = field_pooled(ctx, mk);
     if (arena && mk == GF_MAT32) {
       // two fp32 matrix fields fill one fp64 link-sized block
       const size_t half = field_bytes(ctx->geom, GF_MAT32);
@@ -451,10 +454,10 @@ static gf_stout* stout_new(gf_ctx* ctx, int nlev, const double* rho, int precisi
       st->D[0] = arena_view(ctx, 1, 0, mk);
       st->D[1] = arena_view(ctx, 1, half, mk);
     } else {
-      st->Z = field_new(ctx, mk);
-      st->Dp = field_new(ctx, mk);
-      st->D[0] = field_new(ctx, mk);
-      st->D[1] = field_new(ctx, mk);
+      st->Z = field_pooled(ctx, mk);
+      st->Dp = field_pooled(ctx, mk);
+      st->D[0] = field_pooled(ctx, mk);
+      st->D[1] = field_pooled(ctx, mk);
     }
   } catch (...) {
     gf_stout_destroy(st);

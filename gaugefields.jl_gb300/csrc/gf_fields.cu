@@ -25,47 +25,81 @@ size_t field_bytes(const Geom& g, int kind) {
   throw gf_error(GF_EINVAL, "unknown field kind " + std::to_string(kind));
 }
 
-gf_field* field_new(gf_ctx* ctx, int kind) {
-  size_t bytes = field_bytes(ctx->geom, kind);
+void pool_trim(gf_pool* pool, bool close) {
+  if (!pool) return;
+  std::vector<std::pair<size_t, void*>> kept;
+  {
+    std::lock_guard<std::mutex> hold(pool->lock);
+    kept.swap(pool->kept);
+    pool->bytes = 0;
+    if (close) pool->open = false;
+  }
+  for (auto& k : kept) cudaFree(k.second);
+}
+
+// cudaMalloc, once more after the pool has given back what it keeps
+static void* device_alloc(gf_ctx* ctx, size_t bytes) {
   void* p = nullptr;
   cudaError_t e = cudaMalloc(&p, bytes);
+  if (e == cudaErrorMemoryAllocation && ctx->pool) {
+    cudaGetLastError();
+    pool_trim(ctx->pool.get(), false);
+    e = cudaMalloc(&p, bytes);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     throw gf_error(GF_ENOMEM, "cudaMalloc of " + std::to_string(bytes) + " bytes failed: " + cudaGetErrorString(e));
   }
-  gf_field* f = new gf_field;
-  f->ctx = ctx;
-  f->kind = kind;
-  f->ptr = p;
-  f->bytes = bytes;
-  f->owned = 1;
-  return f;
+  return p;
+}
+
+gf_field* field_new(gf_ctx* ctx, int kind) {
+  const size_t bytes = field_bytes(ctx->geom, kind);
+  return new gf_field{ctx, kind, device_alloc(ctx, bytes), bytes, 1, nullptr};
+}
+
+gf_field* field_pooled(gf_ctx* ctx, int kind) {
+  const size_t bytes = field_bytes(ctx->geom, kind);
+  void* p = nullptr;
+  {
+    std::lock_guard<std::mutex> hold(ctx->pool->lock);
+    auto& kept = ctx->pool->kept;
+    for (size_t i = 0; i < kept.size() && !p; ++i)
+      if (kept[i].first == bytes) {
+        p = kept[i].second;
+        kept[i] = kept.back();
+        kept.pop_back();
+        ctx->pool->bytes -= bytes;
+      }
+  }
+  if (!p) p = device_alloc(ctx, bytes);
+  return new gf_field{ctx, kind, p, bytes, 1, ctx->pool};
 }
 
 gf_field* arena_view(gf_ctx* ctx, int which, size_t off, int kind) {
   const size_t cap = field_bytes(ctx->geom, GF_LINK64);
   if (!ctx->arena[which]) {
-    cudaError_t e = cudaMalloc(&ctx->arena[which], cap);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      ctx->arena[which] = nullptr;
-      throw gf_error(GF_ENOMEM, "cudaMalloc of " + std::to_string(cap) + " bytes failed: " + cudaGetErrorString(e));
-    }
+    ctx->arena[which] = device_alloc(ctx, cap);
   }
   const size_t bytes = field_bytes(ctx->geom, kind);
   if (off + bytes > cap) throw gf_error(GF_EINVAL, "scratch view beyond its block");
-  gf_field* f = new gf_field;
-  f->ctx = ctx;
-  f->kind = kind;
-  f->ptr = (char*)ctx->arena[which] + off;
-  f->bytes = bytes;
-  f->owned = 0;
-  return f;
+  return new gf_field{ctx, kind, (char*)ctx->arena[which] + off, bytes, 0, nullptr};
 }
 
 void field_delete(gf_field* f) {
   if (!f) return;
-  if (f->owned && f->ptr) cudaFree(f->ptr);
+  if (f->owned && f->ptr) {
+    bool back = false;
+    if (f->pool) {
+      std::lock_guard<std::mutex> hold(f->pool->lock);
+      back = f->pool->open && f->pool->bytes + f->bytes <= GF_POOL_CAP;
+      if (back) {
+        f->pool->kept.emplace_back(f->bytes, f->ptr);
+        f->pool->bytes += f->bytes;
+      }
+    }
+    if (!back) cudaFree(f->ptr);
+  }
   delete f;
 }
 
@@ -219,11 +253,7 @@ static void* staging(gf_ctx* ctx, size_t bytes) {
       ctx->d_stage = nullptr;
       ctx->stage_bytes = 0;
     }
-    cudaError_t e = cudaMalloc(&ctx->d_stage, bytes);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      throw gf_error(GF_ENOMEM, std::string("staging allocation failed: ") + cudaGetErrorString(e));
-    }
+    ctx->d_stage = device_alloc(ctx, bytes);
     ctx->stage_bytes = bytes;
   }
   return ctx->d_stage;

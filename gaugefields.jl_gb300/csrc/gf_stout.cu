@@ -680,12 +680,13 @@ void stout_forward(gf_ctx* ctx, gf_stout* st, const gf_field* U, gf_field* Uout)
     // alias the caller's thin links (not owned by the stack)
     gf_field* a = new gf_field(*U);
     a->owned = 0;
+    a->pool = nullptr;
     st->lev_in[0] = a;
     field_delete(old);  // frees storage only if the old entry was owned
   } else if (lk != GF_LINK64 && U->kind == GF_LINK64) {
     // keep an owned copy of the fp64 thin links in the stack's storage
     if (!old || !old->owned) {
-      st->lev_in[0] = field_new(ctx, lk);
+      st->lev_in[0] = field_pooled(ctx, lk);
       field_delete(old);
     }
     copy_field(ctx, st->lev_in[0], U);
