@@ -4,7 +4,7 @@
 // two warps evaluate the Cayley-Hamilton series with a thread per link (real
 // and imaginary parts), exchanging through shared memory. All three kernels
 // are bound by integer multiply-add issue. A two-level smearing with its
-// adjoint at 16^4: 9.65 ms in fp64 arithmetic, 1.74 ms here (1.5 ms of it in
+// adjoint at 16^4: 9.65 ms in fp64 arithmetic, 1.67 ms here (1.4 ms of it in
 // these kernels), at no larger an error (gradient 4.3e-16 against 4.8e-16).
 #include "gf_internal.h"
 #include "fxlat.cuh"
@@ -42,12 +42,12 @@ __device__ __forceinline__ void fx_down_row(fx_acc& v) {
 }
 
 // Ubar = exp(TA(C U^dag)) U, C = rho V stored when Cout is given
-// Blocks per SM, by 32^4 launches: gather 5.72 ms with three or four (168
-// registers), 5.99 with five, 8.25 with six (spills); local adjoint 4.36 with
-// five, 4.46 with three, four or six; forward 2.85 with seven, 2.93 with eight,
-// 3.1 with five or six.
+// Blocks per SM, by 32^4 launches: gather 5.20 ms with four (168 registers),
+// 5.12 with five, 5.82 with six (spills); local adjoint 3.95 with four, 3.91
+// with five, 4.10 with six; forward 2.84 with seven, 2.93 with eight, 3.1 with
+// five or six.
 #ifndef GF_FX_GATHER_MINB
-#define GF_FX_GATHER_MINB 4
+#define GF_FX_GATHER_MINB 5
 #endif
 #ifndef GF_FX_LOCAL_MINB
 #define GF_FX_LOCAL_MINB 5
@@ -107,7 +107,7 @@ static size_t fx_local_bytes(bool top, bool recompute) {
   return offsetof(FxLocal, db) + (recompute ? 2 : (top ? 1 : 0)) * sizeof(FxOperand);
 }
 
-template <bool TOP>
+template <bool TOP, bool RECOMPUTE>
 __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_LOCAL_MINB)
     k_bwd_local_fx(FxField U, FxField F1, FxField Cst, char* __restrict__ Zout, char* __restrict__ Dpout, Geom g,
                    fx_scalar rho, fx_scalar one, fx_scalar one3, fx_scalar halfbeta) {
@@ -118,11 +118,10 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_LOCAL_MINB)
   const int sx = (blockIdx.x >> 2) * GF_FX_LINKS + link, s = min(sx, V - 1);
   const size_t off = fx_offset(mu, s, V);
   const Site st = site_of(g, s);
-  const bool recompute = Cst.p == nullptr;
   const int eu = fx_exp(U, mu, s, V);
   int ec, ed;
   // C U^dag
-  if (recompute) {
+  if (RECOMPUTE) {
     fx_acc c = fx_staple_row(U, g, st, s, mu, r, ec);
     fx_down_row<3>(c);
     fx_scale_row(c, rho);
@@ -284,7 +283,7 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_LOCAL_MINB)
   if (TOP) dp = fx_row_mul<false>(fx_load_row<true>(FxShMat{&sh.db, link}, r), FxShMat{&sh.em, link});
   else dp = fx_row_mul<false>(fx_load_row<false>(fx_mat(F1, mu, s, V), r), FxShMat{&sh.em, link});
   fx_row cr;
-  if (recompute) cr = fx_load_row<true>(FxShMat{&sh.cm, link}, r);
+  if (RECOMPUTE) cr = fx_load_row<true>(FxShMat{&sh.cm, link}, r);
   else cr = fx_load_row<true>(fx_mat(Cst, mu, s, V), r);
   fx_add(dp, ed, fx_row_mul<true>(cr, Y), ec + ey);
   fx_down_row<1>(dp);
@@ -303,6 +302,8 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_LOCAL_MINB)
 //   (c) + (f) [Z_K(x+nu)^dag U_nu(x+K)^dag + U_K(x+nu) Z_nu(x+K)] U_K(x)^dag
 //   (b) U_K(x-K+nu)^dag U_nu(x-K)^dag Z_K(x-K)^dag
 //   (d) + (e) [Z_K(x-K+nu) U_nu(x-K)^dag + U_K(x-K+nu)^dag Z_nu(x-K)] U_K(x-K)
+// The two products with U_nu(x+-K)^dag stand side by side, so that its nine
+// elements are in registers once and not across an axis (5.69 -> 5.12 ms).
 // The last left factor is taken one bit down (the bracketed sums reach two
 // units), and the six terms of an axis sum to at most three units.
 __device__ __forceinline__ void fx_gather_axis(fx_acc& acc, int& ea, const FxField& U, const FxField& Z, const Geom& g,
@@ -314,11 +315,11 @@ __device__ __forceinline__ void fx_gather_axis(fx_acc& acc, int& ea, const FxFie
     const int eun = fx_exp(U, nu, xpk, V), euk = fx_exp(U, K, xpn, V);
     const FxMat un = fx_mat(U, nu, xpk, V);
     const fx_row uk = fx_load_row<false>(fx_mat(U, K, xpn, V), r);
-    fx_acc t = fx_row_mul<true>(uk, un);
-    fx_add(acc, ea, fx_row_mul<false>(fx_operand<1>(t), fx_mat(Z, K, s, V)), euk + eun + fx_exp(Z, K, s, V) + 1);
-    t = fx_row_mul<false>(uk, fx_mat(Z, nu, xpk, V));
-    int et = euk + fx_exp(Z, nu, xpk, V);
-    fx_add(t, et, fx_row_mul<true>(fx_load_row<true>(fx_mat(Z, K, xpn, V), r), un), fx_exp(Z, K, xpn, V) + eun);
+    fx_acc r1 = fx_row_mul<true>(uk, un);
+    fx_acc t = fx_row_mul<true>(fx_load_row<true>(fx_mat(Z, K, xpn, V), r), un);
+    int et = fx_exp(Z, K, xpn, V) + eun;
+    fx_add(acc, ea, fx_row_mul<false>(fx_operand<1>(r1), fx_mat(Z, K, s, V)), euk + eun + fx_exp(Z, K, s, V) + 1);
+    fx_add(t, et, fx_row_mul<false>(uk, fx_mat(Z, nu, xpk, V)), euk + fx_exp(Z, nu, xpk, V));
     fx_add(acc, ea, fx_row_mul<true>(fx_operand<1>(t), fx_mat(U, K, s, V)), et + fx_exp(U, K, s, V) + 1);
   }
   {
@@ -328,11 +329,11 @@ __device__ __forceinline__ void fx_gather_axis(fx_acc& acc, int& ea, const FxFie
     const int eun = fx_exp(U, nu, xmk, V), euk = fx_exp(U, K, xmkn, V);
     const FxMat un = fx_mat(U, nu, xmk, V);
     const fx_row uk = fx_load_row<true>(fx_mat(U, K, xmkn, V), r);
-    fx_acc t = fx_row_mul<true>(uk, un);
-    fx_add(acc, ea, fx_row_mul<true>(fx_operand<1>(t), fx_mat(Z, K, xmk, V)), euk + eun + fx_exp(Z, K, xmk, V) + 1);
-    t = fx_row_mul<false>(uk, fx_mat(Z, nu, xmk, V));
-    int et = euk + fx_exp(Z, nu, xmk, V);
-    fx_add(t, et, fx_row_mul<true>(fx_load_row<false>(fx_mat(Z, K, xmkn, V), r), un), fx_exp(Z, K, xmkn, V) + eun);
+    fx_acc r1 = fx_row_mul<true>(uk, un);
+    fx_acc t = fx_row_mul<true>(fx_load_row<false>(fx_mat(Z, K, xmkn, V), r), un);
+    int et = fx_exp(Z, K, xmkn, V) + eun;
+    fx_add(acc, ea, fx_row_mul<true>(fx_operand<1>(r1), fx_mat(Z, K, xmk, V)), euk + eun + fx_exp(Z, K, xmk, V) + 1);
+    fx_add(t, et, fx_row_mul<false>(uk, fx_mat(Z, nu, xmk, V)), euk + fx_exp(Z, nu, xmk, V));
     fx_add(acc, ea, fx_row_mul<false>(fx_operand<1>(t), fx_mat(U, K, xmk, V)), et + fx_exp(U, K, xmk, V) + 1);
   }
 }
@@ -430,7 +431,8 @@ void stout_backward_fx(gf_ctx* ctx, gf_stout* st, const gf_field* dSdUbar, doubl
       ProfScope prof(ctx, GF_K_BWD_LOCAL64);
       const FxField C = st->store ? fx_view(st->C[l]) : FxField{nullptr};
       const size_t smem = fx_local_bytes(top, !st->store);
-      auto kern = top ? k_bwd_local_fx<true> : k_bwd_local_fx<false>;
+      auto kern = st->store ? (top ? k_bwd_local_fx<true, false> : k_bwd_local_fx<false, false>)
+                            : (top ? k_bwd_local_fx<true, true> : k_bwd_local_fx<false, true>);
       GF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       kern<<<nb, GF_FX_THREADS, smem, ctx->stream>>>(fx_view(st->lev_in[l]),
                                                      fx_view(top ? st->lev_in[l + 1] : st->D[cur]), C,
