@@ -142,7 +142,6 @@ extern "C" int gf_ctx_destroy(gf_ctx* ctx) {
   field_delete(ctx->w_link64b);
   for (int i = 0; i < 4; ++i) field_delete(ctx->w_mom[i]);
   field_delete(ctx->w_link32);
-  field_delete(ctx->w_linkdf);
   field_delete(ctx->w_linkfx);
   if (ctx->w_stout64) gf_stout_destroy(ctx->w_stout64);
   if (ctx->w_stout32) gf_stout_destroy(ctx->w_stout32);

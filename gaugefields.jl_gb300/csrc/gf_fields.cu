@@ -554,7 +554,7 @@ void copy_field(gf_ctx* ctx, gf_field* dst, const gf_field* src) {
   } else if (is_dfn(a) && is_f64_full(b)) {
     k_dfn_to_f64<<<nb, 256, 0, ctx->stream>>>((const float4*)src->ptr, (double2*)dst->ptr, n);
   } else if (is_f64_full(a) && is_fx(b)) {
-    f64_to_fx(ctx, dst, src);
+    to_fx(ctx, dst, src);
     return;
   } else if (is_fx(a) && is_f64_full(b)) {
     fx_to_f64_field(ctx, dst, src);

@@ -91,7 +91,6 @@ struct gf_ctx {
   gf_field* w_link64b;    // W2 of the flow
   gf_field* w_mom[4];     // F0, F1, F2, Ftmp of the RK3 flow (fp64 coefficients)
   gf_field* w_link32;     // fp32 12-real shadow of the thin links (mixed form)
-  gf_field* w_linkdf;     // double-float-native copy of the thin links (double-float rectangle force)
   gf_field* w_linkfx;     // fixed-point copy of the links (fp64-class kernels)
   // Two scratch blocks of one fp64 link field each, shared by the mixed form's
   // internal stacks: the Hamiltonian's double-float level buffers and the
@@ -193,7 +192,7 @@ void field_axpy(gf_ctx* ctx, gf_field* y, double a, const gf_field* x);  // y +=
 void mom_scale(gf_ctx* ctx, gf_field* y, double a);                      // y *= a
 
 // ---- Wilson action pieces (gf_wilson.cu) ----
-double plaquette_sum(gf_ctx* ctx, const gf_field* U, bool df = false);  // sum_x sum_{mu<nu} Re tr P
+double plaquette_sum(gf_ctx* ctx, const gf_field* U);  // sum_x sum_{mu<nu} Re tr P
 // mean over the t = 0 slice of tr prod_t U_T: out = {Re, Im}
 void polyakov_loop(gf_ctx* ctx, const gf_field* U, double out[2]);
 void staple_up(gf_ctx* ctx, const gf_field* U, int mu, gf_field* V);  // construct_staple! (mu field slot)
@@ -206,10 +205,10 @@ void wilson_force_fx(gf_ctx* ctx, const gf_field* U, gf_field* P, double coef, d
 
 double plaquette_sum_fx(gf_ctx* ctx, const gf_field* F);  // of a fixed-point field
 inline FxField fx_view(const gf_field* f) { return FxField{(const char*)f->ptr}; }
-// the context's fixed-point copy of fp64 links
+// the context's fixed-point copy of fp64 or double-float links
 const gf_field* fx_links(gf_ctx* ctx, const gf_field* U);
-// LINK64 / MAT64 <-> fixed-point fields
-void f64_to_fx(gf_ctx* ctx, gf_field* dst, const gf_field* src);
+// LINK64 / MAT64 or double-float pairs -> fixed point, and fixed point -> fp64
+void to_fx(gf_ctx* ctx, gf_field* dst, const gf_field* src);
 void fx_to_f64_field(gf_ctx* ctx, gf_field* dst, const gf_field* src);
 
 // ---- rectangle loops (gf_rect.cu) ----
@@ -221,10 +220,6 @@ void loops_force_coef(gf_ctx* ctx, const gf_field* U, gf_field* P, double cp, do
 // D = cp S + cr R (plaquette and rectangle staples) on a stack's top level:
 // LINK64 -> MAT64, LINK32 -> MAT32, LINKDF -> MATDF (double-float)
 void loops_dsdu(gf_ctx* ctx, const gf_field* Ubar, gf_field* D, double cp, double cr);
-// P <- keep P + coef c(U S), S the six plaquette staples, as a double-float
-// table loop of fixed-grid products on a double-float-native copy of U
-void plaquette_force_df(gf_ctx* ctx, const gf_field* U, gf_field* P, double coef, double keep);
-
 // the same on a fixed-point field (gf_fxrect.cu): the loop sum; the force into
 // P, or D = cp S + cr R into a fixed-point D
 double rectangle_sum_fx(gf_ctx* ctx, const gf_field* F);

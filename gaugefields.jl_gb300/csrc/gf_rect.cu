@@ -1,6 +1,5 @@
-// Rectangle (2x1) loops of the gauge action, fp64 links in fp64 arithmetic:
-// the loop sum, and the force (+ momentum update) of an action with
-// plaquette and rectangle terms, push!(action, c_plaq, plaq U plaq') and
+// Rectangle (2x1) loops of the gauge action: the loop sum, and the force (+
+// momentum update) of an action with plaquette and rectangle terms, push!(action, c_plaq, plaq U plaq') and
 // push!(action, c_rect, rect U rect') (src/action/GaugeActions.jl:48-142; the
 // loops of make_rect, src/autostaples/wilsonloops.jl:304-330).
 //
@@ -16,6 +15,8 @@
 // Each geometric rectangle holding the link appears once, as the six
 // plaquette-staple terms do for the plaquettes, so dS/dU_mu = c_plaq S_plaq +
 // c_rect S_rect and F = -(1/3) TA(U_mu dS/dU_mu), as for the Wilson action.
+// On fp64 links all of it runs in fixed point (gf_fxrect.cu); here are the
+// mixed form's fp32 kernels and the double-float stack's dS/dUbar.
 #include "gf_internal.h"
 #include "stencil.cuh"
 #include "dfslots.cuh"
@@ -34,43 +35,6 @@ __device__ __forceinline__ int site_off(const Geom& g, const Site& st, int mu, i
   if (n < 0) n += g.L[nu];
   lex += (n - c) * g.stride[nu];
   return eo_of_lex(g, lex, st.par ^ ((a + b) & 1));
-}
-
-// Sum over mu < nu of Re tr (R^{1x2}_{mu nu}(x) + R^{2x1}_{mu nu}(x)) at one
-// site, each rectangle as Re tr(A B^+) of its two three-link halves.
-template <class SRC>
-__device__ double rect_site(const SRC& U, const Geom& g, const Site& st, int s) {
-  const int V = g.vol;
-  double v = 0.0;
-#pragma unroll 1
-  for (int p = 0; p < 6; ++p) {
-    const int mu = p < 3 ? 0 : (p < 5 ? 1 : 2);
-    const int nu = p < 3 ? p + 1 : (p < 5 ? p - 1 : 3);
-    // 1x2: A = U_mu(x) U_nu(x+mu) U_nu(x+mu+nu), B = U_nu(x) U_nu(x+nu) U_mu(x+2nu)
-    mat3<double> a = mul_nn(U(mu, s, V), U(nu, site_off(g, st, mu, 1, nu, 0), V));
-    a = mul_nn(a, U(nu, site_off(g, st, mu, 1, nu, 1), V));
-    mat3<double> b = mul_nn(U(nu, s, V), U(nu, site_off(g, st, mu, 0, nu, 1), V));
-    b = mul_nn(b, U(mu, site_off(g, st, mu, 0, nu, 2), V));
-    v += retr_na(a, b);
-    // 2x1: A = U_mu(x) U_mu(x+mu) U_nu(x+2mu), B = U_nu(x) U_mu(x+nu) U_mu(x+mu+nu)
-    a = mul_nn(U(mu, s, V), U(mu, site_off(g, st, mu, 1, nu, 0), V));
-    a = mul_nn(a, U(nu, site_off(g, st, mu, 2, nu, 0), V));
-    b = mul_nn(U(nu, s, V), U(mu, site_off(g, st, mu, 0, nu, 1), V));
-    b = mul_nn(b, U(mu, site_off(g, st, mu, 1, nu, 1), V));
-    v += retr_na(a, b);
-  }
-  return v;
-}
-
-template <class SRC>
-__global__ void __launch_bounds__(128) k_rect_sum(SRC U, Geom g, double* __restrict__ part) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  double v = 0.0;
-  if (s < g.vol) {
-    Site st = site_of(g, s);
-    v = rect_site(U, g, st, s);
-  }
-  block_partial_sum(v, part);
 }
 
 // acc += the six rectangle staples (a)-(f) of U_mu(x) in the mu-nu plane
@@ -164,11 +128,11 @@ __global__ void __launch_bounds__(128) k_dsdu_rect(SRC U, typename LinkFull<R>::
 }
 
 // --------------------------------------------------------------------------
-// The same force in double-float arithmetic (the GF_DFLOAT form: the force
-// on thin links, or dS/dUbar on a stack's top level), as a loop over a table
-// of products with one inlined fixed-grid
-// product (the double-float stencils overflow the instruction cache when
-// their products are inlined). Per plane (mu, nu): ops 0-3 add the two
+// dS/dUbar of the same action in double-float arithmetic on a double-float
+// stack's top level (on thin links the fixed-point force is faster, 4.1 ms
+// against 5.5 ms at 24^4, and more exact), as a loop over a table of products
+// with one inlined fixed-grid product (the double-float stencils overflow the
+// instruction cache when their products are inlined). Per plane (mu, nu): ops 0-3 add the two
 // plaquette staples to S (add_staple_pair), ops 4-27 the six rectangle
 // staples (a)-(f) above to R, four products each. An operand is the link of
 // direction mu or nu at x + mo e_mu + no e_nu (optionally daggered) or the
@@ -216,15 +180,10 @@ __device__ __forceinline__ mat3<dfl> rect_operand(int src, int dir, int mo, int 
   return m;
 }
 
-// P_mu(x) <- keep * P_mu(x) + c(U_mu(x) (cp S_mu(x) + cr R_mu(x))) as
-// k_force_rect, the staples, the combination and the projection in
-// double-float, on double-float-native links; DSDU: D_mu(x) = cp S + cr R
-// (as k_dsdu_rect, double-float-native) instead. NOPS = 4 runs only the
-// plaquette staples (the Wilson force; R stays zero).
-template <bool DSDU, int NOPS>
+// D_mu(x) = cp S_mu(x) + cr R_mu(x) as k_dsdu_rect, staples and combination in
+// double-float, on double-float-native links.
 __global__ void __launch_bounds__(128, 3)
-    k_force_rect_df(const float4* __restrict__ U, double* __restrict__ P, float4* __restrict__ D, Geom g, dfl cp,
-                    dfl cr, double keep) {
+    k_force_rect_df(const float4* __restrict__ U, float4* __restrict__ D, Geom g, dfl cp, dfl cr) {
   extern __shared__ __align__(16) float sm[];  // GF_RECT_SLOTS slots of 36 x 128 floats
   const int tid = threadIdx.x;
   int s, mu;
@@ -237,7 +196,7 @@ __global__ void __launch_bounds__(128, 3)
   for (int k = 1; k < 4; ++k) {
     const int nu = (mu + k) & 3;
 #pragma unroll 1
-    for (int q = 0; q < NOPS; ++q) {
+    for (int q = 0; q < 28; ++q) {
       const DfOpR op = c_rect_ops[q];
       const mat3<dfl> A = rect_operand(op.a_src, op.a_dir, op.a_mo, op.a_no, op.a_dag, sm, tid, U, g, st, mu, nu);
       const mat3<dfl> B = rect_operand(op.b_src, op.b_dir, op.b_mo, op.b_no, op.b_dag, sm, tid, U, g, st, mu, nu);
@@ -256,61 +215,31 @@ __global__ void __launch_bounds__(128, 3)
       dfg_rcterm(a, cr, R.e[i][j]);
       T.e[i][j] = dfg_cend(a);
     }
-  if (DSDU) {
-    LinkDfn::store(D, mu, s, g.vol, T);
-    return;
-  }
-  const mat3<dfl> M = dfg_matmul<false, false, false>(LinkDfn::load(U, mu, s, g.vol), T, nullptr);
-  dfl c[8];
-  ta_coeffs(M, c);
-  double* p = P + (size_t)mu * 8 * g.vol + s;
-#pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    const double old = (keep != 0.0) ? keep * p[(size_t)a * g.vol] : 0.0;
-    p[(size_t)a * g.vol] = old + to_f64(c[a]);
-  }
+  LinkDfn::store(D, mu, s, g.vol, T);
 }
 
-static void rect_df(gf_ctx* ctx, const float4* U, gf_field* P, gf_field* D, double cp, double cr, double keep,
-                    bool plaquette_only = false) {
+static void rect_df(gf_ctx* ctx, const float4* U, gf_field* D, double cp, double cr) {
   const size_t smem = (size_t)GF_RECT_SLOTS * 36 * 128 * sizeof(float);
-  auto kern = plaquette_only ? k_force_rect_df<false, 4> : (D ? k_force_rect_df<true, 28> : k_force_rect_df<false, 28>);
-  GF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid = stencil_grid(ctx->geom.vol, 128);
+  GF_CUDA(cudaFuncSetAttribute(k_force_rect_df, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   ProfScope prof(ctx, GF_K_RECT_DF);
-  kern<<<grid, 128, smem, ctx->stream>>>(U, P ? (double*)P->ptr : nullptr, D ? (float4*)D->ptr : nullptr, ctx->geom,
-                                         dfl(cp), dfl(cr), keep);
+  k_force_rect_df<<<stencil_grid(ctx->geom.vol, 128), 128, smem, ctx->stream>>>(U, (float4*)D->ptr, ctx->geom, dfl(cp),
+                                                                                dfl(cr));
   GF_CHECK_LAUNCH();
-}
-
-template <class SRC>
-static double rect_sum_of(gf_ctx* ctx, SRC src) {
-  const int nb = blocks_for(ctx->geom.vol, 128);
-  ProfScope prof(ctx, GF_K_RECT);
-  k_rect_sum<<<nb, 128, 0, ctx->stream>>>(src, ctx->geom, ctx->d_partials);
-  GF_CHECK_LAUNCH();
-  return finish_reduction(ctx, nb);
 }
 
 double rectangle_sum(gf_ctx* ctx, const gf_field* U) {
-  if (U->kind == GF_LINK64 || U->kind == GF_MAT64) return rectangle_sum_fx(ctx, fx_links(ctx, U));
   if (U->kind == GF_LINKFX) return rectangle_sum_fx(ctx, U);
-  // top level of a double-float stack: fp64 arithmetic on hi + lo
-  if (U->kind == GF_LINKDF) return rect_sum_of(ctx, LinkSrcDfn64{(const float4*)U->ptr});
+  // fp64 links, and the top level of a double-float stack
+  if (U->kind == GF_LINK64 || U->kind == GF_MAT64 || U->kind == GF_LINKDF)
+    return rectangle_sum_fx(ctx, fx_links(ctx, U));
   throw gf_error(GF_EINVAL, "rectangle: links must be LINK64");
 }
 
 void loops_force_coef(gf_ctx* ctx, const gf_field* U, gf_field* P, double cp, double cr, double keep, bool df) {
   if (P->kind != GF_MOM64) throw gf_error(GF_EINVAL, "force: output must be MOM64");
   dim3 grid = stencil_grid(ctx->geom.vol, 128);
-  if (df) {
-    if (U->kind != GF_LINK64) throw gf_error(GF_EINVAL, "force: the double-float rectangle force takes LINK64 links");
-    // a double-float-native copy of the links, converted once per force
-    if (!ctx->w_linkdf) ctx->w_linkdf = field_new(ctx, GF_LINKDF);
-    copy_field(ctx, ctx->w_linkdf, U);
-    rect_df(ctx, (const float4*)ctx->w_linkdf->ptr, P, nullptr, cp, cr, keep);
-    return;
-  }
+  if (df && U->kind != GF_LINK64)
+    throw gf_error(GF_EINVAL, "force: the double-float rectangle force takes LINK64 links");
   if (U->kind == GF_LINK64 || U->kind == GF_MAT64) {
     if (cr == 0.0) wilson_force_coef(ctx, U, P, cp, keep);
     else loops_fx(ctx, fx_links(ctx, U), P, nullptr, cp, cr, keep);
@@ -325,18 +254,10 @@ void loops_force_coef(gf_ctx* ctx, const gf_field* U, gf_field* P, double cp, do
   GF_CHECK_LAUNCH();
 }
 
-void plaquette_force_df(gf_ctx* ctx, const gf_field* U, gf_field* P, double coef, double keep) {
-  if (P->kind != GF_MOM64) throw gf_error(GF_EINVAL, "force: output must be MOM64");
-  if (U->kind != GF_LINK64) throw gf_error(GF_EINVAL, "force: the double-float force takes LINK64 links");
-  if (!ctx->w_linkdf) ctx->w_linkdf = field_new(ctx, GF_LINKDF);
-  copy_field(ctx, ctx->w_linkdf, U);
-  rect_df(ctx, (const float4*)ctx->w_linkdf->ptr, P, nullptr, coef, 0.0, keep, true);
-}
-
 void loops_dsdu(gf_ctx* ctx, const gf_field* Ubar, gf_field* D, double cp, double cr) {
   dim3 grid = stencil_grid(ctx->geom.vol, 128);
   if (Ubar->kind == GF_LINKDF && D->kind == GF_MATDF) {
-    rect_df(ctx, (const float4*)Ubar->ptr, nullptr, D, cp, cr, 0.0);
+    rect_df(ctx, (const float4*)Ubar->ptr, D, cp, cr);
     return;
   }
   if (Ubar->kind == GF_LINKFX && D->kind == GF_MATFX) {
