@@ -112,11 +112,16 @@ extern "C" int gf_ctx_create(const int L[4], int device, gf_ctx** out) {
   ctx->own_stream = 1;
   // at least one partial per resident block of the grid-stride sums
   ctx->partial_cap = std::max(blocks_for((int)V, 128) + 1, ctx->sm_count * 64);
-  GF_CUDA(cudaMalloc(&ctx->d_partials, sizeof(double) * ctx->partial_cap));
-  GF_CUDA(cudaMalloc(&ctx->d_result, sizeof(double) * 4));
-  GF_CUDA(cudaMallocHost(&ctx->h_result, sizeof(double) * 4));
-  GF_CUDA(cudaMalloc(&ctx->d_hash, sizeof(unsigned long long)));
-  GF_CUDA(cudaMallocHost(&ctx->h_hash, sizeof(unsigned long long)));
+  // one device block: partial sums, hash, block count
+  GF_CUDA(cudaMalloc(&ctx->d_partials, sizeof(double) * ((size_t)ctx->partial_cap + 2)));
+  ctx->d_hash = (unsigned long long*)(ctx->d_partials + ctx->partial_cap);
+  ctx->d_count = (unsigned*)(ctx->d_partials + ctx->partial_cap + 1);
+  GF_CUDA(cudaMemsetAsync(ctx->d_count, 0, sizeof(unsigned), ctx->stream));
+  GF_CUDA(cudaMallocHost(&ctx->h_result, sizeof(double) * 5));
+  ctx->h_hash = (unsigned long long*)(ctx->h_result + 4);
+  // the fixed-point copy of the links that most calls make: small ones at
+  // once, so that the first call on a small lattice does not wait for them
+  if (field_bytes(ctx->geom, GF_LINKFX) <= ((size_t)32 << 20)) ctx->w_linkfx = field_new(ctx, GF_LINKFX);
   *out = ctx;
   return GF_OK;
   }
@@ -148,13 +153,10 @@ extern "C" int gf_ctx_destroy(gf_ctx* ctx) {
   if (ctx->w_stoutdf) gf_stout_destroy(ctx->w_stoutdf);
   pool_trim(ctx->pool.get(), true);
   if (ctx->d_partials) cudaFree(ctx->d_partials);
-  if (ctx->d_result) cudaFree(ctx->d_result);
   if (ctx->h_result) cudaFreeHost(ctx->h_result);
-  if (ctx->d_hash) cudaFree(ctx->d_hash);
   if (ctx->d_stage) cudaFree(ctx->d_stage);
   for (int i = 0; i < 2; ++i)
     if (ctx->arena[i]) cudaFree(ctx->arena[i]);
-  if (ctx->h_hash) cudaFreeHost(ctx->h_hash);
   if (ctx->prof_ev) {
     for (int i = 0; i < 2 * GF_PROF_CAP; ++i) cudaEventDestroy(ctx->prof_ev[i]);
     delete[] ctx->prof_ev;
@@ -578,7 +580,9 @@ static gf_stout* ctx_stout(gf_ctx* ctx, const gf_md_params* p, int precision) {
 #ifndef GF_DF_HAMILTONIAN
 #define GF_DF_HAMILTONIAN 1
 #endif
-static double potential(gf_ctx* ctx, const gf_field* U, const gf_md_params* p) {
+// The sums go to slots 0 (plaquettes) and 1 (rectangles) of the context's
+// results; potential_value reads them after the stream has been waited for.
+static void potential_start(gf_ctx* ctx, const gf_field* U, const gf_md_params* p) {
   bool df = (GF_DF_HAMILTONIAN && p->precision == GF_MIXED) || p->precision == GF_DFLOAT;
   const gf_field* links = U;
   if (p->nstout > 0) {
@@ -586,20 +590,34 @@ static double potential(gf_ctx* ctx, const gf_field* U, const gf_md_params* p) {
     stout_forward(ctx, st, U, nullptr);
     links = stout_top(st);
   }
-  double v = -(p->beta / 3.0) * plaquette_sum(ctx, links);
-  if (p->c_rect != 0.0) v -= (2.0 / 3.0) * p->c_rect * rectangle_sum(ctx, links);
+  plaquette_start(ctx, links, 0);
+  if (p->c_rect != 0.0) rectangle_start(ctx, links, 1);
+}
+static double potential_value(const gf_ctx* ctx, const gf_md_params* p) {
+  double v = -(p->beta / 3.0) * ctx->h_result[0];
+  if (p->c_rect != 0.0) v -= (2.0 / 3.0) * p->c_rect * ctx->h_result[1];
   return v;
 }
 
 static double hamiltonian(gf_ctx* ctx, const gf_field* U, const gf_field* P, const gf_md_params* p) {
-  double v = potential(ctx, U, p);
-  return v + 0.5 * kinetic(ctx, P);
+  potential_start(ctx, U, p);
+  kinetic_start(ctx, P, 2);
+  const double k = sum_wait(ctx, 2);
+  return potential_value(ctx, p) + 0.5 * k;
 }
 
-// P += eps * F(U) with the force of the (smeared) Wilson action
-static void mom_update(gf_ctx* ctx, gf_field* P, const gf_field* U, const gf_field* U32, double eps,
+// Whether the drivers keep a fixed-point copy of the links beside them: the
+// link update writes it, and the force and the potential of thin links, and
+// the plain form's stack, read it instead of converting the links each time.
+static bool keeps_fx(const gf_md_params* p) {
+  return p->precision == GF_FP64 || (p->precision == GF_DFLOAT && p->nstout == 0);
+}
+
+// P += eps * F(U) with the force of the (smeared) Wilson action; Ucopy: the
+// fp32 links of the mixed form, or the fixed-point copy (keeps_fx) or null
+static void mom_update(gf_ctx* ctx, gf_field* P, const gf_field* U, const gf_field* Ucopy, double eps,
                        const gf_md_params* p) {
-  const gf_field* links = (p->precision == GF_MIXED) ? U32 : U;
+  const gf_field* links = Ucopy ? Ucopy : U;
   if (p->nstout == 0 && p->c_rect != 0.0) {
     loops_force_coef(ctx, links, P, eps * (-1.0 / 3.0) * (0.5 * p->beta), eps * (-1.0 / 3.0) * p->c_rect, 1.0,
                      p->precision == GF_DFLOAT);
@@ -672,50 +690,64 @@ struct MDResult {
 static MDResult md_run(gf_ctx* ctx, gf_field* U, gf_field* P, const gf_md_params* p) {
   need_kind(U, GF_LINK64, "md: U");
   need_kind(P, GF_MOM64, "md: P");
-  gf_field* U32 = nullptr;
+  gf_field *U32 = nullptr, *Ufx = nullptr;
   if (p->precision == GF_MIXED) {
     if (!ctx->w_link32) ctx->w_link32 = field_new(ctx, GF_LINK32);
     U32 = ctx->w_link32;
     link64_to_32(ctx, U32, U);
   }
+  if (keeps_fx(p)) Ufx = fx_links(ctx, U);
+  const gf_field* Ucopy = U32 ? U32 : Ufx;
+  const gf_field* Upot = Ufx ? Ufx : U;  // the potential never takes the fp32 links
   MDResult r;
-  r.h0 = field_hash(ctx, U);
-  if (!vcache_lookup(ctx, p, r.h0, &r.V0)) r.V0 = potential(ctx, U, p);
-  r.H0 = r.V0 + 0.5 * kinetic(ctx, P);
+  field_hash_start(ctx, U);
+  kinetic_start(ctx, P, 2);
+  const double k0 = sum_wait(ctx, 2);
+  r.h0 = *ctx->h_hash;
+  if (!vcache_lookup(ctx, p, r.h0, &r.V0)) {
+    potential_start(ctx, Upot, p);
+    sum_wait(ctx, 0);
+    r.V0 = potential_value(ctx, p);
+  }
+  r.H0 = r.V0 + 0.5 * k0;
   double eps = p->tau / p->steps;
   // Adjacent half steps of consecutive QPQ (PQP) steps act with the same P
   // (the same U), so they are applied as one full step, as the reference's
   // _md_fast_qpq! does (molecular_dynamics.jl:618-633): n+1 link updates and
   // n forces (QPQ), or n+1 forces and n link updates (PQP). The trajectory
   // is the one of md_step! up to rounding.
-  const bool df = p->precision != GF_FP64;  // link updates in double-float
+  const bool df = p->precision != GF_FP64;  // profiling class of the link updates
   if (p->integrator == GF_QPQ) {
-    link_update(ctx, U, P, 0.5 * eps, p->reunitarize, U32, df);
+    link_update(ctx, U, P, 0.5 * eps, p->reunitarize, U32, df, Ufx);
     for (int n = 0; n < p->steps; ++n) {
-      mom_update(ctx, P, U, U32, eps, p);
-      link_update(ctx, U, P, (n == p->steps - 1) ? 0.5 * eps : eps, p->reunitarize, U32, df);
+      mom_update(ctx, P, U, Ucopy, eps, p);
+      link_update(ctx, U, P, (n == p->steps - 1) ? 0.5 * eps : eps, p->reunitarize, U32, df, Ufx);
     }
   } else if (p->integrator == GF_PQP) {
-    mom_update(ctx, P, U, U32, 0.5 * eps, p);
+    mom_update(ctx, P, U, Ucopy, 0.5 * eps, p);
     for (int n = 0; n < p->steps; ++n) {
-      link_update(ctx, U, P, eps, p->reunitarize, U32, df);
-      mom_update(ctx, P, U, U32, (n == p->steps - 1) ? 0.5 * eps : eps, p);
+      link_update(ctx, U, P, eps, p->reunitarize, U32, df, Ufx);
+      mom_update(ctx, P, U, Ucopy, (n == p->steps - 1) ? 0.5 * eps : eps, p);
     }
   } else {
     // Omelyan PQPQP: P(l eps) Q(eps/2) P((1-2l) eps) Q(eps/2) P(l eps); the
     // closing and opening kicks of consecutive steps merge into P(2 l eps).
     const double lam = p->lambda;
-    mom_update(ctx, P, U, U32, lam * eps, p);
+    mom_update(ctx, P, U, Ucopy, lam * eps, p);
     for (int n = 0; n < p->steps; ++n) {
-      link_update(ctx, U, P, 0.5 * eps, p->reunitarize, U32, df);
-      mom_update(ctx, P, U, U32, (1.0 - 2.0 * lam) * eps, p);
-      link_update(ctx, U, P, 0.5 * eps, p->reunitarize, U32, df);
-      mom_update(ctx, P, U, U32, (n == p->steps - 1 ? 1.0 : 2.0) * lam * eps, p);
+      link_update(ctx, U, P, 0.5 * eps, p->reunitarize, U32, df, Ufx);
+      mom_update(ctx, P, U, Ucopy, (1.0 - 2.0 * lam) * eps, p);
+      link_update(ctx, U, P, 0.5 * eps, p->reunitarize, U32, df, Ufx);
+      mom_update(ctx, P, U, Ucopy, (n == p->steps - 1 ? 1.0 : 2.0) * lam * eps, p);
     }
   }
-  r.V1 = potential(ctx, U, p);
-  r.H1 = r.V1 + 0.5 * kinetic(ctx, P);
-  r.h1 = field_hash(ctx, U);
+  potential_start(ctx, Upot, p);
+  kinetic_start(ctx, P, 2);
+  field_hash_start(ctx, U);
+  const double k1 = sum_wait(ctx, 2);
+  r.V1 = potential_value(ctx, p);
+  r.H1 = r.V1 + 0.5 * k1;
+  r.h1 = *ctx->h_hash;
   return r;
 }
 
@@ -882,13 +914,15 @@ static void flow_steps(gf_ctx* ctx, gf_field* U, double eps, int nsteps, bool df
   gf_field* W2 = ctx->w_link64b;
   gf_field* G = ctx->w_mom[0];
   const double c0 = 17.0 * eps / 36.0;
+  if (nsteps == 0) return;
+  gf_field* F = fx_links(ctx, U);  // the fixed-point copy of U, W1, W2 in turn, written by their updates
   for (int n = 0; n < nsteps; ++n) {
-    flow_force(ctx, U, G, c0, 0.0, df);                 // G = 17eps/36 F0
-    exp_mom_links(ctx, W1, G, -9.0 / 17.0, U, df);      // W1 = exp(-eps/4 F0) U
-    flow_force(ctx, W1, G, -8.0 * eps / 9.0, 1.0, df);  // G = 17eps/36 F0 - 8eps/9 F1
-    exp_mom_links(ctx, W2, G, 1.0, W1, df);             // W2 = exp(G) W1
-    flow_force(ctx, W2, G, -0.75 * eps, -1.0, df);      // G = -G - 3eps/4 F2
-    exp_mom_links(ctx, U, G, 1.0, W2, df);              // U = exp(G) W2
+    flow_force(ctx, F, G, c0, 0.0, df);                // G = 17eps/36 F0
+    exp_mom_links(ctx, W1, G, -9.0 / 17.0, U, df, F);  // W1 = exp(-eps/4 F0) U
+    flow_force(ctx, F, G, -8.0 * eps / 9.0, 1.0, df);  // G = 17eps/36 F0 - 8eps/9 F1
+    exp_mom_links(ctx, W2, G, 1.0, W1, df, F);         // W2 = exp(G) W1
+    flow_force(ctx, F, G, -0.75 * eps, -1.0, df);      // G = -G - 3eps/4 F2
+    exp_mom_links(ctx, U, G, 1.0, W2, df, F);          // U = exp(G) W2
   }
 }
 
@@ -927,13 +961,14 @@ extern "C" int gf_flow_loops(gf_ctx* ctx, gf_field* U, double eps, int nsteps, d
   const double c0 = 17.0 * eps / 36.0;
   const double c1 = -8.0 * eps / 9.0;
   const double c2 = -0.75 * eps;
+  gf_field* F = nsteps ? fx_links(ctx, U) : nullptr;  // of U, W1, W2 in turn
   for (int n = 0; n < nsteps; ++n) {
-    loops_force_coef(ctx, U, G, c0 * c_plaq, c0 * c_rect, 0.0);    // G = 17eps/36 F0
-    exp_mom_links(ctx, W1, G, -9.0 / 17.0, U);                    // W1 = exp(-eps/4 F0) U
-    loops_force_coef(ctx, W1, G, c1 * c_plaq, c1 * c_rect, 1.0);   // G += -8eps/9 F1
-    exp_mom_links(ctx, W2, G, 1.0, W1);                           // W2 = exp(G) W1
-    loops_force_coef(ctx, W2, G, c2 * c_plaq, c2 * c_rect, -1.0);  // G = -G - 3eps/4 F2
-    exp_mom_links(ctx, U, G, 1.0, W2);                            // U = exp(G) W2
+    loops_force_coef(ctx, F, G, c0 * c_plaq, c0 * c_rect, 0.0);   // G = 17eps/36 F0
+    exp_mom_links(ctx, W1, G, -9.0 / 17.0, U, false, F);         // W1 = exp(-eps/4 F0) U
+    loops_force_coef(ctx, F, G, c1 * c_plaq, c1 * c_rect, 1.0);   // G += -8eps/9 F1
+    exp_mom_links(ctx, W2, G, 1.0, W1, false, F);                // W2 = exp(G) W1
+    loops_force_coef(ctx, F, G, c2 * c_plaq, c2 * c_rect, -1.0);  // G = -G - 3eps/4 F2
+    exp_mom_links(ctx, U, G, 1.0, W2, false, F);                 // U = exp(G) W2
   }
   API_END(ctx)
 }

@@ -2,6 +2,7 @@
 // hot starts, Gaussian momenta, field copies/conversions and the deterministic
 // two-stage reductions used by every global sum.
 #include "gf_internal.h"
+#include "stencil.cuh"
 #include <vector>
 
 namespace gf {
@@ -122,27 +123,25 @@ __global__ void k_reduce_final(const double* __restrict__ part, int n, double* _
 }
 
 double finish_reduction(gf_ctx* ctx, int nblocks) {
-  k_reduce_final<<<1, 1024, 0, ctx->stream>>>(ctx->d_partials, nblocks, ctx->d_result);
+  k_reduce_final<<<1, 1024, 0, ctx->stream>>>(ctx->d_partials, nblocks, ctx->h_result);
   GF_CHECK_LAUNCH();
-  GF_CUDA(cudaMemcpyAsync(ctx->h_result, ctx->d_result, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  return sum_wait(ctx, 0);
+}
+// 8^4 plaquette: 29.8 us with a second kernel and a copy, 25.6 us without
+SumOut sum_out(gf_ctx* ctx, int nblocks, int threads, int slot) {
+  return SumOut{ctx->d_partials, nblocks <= 8 * threads ? ctx->d_count : nullptr, ctx->h_result + slot};
+}
+void sum_finish(gf_ctx* ctx, const SumOut& to, int nblocks, int slot) {
+  if (to.count) return;
+  k_reduce_final<<<1, 1024, 0, ctx->stream>>>(ctx->d_partials, nblocks, ctx->h_result + slot);
+  GF_CHECK_LAUNCH();
+}
+double sum_wait(gf_ctx* ctx, int slot) {
   GF_CUDA(cudaStreamSynchronize(ctx->stream));
-  return *ctx->h_result;
+  return ctx->h_result[slot];
 }
 
-__device__ __forceinline__ void block_partial(double v, double* __restrict__ part) {
-  __shared__ double sh[32];
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) sh[w] = v;
-  __syncthreads();
-  if (w == 0) {
-    v = (lane < (int)(blockDim.x >> 5)) ? sh[lane] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) part[blockIdx.x] = v;
-  }
-}
-
-__global__ void k_kinetic(const double* __restrict__ P, int V, double* __restrict__ part) {
+__global__ void k_kinetic(const double* __restrict__ P, int V, SumOut to) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   double v = 0.0;
   if (s < V) {
@@ -154,15 +153,20 @@ __global__ void k_kinetic(const double* __restrict__ P, int V, double* __restric
         v += p * p;
       }
   }
-  block_partial(v, part);
+  block_sum(v, to);
 }
 
-double kinetic(gf_ctx* ctx, const gf_field* P) {
+void kinetic_start(gf_ctx* ctx, const gf_field* P, int slot) {
   int V = ctx->geom.vol;
   int nb = blocks_for(V, 256);
-  k_kinetic<<<nb, 256, 0, ctx->stream>>>((const double*)P->ptr, V, ctx->d_partials);
+  const SumOut to = sum_out(ctx, nb, 256, slot);
+  k_kinetic<<<nb, 256, 0, ctx->stream>>>((const double*)P->ptr, V, to);
   GF_CHECK_LAUNCH();
-  return finish_reduction(ctx, nb);
+  sum_finish(ctx, to, nb, slot);
+}
+double kinetic(gf_ctx* ctx, const gf_field* P) {
+  kinetic_start(ctx, P, 0);
+  return sum_wait(ctx, 0);
 }
 
 __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
@@ -181,14 +185,12 @@ __global__ void k_hash(const unsigned long long* __restrict__ w, size_t n, unsig
   if ((threadIdx.x & 31) == 0) atomicAdd(out, h);
 }
 
-unsigned long long field_hash(gf_ctx* ctx, const gf_field* f) {
+void field_hash_start(gf_ctx* ctx, const gf_field* f) {
   GF_CUDA(cudaMemsetAsync(ctx->d_hash, 0, sizeof(unsigned long long), ctx->stream));
   // a grid-stride loop over the field: eight blocks of 256 threads per SM
   k_hash<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>((const unsigned long long*)f->ptr, f->bytes / 8, ctx->d_hash);
   GF_CHECK_LAUNCH();
   GF_CUDA(cudaMemcpyAsync(ctx->h_hash, ctx->d_hash, sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream));
-  GF_CUDA(cudaStreamSynchronize(ctx->stream));
-  return *ctx->h_hash;
 }
 
 // ---------------------------------------------------------------------------

@@ -59,10 +59,10 @@ void fx_to_f64_field(gf_ctx* ctx, gf_field* dst, const gf_field* src) {
 // block. A work item is one plane of 32 sites; a thread forms row r of
 // U_mu(x) U_nu(x+mu) U_mu(x+nu)^dag and its product with row r of U_nu(x).
 // Integer-issue-bound: 2M sites (32^3 x 64) 7.16 ms in fp64, 1.68 ms here with
-// the conversion (0.4 ms, bandwidth-bound); 8^4 89 -> 31 us, a launch and a
-// wait each for the conversion, the sum and its second stage.
+// the conversion (0.4 ms, bandwidth-bound); 8^4 89 -> 25.6 us, the launches of
+// the conversion and the sum and one wait.
 __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_MINB)
-    k_plaquette_fx(FxField U, Geom g, int items, double* __restrict__ part) {
+    k_plaquette_fx(FxField U, Geom g, int items, SumOut to) {
   const int t = threadIdx.x, V = g.vol;
   const int link = t / 3, r = t - 3 * link;
   double v = 0.0;
@@ -87,16 +87,17 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_MINB)
     }
     v = fma(fx_value(fx_get(d)), fx_unit(1.0, e), v);
   }
-  block_partial_sum(v, part);
+  block_sum(v, to);
 }
 
-double plaquette_sum_fx(gf_ctx* ctx, const gf_field* F) {
+void plaquette_start_fx(gf_ctx* ctx, const gf_field* F, int slot) {
   const int items = 6 * blocks_for(ctx->geom.vol, GF_FX_LINKS);
   // a few waves of resident blocks, so that the second stage stays short
   const int nb = std::min(std::min(items, ctx->sm_count * GF_FX_MINB * 8), ctx->partial_cap);
-  k_plaquette_fx<<<nb, GF_FX_THREADS, 0, ctx->stream>>>(fx_view(F), ctx->geom, items, ctx->d_partials);
+  const SumOut to = sum_out(ctx, nb, GF_FX_THREADS, slot);
+  k_plaquette_fx<<<nb, GF_FX_THREADS, 0, ctx->stream>>>(fx_view(F), ctx->geom, items, to);
   GF_CHECK_LAUNCH();
-  return finish_reduction(ctx, nb);
+  sum_finish(ctx, to, nb, slot);
 }
 
 // P_mu(x) <- keep * P_mu(x) + coef * c(U_mu(x) S_mu(x)) as k_force_ta. The
@@ -129,14 +130,13 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_MINB)
   fx_update_mom(sh, se, P, mu, s0, V, -coef, keep);
 }
 
-const gf_field* fx_links(gf_ctx* ctx, const gf_field* U) {
+gf_field* fx_links(gf_ctx* ctx, const gf_field* U) {
   if (!ctx->w_linkfx) ctx->w_linkfx = field_new(ctx, GF_LINKFX);
   to_fx(ctx, ctx->w_linkfx, U);
   return ctx->w_linkfx;
 }
 
-void wilson_force_fx(gf_ctx* ctx, const gf_field* U, gf_field* P, double coef, double keep) {
-  const gf_field* F = fx_links(ctx, U);
+void wilson_force_fx(gf_ctx* ctx, const gf_field* F, gf_field* P, double coef, double keep) {
   const int nb = 4 * blocks_for(ctx->geom.vol, GF_FX_LINKS);
   k_force_fx<<<nb, GF_FX_THREADS, 0, ctx->stream>>>(fx_view(F), (double*)P->ptr, ctx->geom, coef, keep);
   GF_CHECK_LAUNCH();

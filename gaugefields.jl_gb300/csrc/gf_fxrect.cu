@@ -38,7 +38,7 @@ __device__ __forceinline__ int fx_steps(const Geom& g, const Site& st, int mu, i
 // Sum over sites and planes of Re tr of the 1x2 and 2x1 rectangles, one
 // partial per block; a work item is one plane of 32 sites.
 __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_MINB)
-    k_rect_sum_fx(FxField U, Geom g, int items, double* __restrict__ part) {
+    k_rect_sum_fx(FxField U, Geom g, int items, SumOut to) {
   const int t = threadIdx.x, V = g.vol;
   const int link = t / 3, r = t - 3 * link;
   double v = 0.0;
@@ -71,16 +71,17 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_MINB)
     }
     v = fma(fx_value(fx_get(d)), fx_unit(1.0, c.e), v);
   }
-  block_partial_sum(v, part);
+  block_sum(v, to);
 }
 
-double rectangle_sum_fx(gf_ctx* ctx, const gf_field* F) {
+void rectangle_start_fx(gf_ctx* ctx, const gf_field* F, int slot) {
   const int items = 12 * blocks_for(ctx->geom.vol, GF_FX_LINKS);
   const int nb = std::min(std::min(items, ctx->sm_count * GF_FX_MINB * 8), ctx->partial_cap);
+  const SumOut to = sum_out(ctx, nb, GF_FX_THREADS, slot);
   ProfScope prof(ctx, GF_K_RECT);
-  k_rect_sum_fx<<<nb, GF_FX_THREADS, 0, ctx->stream>>>(fx_view(F), ctx->geom, items, ctx->d_partials);
+  k_rect_sum_fx<<<nb, GF_FX_THREADS, 0, ctx->stream>>>(fx_view(F), ctx->geom, items, to);
   GF_CHECK_LAUNCH();
-  return finish_reduction(ctx, nb);
+  sum_finish(ctx, to, nb, slot);
 }
 
 // acc (+)= [cp t_p + cr (t_1 + t_2)] / 4 as an operand row; cp and cr share

@@ -84,8 +84,8 @@ struct gf_ctx {
   // deterministic reductions: per-block partial sums and a pinned result slot
   double* d_partials;
   int partial_cap;
-  double* d_result;
-  double* h_result;
+  unsigned* d_count;  // blocks that have finished (block_sum)
+  double* h_result;   // four slots, written by the device
   // work fields of the MD / flow drivers, allocated on first use
   gf_field* w_link64;     // backup / W1 of the flow
   gf_field* w_link64b;    // W2 of the flow
@@ -143,6 +143,8 @@ struct gf_stout {
 
 namespace gf {
 
+struct SumOut;
+
 size_t field_bytes(const Geom& g, int kind);
 gf_field* field_new(gf_ctx* ctx, int kind);
 // the same from the context's pool, for buffers that stay inside the library
@@ -170,12 +172,22 @@ struct ProfScope {
 void set_global_error(const std::string& m);
 
 // ---- reductions (gf_fields.cu) ----
-// Deterministic two-stage sum of per-site doubles produced by a kernel that
-// writes one partial per block; returns the total on the host.
+// Deterministic sums of per-site doubles. A kernel writes one partial per
+// block; finish_reduction adds them in a second kernel, waits and returns the
+// total. Kernels that end in block_sum (stencil.cuh) take sum_out: up to eight
+// partials per thread of a block their last block adds up itself, else
+// sum_finish launches the second kernel. Either way the total arrives in slot
+// `slot` (0 .. 3) of h_result once the stream is waited for: no copy, and
+// several sums can share one wait.
 double finish_reduction(gf_ctx* ctx, int nblocks);
+SumOut sum_out(gf_ctx* ctx, int nblocks, int threads, int slot);
+void sum_finish(gf_ctx* ctx, const SumOut& to, int nblocks, int slot);
+double sum_wait(gf_ctx* ctx, int slot);  // waits for the stream
 double kinetic(gf_ctx* ctx, const gf_field* P);
+void kinetic_start(gf_ctx* ctx, const gf_field* P, int slot);
 // order-independent 64-bit hash of a field's bytes (sum of mixed words)
-unsigned long long field_hash(gf_ctx* ctx, const gf_field* f);
+// (in *h_hash once the stream is waited for)
+void field_hash_start(gf_ctx* ctx, const gf_field* f);
 
 // ---- field plumbing (gf_fields.cu) ----
 void upload_links(gf_ctx* ctx, gf_field* U, const double* host);
@@ -200,19 +212,22 @@ void staple_up(gf_ctx* ctx, const gf_field* U, int mu, gf_field* V);  // constru
 // staples (dS/dU order); keep = 0 overwrites P without reading it.
 void wilson_force_coef(gf_ctx* ctx, const gf_field* U, gf_field* P, double coef, double keep, bool df = false);
 
-// the same on fp64 links in fixed-point arithmetic (gf_fixed.cu)
-void wilson_force_fx(gf_ctx* ctx, const gf_field* U, gf_field* P, double coef, double keep);
+// the same on a fixed-point copy of the links (gf_fixed.cu)
+void wilson_force_fx(gf_ctx* ctx, const gf_field* F, gf_field* P, double coef, double keep);
 
-double plaquette_sum_fx(gf_ctx* ctx, const gf_field* F);  // of a fixed-point field
+void plaquette_start_fx(gf_ctx* ctx, const gf_field* F, int slot);  // of a fixed-point field
+// the sum into slot `slot` of h_result: LINK64, fixed-point or double-float links
+void plaquette_start(gf_ctx* ctx, const gf_field* U, int slot);
 inline FxField fx_view(const gf_field* f) { return FxField{(const char*)f->ptr}; }
 // the context's fixed-point copy of fp64 or double-float links
-const gf_field* fx_links(gf_ctx* ctx, const gf_field* U);
+gf_field* fx_links(gf_ctx* ctx, const gf_field* U);
 // LINK64 / MAT64 or double-float pairs -> fixed point, and fixed point -> fp64
 void to_fx(gf_ctx* ctx, gf_field* dst, const gf_field* src);
 void fx_to_f64_field(gf_ctx* ctx, gf_field* dst, const gf_field* src);
 
 // ---- rectangle loops (gf_rect.cu) ----
 double rectangle_sum(gf_ctx* ctx, const gf_field* U);  // sum_x sum_{mu<nu} Re tr (R1x2 + R2x1)
+void rectangle_start(gf_ctx* ctx, const gf_field* U, int slot);
 // P <- keep * P + TA-coefficients(U_mu (cp S_mu + cr R_mu)), S the six
 // plaquette staples and R the eighteen rectangle staples of U_mu.
 void loops_force_coef(gf_ctx* ctx, const gf_field* U, gf_field* P, double cp, double cr, double keep,
@@ -222,16 +237,18 @@ void loops_force_coef(gf_ctx* ctx, const gf_field* U, gf_field* P, double cp, do
 void loops_dsdu(gf_ctx* ctx, const gf_field* Ubar, gf_field* D, double cp, double cr);
 // the same on a fixed-point field (gf_fxrect.cu): the loop sum; the force into
 // P, or D = cp S + cr R into a fixed-point D
-double rectangle_sum_fx(gf_ctx* ctx, const gf_field* F);
+void rectangle_start_fx(gf_ctx* ctx, const gf_field* F, int slot);
 void loops_fx(gf_ctx* ctx, const gf_field* F, gf_field* P, gf_field* D, double cp, double cr, double keep);
 
 // ---- link update (gf_update.cu) ----
 // U <- exp(i eps P) U, optional re-unitarisation, optional fp32 shadow copy.
 // df: double-float arithmetic on the fp32 pipes (the mixed form), else fp64.
+// fx: also write the fixed-point copy of the updated links (a LINKFX field).
 void link_update(gf_ctx* ctx, gf_field* U, const gf_field* P, double eps, int reunit, gf_field* shadow32,
-                 bool df = false);
+                 bool df = false, gf_field* fx = nullptr);
 // W = exp(i a P) U (fp64, or double-float arithmetic on the fp64 fields)
-void exp_mom_links(gf_ctx* ctx, gf_field* W, const gf_field* P, double a, const gf_field* U, bool df = false);
+void exp_mom_links(gf_ctx* ctx, gf_field* W, const gf_field* P, double a, const gf_field* U, bool df = false,
+                   gf_field* fx = nullptr);
 void reunitarize_links(gf_ctx* ctx, gf_field* U);
 void link64_to_32(gf_ctx* ctx, gf_field* dst, const gf_field* src);
 

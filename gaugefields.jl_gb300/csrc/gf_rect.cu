@@ -227,22 +227,26 @@ static void rect_df(gf_ctx* ctx, const float4* U, gf_field* D, double cp, double
   GF_CHECK_LAUNCH();
 }
 
+void rectangle_start(gf_ctx* ctx, const gf_field* U, int slot) {
+  // fp64 links, and the top level of a double-float stack, through a fixed-point copy
+  if (U->kind != GF_LINKFX && U->kind != GF_LINK64 && U->kind != GF_MAT64 && U->kind != GF_LINKDF)
+    throw gf_error(GF_EINVAL, "rectangle: links must be LINK64");
+  rectangle_start_fx(ctx, U->kind == GF_LINKFX ? U : fx_links(ctx, U), slot);
+}
+
 double rectangle_sum(gf_ctx* ctx, const gf_field* U) {
-  if (U->kind == GF_LINKFX) return rectangle_sum_fx(ctx, U);
-  // fp64 links, and the top level of a double-float stack
-  if (U->kind == GF_LINK64 || U->kind == GF_MAT64 || U->kind == GF_LINKDF)
-    return rectangle_sum_fx(ctx, fx_links(ctx, U));
-  throw gf_error(GF_EINVAL, "rectangle: links must be LINK64");
+  rectangle_start(ctx, U, 0);
+  return sum_wait(ctx, 0);
 }
 
 void loops_force_coef(gf_ctx* ctx, const gf_field* U, gf_field* P, double cp, double cr, double keep, bool df) {
   if (P->kind != GF_MOM64) throw gf_error(GF_EINVAL, "force: output must be MOM64");
   dim3 grid = stencil_grid(ctx->geom.vol, 128);
-  if (df && U->kind != GF_LINK64)
+  if (df && U->kind != GF_LINK64 && U->kind != GF_LINKFX)
     throw gf_error(GF_EINVAL, "force: the double-float rectangle force takes LINK64 links");
-  if (U->kind == GF_LINK64 || U->kind == GF_MAT64) {
+  if (U->kind == GF_LINK64 || U->kind == GF_MAT64 || U->kind == GF_LINKFX) {
     if (cr == 0.0) wilson_force_coef(ctx, U, P, cp, keep);
-    else loops_fx(ctx, fx_links(ctx, U), P, nullptr, cp, cr, keep);
+    else loops_fx(ctx, U->kind == GF_LINKFX ? U : fx_links(ctx, U), P, nullptr, cp, cr, keep);
     return;
   } else if (U->kind == GF_LINK32) {
     ProfScope prof(ctx, GF_K_RECT);

@@ -179,7 +179,7 @@ __device__ __forceinline__ int fx_from_f64_fast(const double* m, int4 out[9]) {
 template <bool REUNIT>
 __global__ void __launch_bounds__(128, GF_FX_UPDATE_MINB)
     k_link_update_fx(const double2* Uin, double2* Uout, const double* __restrict__ P, Geom g, fx_scalar eps,
-                     float4* __restrict__ sh32) {
+                     float4* __restrict__ sh32, char* __restrict__ fx) {
   const int V = g.vol, mu = blockIdx.y, s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= V) return;
   constexpr int rows = REUNIT ? 2 : 3;  // re-unitarisation rebuilds row 3
@@ -247,29 +247,55 @@ __global__ void __launch_bounds__(128, GF_FX_UPDATE_MINB)
       q4[(size_t)k * V] =
           make_float4((float)v[2 * k].x, (float)v[2 * k].y, (float)v[2 * k + 1].x, (float)v[2 * k + 1].y);
   }
+  if (fx) {
+    // the fixed-point copy of what was stored, as k_to_fx makes it
+    double m[18];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      m[2 * k] = v[k].x;
+      m[2 * k + 1] = v[k].y;
+    }
+    int4 el[9];
+    const size_t off = fx_offset(mu, s, V);
+    fx_store_exp(fx, off, s, fx_from_f64(m, el));
+#pragma unroll
+    for (int k = 0; k < 9; ++k) *reinterpret_cast<int4*>(fx + off + 512 * k) = el[k];
+  }
 }
 
+// Sites up to which the update itself writes the fixed-point copy. It saves a
+// launch and the copy's pass over the links (8^4 trajectory of 20 steps 784 ->
+// 718 us, 24^4 of 10 steps 11.22 -> 11.13 ms), but in registers it costs the
+// update more than the bandwidth-bound copy kernel once that runs at full rate
+// (32^4 flow, 2 steps: 18.64 against 18.41 ms).
+#ifndef GF_FX_FUSE_MAX
+#define GF_FX_FUSE_MAX (1 << 19)
+#endif
 static void update_links(gf_ctx* ctx, gf_field* W, const gf_field* P, double eps, const gf_field* U, int reunit,
-                         gf_field* shadow32) {
+                         gf_field* shadow32, gf_field* fx) {
   dim3 grid(blocks_for(ctx->geom.vol, 128), 4);
+  const bool fused = ctx->geom.vol <= GF_FX_FUSE_MAX;
   auto kern = reunit ? k_link_update_fx<true> : k_link_update_fx<false>;
   kern<<<grid, 128, 0, ctx->stream>>>((const double2*)U->ptr, (double2*)W->ptr, (const double*)P->ptr, ctx->geom,
-                                      fx_scalar_of(eps), shadow32 ? (float4*)shadow32->ptr : nullptr);
+                                      fx_scalar_of(eps), shadow32 ? (float4*)shadow32->ptr : nullptr,
+                                      fx && fused ? (char*)fx->ptr : nullptr);
   GF_CHECK_LAUNCH();
+  if (fx && !fused) to_fx(ctx, fx, W);
 }
 
-void link_update(gf_ctx* ctx, gf_field* U, const gf_field* P, double eps, int reunit, gf_field* shadow32, bool df) {
+void link_update(gf_ctx* ctx, gf_field* U, const gf_field* P, double eps, int reunit, gf_field* shadow32, bool df,
+                 gf_field* fx) {
   if (U->kind != GF_LINK64) throw gf_error(GF_EINVAL, "link update: U must be LINK64");
   if (P->kind != GF_MOM64) throw gf_error(GF_EINVAL, "link update: P must be MOM64");
   ProfScope prof(ctx, df ? GF_K_LINK_UPDATE_DF : GF_K_LINK_UPDATE);
-  update_links(ctx, U, P, eps, U, reunit, shadow32);
+  update_links(ctx, U, P, eps, U, reunit, shadow32, fx);
 }
 
 // exp_aF_U!(W, a, F, U) (src/AbstractGaugefields.jl:2810-2842): W_mu = exp(a F_mu) U_mu
 // with F in su(3) coefficients, i.e. exp(i a sum_a F_a lambda_a / 2) U.
-void exp_mom_links(gf_ctx* ctx, gf_field* W, const gf_field* P, double a, const gf_field* U, bool df) {
+void exp_mom_links(gf_ctx* ctx, gf_field* W, const gf_field* P, double a, const gf_field* U, bool df, gf_field* fx) {
   ProfScope prof(ctx, df ? GF_K_LINK_UPDATE_DF : GF_K_LINK_UPDATE);
-  update_links(ctx, W, P, a, U, 0, nullptr);
+  update_links(ctx, W, P, a, U, 0, nullptr, fx);
 }
 
 __global__ void k_reunit(double2* __restrict__ U, int V) {

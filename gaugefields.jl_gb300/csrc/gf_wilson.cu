@@ -24,13 +24,20 @@ __global__ void __launch_bounds__(128, GF_MINB(R)) k_plaquette(SRC U, Geom g, do
   block_partial_sum(v, part);
 }
 
-double plaquette_sum(gf_ctx* ctx, const gf_field* U) {
+void plaquette_start(gf_ctx* ctx, const gf_field* U, int slot) {
   ProfScope prof(ctx, GF_K_PLAQ);
-  if (U->kind == GF_LINKFX) return plaquette_sum_fx(ctx, U);
-  // fp64 links, and the top level of a double-float stack
-  if (U->kind == GF_LINK64 || U->kind == GF_MAT64 || U->kind == GF_LINKDF) return plaquette_sum_fx(ctx, fx_links(ctx, U));
+  // fp64 links, and the top level of a double-float stack, through a fixed-point copy
+  plaquette_start_fx(ctx, U->kind == GF_LINKFX ? U : fx_links(ctx, U), slot);
+}
+
+double plaquette_sum(gf_ctx* ctx, const gf_field* U) {
+  if (U->kind == GF_LINK64 || U->kind == GF_MAT64 || U->kind == GF_LINKDF || U->kind == GF_LINKFX) {
+    plaquette_start(ctx, U, 0);
+    return sum_wait(ctx, 0);
+  }
   if (U->kind != GF_LINK32) throw gf_error(GF_EINVAL, "plaquette: links must be LINK64 or LINK32");
   const int nb = blocks_for(ctx->geom.vol, 128);
+  ProfScope prof(ctx, GF_K_PLAQ);
   Src32 src{(const float4*)U->ptr};
   k_plaquette<float><<<nb, 128, 0, ctx->stream>>>(src, ctx->geom, ctx->d_partials);
   GF_CHECK_LAUNCH();
@@ -129,9 +136,12 @@ void wilson_force_coef(gf_ctx* ctx, const gf_field* U, gf_field* P, double coef,
   if (P->kind != GF_MOM64) throw gf_error(GF_EINVAL, "force: output must be MOM64");
   dim3 grid = stencil_grid(ctx->geom.vol, 128);
   ProfScope prof(ctx, df ? GF_K_FORCE_DF : GF_K_FORCE);
-  if (df && U->kind != GF_LINK64) {
+  if (df && U->kind != GF_LINK64 && U->kind != GF_LINKFX) {
     throw gf_error(GF_EINVAL, "force: the double-float force needs LINK64 links");
   } else if (U->kind == GF_LINK64) {
+    wilson_force_fx(ctx, fx_links(ctx, U), P, coef, keep);
+    return;
+  } else if (U->kind == GF_LINKFX) {
     wilson_force_fx(ctx, U, P, coef, keep);
     return;
   } else if (U->kind == GF_LINK32) {

@@ -128,4 +128,47 @@ __device__ __forceinline__ void block_partial_sum(double v, double* __restrict__
   }
 }
 
+// Where a global sum goes: the blocks' partials, and (count set) the total,
+// which the last block to finish adds up in the order of the blocks, so that
+// the result does not depend on which one that is, and writes to *out (pinned
+// host memory). count is zero before and after.
+struct SumOut {
+  double* part;
+  unsigned* count;
+  double* out;
+};
+__device__ __forceinline__ void block_sum(double v, const SumOut& to) {
+  __shared__ double sh[32];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll 1
+  for (int round = 0; round < 2; ++round) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) sh[w] = v;
+    __syncthreads();
+    if (w == 0) {
+      v = lane < nw ? sh[lane] : 0.0;
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+      if (lane == 0) {
+        if (round == 1) {
+          *to.out = v;
+          *to.count = 0;
+        } else {
+          to.part[blockIdx.x] = v;
+          if (to.count) {
+            __threadfence();
+            last = atomicAdd(to.count, 1u) == gridDim.x - 1;
+          }
+        }
+      }
+    }
+    if (round == 1 || !to.count) return;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    v = 0.0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) v += __ldcg(to.part + i);
+  }
+}
+
 }  // namespace gf

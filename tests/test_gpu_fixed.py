@@ -202,3 +202,42 @@ def test_link_update_keeps_bad_values_where_they_are(pkg, exact_exp_oracle):
     hit = ~np.isfinite(got).all(axis=(-1, -2))
     assert sorted(zip(*np.nonzero(hit))) == [(0, 5), (1, 60), (3, 100)]
     close(got[~hit], ref[~hit], 1e-12)
+
+
+@pytest.mark.parametrize("L", SIZES + [(8, 8, 16, 18)])
+def test_sums_of_few_and_many_blocks(pkg, oracle, L):
+    """A sum whose last block adds up the partials and one that needs the
+    second kernel (8 x 8 x 16 x 18: 3,456 plaquette items), twice over: bitwise
+    repeatable, and P P against numpy."""
+    U, Uh = start(pkg, oracle, L, "unitary")
+    p = [pkg.calculate_Plaquette(U) for _ in range(3)]
+    r = [pkg.rectangle_sum(U) for _ in range(3)]
+    assert len(set(p)) == 1 and len(set(r)) == 1
+    assert abs(p[0] - oracle.plaquette(list(L), Uh)) <= 1e-13 * abs(18 * np.prod(L))
+    assert abs(r[0] - oracle.rectangle_sum(list(L), Uh)) <= 1e-13 * abs(36 * np.prod(L))
+    P = pkg.gaussian_momenta(U, seed=3)
+    k = (P.to_host() ** 2).sum()
+    assert abs(P * P - k) <= 1e-13 * k
+
+
+@pytest.mark.parametrize("L", [(4, 6, 10, 14), (34, 2, 2, 6)])
+@pytest.mark.parametrize("c_rect", [0.0, -0.1])
+def test_drivers_copy_equals_a_fresh_conversion(pkg, oracle, L, c_rect):
+    """The fixed-point copy that the link update keeps for the next force is
+    bitwise what converting the stored links gives: the one-call trajectory and
+    the one stepped through md_step_ (which converts each time) agree bitwise
+    where they take the same steps (PQP: no half steps merge for one step)."""
+    out = []
+    for whole in (True, False):
+        U, _ = start(pkg, oracle, L, "unitary")
+        P = pkg.gaussian_momenta(U, seed=9)
+        action = pkg.GaugeAction(U)
+        pkg.push_(action, 3.0, "plaquette")
+        pkg.push_(action, c_rect, "rectangular")
+        drv = pkg.md_driver(U, action, steps=1, trajectory_length=0.3, integrator=pkg.PQP())
+        if whole:
+            pkg.md_trajectory_(U, P, drv)
+        else:
+            pkg.md_step_(pkg.PQP(), U, P, 0.3, drv)
+        out.append((U.to_host(), P.to_host()))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
