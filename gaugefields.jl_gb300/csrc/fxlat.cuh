@@ -198,6 +198,65 @@ __device__ __forceinline__ void fx_add_staples(fx_acc& acc, int& ea, const FxFie
   }
 }
 
+// Small lattices do not fill the GPU with three threads per link, and a call
+// takes as long as one thread's chain of products. The stencil kernels then
+// run three times as many, one group of 96 per axis nu != mu (thread t: axis
+// t / 96), and sum the groups' rows through shared memory. 20-step Wilson
+// trajectories and two-level stout forces, one group against three: 4^4 629
+// and 105 us against 506 and 88, 6^4 653 and 120 against 570 and 112, 8^4 718
+// and 158 against 759 and 175 (the GPU is full, and the exchange costs).
+#ifndef GF_FX_SPLIT_MAX
+#define GF_FX_SPLIT_MAX 2048
+#endif
+template <int AXES>
+struct FxAxes {  // rows of the axes 1 .. AXES - 1
+  FxRaw v[AXES > 1 ? AXES - 1 : 1];
+  int e[AXES > 1 ? AXES - 1 : 1][GF_FX_LINKS];
+};
+template <>
+struct FxAxes<1> {};
+// acc of the other axes added to the first one's; every thread of the block
+// calls it, those of axis 0 return the sum
+template <int AXES>
+__device__ __forceinline__ void fx_sum_axes(FxAxes<AXES>& sh, int axis, int link, int r, fx_acc& acc, int& ea) {
+  if constexpr (AXES > 1) {
+    if (axis > 0) {
+      fx_share(sh.v[axis - 1], link, r, acc);
+      if (r == 0) sh.e[axis - 1][link] = ea;
+    }
+    __syncthreads();
+    if (axis == 0) {
+#pragma unroll
+      for (int a = 0; a < AXES - 1; ++a) {
+        fx_acc o;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          o.re[j] = sh.v[a].v[2 * (3 * r + j)][link];
+          o.im[j] = sh.v[a].v[2 * (3 * r + j) + 1][link];
+        }
+        fx_add(acc, ea, o, sh.e[a][link]);
+      }
+    }
+  }
+}
+// rows of V = S^dag of a field at s: the staple sum, |V| <= 6 2^ea (axis 0's
+// threads when AXES = 3)
+template <int AXES>
+__device__ __forceinline__ fx_acc fx_staple_row(FxAxes<AXES>& sh, const FxField& U, const Geom& g, const Site& st,
+                                                int s, int mu, int axis, int link, int r, int& ea) {
+  fx_acc acc = {{0, 0, 0}, {0, 0, 0}};
+  ea = -GF_FX_BAD;
+  const int mu_up = fx_up(g, st, mu);
+  if (AXES > 1) {
+    fx_add_staples(acc, ea, U, g, st, s, mu, (mu + 1 + axis) & 3, mu_up, r);
+  } else {
+#pragma unroll 1
+    for (int k = 1; k < 4; ++k) fx_add_staples(acc, ea, U, g, st, s, mu, (mu + k) & 3, mu_up, r);
+  }
+  fx_sum_axes<AXES>(sh, axis, link, r, acc, ea);
+  return acc;
+}
+
 // ---------------------------------------------------------------------------
 // exp(iX) of the block's links
 // ---------------------------------------------------------------------------

@@ -107,27 +107,28 @@ void plaquette_start_fx(gf_ctx* ctx, const gf_field* F, int slot) {
 // four cycles: 81 per row product, 13 products). 24^4, conversion included:
 // 4.71 ms in fp64 arithmetic, 0.70 ms here. Seven blocks per SM (80
 // registers) measured 0.70 ms, six 0.73, five 0.74, eight (spills) 0.72.
-__global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_MINB)
+template <int AXES>
+__global__ void __launch_bounds__(GF_FX_THREADS * AXES, AXES > 1 ? 2 : GF_FX_MINB)
     k_force_fx(FxField U, double* __restrict__ P, Geom g, double coef, double keep) {
   __shared__ FxRaw sh;
+  __shared__ FxAxes<AXES> ax;
   __shared__ int se[GF_FX_LINKS];
-  const int t = threadIdx.x, mu = blockIdx.x & 3, V = g.vol;
-  const int s0 = (blockIdx.x >> 2) * GF_FX_LINKS;
+  const int axis = AXES > 1 ? threadIdx.x / GF_FX_THREADS : 0, t = threadIdx.x - axis * GF_FX_THREADS;
+  const int mu = blockIdx.x & 3, V = g.vol, s0 = (blockIdx.x >> 2) * GF_FX_LINKS;
   {
     const int link = t / 3, r = t - 3 * link;
     const int s = min(s0 + link, V - 1);
     const Site st = site_of(g, s);
-    const int mu_up = fx_up(g, st, mu);
-    fx_acc acc = {{0, 0, 0}, {0, 0, 0}};
-    int ea = -GF_FX_BAD;
-#pragma unroll 1
-    for (int k = 1; k < 4; ++k) fx_add_staples(acc, ea, U, g, st, s, mu, (mu + k) & 3, mu_up, r);
-    // |V| <= 6: three bits down to serve as an operand
-    fx_share(sh, link, r, fx_row_mul<true>(fx_operand<3>(acc), fx_mat(U, mu, s, V)));
-    if (r == 0) se[link] = ea + 3 + fx_exp(U, mu, s, V);
+    int ea;
+    const fx_acc acc = fx_staple_row<AXES>(ax, U, g, st, s, mu, axis, link, r, ea);
+    if (axis == 0) {
+      // |V| <= 6: three bits down to serve as an operand
+      fx_share(sh, link, r, fx_row_mul<true>(fx_operand<3>(acc), fx_mat(U, mu, s, V)));
+      if (r == 0) se[link] = ea + 3 + fx_exp(U, mu, s, V);
+    }
   }
   __syncthreads();
-  fx_update_mom(sh, se, P, mu, s0, V, -coef, keep);
+  if (axis == 0) fx_update_mom(sh, se, P, mu, s0, V, -coef, keep);
 }
 
 gf_field* fx_links(gf_ctx* ctx, const gf_field* U) {
@@ -138,7 +139,9 @@ gf_field* fx_links(gf_ctx* ctx, const gf_field* U) {
 
 void wilson_force_fx(gf_ctx* ctx, const gf_field* F, gf_field* P, double coef, double keep) {
   const int nb = 4 * blocks_for(ctx->geom.vol, GF_FX_LINKS);
-  k_force_fx<<<nb, GF_FX_THREADS, 0, ctx->stream>>>(fx_view(F), (double*)P->ptr, ctx->geom, coef, keep);
+  const int axes = ctx->geom.vol <= GF_FX_SPLIT_MAX ? 3 : 1;
+  auto kern = axes == 3 ? k_force_fx<3> : k_force_fx<1>;
+  kern<<<nb, axes * GF_FX_THREADS, 0, ctx->stream>>>(fx_view(F), (double*)P->ptr, ctx->geom, coef, keep);
   GF_CHECK_LAUNCH();
 }
 

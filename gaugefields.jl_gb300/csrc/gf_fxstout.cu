@@ -12,16 +12,6 @@
 
 namespace gf {
 
-// rows of V = S^dag of a field at s: the staple sum, |V| <= 6 2^ea
-__device__ __forceinline__ fx_acc fx_staple_row(const FxField& U, const Geom& g, const Site& st, int s, int mu, int r,
-                                                int& ea) {
-  fx_acc acc = {{0, 0, 0}, {0, 0, 0}};
-  ea = -GF_FX_BAD;
-  const int mu_up = fx_up(g, st, mu);
-#pragma unroll 1
-  for (int k = 1; k < 4; ++k) fx_add_staples(acc, ea, U, g, st, s, mu, (mu + k) & 3, mu_up, r);
-  return acc;
-}
 // a raw row from an operand row of a field
 __device__ __forceinline__ fx_acc fx_raw_row(const fx_row& a) {
   fx_acc v;
@@ -55,36 +45,48 @@ __device__ __forceinline__ void fx_down_row(fx_acc& v) {
 #ifndef GF_FX_FWD_MINB
 #define GF_FX_FWD_MINB 7
 #endif
-__global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_FWD_MINB)
+template <int AXES>
+__global__ void __launch_bounds__(GF_FX_THREADS * AXES, AXES > 1 ? 2 : GF_FX_FWD_MINB)
     k_stout_fwd_fx(FxField U, char* __restrict__ Uout, char* __restrict__ Cout, Geom g, fx_scalar rho,
                    fx_scalar rho3) {
   __shared__ FxExp sh;
-  const int t = threadIdx.x, mu = blockIdx.x & 3, V = g.vol;
+  __shared__ FxAxes<AXES> ax;
+  const int axis = AXES > 1 ? threadIdx.x / GF_FX_THREADS : 0, t = threadIdx.x - axis * GF_FX_THREADS;
+  const int mu = blockIdx.x & 3, V = g.vol;
   const int link = t / 3, r = t - 3 * link;
   const int sx = (blockIdx.x >> 2) * GF_FX_LINKS + link, s = min(sx, V - 1);
   const size_t off = fx_offset(mu, s, V);
   {
     const Site st = site_of(g, s);
     int ev;
-    fx_acc v = fx_staple_row(U, g, st, s, mu, r, ev);
-    const fx_row vr = fx_operand<3>(v);
-    fx_share(sh.m, link, r, fx_row_mul<true>(vr, fx_mat(U, mu, s, V)));
-    if (r == 0) sh.e[link] = ev + 3 + fx_exp(U, mu, s, V);
-    if (Cout && sx < V) {
-      fx_down_row<3>(v);
-      fx_scale_row(v, rho);
-      fx_store_row(Cout, off, r, v);
-      if (r == 0) fx_store_exp(Cout, off, s, ev + 3 + rho.e);
+    fx_acc v = fx_staple_row<AXES>(ax, U, g, st, s, mu, axis, link, r, ev);
+    if (axis == 0) {
+      const fx_row vr = fx_operand<3>(v);
+      fx_share(sh.m, link, r, fx_row_mul<true>(vr, fx_mat(U, mu, s, V)));
+      if (r == 0) sh.e[link] = ev + 3 + fx_exp(U, mu, s, V);
+      if (Cout && sx < V) {
+        fx_down_row<3>(v);
+        fx_scale_row(v, rho);
+        fx_store_row(Cout, off, r, v);
+        if (r == 0) fx_store_exp(Cout, off, s, ev + 3 + rho.e);
+      }
     }
   }
   __syncthreads();
   const int E0 = sh.e[link];
-  if (t < 64) {
+  if (threadIdx.x < 64) {
     int e;
     const fx_herm q = fx_ta_herm(sh, t & 31, rho, rho3, e);
     fx_exp_coefficients<false>(sh, nullptr, t & 31, t >> 5, q, e);
   }
   __syncthreads();
+  if (AXES > 1) {
+    // the other axes' threads only keep step with the squarings' barriers
+    if (axis > 0) {
+      for (int k = 0; k < 2 * sh.most; ++k) __syncthreads();
+      return;
+    }
+  }
   const fx_acc E = fx_exp_row_squared(sh, link, r);
   const fx_acc W = fx_row_mul<false>(fx_operand<0>(E), fx_mat(U, mu, s, V));
   if (sx >= V) return;
@@ -122,7 +124,8 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_LOCAL_MINB)
   int ec, ed;
   // C U^dag
   if (RECOMPUTE) {
-    fx_acc c = fx_staple_row(U, g, st, s, mu, r, ec);
+    FxAxes<1> none;
+    fx_acc c = fx_staple_row<1>(none, U, g, st, s, mu, 0, link, r, ec);
     fx_down_row<3>(c);
     fx_scale_row(c, rho);
     ec += 3 + rho.e;
@@ -134,7 +137,8 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_LOCAL_MINB)
   }
   if (r == 0) sh.x.e[link] = ec + eu;
   if (TOP) {
-    fx_acc v = fx_staple_row(F1, g, st, s, mu, r, ed);
+    FxAxes<1> none;
+    fx_acc v = fx_staple_row<1>(none, F1, g, st, s, mu, 0, link, r, ed);
     fx_down_row<3>(v);
     fx_scale_row(v, halfbeta);
     ed += 3 + halfbeta.e;
@@ -340,8 +344,8 @@ __device__ __forceinline__ void fx_gather_axis(fx_acc& acc, int& ea, const FxFie
 
 // D = Dp + rho (pull-back). OUT 0: fixed-point Dout; 1: fp64 Dout (MAT64);
 // 2: the thin-link momentum update P += coef c(U D) instead.
-template <int OUT>
-__global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_GATHER_MINB)
+template <int OUT, int AXES>
+__global__ void __launch_bounds__(GF_FX_THREADS * AXES, AXES > 1 ? 2 : GF_FX_GATHER_MINB)
     k_bwd_gather_fx(FxField U, FxField Z, FxField Dp, char* __restrict__ Dout, double* __restrict__ P, Geom g,
                     fx_scalar rho, double coef) {
   __shared__ union {
@@ -350,15 +354,21 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_GATHER_MINB)
     float n[3][GF_FX_LINKS];
   } sh;
   __shared__ int se[GF_FX_LINKS];
-  const int t = threadIdx.x, nu = blockIdx.x & 3, V = g.vol;
+  __shared__ FxAxes<AXES> ax;
+  const int axis = AXES > 1 ? threadIdx.x / GF_FX_THREADS : 0, t = threadIdx.x - axis * GF_FX_THREADS;
+  const int nu = blockIdx.x & 3, V = g.vol;
   const int link = t / 3, r = t - 3 * link, s0 = (blockIdx.x >> 2) * GF_FX_LINKS;
   const int sx = s0 + link, s = min(sx, V - 1);
   const Site st = site_of(g, s);
   const int nu_up = fx_up(g, st, nu);
-  fx_acc d = fx_raw_row(fx_load_row<false>(fx_mat(Dp, nu, s, V), r));
-  int ed = fx_exp(Dp, nu, s, V);
+  fx_acc d = {{0, 0, 0}, {0, 0, 0}};
+  int ed = -GF_FX_BAD;
+  if (axis == 0) {
+    d = fx_raw_row(fx_load_row<false>(fx_mat(Dp, nu, s, V), r));
+    ed = fx_exp(Dp, nu, s, V);
+  }
 #pragma unroll 1
-  for (int k = 1; k < 4; ++k) {
+  for (int k = 1 + axis; k < 4; k += AXES) {
     fx_acc acc = {{0, 0, 0}, {0, 0, 0}};
     int ea = -GF_FX_BAD;
     fx_gather_axis(acc, ea, U, Z, g, st, s, nu, nu_up, (nu + k) & 3, r);
@@ -366,15 +376,20 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_GATHER_MINB)
     fx_scale_row(acc, rho);
     fx_add(d, ed, acc, ea + 1 + rho.e);  // |d| <= 1 + 3 * 1.5
   }
+  fx_sum_axes<AXES>(ax, axis, link, r, d, ed);
+  if (AXES > 1 && axis > 0 && OUT == 1) return;
   if (OUT == 2) {
-    fx_share<3>(sh.d, link, r, d);
+    if (axis == 0) fx_share<3>(sh.d, link, r, d);
     __syncthreads();
-    const fx_acc m = fx_row_mul<false>(fx_load_row<false>(fx_mat(U, nu, s, V), r), FxShMat{&sh.d, link});
+    fx_acc m;
+    if (axis == 0) m = fx_row_mul<false>(fx_load_row<false>(fx_mat(U, nu, s, V), r), FxShMat{&sh.d, link});
     __syncthreads();
-    fx_share(sh.m, link, r, m);
-    if (r == 0) se[link] = ed + 3 + fx_exp(U, nu, s, V);
+    if (axis == 0) {
+      fx_share(sh.m, link, r, m);
+      if (r == 0) se[link] = ed + 3 + fx_exp(U, nu, s, V);
+    }
     __syncthreads();
-    fx_update_mom(sh.m, se, P, nu, s0, V, coef, 1.0);
+    if (axis == 0) fx_update_mom(sh.m, se, P, nu, s0, V, coef, 1.0);
   } else if (OUT == 1) {
     if (sx >= V) return;
     double2* o = reinterpret_cast<double2*>(Dout) + (size_t)nu * 9 * V + s;
@@ -382,9 +397,9 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_GATHER_MINB)
     for (int j = 0; j < 3; ++j)
       o[(size_t)(3 * r + j) * V] = make_double2(fx_to_f64(d.re[j], ed), fx_to_f64(d.im[j], ed));
   } else {
-    sh.n[r][link] = fx_square(d);
+    if (axis == 0) sh.n[r][link] = fx_square(d);
     __syncthreads();
-    if (sx >= V) return;
+    if (sx >= V || axis > 0) return;
     const int k = fx_norm_shift(sh.n[0][link] + sh.n[1][link] + sh.n[2][link], ed);
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
@@ -409,13 +424,17 @@ static fx_scalar third_of(double c) {
   return r;
 }
 
+static int axes_of(const gf_ctx* ctx) { return ctx->geom.vol <= GF_FX_SPLIT_MAX ? 3 : 1; }
+
 void stout_forward_fx(gf_ctx* ctx, gf_stout* st) {
   const int nb = 4 * blocks_for(ctx->geom.vol, GF_FX_LINKS);
   for (int l = 0; l < st->nlev; ++l) {
     ProfScope prof(ctx, GF_K_STOUT_FWD64);
-    k_stout_fwd_fx<<<nb, GF_FX_THREADS, 0, ctx->stream>>>(fx_view(st->lev_in[l]), (char*)st->lev_in[l + 1]->ptr,
-                                                          st->store ? (char*)st->C[l]->ptr : nullptr, ctx->geom,
-                                                          fx_scalar_of(st->rho[l]), third_of(st->rho[l]));
+    const int axes = axes_of(ctx);
+    auto kern = axes == 3 ? k_stout_fwd_fx<3> : k_stout_fwd_fx<1>;
+    kern<<<nb, axes * GF_FX_THREADS, 0, ctx->stream>>>(fx_view(st->lev_in[l]), (char*)st->lev_in[l + 1]->ptr,
+                                                       st->store ? (char*)st->C[l]->ptr : nullptr, ctx->geom,
+                                                       fx_scalar_of(st->rho[l]), third_of(st->rho[l]));
     GF_CHECK_LAUNCH();
   }
 }
@@ -446,15 +465,17 @@ void stout_backward_fx(gf_ctx* ctx, gf_stout* st, const gf_field* dSdUbar, doubl
     ProfScope prof(ctx, GF_K_BWD_GATHER64);
     const FxField u = fx_view(st->lev_in[l]), z = fx_view(st->Z), dp = fx_view(st->Dp);
     const fx_scalar rho = fx_scalar_of(st->rho[l]);
+    const bool split = axes_of(ctx) == 3;
+    const int nt = (split ? 3 : 1) * GF_FX_THREADS;
     if (l == 0 && P)
-      k_bwd_gather_fx<2><<<nb, GF_FX_THREADS, 0, ctx->stream>>>(u, z, dp, nullptr, (double*)P->ptr, ctx->geom, rho,
-                                                                -eps / 3.0);
+      (split ? k_bwd_gather_fx<2, 3> : k_bwd_gather_fx<2, 1>)<<<nb, nt, 0, ctx->stream>>>(
+          u, z, dp, nullptr, (double*)P->ptr, ctx->geom, rho, -eps / 3.0);
     else if (l == 0 && dSdU)
-      k_bwd_gather_fx<1><<<nb, GF_FX_THREADS, 0, ctx->stream>>>(u, z, dp, (char*)dSdU->ptr, nullptr, ctx->geom, rho,
-                                                                0.0);
+      (split ? k_bwd_gather_fx<1, 3> : k_bwd_gather_fx<1, 1>)<<<nb, nt, 0, ctx->stream>>>(
+          u, z, dp, (char*)dSdU->ptr, nullptr, ctx->geom, rho, 0.0);
     else
-      k_bwd_gather_fx<0><<<nb, GF_FX_THREADS, 0, ctx->stream>>>(u, z, dp, (char*)st->D[nxt]->ptr, nullptr, ctx->geom,
-                                                                rho, 0.0);
+      (split ? k_bwd_gather_fx<0, 3> : k_bwd_gather_fx<0, 1>)<<<nb, nt, 0, ctx->stream>>>(
+          u, z, dp, (char*)st->D[nxt]->ptr, nullptr, ctx->geom, rho, 0.0);
     GF_CHECK_LAUNCH();
     cur = nxt;
   }
