@@ -427,21 +427,19 @@ GF_HD float fx_leading(double d, int emax) {
   return (e == 0 || ef <= 0) ? 0.f : fx_float_bits(sg | ((unsigned int)ef << 23) | man);
 }
 
-// One matrix to fixed point; returns its exponent. A bound on the squared
-// spectral norm, max_i sum_j |(M^dag M)_ij|, is formed in fp32 from the
-// leading bits; it is 1 for a unitary matrix.
-GF_HD int fx_from_f64(const double* m /* 18, row-major, re im */, int4 out[9]) {
-  int emax = 1;
+// Exponent emax - 1023 + up of a matrix: the smallest for which a bound on the
+// spectral norm, max_i sum_j |(M^dag M)_ij| in fp32 from the leading bits, is
+// at most 1 (1 + 2^-10). It is 1 for a unitary matrix. False for a matrix that
+// is not finite.
+GF_HD bool fx_exponent_of(const double* m /* 18, row-major, re im */, int& emax, int& up) {
+  emax = 1;
+  up = 0;
 #pragma unroll
   for (int i = 0; i < 18; ++i) {
     const int e = fx_exponent_field(m[i]);
     emax = e > emax ? e : emax;
   }
-  if (emax == 0x7FF) {
-#pragma unroll
-    for (int i = 0; i < 9; ++i) out[i] = make_int4(0, 0, 0, 0);
-    return GF_FX_BAD;
-  }
+  if (emax == 0x7FF) return false;
   float f[18];
 #pragma unroll
   for (int i = 0; i < 18; ++i) f[i] = fx_leading(m[i], emax);
@@ -463,17 +461,20 @@ GF_HD int fx_from_f64(const double* m /* 18, row-major, re im */, int4 out[9]) {
     }
     bound = fmaxf(bound, s);
   }
-  // smallest E2 with bound <= 4^E2 (1 + 2^-10); bound < 3 * 72 < 4^4
-  const int E2 = (bound > 1.0009765625f) + (bound > 4.00390625f) + (bound > 16.015625f) + (bound > 64.0625f);
-  i64 R[18];
-#pragma unroll
-  for (int i = 0; i < 18; ++i) R[i] = fx_mantissa(m[i], emax, E2);
+  // bound < 3 * 72 < 4^4
+  up = (bound > 1.0009765625f) + (bound > 4.00390625f) + (bound > 16.015625f) + (bound > 64.0625f);
+  return true;
+}
+// One matrix to fixed point; returns its exponent.
+GF_HD int fx_from_f64(const double* m, int4 out[9]) {
+  int emax, up;
+  const bool ok = fx_exponent_of(m, emax, up);
 #pragma unroll
   for (int i = 0; i < 9; ++i) {
-    fx_split<0>(R[2 * i], out[i].x, out[i].y);
-    fx_split<0>(R[2 * i + 1], out[i].z, out[i].w);
+    fx_split<0>(ok ? fx_mantissa(m[2 * i], emax, up) : 0, out[i].x, out[i].y);
+    fx_split<0>(ok ? fx_mantissa(m[2 * i + 1], emax, up) : 0, out[i].z, out[i].w);
   }
-  return emax - 1023 + E2;
+  return ok ? emax - 1023 + up : GF_FX_BAD;
 }
 
 // real and imaginary parts of the f_j, side by side: f at [2 j + im]

@@ -100,47 +100,53 @@ __device__ __forceinline__ fx_herm fx_mom_herm(const double* __restrict__ P, int
   return q;
 }
 
-// rows a, b -> orthonormal, c = conj(a x b) (normalize3!,
-// src/AbstractGaugefields.jl:3378). Returns how many rows are defined.
-__device__ __forceinline__ int fx_unitarise(fx_acc w[3]) {
-  if (!fx_unit_row(w[0])) return 0;
-  fx_num ar[3], ai[3], br[3], bi[3];
-  // row 2 relative to its own size, so that the projection keeps its digits
-  const int d = fx_norm_shift(fx_square(w[1]), 0);
+// b <- unit row of b - <a, b> a, a a unit row; false when nothing is left
+__device__ __forceinline__ bool fx_orthonormal_row(fx_acc& b, const fx_acc& a) {
+  fx_num ar[3], ai[3];
+  // relative to its own size, so that the projection keeps its digits
+  const int d = fx_norm_shift(fx_square(b), 0);
   fx_sum pr = fx_zero_sum(), pi = fx_zero_sum();
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
-    w[1].re[j] = fx_shift(w[1].re[j], d);
-    w[1].im[j] = fx_shift(w[1].im[j], d);
-    br[j] = fx_pre(w[1].re[j]);
-    bi[j] = fx_pre(w[1].im[j]);
-    ar[j] = fx_pre(w[0].re[j]);
-    ai[j] = fx_pre(w[0].im[j]);
-    fx_cmac(pr, pi, br[j], bi[j], ar[j], fx_neg(ai[j]));
+    b.re[j] = fx_shift(b.re[j], d);
+    b.im[j] = fx_shift(b.im[j], d);
+    ar[j] = fx_pre(a.re[j]);
+    ai[j] = fx_pre(a.im[j]);
+    fx_cmac(pr, pi, fx_pre(b.re[j]), fx_pre(b.im[j]), ar[j], fx_neg(ai[j]));
   }
   const fx_num xr = fx_pre(fx_get(pr)), xi = fx_pre(fx_get(pi));
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
     fx_sum yr = fx_zero_sum(), yi = fx_zero_sum();
     fx_cmac(yr, yi, xr, xi, ar[j], ai[j]);
-    w[1].re[j] -= fx_get(yr);
-    w[1].im[j] -= fx_get(yi);
+    b.re[j] -= fx_get(yr);
+    b.im[j] -= fx_get(yi);
   }
-  if (!fx_unit_row(w[1])) return 1;
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    br[j] = fx_pre(w[1].re[j]);
-    bi[j] = fx_pre(w[1].im[j]);
-  }
+  return fx_unit_row(b);
+}
+// conj(a x b)
+__device__ __forceinline__ fx_acc fx_cross_row(const fx_acc& a, const fx_acc& b) {
+  const fx_row x = fx_operand<0>(a), y = fx_operand<0>(b);
+  fx_acc c;
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
     const int k = (j + 1) % 3, l = (j + 2) % 3;
+    const fx_num ark{x.ah[k], x.al[k]}, aik{x.bh[k], x.bl[k]}, arl{x.ah[l], x.al[l]}, ail{x.bh[l], x.bl[l]};
+    const fx_num brk{y.ah[k], y.al[k]}, bik{y.bh[k], y.bl[k]}, brl{y.ah[l], y.al[l]}, bil{y.bh[l], y.bl[l]};
     fx_sum re = fx_zero_sum(), im = fx_zero_sum();
-    fx_cmac(re, im, ar[k], ai[k], br[l], bi[l]);
-    fx_cmac(re, im, fx_neg(ar[l]), fx_neg(ai[l]), br[k], bi[k]);
-    w[2].re[j] = fx_get(re);
-    w[2].im[j] = -fx_get(im);
+    fx_cmac(re, im, ark, aik, brl, bil);
+    fx_cmac(re, im, fx_neg(arl), fx_neg(ail), brk, bik);
+    c.re[j] = fx_get(re);
+    c.im[j] = -fx_get(im);
   }
+  return c;
+}
+// rows a, b -> orthonormal, c = conj(a x b) (normalize3!,
+// src/AbstractGaugefields.jl:3378). Returns how many rows are defined.
+__device__ __forceinline__ int fx_unitarise(fx_acc w[3]) {
+  if (!fx_unit_row(w[0])) return 0;
+  if (!fx_orthonormal_row(w[1], w[0])) return 1;
+  w[2] = fx_cross_row(w[0], w[1]);
   return 3;
 }
 
@@ -163,6 +169,23 @@ __device__ __forceinline__ int fx_from_f64_fast(const double* m, int4 out[9]) {
     fx_split<0>(bad ? 0 : fx_mantissa(m[2 * i + 1], emax, up), out[i].z, out[i].w);
   }
   return bad ? GF_FX_BAD : emax - 1023 + up;
+}
+
+// an element of a unitary matrix, exponent 0
+__device__ __forceinline__ int4 fx_unitary_element(double2 v, bool ok) {
+  int4 o;
+  fx_split<0>(ok ? fx_mantissa(v.x, 1023, 0) : 0, o.x, o.y);
+  fx_split<0>(ok ? fx_mantissa(v.y, 1023, 0) : 0, o.z, o.w);
+  return o;
+}
+__device__ __forceinline__ fx_acc fx_shared_row(const FxRaw& m, int link, int r) {
+  fx_acc v;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    v.re[j] = m.v[2 * (3 * r + j)][link];
+    v.im[j] = m.v[2 * (3 * r + j) + 1][link];
+  }
+  return v;
 }
 
 // blocks per SM of the link update
@@ -249,34 +272,169 @@ __global__ void __launch_bounds__(128, GF_FX_UPDATE_MINB)
   }
   if (fx) {
     // the fixed-point copy of what was stored, as k_to_fx makes it
-    double m[18];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-      m[2 * k] = v[k].x;
-      m[2 * k + 1] = v[k].y;
-    }
     int4 el[9];
     const size_t off = fx_offset(mu, s, V);
-    fx_store_exp(fx, off, s, fx_from_f64(m, el));
+    if (REUNIT) {
+      // a unitary matrix has exponent 0
+#pragma unroll
+      for (int k = 0; k < 9; ++k) el[k] = fx_unitary_element(v[k], fine == 3);
+      fx_store_exp(fx, off, s, fine == 3 ? 0 : GF_FX_BAD);
+    } else {
+      double m[18];
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        m[2 * k] = v[k].x;
+        m[2 * k + 1] = v[k].y;
+      }
+      fx_store_exp(fx, off, s, fx_from_f64(m, el));
+    }
 #pragma unroll
     for (int k = 0; k < 9; ++k) *reinterpret_cast<int4*>(fx + off + 512 * k) = el[k];
   }
 }
 
+// The same with a warp per row of 32 links, for lattices that do not fill the
+// GPU with a thread per link: there the update takes as long as one thread's
+// instructions, some 6,000 of them (GF_FX_ROWS_MAX has the figures). Warps 0 and 1 form the real and imaginary parts of the series
+// while warp 2 brings U to fixed point. Same results as above.
+struct FxUpdateRows {
+  FxExp x;      // x.m: the finished rows
+  FxOperand u;  // U, then (no re-unitarisation) the fp64 result
+  int eu[GF_FX_LINKS];
+  int fine[GF_FX_LINKS];
+};
+template <bool REUNIT>
+__global__ void __launch_bounds__(GF_FX_THREADS, 4)
+    k_link_update_rows_fx(const double2* Uin, double2* Uout, const double* __restrict__ P, Geom g, fx_scalar eps,
+                          float4* __restrict__ sh32, char* __restrict__ fx) {
+  __shared__ FxUpdateRows sh;
+  const int V = g.vol, mu = blockIdx.y, link = threadIdx.x & 31, r = threadIdx.x >> 5;
+  const int sx = blockIdx.x * GF_FX_LINKS + link, s = min(sx, V - 1);
+  if (r < 2) {
+    int e;
+    fx_herm q = fx_mom_herm(P, mu, s, V, eps, e);
+    const fx_plan plan = fx_exp_plan<false>(q, e);
+    i64 c0, c1, f[3], b1[3], b2[3];
+    fx_invariants(q, c0, c1);
+    fx_ch<false>(c_fx_kappa.k[plan.series], plan.guard - fx_kappa_base(plan.series), plan.terms, r, c0, c1, f, b1, b2);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) sh.x.f[2 * j + r][link] = f[j];
+    if (r == 0) {
+#pragma unroll
+      for (int el = 0; el < 9; ++el) sh.x.q.v[el][link] = fx_herm_element(q, el / 3, el % 3);
+      sh.x.e[link] = e;
+      sh.x.g[link] = plan.guard;
+      sh.x.sq[link] = plan.squares;
+      const int most = __reduce_max_sync(0xffffffffu, plan.squares);
+      if (link == 0) sh.x.most = most;
+    }
+  } else {
+    const double2* b = Uin + (size_t)mu * 9 * V + s;
+    double m[18];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      const double2 v = b[(size_t)k * V];
+      m[2 * k] = v.x;
+      m[2 * k + 1] = v.y;
+    }
+    int4 u[9];
+    sh.eu[link] = fx_from_f64_fast(m, u);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) sh.u.v[k][link] = u[k];
+  }
+  __syncthreads();
+  const fx_acc E = fx_exp_row_squared(sh.x, link, r);
+  fx_acc w = {{0, 0, 0}, {0, 0, 0}};
+  if (!REUNIT || r < 2) w = fx_row_mul<false>(fx_operand<0>(E), FxShMat{&sh.u, link});
+  int eu = sh.x.e[link] > GF_FX_BAD / 2 ? GF_FX_BAD : sh.eu[link], fine = 3;
+  if (REUNIT) {
+    if (r == 0) {
+      const bool ok = fx_unit_row(w);
+      sh.fine[link] = ok && eu <= GF_FX_BAD / 2 ? 3 : 0;
+      fx_share(sh.x.m, link, 0, w);
+    }
+    __syncthreads();
+    if (r == 1) {
+      if (!fx_orthonormal_row(w, fx_shared_row(sh.x.m, link, 0)) && sh.fine[link] == 3) sh.fine[link] = 1;
+      fx_share(sh.x.m, link, 1, w);
+    }
+    __syncthreads();
+    if (r == 2) w = fx_cross_row(fx_shared_row(sh.x.m, link, 0), fx_shared_row(sh.x.m, link, 1));
+    fine = sh.fine[link];
+    eu = 0;
+  }
+  double2 v[3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const int ew = r < fine ? eu : GF_FX_BAD;
+    v[j] = make_double2(fx_to_f64(w.re[j], ew), fx_to_f64(w.im[j], ew));
+  }
+  const size_t off = fx_offset(mu, s, V);
+  int4 el[3];
+  int ef = fine == 3 ? 0 : GF_FX_BAD;
+  if (fx && REUNIT) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) el[j] = fx_unitary_element(v[j], fine == 3);
+  } else if (fx) {
+    double2* x = reinterpret_cast<double2*>(sh.u.v) + link;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 3; ++j) x[(3 * r + j) * GF_FX_LINKS] = v[j];
+    __syncthreads();
+    double m[18];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      m[2 * k] = x[k * GF_FX_LINKS].x;
+      m[2 * k + 1] = x[k * GF_FX_LINKS].y;
+    }
+    int emax, up;
+    const bool bad = !fx_exponent_of(m, emax, up);
+    ef = bad ? GF_FX_BAD : emax - 1023 + up;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      fx_split<0>(bad ? 0 : fx_mantissa(v[j].x, emax, up), el[j].x, el[j].y);
+      fx_split<0>(bad ? 0 : fx_mantissa(v[j].y, emax, up), el[j].z, el[j].w);
+    }
+  }
+  if (sx >= V) return;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const int k = 3 * r + j;
+    Uout[((size_t)mu * 9 + k) * V + s] = v[j];
+    if (sh32 && r < 2)  // complex element k of float4 [3][V]
+      reinterpret_cast<float2*>(sh32)[2 * ((size_t)(mu * 3 + k / 2) * V + s) + (k & 1)] =
+          make_float2((float)v[j].x, (float)v[j].y);
+    if (fx) *reinterpret_cast<int4*>(fx + off + 512 * k) = el[j];
+  }
+  if (fx && r == 0) fx_store_exp(fx, off, s, ef);
+}
+
 // Sites up to which the update itself writes the fixed-point copy. It saves a
-// launch and the copy's pass over the links (8^4 trajectory of 20 steps 784 ->
-// 718 us, 24^4 of 10 steps 11.22 -> 11.13 ms), but in registers it costs the
+// launch and the copy's pass over the links (8^4 trajectory of 20 steps, a
+// thread per link, 784 -> 718 us, 24^4 of 10 steps 11.22 -> 11.13 ms), but in registers it costs the
 // update more than the bandwidth-bound copy kernel once that runs at full rate
 // (32^4 flow, 2 steps: 18.64 against 18.41 ms).
 #ifndef GF_FX_FUSE_MAX
 #define GF_FX_FUSE_MAX (1 << 19)
 #endif
+// Sites up to which a link gets a warp lane in each of three warps. Trajectory
+// of 20 steps (without re-unitarisation, flow of 5 steps), a thread per link
+// against rows: 4^4 502 (311) against 462 (251) us, 6^4 572 (343) against 522
+// (282), 8^4 710 (437) against 674 (406); at 10^4 the GPU is full and the
+// rows' barriers cost, 1134 (737) against 1167 (763), at 32^4 the update takes
+// 0.91 against 1.54 ms.
+#ifndef GF_FX_ROWS_MAX
+#define GF_FX_ROWS_MAX 6144
+#endif
 static void update_links(gf_ctx* ctx, gf_field* W, const gf_field* P, double eps, const gf_field* U, int reunit,
                          gf_field* shadow32, gf_field* fx) {
-  dim3 grid(blocks_for(ctx->geom.vol, 128), 4);
-  const bool fused = ctx->geom.vol <= GF_FX_FUSE_MAX;
-  auto kern = reunit ? k_link_update_fx<true> : k_link_update_fx<false>;
-  kern<<<grid, 128, 0, ctx->stream>>>((const double2*)U->ptr, (double2*)W->ptr, (const double*)P->ptr, ctx->geom,
+  const int V = ctx->geom.vol;
+  const bool fused = V <= GF_FX_FUSE_MAX, rows = V <= GF_FX_ROWS_MAX;
+  const int threads = rows ? GF_FX_THREADS : 128;
+  dim3 grid(blocks_for(V, rows ? GF_FX_LINKS : 128), 4);
+  auto kern = rows ? (reunit ? k_link_update_rows_fx<true> : k_link_update_rows_fx<false>)
+                   : (reunit ? k_link_update_fx<true> : k_link_update_fx<false>);
+  kern<<<grid, threads, 0, ctx->stream>>>((const double2*)U->ptr, (double2*)W->ptr, (const double*)P->ptr, ctx->geom,
                                       fx_scalar_of(eps), shadow32 ? (float4*)shadow32->ptr : nullptr,
                                       fx && fused ? (char*)fx->ptr : nullptr);
   GF_CHECK_LAUNCH();

@@ -220,9 +220,10 @@ def test_sums_of_few_and_many_blocks(pkg, oracle, L):
     assert abs(P * P - k) <= 1e-13 * k
 
 
-@pytest.mark.parametrize("L", [(4, 6, 10, 14), (34, 2, 2, 6)])
+@pytest.mark.parametrize("L", [(4, 6, 10, 14), (34, 2, 2, 6), (14, 8, 8, 8)])
 @pytest.mark.parametrize("c_rect", [0.0, -0.1])
-def test_drivers_copy_equals_a_fresh_conversion(pkg, oracle, L, c_rect):
+@pytest.mark.parametrize("reunit", [False, True])
+def test_drivers_copy_equals_a_fresh_conversion(pkg, oracle, L, c_rect, reunit):
     """The fixed-point copy that the link update keeps for the next force is
     bitwise what converting the stored links gives: the one-call trajectory and
     the one stepped through md_step_ (which converts each time) agree bitwise
@@ -234,10 +235,44 @@ def test_drivers_copy_equals_a_fresh_conversion(pkg, oracle, L, c_rect):
         action = pkg.GaugeAction(U)
         pkg.push_(action, 3.0, "plaquette")
         pkg.push_(action, c_rect, "rectangular")
-        drv = pkg.md_driver(U, action, steps=1, trajectory_length=0.3, integrator=pkg.PQP())
+        drv = pkg.md_driver(U, action, steps=1, trajectory_length=0.3, integrator=pkg.PQP(), reunitarize=reunit)
         if whole:
             pkg.md_trajectory_(U, P, drv)
         else:
             pkg.md_step_(pkg.PQP(), U, P, 0.3, drv)
         out.append((U.to_host(), P.to_host()))
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("eps", [0.05, -3.0])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("reunit", [False, True])
+@pytest.mark.parametrize("kind", ["unitary", "scaled"])
+def test_link_update_does_not_depend_on_the_lattice(pkg, oracle, kind, reunit, precision, eps):
+    """Up to 6144 sites the update runs a link's rows in three threads, beyond
+    in one. A link's result depends on nothing else, so a small lattice's links
+    and momenta, repeated over one of 7168 sites, come out bitwise the same,
+    NaNs included."""
+    S, B = (14, 2, 4, 2), (14, 8, 8, 8)
+    n, N = int(np.prod(S)), int(np.prod(B))
+    assert n <= 6144 < N
+    _, Uh = start(pkg, oracle, S, kind)
+    Ph = np.random.RandomState(8).normal(size=(4, n, 8))
+    Uh[1, 7] = 0.0
+    Uh[2, 9, 1, 1] = np.nan
+    Uh[3, 11, 1] = Uh[3, 11, 0]  # rank two: row 2 vanishes under the projection
+    Ph[0, 13, 4] = np.inf
+    reps = -(-N // n)
+    got = []
+    for L, k in ((S, 1), (B, reps)):
+        V = int(np.prod(L))
+        U = pkg.gauge_configuration(L, start="cold")
+        U.from_host(np.tile(Uh, (1, k, 1, 1))[:, :V])
+        P = pkg.gauge_momenta(U).from_host(np.tile(Ph, (1, k, 1))[:, :V])
+        action = pkg.GaugeAction(U)
+        pkg.push_(action, 3.0, "plaquette")
+        drv = pkg.md_driver(U, action, steps=1, reunitarize=reunit, precision=precision)
+        pkg.update_gaugefields_(U, P, eps, drv)
+        got.append(U.to_host())
+    want = np.tile(got[0], (1, reps, 1, 1))[:, :N]
+    assert np.array_equal(got[1], want, equal_nan=True)
