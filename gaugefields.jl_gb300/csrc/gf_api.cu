@@ -409,6 +409,21 @@ extern "C" int gf_staple(gf_ctx* ctx, const gf_field* U, int mu, gf_field* V) {
 // ---------------------------------------------------------------------------
 // stout workspace
 // ---------------------------------------------------------------------------
+// Sites up to which the double-float form's stacks are fixed-point ones, as
+// the plain form's. Two-level force, double-float tables against fixed point:
+// 4^4 207 / 89 us, 8^4 213 / 159, 12^4 698 / 537, 16^4 1684 / 1542, 24^4 7.95 /
+// 7.54 ms, 32^4 24.9 / 23.9: the tables give a link one thread, which leaves a
+// small lattice's last wave nearly empty, and at 32^4 still read and normalise
+// more. Beyond, where a field takes over 1.2 GB, the 4% are left for the
+// tables' 144 bytes a matrix (fixed point: 148): a stack that fills the memory
+// keeps its size.
+#ifndef GF_FX_STACK_MAX
+#define GF_FX_STACK_MAX (1 << 21)
+#endif
+static bool fx_stack(const gf_ctx* ctx, int precision) {
+  return precision == GF_FP64 || (precision == GF_PREC_DF && ctx->geom.vol <= GF_FX_STACK_MAX);
+}
+
 static gf_stout* stout_new(gf_ctx* ctx, int nlev, const double* rho, int precision, int store,
                            bool fwd_only = false, bool arena = false) {
   need(nlev >= 1 && nlev <= GF_MAX_STOUT, "stout: number of levels must be 1..GF_MAX_STOUT");
@@ -419,6 +434,7 @@ static gf_stout* stout_new(gf_ctx* ctx, int nlev, const double* rho, int precisi
   st->ctx = ctx;
   st->nlev = nlev;
   for (int l = 0; l < nlev; ++l) st->rho[l] = rho[l];
+  if (!fwd_only && fx_stack(ctx, precision)) precision = GF_FP64;
   st->precision = precision;
   st->store = store ? 1 : 0;
   // double-float stacks keep their levels and adjoint fields as fp32 hi/lo
@@ -553,7 +569,7 @@ static void check_md(const gf_md_params* p) {
 
 // The context's stack for a stack precision. The mixed form's Hamiltonian
 // uses a forward-only double-float stack; the GF_DFLOAT form shares one full
-// double-float stack between its force and its Hamiltonian.
+// stack between its force and its Hamiltonian.
 static gf_stout* ctx_stout(gf_ctx* ctx, const gf_md_params* p, int precision) {
   gf_stout** slot = precision == GF_FP64 ? &ctx->w_stout64
                     : (precision == GF_MIXED ? &ctx->w_stout32 : &ctx->w_stoutdf);
@@ -571,12 +587,11 @@ static gf_stout* ctx_stout(gf_ctx* ctx, const gf_md_params* p, int precision) {
   return *slot;
 }
 
-// The potential on the (smeared) fp64 links, plaquette and rectangle loops.
-// The plain form evaluates it in fp64. The mixed and double-float forms smear
-// in double-float arithmetic (compensated products, ~1e-13 of the operands'
-// norms) on the fp32 pipes, which on GB300 is 2.1x faster than the fp64 stout
-// forward; the loop sums over the smeared links stay fp64
-// (GF_DF_HAMILTONIAN=0 keeps the mixed form's potential fp64).
+// The potential on the (smeared) links, plaquette and rectangle loops, the
+// sums of fp64 class in every form. The mixed form smears them in double-float
+// arithmetic (compensated products, ~1e-13 of the operands' norms) in two
+// scratch fields, reading the thin links in place (GF_DF_HAMILTONIAN=0: with a
+// plain-form stack of its own).
 #ifndef GF_DF_HAMILTONIAN
 #define GF_DF_HAMILTONIAN 1
 #endif
@@ -608,9 +623,9 @@ static double hamiltonian(gf_ctx* ctx, const gf_field* U, const gf_field* P, con
 
 // Whether the drivers keep a fixed-point copy of the links beside them: the
 // link update writes it, and the force and the potential of thin links, and
-// the plain form's stack, read it instead of converting the links each time.
-static bool keeps_fx(const gf_md_params* p) {
-  return p->precision == GF_FP64 || (p->precision == GF_DFLOAT && p->nstout == 0);
+// a fixed-point stack, read it instead of converting the links each time.
+static bool keeps_fx(const gf_ctx* ctx, const gf_md_params* p) {
+  return fx_stack(ctx, p->precision) || (p->precision == GF_DFLOAT && p->nstout == 0);
 }
 
 // P += eps * F(U) with the force of the (smeared) Wilson action; Ucopy: the
@@ -696,7 +711,7 @@ static MDResult md_run(gf_ctx* ctx, gf_field* U, gf_field* P, const gf_md_params
     U32 = ctx->w_link32;
     link64_to_32(ctx, U32, U);
   }
-  if (keeps_fx(p)) Ufx = fx_links(ctx, U);
+  if (keeps_fx(ctx, p)) Ufx = fx_links(ctx, U);
   const gf_field* Ucopy = U32 ? U32 : Ufx;
   const gf_field* Upot = Ufx ? Ufx : U;  // the potential never takes the fp32 links
   MDResult r;

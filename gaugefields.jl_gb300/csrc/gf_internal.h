@@ -37,8 +37,8 @@ void count_launch();
 
 #define GF_PROF_CAP 4096
 
-// Stack precision with double-float arithmetic: the GF_DFLOAT form, and the
-// Hamiltonian of the mixed form (forward only).
+// Stack precision with double-float arithmetic: the GF_DFLOAT form on large
+// lattices, and the Hamiltonian of the mixed form (forward only).
 #define GF_PREC_DF GF_DFLOAT
 
 // Internal field kinds of double-float stacks: 18-real links and general
@@ -130,7 +130,7 @@ struct gf_stout {
   gf_ctx* ctx;
   int nlev;
   double rho[GF_MAX_STOUT];
-  int precision;  // GF_FP64, GF_MIXED or GF_PREC_DF
+  int precision;  // of the storage and the kernels: GF_FP64 (fixed point), GF_MIXED or GF_PREC_DF
   int store;      // 1: keep C of every level from the forward pass
   int fwd_only;   // 1: no adjoint buffers (a Hamiltonian-only stack)
   gf_field* lev_in[GF_MAX_STOUT + 1];  // lev_in[0] aliases the thin links

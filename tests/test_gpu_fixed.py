@@ -15,6 +15,7 @@ pytestmark = pytest.mark.gpu
 
 SIZES = [(2, 2, 2, 2), (2, 4, 2, 6), (6, 2, 10, 2), (4, 6, 10, 14), (34, 2, 2, 6)]
 TOL = 1e-13
+LARGE = (48, 48, 32, 32)  # 9 2^18 sites, more than 2^21
 
 
 def start(pkg, oracle, L, kind):
@@ -276,3 +277,51 @@ def test_link_update_does_not_depend_on_the_lattice(pkg, oracle, kind, reunit, p
         got.append(U.to_host())
     want = np.tile(got[0], (1, reps, 1, 1))[:, :N]
     assert np.array_equal(got[1], want, equal_nan=True)
+
+
+@pytest.mark.parametrize("c_rect,recompute", [(0.0, True), (-0.1, False)])
+def test_double_float_stacks_of_large_lattices(pkg, c_rect, recompute):
+    """Beyond 2^21 sites the double-float form's stacks run through the
+    double-float tables, up to there in fixed point. 1e-11 between the forms'
+    forces and 5e-13 between their energies, as at the other sizes."""
+    U = pkg.gauge_configuration(LARGE, start="hot", seed=3)
+    action = pkg.GaugeAction(U)
+    pkg.push_(action, 3.0, "plaquette")
+    pkg.push_(action, c_rect, "rectangular")
+    net = pkg.CovNeuralnet(U)
+    for rho in (0.1, 0.08):
+        pkg.push_(net, pkg.STOUT_Layer("plaquette", rho))
+    force, energy = [], []
+    for precision in ("fp64", "dfloat"):
+        P = pkg.gauge_momenta(U)
+        drv = pkg.md_driver(U, action, steps=1, smearing=net, precision=precision, recompute=recompute)
+        pkg.update_momenta_(P, U, 1.0, drv)
+        energy.append(pkg.md_hamiltonian(U, P, drv))
+        force.append(P.to_host())
+    assert np.linalg.norm(force[1] - force[0]) <= 1e-11 * np.linalg.norm(force[0])
+    assert abs(energy[1] - energy[0]) <= 5e-13 * abs(energy[0])
+
+
+def test_double_float_adjoint_of_large_lattices(pkg):
+    """The same for the pull-back of a caller's dS/dUbar, and 1e-11 a link for
+    dS/drho, a sum over the links."""
+    from gaugefields_gb300 import _lib
+    from gaugefields_gb300.api import _StoutStack
+    V = int(np.prod(LARGE))
+    U = pkg.gauge_configuration(LARGE, start="hot", seed=3)
+    rng = np.random.RandomState(5)
+    few = rng.randn(4, 9 << 10, 3, 3) + 1j * rng.randn(4, 9 << 10, 3, 3)
+    D = pkg.Gaugefields4D(U.ctx, _lib.GF_MAT64)
+    D.from_host(np.tile(few, (1, V // few.shape[1], 1, 1)))
+    net = pkg.CovNeuralnet(U)
+    pkg.push_(net, pkg.STOUT_Layer("plaquette", 0.1))
+    grad, drho = [], []
+    for precision in ("fp64", "dfloat"):
+        stack = _StoutStack(U.ctx, [0.1], precision)
+        _lib.check(_lib.load().gf_stout_forward(U.ctx.h, stack.h, U.field.h, None), U.ctx.h)
+        out = pkg.Gaugefields4D(U.ctx, _lib.GF_MAT64)
+        _lib.check(_lib.load().gf_stout_backward(U.ctx.h, stack.h, D.field.h, out.field.h), U.ctx.h)
+        grad.append(out.to_host())
+        drho.append(pkg.get_parameter_derivatives(D, net, U, precision)[0])
+    assert np.linalg.norm(grad[1] - grad[0]) <= 1e-11 * np.linalg.norm(grad[0])
+    assert abs(drho[1] - drho[0]) <= 1e-11 * 4 * V
