@@ -62,14 +62,6 @@ GF_HD fx_row fx_operand(const fx_acc& v) {
   }
   return r;
 }
-// row r of the conjugate: the imaginary part negated limb by limb
-GF_HD void fx_conj(fx_row& r) {
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    r.bh[j] = -r.bh[j];
-    r.bl[j] = -r.bl[j];
-  }
-}
 
 // a b + c as one IMAD.WIDE. The product is written in PTX: knowing that a limb
 // is not negative, the compiler widens it as unsigned, finds no 32 x 32 form

@@ -1,12 +1,29 @@
 // Plaquette + rectangle action (the loops of gf_rect.cu) in block fixed point
 // by rows: the loop sum, the force, and dS/dUbar on a stack's top level. Bound
 // by integer multiply-add issue; the force on 65,520 sites: 5.95 ms in fp64
-// arithmetic, 0.82 ms here.
+// arithmetic, 0.65 ms here.
 #include "gf_internal.h"
 #include "stencil.cuh"
 #include <algorithm>
 
 namespace gf {
+
+// the imaginary parts of a row negated
+__device__ __forceinline__ void fx_conj(fx_row& a) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    a.bh[k] = -a.bh[k];
+    a.bl[k] = -a.bl[k];
+  }
+}
+// a matrix of a field or its transpose: distances of its rows and columns
+struct FxTurned {
+  const char* p;
+  int row, column;
+  __device__ __forceinline__ int4 operator()(int el) const {
+    return __ldg(reinterpret_cast<const int4*>(p + (el / 3) * row + (el % 3) * column));
+  }
+};
 
 // A running row of a product of links, with its exponent.
 struct FxChain {
@@ -24,7 +41,38 @@ struct FxChain {
   __device__ __forceinline__ FxChain& mul(int dir, int site) {
     return mul<DAG>(fx_operand<0>(v), dir, site);
   }
+  // the same with the dagger chosen at run time, one copy of the product for
+  // both: a U^dag = conj(conj(a) U^T)
+  __device__ __forceinline__ FxChain& mul(fx_row a, int dir, int site, bool dag) {
+    const FxTurned u{fx_mat(U, dir, site, V).p, dag ? 512 : 3 * 512, dag ? 3 * 512 : 512};
+    if (dag) fx_conj(a);
+    v = fx_row_mul<false>(a, u);
+    if (dag) {
+#pragma unroll
+      for (int j = 0; j < 3; ++j) v.im[j] = -v.im[j];
+    }
+    e += fx_exp(U, dir, site, V);
+    return *this;
+  }
+  __device__ __forceinline__ FxChain& mul(int dir, int site, bool dag) {
+    return mul(fx_operand<0>(v), dir, site, dag);
+  }
 };
+// row r of a link, or of its dagger, chosen at run time
+__device__ __forceinline__ fx_row fx_load_row(const FxMat& M, int r, bool dag) {
+  const FxTurned u{M.p, dag ? 512 : 3 * 512, dag ? 3 * 512 : 512};
+  fx_row a;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int4 v = __ldg(reinterpret_cast<const int4*>(u.p + r * u.row + k * u.column));
+    a.ah[k] = v.x;
+    a.al[k] = v.y;
+    a.bh[k] = v.z;
+    a.bl[k] = v.w;
+  }
+  if (dag) fx_conj(a);
+  return a;
+}
 
 // lexicographic offset of d steps (|d| <= 2) along mu; extents are at least 2
 __device__ __forceinline__ int fx_steps(const Geom& g, const Site& st, int mu, int d) {
@@ -84,30 +132,38 @@ void rectangle_start_fx(gf_ctx* ctx, const gf_field* F, int slot) {
   sum_finish(ctx, to, nb, slot);
 }
 
-// acc (+)= [cp t_p + cr (t_1 + t_2)] / 4 as an operand row; cp and cr share
-// one exponent (cp.e). |t| <= 1, so the bracket is below 3 units.
-__device__ __forceinline__ fx_row fx_weighted(const FxChain& tp, FxChain t1, const FxChain& t2, fx_scalar cp,
-                                              fx_scalar cr, int& e) {
-  fx_add(t1.v, t1.e, t2.v, t2.e);
-  fx_acc p = tp.v;
-  int ep = tp.e;
+// [cp p + cr t] / 4 as an operand row; cp and cr share one exponent (cp.e).
+// |p| <= 1 and |t| <= 2, so the bracket is below 3 units.
+__device__ __forceinline__ fx_row fx_weighted(const FxChain& p, const FxChain& t, fx_scalar cp, fx_scalar cr, int& e) {
   // one exponent for both summands
-  fx_acc zero = {{0, 0, 0}, {0, 0, 0}};
-  fx_add(p, ep, zero, t1.e);
-  fx_add(t1.v, t1.e, zero, ep);
+  const fx_acc zero = {{0, 0, 0}, {0, 0, 0}};
+  fx_acc a = p.v, b = t.v;
+  int ea = p.e, eb = t.e;
+  fx_add(a, ea, zero, t.e);
+  fx_add(b, eb, zero, ea);
   fx_acc out;
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
     fx_sum re = fx_zero_sum(), im = fx_zero_sum();
-    fx_mac(re, fx_pre(p.re[j] >> 1), fx_num_of(cp));
-    fx_mac(re, fx_pre(t1.v.re[j] >> 1), fx_num_of(cr));
-    fx_mac(im, fx_pre(p.im[j] >> 1), fx_num_of(cp));
-    fx_mac(im, fx_pre(t1.v.im[j] >> 1), fx_num_of(cr));
+    fx_mac(re, fx_pre(a.re[j] >> 1), fx_num_of(cp));
+    fx_mac(re, fx_pre(b.re[j] >> 1), fx_num_of(cr));
+    fx_mac(im, fx_pre(a.im[j] >> 1), fx_num_of(cp));
+    fx_mac(im, fx_pre(b.im[j] >> 1), fx_num_of(cr));
     out.re[j] = fx_get(re);
     out.im[j] = fx_get(im);
   }
-  e = ep + 2 + cp.e;
+  e = ea + 2 + cp.e;
   return fx_operand<1>(out);
+}
+
+__device__ __forceinline__ fx_acc fx_parked(const i64* park) {
+  fx_acc v;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    v.re[j] = park[2 * j * GF_FX_THREADS];
+    v.im[j] = park[(2 * j + 1) * GF_FX_THREADS];
+  }
+  return v;
 }
 
 // Rows of (cp S + cr R)^dag, S the six plaquette and R the eighteen rectangle
@@ -115,61 +171,63 @@ __device__ __forceinline__ fx_row fx_weighted(const FxChain& tp, FxChain t1, con
 // the left. Shared factors: per plane and side the plaquette staple and (a),
 // (e) (or (b), (f)) end in the same link, (c) and (d) start as the plaquette
 // staples do, and all (c), (d) end in U_mu(x+mu)^dag, which is applied once:
-// 61 products instead of 84. The sum is below 8 units of 2^ea.
+// 61 products instead of 84. The sum is below 8 units of 2^ea. One loop body
+// of ten products serves both sides: with a body for each, 96 KB of code,
+// warps waited for instructions three times as long as they issued (24^4: 4.22
+// ms; one body 3.71). (a), (b), (e), (f) first, so that the least stays alive:
+// 3.40 ms; the sum of (c), (d) parked in shared memory (park, this thread's
+// six words): 3.30 ms.
 __device__ __forceinline__ fx_acc fx_loops_row(const FxField& U, const Geom& g, const Site& st, int s, int mu, int r,
-                                               fx_scalar cp, fx_scalar cr, int& ea) {
+                                               fx_scalar cp, fx_scalar cr, int& ea, i64* park) {
   const int V = g.vol;
-  fx_acc acc = {{0, 0, 0}, {0, 0, 0}}, far = {{0, 0, 0}, {0, 0, 0}};
+  fx_acc acc = {{0, 0, 0}, {0, 0, 0}};
+#pragma unroll
+  for (int j = 0; j < 6; ++j) park[j * GF_FX_THREADS] = 0;
   ea = -GF_FX_BAD;
   int ef = -GF_FX_BAD;
   const int m1 = fx_steps(g, st, mu, 1), m2 = fx_steps(g, st, mu, 2), mm = fx_steps(g, st, mu, -1);
   const int xm = eo_of_lex(g, st.lex + m1, st.par ^ 1), x2m = eo_of_lex(g, st.lex + m2, st.par);
   const int xmm = eo_of_lex(g, st.lex + mm, st.par ^ 1);
 #pragma unroll 1
-  for (int k = 1; k < 4; ++k) {
-    const int nu = (mu + k) & 3;
+  for (int k = 2; k < 8; ++k) {
+    // above (even k) or below the link
+    const int nu = (mu + (k >> 1)) & 3;
+    const bool low = k & 1;
+    const int n1 = fx_steps(g, st, nu, low ? -1 : 1), n2 = fx_steps(g, st, nu, low ? -2 : 2);
+    const int xn = eo_of_lex(g, st.lex + n1, st.par ^ 1), x2n = eo_of_lex(g, st.lex + n2, st.par);
+    const int xmn = eo_of_lex(g, st.lex + m1 + n1, st.par), xmmn = eo_of_lex(g, st.lex + mm + n1, st.par);
+    const int start = low ? xn : s;
+    const FxMat first = fx_mat(U, nu, start, V);
+    const int e0 = fx_exp(U, nu, start, V);
+    FxChain t{U, V, {}, e0};  // (a), (b)
+    t.mul(fx_load_row(first, r, low), nu, low ? x2n : xn, low).mul<false>(mu, x2n);
+    t.mul(nu, low ? eo_of_lex(g, st.lex + m1 + n2, st.par ^ 1) : xmn, !low);
     {
-      const int n1 = fx_steps(g, st, nu, 1), n2 = fx_steps(g, st, nu, 2);
-      const int xn = eo_of_lex(g, st.lex + n1, st.par ^ 1), x2n = eo_of_lex(g, st.lex + n2, st.par);
-      const int xmn = eo_of_lex(g, st.lex + m1 + n1, st.par), xmmn = eo_of_lex(g, st.lex + mm + n1, st.par);
-      const fx_row a = fx_load_row<false>(fx_mat(U, nu, s, V), r);
-      const int e0 = fx_exp(U, nu, s, V);
-      FxChain p{U, V, {}, e0};
-      p.mul<false>(a, mu, xn);
-      FxChain c = p;  // (c)
-      c.mul<false>(mu, xmn).mul<true>(nu, x2m);
-      fx_add(far, ef, c.v, c.e);
-      FxChain ta{U, V, {}, e0};  // (a)
-      ta.mul<false>(a, nu, xn).mul<false>(mu, x2n).mul<true>(nu, xmn);
-      FxChain te{U, V, {}, fx_exp(U, mu, xmm, V)};  // (e)
-      te.mul<false>(fx_load_row<true>(fx_mat(U, mu, xmm, V), r), nu, xmm).mul<false>(mu, xmmn).mul<false>(mu, xn);
-      FxChain f{U, V, {}, 0};
-      const fx_row w = fx_weighted(p, ta, te, cp, cr, f.e);
-      f.mul<true>(w, nu, xm);
-      fx_add(acc, ea, f.v, f.e);
+      FxChain te{U, V, {}, fx_exp(U, mu, xmm, V)};  // (e), (f)
+      te.mul(fx_load_row<true>(fx_mat(U, mu, xmm, V), r), nu, low ? xmmn : xmm, low);
+      te.mul<false>(mu, xmmn).mul<false>(mu, xn);
+      fx_add(t.v, t.e, te.v, te.e);
     }
+    FxChain p{U, V, {}, e0};
+    p.mul<false>(fx_load_row(first, r, low), mu, xn);
     {
-      const int n1 = fx_steps(g, st, nu, -1), n2 = fx_steps(g, st, nu, -2);
-      const int xn = eo_of_lex(g, st.lex + n1, st.par ^ 1), x2n = eo_of_lex(g, st.lex + n2, st.par);
-      const int xmn = eo_of_lex(g, st.lex + m1 + n1, st.par), xmmn = eo_of_lex(g, st.lex + mm + n1, st.par);
-      const int xm2n = eo_of_lex(g, st.lex + m1 + n2, st.par ^ 1), x2mn = eo_of_lex(g, st.lex + m2 + n1, st.par ^ 1);
-      const fx_row a = fx_load_row<true>(fx_mat(U, nu, xn, V), r);
-      const int e0 = fx_exp(U, nu, xn, V);
-      FxChain p{U, V, {}, e0};
-      p.mul<false>(a, mu, xn);
-      FxChain c = p;  // (d)
-      c.mul<false>(mu, xmn).mul<false>(nu, x2mn);
+      FxChain c = p;  // (c), (d)
+      c.mul<false>(mu, xmn);
+      c.mul(nu, low ? eo_of_lex(g, st.lex + m2 + n1, st.par ^ 1) : x2m, !low);
+      fx_acc far = fx_parked(park);
       fx_add(far, ef, c.v, c.e);
-      FxChain tb{U, V, {}, e0};  // (b)
-      tb.mul<true>(a, nu, x2n).mul<false>(mu, x2n).mul<false>(nu, xm2n);
-      FxChain tf{U, V, {}, fx_exp(U, mu, xmm, V)};  // (f)
-      tf.mul<true>(fx_load_row<true>(fx_mat(U, mu, xmm, V), r), nu, xmmn).mul<false>(mu, xmmn).mul<false>(mu, xn);
-      FxChain f{U, V, {}, 0};
-      const fx_row w = fx_weighted(p, tb, tf, cp, cr, f.e);
-      f.mul<false>(w, nu, xmn);
-      fx_add(acc, ea, f.v, f.e);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        park[2 * j * GF_FX_THREADS] = far.re[j];
+        park[(2 * j + 1) * GF_FX_THREADS] = far.im[j];
+      }
     }
+    FxChain f{U, V, {}, 0};
+    const fx_row w = fx_weighted(p, t, cp, cr, f.e);
+    f.mul(w, nu, low ? xmn : xm, !low);
+    fx_add(acc, ea, f.v, f.e);
   }
+  fx_acc far = fx_parked(park);
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
     far.re[j] >>= 3;
@@ -182,9 +240,10 @@ __device__ __forceinline__ fx_acc fx_loops_row(const FxField& U, const Geom& g, 
   return acc;
 }
 
-// P <- keep P + c(U (cp S + cr R)), or (DSDU) D = cp S + cr R
+// P <- keep P + c(U (cp S + cr R)), or (DSDU) D = cp S + cr R. Four blocks per
+// SM (168 registers): 3.30 ms at 24^4, five 3.36, six 3.81.
 #ifndef GF_FX_LOOPS_MINB
-#define GF_FX_LOOPS_MINB 5
+#define GF_FX_LOOPS_MINB 4
 #endif
 template <bool DSDU>
 __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_LOOPS_MINB)
@@ -194,13 +253,14 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_LOOPS_MINB)
     FxRaw m;
     float n[3][GF_FX_LINKS];
   } sh;
+  __shared__ i64 park[6][GF_FX_THREADS];
   __shared__ int se[GF_FX_LINKS];
   const int t = threadIdx.x, mu = blockIdx.x & 3, V = g.vol;
   const int link = t / 3, r = t - 3 * link, s0 = (blockIdx.x >> 2) * GF_FX_LINKS;
   const int sx = s0 + link, s = min(sx, V - 1);
   const Site st = site_of(g, s);
   int ea;
-  fx_acc a = fx_loops_row(U, g, st, s, mu, r, cp, cr, ea);
+  fx_acc a = fx_loops_row(U, g, st, s, mu, r, cp, cr, ea, park[0] + t);
   if (DSDU) {
     sh.n[r][link] = fx_square(a);
     __syncthreads();

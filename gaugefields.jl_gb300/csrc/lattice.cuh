@@ -77,8 +77,7 @@ GF_HD int nbr2(const Geom& g, const Site& st, int d0, int d1) {
 
 // Minimum resident blocks per SM requested for the stencil kernels (register
 // budget 65536 / (128 threads * min blocks)): fp32 and double-float kernels are
-// latency-bound and gain from occupancy; fp64 kernels are fp64-issue-bound and
-// keep the full register file.
+// latency-bound and gain from occupancy.
 #ifndef GF_FP32_MINB
 #define GF_FP32_MINB 4
 #endif

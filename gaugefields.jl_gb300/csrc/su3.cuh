@@ -244,24 +244,6 @@ GF_HD void ta_coeffs(const mat3<R>& m, R c[8]) {
   c[7] = sr3i * (d1 + d2 - R(2) * d3);
 }
 
-// Hermitian matrix Q = sum_a p_a lambda_a / 2 (Gell-Mann basis).
-template <typename R>
-GF_HD mat3<R> herm_from_coeffs(const R p[8]) {
-  constexpr R sr3i = R(0.57735026918962576451);
-  constexpr R h = R(0.5), two = R(2.0);
-  mat3<R> q;
-  q.e[0][0] = mk<R>(h * (p[2] + sr3i * p[7]), R(0));
-  q.e[1][1] = mk<R>(h * (-p[2] + sr3i * p[7]), R(0));
-  q.e[2][2] = mk<R>(-h * two * sr3i * p[7], R(0));
-  q.e[0][1] = mk<R>(h * p[0], -h * p[1]);
-  q.e[1][0] = mk<R>(h * p[0], h * p[1]);
-  q.e[0][2] = mk<R>(h * p[3], -h * p[4]);
-  q.e[2][0] = mk<R>(h * p[3], h * p[4]);
-  q.e[1][2] = mk<R>(h * p[5], -h * p[6]);
-  q.e[2][1] = mk<R>(h * p[5], h * p[6]);
-  return q;
-}
-
 // Third row of an SU(3) matrix from its first two rows: row3 = conj(row1 x row2)
 // (m3complv3! of src/AbstractGaugefields.jl:3431).
 template <typename R>
