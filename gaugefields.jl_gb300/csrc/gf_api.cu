@@ -473,7 +473,8 @@ static gf_stout* stout_new(gf_ctx* ctx, int nlev, const double* rho, int precisi
     } else {
       st->Z = field_pooled(ctx, mk);
       st->Dp = field_pooled(ctx, mk);
-      st->D[0] = field_pooled(ctx, mk);
+      // a fixed-point level's gather writes D after the level's local kernel has read it: one buffer
+      if (mk != GF_MATFX) st->D[0] = field_pooled(ctx, mk);
       st->D[1] = field_pooled(ctx, mk);
     }
   } catch (...) {
@@ -711,7 +712,8 @@ static MDResult md_run(gf_ctx* ctx, gf_field* U, gf_field* P, const gf_md_params
     U32 = ctx->w_link32;
     link64_to_32(ctx, U32, U);
   }
-  if (keeps_fx(ctx, p)) Ufx = fx_links(ctx, U);
+  const FxHold hold(ctx);
+  if (keeps_fx(ctx, p)) Ufx = fx_links(ctx, U);  // null: no memory for it
   const gf_field* Ucopy = U32 ? U32 : Ufx;
   const gf_field* Upot = Ufx ? Ufx : U;  // the potential never takes the fp32 links
   MDResult r;
@@ -930,14 +932,16 @@ static void flow_steps(gf_ctx* ctx, gf_field* U, double eps, int nsteps, bool df
   gf_field* G = ctx->w_mom[0];
   const double c0 = 17.0 * eps / 36.0;
   if (nsteps == 0) return;
-  gf_field* F = fx_links(ctx, U);  // the fixed-point copy of U, W1, W2 in turn, written by their updates
+  // the fixed-point copy of U, W1, W2 in turn, written by their updates (null: no memory for it)
+  const FxHold hold(ctx);
+  gf_field* F = fx_links(ctx, U);
   for (int n = 0; n < nsteps; ++n) {
-    flow_force(ctx, F, G, c0, 0.0, df);                // G = 17eps/36 F0
-    exp_mom_links(ctx, W1, G, -9.0 / 17.0, U, df, F);  // W1 = exp(-eps/4 F0) U
-    flow_force(ctx, F, G, -8.0 * eps / 9.0, 1.0, df);  // G = 17eps/36 F0 - 8eps/9 F1
-    exp_mom_links(ctx, W2, G, 1.0, W1, df, F);         // W2 = exp(G) W1
-    flow_force(ctx, F, G, -0.75 * eps, -1.0, df);      // G = -G - 3eps/4 F2
-    exp_mom_links(ctx, U, G, 1.0, W2, df, F);          // U = exp(G) W2
+    flow_force(ctx, F ? F : U, G, c0, 0.0, df);                 // G = 17eps/36 F0
+    exp_mom_links(ctx, W1, G, -9.0 / 17.0, U, df, F);           // W1 = exp(-eps/4 F0) U
+    flow_force(ctx, F ? F : W1, G, -8.0 * eps / 9.0, 1.0, df);  // G = 17eps/36 F0 - 8eps/9 F1
+    exp_mom_links(ctx, W2, G, 1.0, W1, df, F);                  // W2 = exp(G) W1
+    flow_force(ctx, F ? F : W2, G, -0.75 * eps, -1.0, df);      // G = -G - 3eps/4 F2
+    exp_mom_links(ctx, U, G, 1.0, W2, df, F);                   // U = exp(G) W2
   }
 }
 
@@ -976,13 +980,14 @@ extern "C" int gf_flow_loops(gf_ctx* ctx, gf_field* U, double eps, int nsteps, d
   const double c0 = 17.0 * eps / 36.0;
   const double c1 = -8.0 * eps / 9.0;
   const double c2 = -0.75 * eps;
+  const FxHold hold(ctx);
   gf_field* F = nsteps ? fx_links(ctx, U) : nullptr;  // of U, W1, W2 in turn
   for (int n = 0; n < nsteps; ++n) {
-    loops_force_coef(ctx, F, G, c0 * c_plaq, c0 * c_rect, 0.0);   // G = 17eps/36 F0
+    loops_force_coef(ctx, F ? F : U, G, c0 * c_plaq, c0 * c_rect, 0.0);  // G = 17eps/36 F0
     exp_mom_links(ctx, W1, G, -9.0 / 17.0, U, false, F);         // W1 = exp(-eps/4 F0) U
-    loops_force_coef(ctx, F, G, c1 * c_plaq, c1 * c_rect, 1.0);   // G += -8eps/9 F1
+    loops_force_coef(ctx, F ? F : W1, G, c1 * c_plaq, c1 * c_rect, 1.0);  // G += -8eps/9 F1
     exp_mom_links(ctx, W2, G, 1.0, W1, false, F);                // W2 = exp(G) W1
-    loops_force_coef(ctx, F, G, c2 * c_plaq, c2 * c_rect, -1.0);  // G = -G - 3eps/4 F2
+    loops_force_coef(ctx, F ? F : W2, G, c2 * c_plaq, c2 * c_rect, -1.0);  // G = -G - 3eps/4 F2
     exp_mom_links(ctx, U, G, 1.0, W2, false, F);                 // U = exp(G) W2
   }
   API_END(ctx)

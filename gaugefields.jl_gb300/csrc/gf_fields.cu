@@ -38,7 +38,8 @@ void pool_trim(gf_pool* pool, bool close) {
   for (auto& k : kept) cudaFree(k.second);
 }
 
-// cudaMalloc, once more after the pool has given back what it keeps
+// cudaMalloc, once more after the pool, and then the fixed-point copy of the
+// links, have given back what they keep
 static void* device_alloc(gf_ctx* ctx, size_t bytes) {
   void* p = nullptr;
   cudaError_t e = cudaMalloc(&p, bytes);
@@ -46,6 +47,12 @@ static void* device_alloc(gf_ctx* ctx, size_t bytes) {
     cudaGetLastError();
     pool_trim(ctx->pool.get(), false);
     e = cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation && ctx->w_linkfx && !ctx->fx_hold) {
+      cudaGetLastError();
+      field_delete(ctx->w_linkfx);  // cudaFree waits for the kernels that read it
+      ctx->w_linkfx = nullptr;
+      e = cudaMalloc(&p, bytes);
+    }
   }
   if (e != cudaSuccess) {
     cudaGetLastError();

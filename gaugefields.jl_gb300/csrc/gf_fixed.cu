@@ -132,7 +132,14 @@ __global__ void __launch_bounds__(GF_FX_THREADS * AXES, AXES > 1 ? 2 : GF_FX_MIN
 }
 
 gf_field* fx_links(gf_ctx* ctx, const gf_field* U) {
-  if (!ctx->w_linkfx) ctx->w_linkfx = field_new(ctx, GF_LINKFX);
+  if (!ctx->w_linkfx) {
+    try {
+      ctx->w_linkfx = field_new(ctx, GF_LINKFX);
+    } catch (const gf_error& e) {
+      if (e.code != GF_ENOMEM) throw;
+      return nullptr;
+    }
+  }
   to_fx(ctx, ctx->w_linkfx, U);
   return ctx->w_linkfx;
 }

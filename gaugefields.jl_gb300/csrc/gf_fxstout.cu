@@ -443,7 +443,6 @@ void stout_backward_fx(gf_ctx* ctx, gf_stout* st, const gf_field* dSdUbar, doubl
                        double eps, double* dsdrho) {
   const int nb = 4 * blocks_for(ctx->geom.vol, GF_FX_LINKS);
   if (dSdUbar && dSdUbar != st->D[1]) copy_field(ctx, st->D[1], dSdUbar);
-  int cur = 1;
   for (int l = st->nlev - 1; l >= 0; --l) {
     const bool top = (l == st->nlev - 1) && dSdUbar == nullptr;
     {
@@ -454,14 +453,13 @@ void stout_backward_fx(gf_ctx* ctx, gf_stout* st, const gf_field* dSdUbar, doubl
                             : (top ? k_bwd_local_fx<true, true> : k_bwd_local_fx<false, true>);
       GF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       kern<<<nb, GF_FX_THREADS, smem, ctx->stream>>>(fx_view(st->lev_in[l]),
-                                                     fx_view(top ? st->lev_in[l + 1] : st->D[cur]), C,
+                                                     fx_view(top ? st->lev_in[l + 1] : st->D[1]), C,
                                                      (char*)st->Z->ptr, (char*)st->Dp->ptr, ctx->geom,
                                                      fx_scalar_of(st->rho[l]), fx_scalar_of(1.0), third_of(1.0),
                                                      fx_scalar_of(0.5 * beta));
       GF_CHECK_LAUNCH();
     }
     if (dsdrho) dsdrho[l] = level_dsdrho(ctx, st, l);
-    const int nxt = cur ^ 1;
     ProfScope prof(ctx, GF_K_BWD_GATHER64);
     const FxField u = fx_view(st->lev_in[l]), z = fx_view(st->Z), dp = fx_view(st->Dp);
     const fx_scalar rho = fx_scalar_of(st->rho[l]);
@@ -475,9 +473,8 @@ void stout_backward_fx(gf_ctx* ctx, gf_stout* st, const gf_field* dSdUbar, doubl
           u, z, dp, (char*)dSdU->ptr, nullptr, ctx->geom, rho, 0.0);
     else
       (split ? k_bwd_gather_fx<0, 3> : k_bwd_gather_fx<0, 1>)<<<nb, nt, 0, ctx->stream>>>(
-          u, z, dp, (char*)st->D[nxt]->ptr, nullptr, ctx->geom, rho, 0.0);
+          u, z, dp, (char*)st->D[1]->ptr, nullptr, ctx->geom, rho, 0.0);
     GF_CHECK_LAUNCH();
-    cur = nxt;
   }
 }
 

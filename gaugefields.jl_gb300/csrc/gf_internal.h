@@ -92,6 +92,7 @@ struct gf_ctx {
   gf_field* w_mom[4];     // F0, F1, F2, Ftmp of the RK3 flow (fp64 coefficients)
   gf_field* w_link32;     // fp32 12-real shadow of the thin links (mixed form)
   gf_field* w_linkfx;     // fixed-point copy of the links (fp64-class kernels)
+  int fx_hold;            // drivers that keep w_linkfx across other calls (FxHold)
   // Two scratch blocks of one fp64 link field each, shared by the mixed form's
   // internal stacks: the Hamiltonian's double-float level buffers and the
   // force adjoint's Z, Dp, D[0], D[1] (fp32). They are never live together:
@@ -212,15 +213,23 @@ void staple_up(gf_ctx* ctx, const gf_field* U, int mu, gf_field* V);  // constru
 // staples (dS/dU order); keep = 0 overwrites P without reading it.
 void wilson_force_coef(gf_ctx* ctx, const gf_field* U, gf_field* P, double coef, double keep, bool df = false);
 
-// the same on a fixed-point copy of the links (gf_fixed.cu)
+// the same on fixed-point links (gf_fixed.cu)
 void wilson_force_fx(gf_ctx* ctx, const gf_field* F, gf_field* P, double coef, double keep);
-
-void plaquette_start_fx(gf_ctx* ctx, const gf_field* F, int slot);  // of a fixed-point field
+void plaquette_start_fx(gf_ctx* ctx, const gf_field* F, int slot);
 // the sum into slot `slot` of h_result: LINK64, fixed-point or double-float links
 void plaquette_start(gf_ctx* ctx, const gf_field* U, int slot);
 inline FxField fx_view(const gf_field* f) { return FxField{(const char*)f->ptr}; }
-// the context's fixed-point copy of fp64 or double-float links
+// the context's fixed-point copy of fp64 or double-float links, made anew;
+// null when there is no memory for it, and the
+// fp64 kernels, a fifth as fast, read the links in place. Another allocation of
+// the context that finds none may take it back, but not while a driver holds it.
 gf_field* fx_links(gf_ctx* ctx, const gf_field* U);
+struct FxHold {
+  gf_ctx* ctx;
+  explicit FxHold(gf_ctx* c) : ctx(c) { ++ctx->fx_hold; }
+  FxHold(const FxHold&) = delete;
+  ~FxHold() { --ctx->fx_hold; }
+};
 // LINK64 / MAT64 or double-float pairs -> fixed point, and fixed point -> fp64
 void to_fx(gf_ctx* ctx, gf_field* dst, const gf_field* src);
 void fx_to_f64_field(gf_ctx* ctx, gf_field* dst, const gf_field* src);

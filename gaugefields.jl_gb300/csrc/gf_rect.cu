@@ -37,6 +37,29 @@ __device__ __forceinline__ int site_off(const Geom& g, const Site& st, int mu, i
   return eo_of_lex(g, lex, st.par ^ ((a + b) & 1));
 }
 
+// Sum over mu < nu of Re tr (R^{1x2}_{mu nu}(x) + R^{2x1}_{mu nu}(x)), one
+// partial per block, each rectangle as Re tr(A B^+) of its two halves:
+// U_mu(x) U_nu(x+mu) U_nu(x+mu+nu) and U_nu(x) U_nu(x+nu) U_mu(x+2nu), the 2x1
+// one as the 1x2 one of the other orientation, reversed.
+template <class SRC>
+__global__ void __launch_bounds__(128) k_rect_sum(SRC U, Geom g, SumOut to) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x, V = g.vol;
+  double v = 0.0;
+  if (s < V) {
+    const Site st = site_of(g, s);
+#pragma unroll 1
+    for (int p = 0; p < 12; ++p) {
+      const int mu = p & 3, nu = (mu + 1 + (p >> 2)) & 3;
+      mat3<double> a = mul_nn(U(mu, s, V), U(nu, site_off(g, st, mu, 1, nu, 0), V));
+      a = mul_nn(a, U(nu, site_off(g, st, mu, 1, nu, 1), V));
+      mat3<double> b = mul_nn(U(nu, s, V), U(nu, site_off(g, st, mu, 0, nu, 1), V));
+      b = mul_nn(b, U(mu, site_off(g, st, mu, 0, nu, 2), V));
+      v += retr_na(a, b);
+    }
+  }
+  block_sum(v, to);
+}
+
 // acc += the six rectangle staples (a)-(f) of U_mu(x) in the mu-nu plane
 template <typename R, class SRC>
 __device__ __forceinline__ void add_rect_staples(mat3<R>& acc, const SRC& U, const Geom& g, const Site& st, int s,
@@ -228,10 +251,23 @@ static void rect_df(gf_ctx* ctx, const float4* U, gf_field* D, double cp, double
 }
 
 void rectangle_start(gf_ctx* ctx, const gf_field* U, int slot) {
-  // fp64 links, and the top level of a double-float stack, through a fixed-point copy
   if (U->kind != GF_LINKFX && U->kind != GF_LINK64 && U->kind != GF_MAT64 && U->kind != GF_LINKDF)
     throw gf_error(GF_EINVAL, "rectangle: links must be LINK64");
-  rectangle_start_fx(ctx, U->kind == GF_LINKFX ? U : fx_links(ctx, U), slot);
+  // fp64 links, and the top level of a double-float stack, through a fixed-point copy
+  const gf_field* F = U->kind == GF_LINKFX ? U : fx_links(ctx, U);
+  if (F) {
+    rectangle_start_fx(ctx, F, slot);
+    return;
+  }
+  const int nb = blocks_for(ctx->geom.vol, 128);
+  const SumOut to = sum_out(ctx, nb, 128, slot);
+  ProfScope prof(ctx, GF_K_RECT);
+  if (U->kind == GF_LINKDF)
+    k_rect_sum<<<nb, 128, 0, ctx->stream>>>(LinkSrcDfn64{(const float4*)U->ptr}, ctx->geom, to);
+  else
+    k_rect_sum<<<nb, 128, 0, ctx->stream>>>(LinkSrc<double, false>{(const double2*)U->ptr}, ctx->geom, to);
+  GF_CHECK_LAUNCH();
+  sum_finish(ctx, to, nb, slot);
 }
 
 double rectangle_sum(gf_ctx* ctx, const gf_field* U) {
@@ -245,9 +281,18 @@ void loops_force_coef(gf_ctx* ctx, const gf_field* U, gf_field* P, double cp, do
   if (df && U->kind != GF_LINK64 && U->kind != GF_LINKFX)
     throw gf_error(GF_EINVAL, "force: the double-float rectangle force takes LINK64 links");
   if (U->kind == GF_LINK64 || U->kind == GF_MAT64 || U->kind == GF_LINKFX) {
-    if (cr == 0.0) wilson_force_coef(ctx, U, P, cp, keep);
-    else loops_fx(ctx, U->kind == GF_LINKFX ? U : fx_links(ctx, U), P, nullptr, cp, cr, keep);
-    return;
+    if (cr == 0.0 && U->kind != GF_MAT64) {
+      wilson_force_coef(ctx, U, P, cp, keep);
+      return;
+    }
+    const gf_field* F = U->kind == GF_LINKFX ? U : fx_links(ctx, U);
+    if (F) {
+      loops_fx(ctx, F, P, nullptr, cp, cr, keep);
+      return;
+    }
+    ProfScope prof(ctx, GF_K_RECT);
+    k_force_rect<double><<<grid, 128, 0, ctx->stream>>>(LinkSrc<double, false>{(const double2*)U->ptr}, (double*)P->ptr,
+                                                        ctx->geom, cp, cr, keep);
   } else if (U->kind == GF_LINK32) {
     ProfScope prof(ctx, GF_K_RECT);
     k_force_rect<float><<<grid, 128, 0, ctx->stream>>>(LinkSrc<float, true>{(const float4*)U->ptr}, (double*)P->ptr,

@@ -14,34 +14,42 @@ typedef LinkSrc<float, true> Src32;
 // Per-site plaquette sum, one partial per block (calculate_Plaquette,
 // src/AbstractGaugefields.jl:2684-2699, evaluated plaquette by plaquette).
 template <typename R, class SRC>
-__global__ void __launch_bounds__(128, GF_MINB(R)) k_plaquette(SRC U, Geom g, double* __restrict__ part) {
+__global__ void __launch_bounds__(128, GF_MINB(R)) k_plaquette(SRC U, Geom g, SumOut to) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   double v = 0.0;
   if (s < g.vol) {
     Site st = site_of(g, s);
     v = (double)plaq_site<R>(U, g, st, s);
   }
-  block_partial_sum(v, part);
+  block_sum(v, to);
 }
 
 void plaquette_start(gf_ctx* ctx, const gf_field* U, int slot) {
+  if (U->kind != GF_LINK64 && U->kind != GF_MAT64 && U->kind != GF_LINKDF && U->kind != GF_LINKFX &&
+      U->kind != GF_LINK32)
+    throw gf_error(GF_EINVAL, "plaquette: links must be LINK64 or LINK32");
   ProfScope prof(ctx, GF_K_PLAQ);
   // fp64 links, and the top level of a double-float stack, through a fixed-point copy
-  plaquette_start_fx(ctx, U->kind == GF_LINKFX ? U : fx_links(ctx, U), slot);
+  const gf_field* F = U->kind == GF_LINKFX ? U : (U->kind == GF_LINK32 ? nullptr : fx_links(ctx, U));
+  if (F) {
+    plaquette_start_fx(ctx, F, slot);
+    return;
+  }
+  const int nb = blocks_for(ctx->geom.vol, 128);
+  const SumOut to = sum_out(ctx, nb, 128, slot);
+  if (U->kind == GF_LINK32)
+    k_plaquette<float><<<nb, 128, 0, ctx->stream>>>(Src32{(const float4*)U->ptr}, ctx->geom, to);
+  else if (U->kind == GF_LINKDF)
+    k_plaquette<double><<<nb, 128, 0, ctx->stream>>>(LinkSrcDfn64{(const float4*)U->ptr}, ctx->geom, to);
+  else
+    k_plaquette<double><<<nb, 128, 0, ctx->stream>>>(Src64{(const double2*)U->ptr}, ctx->geom, to);
+  GF_CHECK_LAUNCH();
+  sum_finish(ctx, to, nb, slot);
 }
 
 double plaquette_sum(gf_ctx* ctx, const gf_field* U) {
-  if (U->kind == GF_LINK64 || U->kind == GF_MAT64 || U->kind == GF_LINKDF || U->kind == GF_LINKFX) {
-    plaquette_start(ctx, U, 0);
-    return sum_wait(ctx, 0);
-  }
-  if (U->kind != GF_LINK32) throw gf_error(GF_EINVAL, "plaquette: links must be LINK64 or LINK32");
-  const int nb = blocks_for(ctx->geom.vol, 128);
-  ProfScope prof(ctx, GF_K_PLAQ);
-  Src32 src{(const float4*)U->ptr};
-  k_plaquette<float><<<nb, 128, 0, ctx->stream>>>(src, ctx->geom, ctx->d_partials);
-  GF_CHECK_LAUNCH();
-  return finish_reduction(ctx, nb);
+  plaquette_start(ctx, U, 0);
+  return sum_wait(ctx, 0);
 }
 
 // Polyakov loop (calculate_Polyakov_loop, src/AbstractGaugefields.jl:
@@ -138,12 +146,14 @@ void wilson_force_coef(gf_ctx* ctx, const gf_field* U, gf_field* P, double coef,
   ProfScope prof(ctx, df ? GF_K_FORCE_DF : GF_K_FORCE);
   if (df && U->kind != GF_LINK64 && U->kind != GF_LINKFX) {
     throw gf_error(GF_EINVAL, "force: the double-float force needs LINK64 links");
-  } else if (U->kind == GF_LINK64) {
-    wilson_force_fx(ctx, fx_links(ctx, U), P, coef, keep);
-    return;
-  } else if (U->kind == GF_LINKFX) {
-    wilson_force_fx(ctx, U, P, coef, keep);
-    return;
+  } else if (U->kind == GF_LINK64 || U->kind == GF_LINKFX) {
+    const gf_field* F = U->kind == GF_LINKFX ? U : fx_links(ctx, U);
+    if (F) {
+      wilson_force_fx(ctx, F, P, coef, keep);
+      return;
+    }
+    k_force_ta<double><<<grid, 128, 0, ctx->stream>>>(Src64{(const double2*)U->ptr}, (double*)P->ptr, ctx->geom, coef,
+                                                      keep);
   } else if (U->kind == GF_LINK32) {
     Src32 src{(const float4*)U->ptr};
     k_force_ta<float><<<grid, 128, 0, ctx->stream>>>(src, (double*)P->ptr, ctx->geom, coef, keep);

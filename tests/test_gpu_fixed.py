@@ -6,6 +6,8 @@ over many orders of magnitude), and a NaN.
 Tolerances: 1e-13 of the largest entry, two orders above fp64 rounding of the
 sums involved (the oracle's own).
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -325,3 +327,63 @@ def test_double_float_adjoint_of_large_lattices(pkg):
         drho.append(pkg.get_parameter_derivatives(D, net, U, precision)[0])
     assert np.linalg.norm(grad[1] - grad[0]) <= 1e-11 * np.linalg.norm(grad[0])
     assert abs(drho[1] - drho[0]) <= 1e-11 * 4 * V
+
+
+def test_without_memory_for_the_copy(pkg):
+    """The fixed-point copy of the links is what goes when memory is short: a
+    field takes its place, and the calls that made it read the links as they
+    are, in fp64 or (the mixed form's energy) double-float storage. The same
+    numbers to 1e-13, and the copy is back when there is memory again."""
+    from gaugefields_gb300 import _lib
+    torch = pytest.importorskip("torch")
+    U = pkg.gauge_configuration((24, 24, 24, 24), start="hot", seed=11)
+    V, P = U.similar(), pkg.gauge_momenta(U)
+    P0 = pkg.gaussian_momenta(U, seed=3)
+    wilson, loops = pkg.GaugeAction(U), pkg.GaugeAction(U)
+    pkg.push_(wilson, 3.0, "plaquette")
+    pkg.push_(loops, 3.0, "plaquette")
+    pkg.push_(loops, -0.1, "rectangular")
+    net = pkg.CovNeuralnet(U)
+    pkg.push_(net, pkg.STOUT_Layer("plaquette", 0.1))
+    smeared = pkg.md_driver(U, loops, steps=1, smearing=net, precision="mixed")
+
+    def launches():
+        n = ctypes.c_longlong()
+        _lib.check(_lib.load().gf_launch_count(ctypes.byref(n)))
+        return n.value
+
+    def numbers():
+        out = [pkg.calculate_Plaquette(U), pkg.rectangle_sum(U), pkg.md_hamiltonian(U, P0, smeared)]
+        for action in (wilson, loops):
+            pkg.md_force_(P, action, U)
+            out.append(P.to_host())
+        pkg.substitute_U_(V, U)
+        P.from_host(P0.to_host())
+        r = pkg.md_trajectory_(V, P, pkg.md_driver(U, wilson, steps=1, trajectory_length=0.1))
+        out += [V.to_host(), P.to_host(), r.initial_hamiltonian, r.final_hamiltonian]
+        pkg.substitute_U_(V, U)
+        pkg.flow_(V, pkg.gradient_flow(V, steps=1, step_size=0.01))
+        out.append(V.to_host())
+        return out
+
+    def plaquette_launches():
+        before = launches()
+        pkg.calculate_Plaquette(U)
+        return launches() - before
+
+    ref = numbers()
+    usual = plaquette_launches()
+    size = 4 * 24 ** 4 * 144
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - size // 2, dtype=torch.uint8, device="cuda")
+    try:
+        W = U.similar()  # takes the copy's place
+        assert plaquette_launches() == usual - 1  # no conversion before the sum
+        got = numbers()
+        del W
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    for a, b in zip(got, ref):
+        close(np.asarray(a), np.asarray(b))
+    for a, b in zip(numbers(), ref):
+        assert np.array_equal(np.asarray(a), np.asarray(b))
