@@ -489,7 +489,17 @@ extern "C" int gf_stout_create(gf_ctx* ctx, int nlev, const double* rho, int pre
   need(ctx && rho && out, "gf_stout_create: null argument");
   need(precision == GF_FP64 || precision == GF_MIXED || precision == GF_DFLOAT,
        "gf_stout_create: precision must be GF_FP64, GF_MIXED or GF_DFLOAT");
-  *out = stout_new(ctx, nlev, rho, precision, store);
+  gf_stout* st = stout_new(ctx, nlev, rho, precision, store);
+  if (st->precision == GF_FP64) {
+    // the level-0 copy at once: forward passes then allocate nothing
+    try {
+      st->lev_in[0] = field_pooled(ctx, GF_LINKFX);
+    } catch (...) {
+      gf_stout_destroy(st);
+      throw;
+    }
+  }
+  *out = st;
   API_END(ctx)
 }
 

@@ -47,7 +47,7 @@ static void* device_alloc(gf_ctx* ctx, size_t bytes) {
     cudaGetLastError();
     pool_trim(ctx->pool.get(), false);
     e = cudaMalloc(&p, bytes);
-    if (e == cudaErrorMemoryAllocation && ctx->w_linkfx && !ctx->fx_hold) {
+    if (e == cudaErrorMemoryAllocation && ctx->w_linkfx && !ctx->fx_hold && !ctx->fx_graph) {
       cudaGetLastError();
       field_delete(ctx->w_linkfx);  // cudaFree waits for the kernels that read it
       ctx->w_linkfx = nullptr;

@@ -93,6 +93,7 @@ struct gf_ctx {
   gf_field* w_link32;     // fp32 12-real shadow of the thin links (mixed form)
   gf_field* w_linkfx;     // fixed-point copy of the links (fp64-class kernels)
   int fx_hold;            // drivers that keep w_linkfx across other calls (FxHold)
+  int fx_graph;           // 1: a captured graph uses w_linkfx
   // Two scratch blocks of one fp64 link field each, shared by the mixed form's
   // internal stacks: the Hamiltonian's double-float level buffers and the
   // force adjoint's Z, Dp, D[0], D[1] (fp32). They are never live together:
@@ -219,10 +220,11 @@ void plaquette_start_fx(gf_ctx* ctx, const gf_field* F, int slot);
 // the sum into slot `slot` of h_result: LINK64, fixed-point or double-float links
 void plaquette_start(gf_ctx* ctx, const gf_field* U, int slot);
 inline FxField fx_view(const gf_field* f) { return FxField{(const char*)f->ptr}; }
-// the context's fixed-point copy of fp64 or double-float links, made anew;
-// null when there is no memory for it, and the
-// fp64 kernels, a fifth as fast, read the links in place. Another allocation of
-// the context that finds none may take it back, but not while a driver holds it.
+// the context's fixed-point copy of fp64 or double-float links, made anew; null
+// when there is no memory for it (or a graph is being captured and there is
+// none yet): the fp64 kernels, a fifth as fast, then read the links in place.
+// An allocation of the context that fails takes it back, but not while a
+// driver holds it or once a graph has captured it.
 gf_field* fx_links(gf_ctx* ctx, const gf_field* U);
 struct FxHold {
   gf_ctx* ctx;

@@ -387,3 +387,42 @@ def test_without_memory_for_the_copy(pkg):
         close(np.asarray(a), np.asarray(b))
     for a, b in zip(numbers(), ref):
         assert np.array_equal(np.asarray(a), np.asarray(b))
+
+
+@pytest.mark.parametrize("warm", [False, True])
+def test_forces_and_smearing_in_a_graph(pkg, warm):
+    """Calls that read nothing back can be captured, with the fixed-point copy
+    in place or (lattices whose copy a first call allocates) without one, and a
+    replay follows the links."""
+    from gaugefields_gb300 import _lib
+    from gaugefields_gb300.api import _StoutStack
+    torch = pytest.importorskip("torch")
+    L = (16, 16, 16, 16)
+    U = pkg.gauge_configuration(L, start="hot", seed=5)
+    W = pkg.gauge_configuration(L, start="hot", seed=6)
+    wilson = pkg.GaugeAction(U)
+    pkg.push_(wilson, 3.0, "plaquette")
+    stack, top, F = _StoutStack(U.ctx, [0.1], "fp64"), U.similar(), pkg.gauge_momenta(U)
+    host = W.to_host()
+
+    def calls():
+        pkg.md_force_(F, wilson, U)
+        _lib.check(_lib.load().gf_stout_forward(U.ctx.h, stack.h, U.field.h, top.field.h), U.ctx.h)
+
+    stream = torch.cuda.Stream()
+    U.ctx.set_stream(stream.cuda_stream)
+    U.ctx.torch_stream = stream  # alive as long as the context
+    if warm:
+        calls()
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        calls()
+    U.from_host(host)
+    torch.cuda.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    got = F.to_host(), top.to_host()
+    calls()
+    close(got[0], F.to_host())
+    close(got[1], top.to_host())
