@@ -460,13 +460,17 @@ GF_HD bool fx_exponent_of(const double* m /* 18, row-major, re im */, int& emax,
 // One matrix to fixed point; returns its exponent.
 GF_HD int fx_from_f64(const double* m, int4 out[9]) {
   int emax, up;
-  const bool ok = fx_exponent_of(m, emax, up);
+  if (!fx_exponent_of(m, emax, up)) {
+#pragma unroll
+    for (int i = 0; i < 9; ++i) out[i] = make_int4(0, 0, 0, 0);
+    return GF_FX_BAD;
+  }
 #pragma unroll
   for (int i = 0; i < 9; ++i) {
-    fx_split<0>(ok ? fx_mantissa(m[2 * i], emax, up) : 0, out[i].x, out[i].y);
-    fx_split<0>(ok ? fx_mantissa(m[2 * i + 1], emax, up) : 0, out[i].z, out[i].w);
+    fx_split<0>(fx_mantissa(m[2 * i], emax, up), out[i].x, out[i].y);
+    fx_split<0>(fx_mantissa(m[2 * i + 1], emax, up), out[i].z, out[i].w);
   }
-  return ok ? emax - 1023 + up : GF_FX_BAD;
+  return emax - 1023 + up;
 }
 
 // real and imaginary parts of the f_j, side by side: f at [2 j + im]

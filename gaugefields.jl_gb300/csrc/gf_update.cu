@@ -409,13 +409,15 @@ __global__ void __launch_bounds__(GF_FX_THREADS, 4)
   if (fx && r == 0) fx_store_exp(fx, off, s, ef);
 }
 
-// Sites up to which the update itself writes the fixed-point copy. It saves a
-// launch and the copy's pass over the links (8^4 trajectory of 20 steps, a
-// thread per link, 784 -> 718 us, 24^4 of 10 steps 11.22 -> 11.13 ms), but in registers it costs the
-// update more than the bandwidth-bound copy kernel once that runs at full rate
-// (32^4 flow, 2 steps: 18.64 against 18.41 ms).
-#ifndef GF_FX_FUSE_MAX
-#define GF_FX_FUSE_MAX (1 << 19)
+// The update writes the fixed-point copy itself: a launch and the copy's pass
+// over the links less. A copy kernel after it against this one: trajectories
+// 8^4 (10 steps) 445 / 389 us, 16^4 2.37 / 2.31 ms, 24^4 11.25 / 10.92, 40^4 (2
+// steps) 22.0 / 21.6. Without re-unitarisation (flows) the copy needs the
+// bound of its exponent, for which this kernel has no registers left: 8^4 (3 steps)
+// 284 / 247 us, 12^4 742 / 706, 16^4 1.86 / 1.85 ms, but on 166,320 sites (5
+// steps) 7.17 / 7.25, 32^4 (2 steps) 18.52 / 18.62.
+#ifndef GF_FX_FUSE_PLAIN_MAX
+#define GF_FX_FUSE_PLAIN_MAX (1 << 16)
 #endif
 // Sites up to which a link gets a warp lane in each of three warps. Trajectory
 // of 20 steps (without re-unitarisation, flow of 5 steps), a thread per link
@@ -429,7 +431,7 @@ __global__ void __launch_bounds__(GF_FX_THREADS, 4)
 static void update_links(gf_ctx* ctx, gf_field* W, const gf_field* P, double eps, const gf_field* U, int reunit,
                          gf_field* shadow32, gf_field* fx) {
   const int V = ctx->geom.vol;
-  const bool fused = V <= GF_FX_FUSE_MAX, rows = V <= GF_FX_ROWS_MAX;
+  const bool rows = V <= GF_FX_ROWS_MAX, fused = reunit || V <= GF_FX_FUSE_PLAIN_MAX;
   const int threads = rows ? GF_FX_THREADS : 128;
   dim3 grid(blocks_for(V, rows ? GF_FX_LINKS : 128), 4);
   auto kern = rows ? (reunit ? k_link_update_rows_fx<true> : k_link_update_rows_fx<false>)
