@@ -615,6 +615,15 @@ static void potential_start(gf_ctx* ctx, const gf_field* U, const gf_md_params* 
     gf_stout* st = ctx_stout(ctx, p, df ? GF_PREC_DF : GF_FP64);
     stout_forward(ctx, st, U, nullptr);
     links = stout_top(st);
+    if (st->fwd_only) {
+      // the levels take the two scratch blocks in turn: the top's copy goes to the other one
+      gf_field* F = arena_view(ctx, p->nstout & 1, 0, GF_LINKFX);
+      to_fx(ctx, F, links);
+      plaquette_start(ctx, F, 0);
+      if (p->c_rect != 0.0) rectangle_start(ctx, F, 1);
+      field_delete(F);
+      return;
+    }
   }
   plaquette_start(ctx, links, 0);
   if (p->c_rect != 0.0) rectangle_start(ctx, links, 1);

@@ -1,6 +1,7 @@
 // Field allocation, host<->device transfer in the reference layout, cold and
 // hot starts, Gaussian momenta, field copies/conversions and the deterministic
 // two-stage reductions used by every global sum.
+#include <algorithm>
 #include "gf_internal.h"
 #include "stencil.cuh"
 #include <vector>
@@ -85,7 +86,7 @@ gf_field* field_pooled(gf_ctx* ctx, int kind) {
 }
 
 gf_field* arena_view(gf_ctx* ctx, int which, size_t off, int kind) {
-  const size_t cap = field_bytes(ctx->geom, GF_LINK64);
+  const size_t cap = std::max(field_bytes(ctx->geom, GF_LINK64), field_bytes(ctx->geom, GF_LINKFX));
   if (!ctx->arena[which]) {
     ctx->arena[which] = device_alloc(ctx, cap);
   }

@@ -253,8 +253,10 @@ static void rect_df(gf_ctx* ctx, const float4* U, gf_field* D, double cp, double
 void rectangle_start(gf_ctx* ctx, const gf_field* U, int slot) {
   if (U->kind != GF_LINKFX && U->kind != GF_LINK64 && U->kind != GF_MAT64 && U->kind != GF_LINKDF)
     throw gf_error(GF_EINVAL, "rectangle: links must be LINK64");
-  // fp64 links, and the top level of a double-float stack, through a fixed-point copy
-  const gf_field* F = U->kind == GF_LINKFX ? U : fx_links(ctx, U);
+  // fp64 links through a fixed-point copy; those of a double-float stack as they are
+  const gf_field* F = U;
+  if (U->kind == GF_LINKDF) F = nullptr;
+  else if (U->kind != GF_LINKFX) F = fx_links(ctx, U);
   if (F) {
     rectangle_start_fx(ctx, F, slot);
     return;

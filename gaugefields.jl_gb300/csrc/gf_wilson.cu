@@ -29,8 +29,10 @@ void plaquette_start(gf_ctx* ctx, const gf_field* U, int slot) {
       U->kind != GF_LINK32)
     throw gf_error(GF_EINVAL, "plaquette: links must be LINK64 or LINK32");
   ProfScope prof(ctx, GF_K_PLAQ);
-  // fp64 links, and the top level of a double-float stack, through a fixed-point copy
-  const gf_field* F = U->kind == GF_LINKFX ? U : (U->kind == GF_LINK32 ? nullptr : fx_links(ctx, U));
+  // fp64 links through a fixed-point copy; those of a double-float stack as they are
+  const gf_field* F = U;
+  if (U->kind == GF_LINK32 || U->kind == GF_LINKDF) F = nullptr;
+  else if (U->kind != GF_LINKFX) F = fx_links(ctx, U);
   if (F) {
     plaquette_start_fx(ctx, F, slot);
     return;

@@ -332,7 +332,7 @@ def test_double_float_adjoint_of_large_lattices(pkg):
 def test_without_memory_for_the_copy(pkg):
     """The fixed-point copy of the links is what goes when memory is short: a
     field takes its place, and the calls that made it read the links as they
-    are, in fp64 or (the mixed form's energy) double-float storage. The same
+    are. The same
     numbers to 1e-13, and the copy is back when there is memory again."""
     from gaugefields_gb300 import _lib
     torch = pytest.importorskip("torch")
