@@ -132,8 +132,9 @@ __global__ void __launch_bounds__(GF_FX_THREADS * AXES, AXES > 1 ? 2 : GF_FX_MIN
 }
 
 gf_field* fx_links(gf_ctx* ctx, const gf_field* U) {
-  cudaStreamCaptureStatus capture;
-  GF_CUDA(cudaStreamIsCapturing(ctx->stream, &capture));
+  // the context's own stream is not given out, so only a caller's is captured
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (!ctx->own_stream) GF_CUDA(cudaStreamIsCapturing(ctx->stream, &capture));
   if (capture != cudaStreamCaptureStatusNone) {
     // a graph can neither allocate the copy nor see it taken back
     if (!ctx->w_linkfx) return nullptr;

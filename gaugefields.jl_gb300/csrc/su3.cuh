@@ -606,39 +606,28 @@ GF_HD void herm_invariants(const mat3<R>& q, R& c0, R& c1) {
   c0 = q11 * q22 * q33 + R(2) * re3 - q11 * a23 - q22 * a13 - q33 * a12;
 }
 
-// Entry (i,j) of f0 + f1 Q + f2 Q^2 with the type's operators
+// Entry (i,j) of f0 + f1 Q + f2 Q^2
 template <typename R>
-__device__ __forceinline__ cplx<R> ch_combine_ops(const ch_coef<R>& cc, const mat3<R>& q, const mat3<R>& q2, int i,
-                                                  int j) {
+__device__ __forceinline__ cplx<R> ch_combine(const ch_coef<R>& cc, const mat3<R>& q, const mat3<R>& q2, int i, int j) {
   cplx<R> v = cc.f[1] * q.e[i][j];
   fma_(v, cc.f[2], q2.e[i][j]);
   if (i == j) v = v + cc.f[0];
   return v;
 }
-template <typename R>
-__device__ __forceinline__ cplx<R> ch_combine(const ch_coef<R>& cc, const mat3<R>& q, const mat3<R>& q2, int i, int j) {
-  return ch_combine_ops(cc, q, q2, i, j);
-}
-// exp(iQ) for traceless Hermitian Q. Q2 receives Q^2 (callers reuse it).
-// ROWS = 2 forms rows 1-2 only (row 3 left zero), for products whose row 3 is
-// rebuilt or not stored. OPS = true combines f0 + f1 Q + f2 Q^2 with the
-// type's operators (for double-float: the accurate double-word sums, ~2^-48,
-// which chains of link updates keep to 1e-12 of fp64), false with the
-// fixed-grid sum (rms ~2^-43 of the bound) where one is given.
-template <typename R, int ROWS = 3, bool OPS = false>
-__device__ __forceinline__ mat3<R> expiq(const mat3<R>& q, mat3<R>* q2out = nullptr) {
+// exp(iQ) for traceless Hermitian Q. ROWS = 2 forms rows 1-2 only (row 3 left
+// zero), for products whose row 3 is rebuilt or not stored.
+template <typename R, int ROWS = 3>
+__device__ __forceinline__ mat3<R> expiq(const mat3<R>& q) {
   R c0, c1;
   herm_invariants(q, c0, c1);
   ch_coef<R> cc;
   ch_coefficients<R, false>(c0, c1, cc);
-  // OPS: the generic (operator) square as well; otherwise the type's best
-  mat3<R> q2 = OPS ? herm_square<R>(q) : herm_square(q);
+  const mat3<R> q2 = herm_square(q);
   mat3<R> e = zero3<R>();
 #pragma unroll
   for (int i = 0; i < ROWS; ++i)
 #pragma unroll
-    for (int j = 0; j < 3; ++j) e.e[i][j] = OPS ? ch_combine_ops(cc, q, q2, i, j) : ch_combine(cc, q, q2, i, j);
-  if (q2out) *q2out = q2;
+    for (int j = 0; j < 3; ++j) e.e[i][j] = ch_combine(cc, q, q2, i, j);
   return e;
 }
 
