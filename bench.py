@@ -6,12 +6,11 @@ Workload (one "step" = one HMC trajectory): 32^4 lattice, Haar-random start
 (rho = 0.1), tau = 1 with 20 QPQ steps, momentum refresh + Metropolis test.
 
 The headline form is the fastest one whose Delta H stays within 1e-4 of the
-plain fp64 form's: the double-float form (force, stout forward and adjoint
-and link updates in fp32-pair arithmetic on the fp32 pipes, every field
-stored in fp64, the Hamiltonian sums, Delta H and Metropolis in fp64). The
-mixed form (fp32 force on 12-real links) is timed beside it and labelled
-non-compliant: its Delta H moves by ~5e-4 at 32^4. The plain fp64 form is
-timed as well.
+plain form's: the double-float form, which at this size runs the plain form's
+fixed-point kernels (64-bit block fixed point on the integer pipes, every
+field stored in fp64, errors of fp64 class) and equals it. The mixed form
+(fp32 force on 12-real links) is timed beside it and labelled non-compliant:
+its Delta H moves by ~5e-4 at 32^4. The plain form is timed as well.
 
   python bench.py [--gpus N --steps K --warmup W]      # this library
   python bench.py --impl reference [...]               # CPU oracle port
@@ -189,8 +188,8 @@ def read_peaks():
 
 def read_utilisation(kclass):
     """The binding unit's utilisation of a kernel class (issue slots for the
-    double-float kernels, the fp64 pipe for the fp64 ones) from the committed
-    ncu summaries, as [metric, fraction]."""
+    double-float kernels, the multiply pipe for the fixed-point ones) from the
+    committed ncu summaries, as [metric, fraction]."""
     p = os.path.join(ROOT, "profiles", "utilisation.json")
     if not os.path.exists(p):
         return None
@@ -412,7 +411,8 @@ def roofline_of(kern, V, L, peaks, hbm_peak, hbm_note):
     """The HBM roofline and the compute fraction of the dominant kernel class
     of `kern` (CUDA-event totals per class); adds share and avg_ms to `kern`.
     Compute peaks are the cuBLAS rates measured in the run: sgemm for fp32,
-    dgemm for fp64. Double-float kernels count fp64-class flops (a 3x3
+    dgemm for fp64 class (a fraction above 1: the fixed-point kernels run on
+    the integer pipes). Double-float kernels count fp64-class flops (a 3x3
     complex product = 198) against dgemm, and the fp32 operations those flops
     take in the fixed-grid product (six per real multiply-add) against sgemm's
     fp32 rate."""
@@ -435,11 +435,11 @@ def roofline_of(kern, V, L, peaks, hbm_peak, hbm_note):
     fl = algorithmic_flops_per_link(dom) * 4 * V
     tf = fl / per_launch_s / 1e12
     pk = peaks["fp32_tflops"] if prec == "fp32" else peaks["fp64_tflops"]
-    note = {"fp64": "cuBLAS dgemm measured in this run", "fp32": "cuBLAS sgemm (no TF32) measured in this run",
+    note = {"fp64": "cuBLAS dgemm measured in this run (the kernel runs on the integer pipes)", "fp32": "cuBLAS sgemm (no TF32) measured in this run",
             "df": "double-float flops (fp64-class) against the cuBLAS dgemm rate measured in this run"}[prec]
     compute = {"kernel": dom, "precision": prec, "achieved_tflops": tf, "peak_tflops": pk, "peak_note": note,
                "flops_per_launch": fl, "frac": tf / pk,
-               "binding": {"fp64": "fp64 issue", "fp32": "fp32 issue / L1", "df": "fp32 issue"}[prec]}
+               "binding": {"fp64": "integer multiply-add issue", "fp32": "fp32 issue / L1", "df": "fp32 issue"}[prec]}
     util = read_utilisation(dom)
     if util:
         compute["ncu_utilisation"] = {"metric": util[0], "value": util[1],
@@ -850,11 +850,11 @@ def main():
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": 1e3 * tmax / args.steps, "higher_is_better": True,
-            "scaling": "weak", "vs_baseline": None, "dtype": "f32 pairs (double-float) + f64 sums",
+            "scaling": "weak", "vs_baseline": None, "dtype": "f64 (64-bit block fixed point arithmetic)",
             "data": "synthetic (Haar-random SU(3) start, seed 7; Gaussian momenta per trajectory)",
             "config": bench_config(L),
-            "form": "double-float: force, stout forward/adjoint and link updates in fp32-pair arithmetic on fp64 "
-                    "fields; Hamiltonian, Delta H and Metropolis in fp64 (meets |dH - dH_fp64| <= 1e-4: dH_check)",
+            "form": "double-float, at this size in the plain form's arithmetic: 64-bit block fixed point of fp64 "
+                    "class on fp64 fields throughout (meets |dH - dH_fp64| <= 1e-4: dH_check)",
             "replicas": world,
             "e2e": e2e, "gpu_launches": launches, "roofline": roof, "compute": compute, "cpu_baseline": cpu,
             "clocks": clocks, "mixed_form": mixed, "fp64_form": fp64,

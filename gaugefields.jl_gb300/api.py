@@ -648,8 +648,8 @@ def md_driver(U, action, steps, trajectory_length=1.0, integrator=None, smearing
     the smeared links and the force is back-propagated to the thin links.
     precision: "fp64" (plain form), "mixed" (fp32 force and stout on 12-real
     links; fp64-class Hamiltonian, Delta H, link updates and re-unitarisation)
-    or "dfloat" (force, stout and link updates in double-float arithmetic on
-    the fp32 pipes, fp64 links; fp64 Hamiltonian).
+    or "dfloat" (as "fp64", but the stout stacks of lattices of more than 2^21
+    sites in double-float arithmetic).
     recompute: the stout adjoint rebuilds each level's staple sum C instead of
     keeping it from the forward pass (less device memory).
     An integrator without an md_step! (neither a builtin, a SextonWeingarten
@@ -722,8 +722,9 @@ def md_hamiltonian(U, P, driver):
 
 
 def update_gaugefields_(U, P, step_size, driver):
-    """U_mu <- exp(step_size P_mu) U_mu (molecular_dynamics.jl:513-531), in the
-    driver's precision (double-float for the mixed and double-float forms)."""
+    """U_mu <- exp(step_size P_mu) U_mu (molecular_dynamics.jl:513-531), in
+    arithmetic of fp64 class in every form; the mixed form's writes its fp32
+    copy too."""
     if not math.isfinite(step_size):
         raise ValueError("the gauge-field step size must be finite; got %s" % step_size)
     p = driver.params()
@@ -956,9 +957,8 @@ def get_parameter_derivatives(dSdUbar, smearing, U, precision="fp64"):
 # ---------------------------------------------------------------------------
 class Gradientflow:
     """Wilson flow with the Luescher RK3 integrator (gradientflow.jl:118-161).
-    precision: "fp64" (the reference's arithmetic) or "dfloat" (the force and
-    the exponentials in double-float arithmetic on the fp32 pipes, fp64
-    fields)."""
+    precision: "fp64" or "dfloat", both the same fp64-class arithmetic on fp64
+    fields (timed as different kernel classes)."""
 
     def __init__(self, U, Nflow=1, eps=0.01, precision="fp64"):
         if precision not in ("fp64", "dfloat"):
@@ -997,7 +997,7 @@ class Gradientflow_general:
 def gradient_flow(U, loops=None, coefficients=None, steps=1, step_size=0.01, precision="fp64"):
     """gradient_flow(U; steps, step_size) and gradient_flow(U, loops,
     coefficients; steps, step_size) (src/API.jl:420-438); precision "dfloat"
-    selects the double-float Wilson flow (plaquette action only)."""
+    selects the double-float form (plaquette action only)."""
     if steps <= 0:
         raise ValueError("steps must be positive; got %d" % steps)
     if step_size <= 0:

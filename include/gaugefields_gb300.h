@@ -43,13 +43,13 @@ extern "C" {
 #define GF_MAT32 5  /* general 3x3 complex per link, fp32 */
 
 /* precision of the force / stout path */
-#define GF_FP64 0  /* plain form: fp64 throughout */
+#define GF_FP64 0  /* plain form: fp64 fields, arithmetic of fp64 class (errors
+                       no larger than fp64's, in 64-bit block fixed point) */
 #define GF_MIXED 1 /* fp32 force and stout (12-real links), fp64 H / updates */
-#define GF_DFLOAT 2 /* force, stout forward/adjoint and link updates in
-                       double-float arithmetic (fp32 pairs, ~48-bit
-                       significand, on the fp32 pipes) on fp64 links; fp64
-                       H, Delta H and Metropolis. No counterpart in the
-                       reference: a third form between GF_FP64 and GF_MIXED */
+#define GF_DFLOAT 2 /* as GF_FP64, but the stout stacks of lattices of more
+                       than 2^21 sites in double-float arithmetic (fp32 pairs,
+                       ~48-bit significand). No counterpart in the reference:
+                       a third form between GF_FP64 and GF_MIXED */
 
 /* integrators of the MD driver (molecular_dynamics.jl:604-616); GF_OMELYAN is
  * the second-order minimum-norm PQPQP scheme of the reference's custom
@@ -205,7 +205,7 @@ int gf_md_mom_update(gf_ctx* ctx, gf_field* P, const gf_field* U, double eps, co
 int gf_md_link_update(gf_ctx* ctx, gf_field* U, const gf_field* P, double eps, const gf_md_params* prm);
 /* md_trajectory!(U, P, driver) (molecular_dynamics.jl:712-730): one QPQ/PQP
  * trajectory. out[0..2] = initial H, final H, Delta H. prm->precision selects
- * the plain fp64, the mixed or the double-float form. */
+ * the plain, the mixed or the double-float form. */
 int gf_md_trajectory(gf_ctx* ctx, gf_field* U, gf_field* P, const gf_md_params* prm, double out[3]);
 /* One HMC update of the application loop (docs/src/hmc.md:22-81): momenta
  * refresh (seed, sweep), md_trajectory!, Metropolis test with the uniform
@@ -216,8 +216,8 @@ int gf_hmc_update(gf_ctx* ctx, gf_field* U, gf_field* P, const gf_md_params* prm
 /* ---- stout smearing ----------------------------------------------------- */
 /* STOUT_Layer stack (stout_fast.jl:6-121) / CovNeuralnet of nlev plaquette
  * layers with coefficients rho[0..nlev-1]. precision GF_FP64, GF_MIXED
- * (fp32 12-real links) or GF_DFLOAT (fp64 links and MAT64 derivatives,
- * double-float arithmetic); store != 0 keeps C_mu of every level from the
+ * (fp32 12-real links) or GF_DFLOAT (fp64 links and MAT64 derivatives, as
+ * GF_FP64 up to 2^21 sites, beyond in double-float arithmetic); store != 0 keeps C_mu of every level from the
  * forward pass, store == 0 recomputes it in the backward pass. */
 int gf_stout_create(gf_ctx* ctx, int nlev, const double* rho, int precision, int store, gf_stout** out);
 int gf_stout_destroy(gf_stout* st);
@@ -244,9 +244,9 @@ int gf_stout_mom_update(gf_ctx* ctx, gf_stout* st, gf_field* P, const gf_field* 
 /* flow!(U, ::Gradientflow) (smearing/gradientflow.jl:171-238): nsteps RK3
  * Wilson-flow steps of size eps. */
 int gf_flow(gf_ctx* ctx, gf_field* U, double eps, int nsteps);
-/* The same flow with the force and the exponentials in double-float
- * arithmetic on the fp32 pipes (precision GF_DFLOAT; the fields stay fp64)
- * or in fp64 (GF_FP64, = gf_flow). */
+/* The same flow by precision: GF_FP64 and GF_DFLOAT give the same (fp64
+ * fields, arithmetic of fp64 class); their launches are timed as different
+ * kernel classes. */
 int gf_flow_precision(gf_ctx* ctx, gf_field* U, double eps, int nsteps, int precision);
 /* flow!(U, ::Gradientflow_general) (smearing/gradientflow.jl:240-336) for the
  * action with the plaquette loops at c_plaq and the rectangle loops at c_rect
@@ -281,23 +281,23 @@ int gf_plaquette_noalloc(const void* links, const int L[4], double* out, void* s
 
 /* ---- instrumentation (no counterpart in the reference) ----------------- */
 /* Kernel classes timed by gf_prof_*: */
-#define GF_K_PLAQ 0         /* plaquette / action reduction (fp64) */
+#define GF_K_PLAQ 0         /* plaquette / action reduction */
 #define GF_K_FORCE 1        /* Wilson staple force (+ momentum update) */
-#define GF_K_LINK_UPDATE 2  /* exp(i eps P) U link update (fp64) */
+#define GF_K_LINK_UPDATE 2  /* exp(i eps P) U link update, plain form */
 #define GF_K_STOUT_FWD 3    /* stout forward level, fp32 */
 #define GF_K_BWD_LOCAL 4    /* stout adjoint, local part, fp32 */
 #define GF_K_BWD_GATHER 5   /* stout adjoint, pull-back gather (+ force), fp32 */
-#define GF_K_STOUT_FWD64 6  /* the same three stages in fp64 */
+#define GF_K_STOUT_FWD64 6  /* the same three stages in fixed point (fp64 class) */
 #define GF_K_BWD_LOCAL64 7
 #define GF_K_BWD_GATHER64 8
 #define GF_K_OTHER 9        /* starts, conversions, kinetic, copies */
-#define GF_K_LINK_UPDATE_DF 10  /* link update in double-float (mixed form) */
-#define GF_K_STOUT_FWD_DF 11    /* stout forward in double-float (Hamiltonian, GF_DFLOAT force) */
-#define GF_K_FORCE_DF 12        /* Wilson staple force in double-float */
+#define GF_K_LINK_UPDATE_DF 10  /* link update of the mixed and double-float forms */
+#define GF_K_STOUT_FWD_DF 11    /* stout forward in double-float (mixed Hamiltonian, large GF_DFLOAT stacks) */
+#define GF_K_FORCE_DF 12        /* Wilson staple force of the double-float form */
 #define GF_K_BWD_LOCAL_DF 13    /* stout adjoint, local part, double-float */
 #define GF_K_BWD_GATHER_DF 14   /* stout adjoint, gather (+ force), double-float */
-#define GF_K_RECT 15            /* rectangle loop sum and plaquette + rectangle force (fp64) */
-#define GF_K_RECT_DF 16         /* plaquette + rectangle force in double-float */
+#define GF_K_RECT 15            /* rectangle loop sum and plaquette + rectangle force */
+#define GF_K_RECT_DF 16         /* dS/dUbar of that action on a double-float stack */
 #define GF_K_COUNT 17
 /* Enable (on != 0) or disable CUDA-event timing of every kernel launch on the
  * context's stream; enabling clears the accumulators. */

@@ -423,8 +423,8 @@ An MD action provider: the Wilson action `push!(action, beta/2, plaq ∪ plaq')`
 (with `c_rect` ≠ 0 also `push!(action, c_rect, rect ∪ rect')`, e.g. Iwasaki)
 evaluated on `length(rho)` plaquette stout levels of the thin links. The
 force runs the hand-written stout adjoint on the device. `precision` selects
-the plain fp64 form (`GF_FP64`), the double-float form (`GF_DFLOAT`, Delta H
-within ~1e-7 of fp64 at 32^4) or the mixed fp32-force form (`GF_MIXED`).
+the plain form (`GF_FP64`), the double-float form (`GF_DFLOAT`: the plain one
+up to 2^21 sites, beyond within ~1e-6 of its Delta H) or the mixed fp32-force form (`GF_MIXED`).
 """
 struct StoutWilsonAction_GB300
     beta::Float64
@@ -605,9 +605,8 @@ end
 # ---------------------------------------------------------------------------
 # gradient flow (src/smearing/gradientflow.jl:171-238)
 # ---------------------------------------------------------------------------
-# precision = GF_DFLOAT runs the force and the exponentials in double-float
-# arithmetic on the fp32 pipes (the fields stay fp64); GF_FP64 is the
-# reference's arithmetic
+# precision GF_FP64 and GF_DFLOAT give the same flow (fp64 fields, arithmetic of
+# fp64 class)
 function flow!(U::GB300Config, g::Gradientflow; precision::Integer=GF_FP64)
     ctx = U[1].ctx
     check(ccall((:gf_flow_precision, libgf), Cint, (Ptr{Cvoid}, Ptr{Cvoid}, Cdouble, Cint, Cint), ctx.h,
