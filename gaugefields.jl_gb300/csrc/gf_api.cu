@@ -939,9 +939,8 @@ extern "C" int gf_flow_force(gf_ctx* ctx, const gf_field* U, gf_field* F, double
   API_END(ctx)
 }
 
-// RK3 Wilson-flow steps (flow!, src/smearing/gradientflow.jl:171-238) in fp64
-// or, df, with the force and the exponentials in double-float arithmetic on
-// the fp64 fields
+// RK3 Wilson-flow steps (flow!, src/smearing/gradientflow.jl:171-238); df: the
+// kernel classes that the launches are timed as
 static void flow_steps(gf_ctx* ctx, gf_field* U, double eps, int nsteps, bool df) {
   if (!ctx->w_link64) ctx->w_link64 = field_new(ctx, GF_LINK64);
   if (!ctx->w_link64b) ctx->w_link64b = field_new(ctx, GF_LINK64);

@@ -17,12 +17,13 @@
 //
 // Two kernels per backward level: k_bwd_local (Lambda .. Dp, Z) and
 // k_bwd_gather (the pull-back through C, fused with the thin-link MD force
-// and momentum update at the bottom level).
+// and momentum update at the bottom level). Here in fp32 (the mixed form) and
+// in double-float (large stacks of that form, the mixed form's Hamiltonian);
+// the fixed-point ones are in gf_fxstout.cu.
 #include "gf_internal.h"
 #include "stencil.cuh"
 #include "dfslots.cuh"
 #include <type_traits>
-
 
 
 namespace gf {

@@ -206,7 +206,7 @@ struct LinkFull<float> {
   }
 };
 
-// fp64 storage, double-float arithmetic (the mixed form's fp64-class kernels)
+// fp64 storage, double-float arithmetic
 template <>
 struct LinkFull<dfl> {
   typedef double2 elem;
