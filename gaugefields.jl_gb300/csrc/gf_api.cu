@@ -598,6 +598,13 @@ static gf_stout* ctx_stout(gf_ctx* ctx, const gf_md_params* p, int precision) {
   return *slot;
 }
 
+// The thin links for a forward pass of one of the context's stacks: a
+// fixed-point one reads the context's copy and needs none of its own.
+static const gf_field* stack_links(gf_ctx* ctx, const gf_stout* st, const gf_field* U) {
+  const gf_field* F = st->precision == GF_FP64 && U->kind == GF_LINK64 ? fx_links(ctx, U) : nullptr;
+  return F ? F : U;
+}
+
 // The potential on the (smeared) links, plaquette and rectangle loops, the
 // sums of fp64 class in every form. The mixed form smears them in double-float
 // arithmetic (compensated products, ~1e-13 of the operands' norms) in two
@@ -613,7 +620,7 @@ static void potential_start(gf_ctx* ctx, const gf_field* U, const gf_md_params* 
   const gf_field* links = U;
   if (p->nstout > 0) {
     gf_stout* st = ctx_stout(ctx, p, df ? GF_PREC_DF : GF_FP64);
-    stout_forward(ctx, st, U, nullptr);
+    stout_forward(ctx, st, stack_links(ctx, st, U), nullptr);
     links = stout_top(st);
     if (st->fwd_only) {
       // the levels take the two scratch blocks in turn: the top's copy goes to the other one
@@ -662,7 +669,7 @@ static void mom_update(gf_ctx* ctx, gf_field* P, const gf_field* U, const gf_fie
     // smeared plaquette + rectangle action: dS/dUbar = beta/2 S + c_rect R on
     // the top level, written into the stack's D[1] and back-propagated
     gf_stout* st = ctx_stout(ctx, p, p->precision);
-    stout_forward(ctx, st, links, nullptr);
+    stout_forward(ctx, st, stack_links(ctx, st, links), nullptr);
     loops_dsdu(ctx, stout_top(st), st->D[1], 0.5 * p->beta, p->c_rect);
     stout_backward(ctx, st, st->D[1], p->beta, nullptr, P, eps);
     return;
@@ -672,7 +679,7 @@ static void mom_update(gf_ctx* ctx, gf_field* P, const gf_field* U, const gf_fie
     return;
   }
   gf_stout* st = ctx_stout(ctx, p, p->precision);
-  stout_forward(ctx, st, links, nullptr);
+  stout_forward(ctx, st, stack_links(ctx, st, links), nullptr);
   stout_backward(ctx, st, nullptr, p->beta, nullptr, P, eps);
 }
 

@@ -426,3 +426,38 @@ def test_forces_and_smearing_in_a_graph(pkg, warm):
     calls()
     close(got[0], F.to_host())
     close(got[1], top.to_host())
+
+
+@pytest.mark.parametrize("precision", ["fp64", "dfloat"])
+def test_smeared_driver_calls_in_any_order(pkg, precision):
+    """The context's stacks read the context's copy of whatever links a call
+    is given; energies, forces and trajectories on two configurations in turn
+    are bitwise those of fresh contexts."""
+    L = (4, 6, 4, 8)
+
+    def run(seeds):
+        U = pkg.gauge_configuration(L, start="hot", seed=1)
+        other = {k: pkg.gauge_configuration(L, start="hot", seed=k).to_host() for k in set(seeds)}
+        action = pkg.GaugeAction(U)
+        pkg.push_(action, 3.0, "plaquette")
+        pkg.push_(action, -0.1, "rectangular")
+        net = pkg.CovNeuralnet(U)
+        pkg.push_(net, pkg.STOUT_Layer("plaquette", 0.1))
+        pkg.push_(net, pkg.STOUT_Layer("plaquette", 0.08))
+        drv = pkg.md_driver(U, action, steps=2, trajectory_length=0.2, smearing=net, precision=precision)
+        out = []
+        for k in seeds:
+            U.from_host(other[k])
+            P = pkg.gaussian_momenta(U, seed=k)
+            h = pkg.md_hamiltonian(U, P, drv)
+            pkg.calculate_Plaquette(U)
+            r = pkg.md_trajectory_(U, P, drv)
+            pkg.update_momenta_(P, U, 0.1, drv)
+            out.append((h, r.initial_hamiltonian, r.final_hamiltonian, U.to_host(), P.to_host()))
+        return out
+
+    turns = run([3, 5, 3])
+    for got, k in zip(turns, [3, 5, 3]):
+        want = run([k])[0]
+        assert got[0] == got[1]
+        assert all(np.array_equal(np.asarray(a), np.asarray(b)) for a, b in zip(got, want))
