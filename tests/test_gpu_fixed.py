@@ -461,3 +461,28 @@ def test_smeared_driver_calls_in_any_order(pkg, precision):
         want = run([k])[0]
         assert got[0] == got[1]
         assert all(np.array_equal(np.asarray(a), np.asarray(b)) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("levels,recompute", [(1, False), (2, True)])
+def test_smeared_force_forms_its_top_derivative_either_way(pkg, levels, recompute):
+    """Above 40,000 sites dS/dUbar of the Wilson action is formed in a kernel
+    of its own, below in the adjoint. A lattice of 2 x 20,480 sites that
+    repeats one of 20,480 along T has the same force, up to the exponents that
+    the two paths choose: 1e-14 of the largest entry."""
+    S, B = (16, 10, 8, 16), (16, 10, 8, 32)
+    n = int(np.prod(S))
+    assert n < 40000 < 2 * n
+    Uh = pkg.gauge_configuration(S, start="hot", seed=2).to_host()
+    out = []
+    for L, k in ((S, 1), (B, 2)):
+        U = pkg.gauge_configuration(L, start="cold")
+        U.from_host(np.tile(Uh, (1, k, 1, 1)))
+        action = pkg.GaugeAction(U)
+        pkg.push_(action, 3.0, "plaquette")
+        net = pkg.CovNeuralnet(U)
+        for rho in (0.1, 0.08)[:levels]:
+            pkg.push_(net, pkg.STOUT_Layer("plaquette", rho))
+        P = pkg.gauge_momenta(U)
+        pkg.update_momenta_(P, U, 1.0, pkg.md_driver(U, action, steps=1, smearing=net, recompute=recompute))
+        out.append(P.to_host())
+    close(out[1], np.tile(out[0], (1, 2, 1)), 1e-14)
