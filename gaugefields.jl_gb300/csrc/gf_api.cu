@@ -411,12 +411,11 @@ extern "C" int gf_staple(gf_ctx* ctx, const gf_field* U, int mu, gf_field* V) {
 // ---------------------------------------------------------------------------
 // Sites up to which the double-float form's stacks are fixed-point ones, as
 // the plain form's. Two-level force, double-float tables against fixed point:
-// 4^4 207 / 89 us, 8^4 213 / 159, 12^4 698 / 537, 16^4 1684 / 1542, 24^4 7.95 /
-// 7.54 ms, 32^4 24.9 / 23.9: the tables give a link one thread, which leaves a
-// small lattice's last wave nearly empty, and at 32^4 still read and normalise
-// more. Beyond, where a field takes over 1.2 GB, the 4% are left for the
-// tables' 144 bytes a matrix (fixed point: 148): a stack that fills the memory
-// keeps its size.
+// 4^4 207 / 89 us, 8^4 213 / 158, 12^4 698 / 537, 16^4 1684 / 1529, 32^4 24.9 /
+// 23.5 ms: the tables give a link one thread, which leaves a small lattice's
+// last wave nearly empty, and at 32^4 still read and normalise more. Beyond,
+// where a field takes over 1.2 GB, the 6% are left for the tables' 144 bytes a
+// matrix (fixed point: 148): a stack that fills the memory keeps its size.
 #ifndef GF_FX_STACK_MAX
 #define GF_FX_STACK_MAX (1 << 21)
 #endif

@@ -2,7 +2,7 @@
 // by rows: fp64-class results at integer-pipe rates. A block serves 32 links;
 // thread 3 link + row carries a row of each matrix through the products, and
 // two warps evaluate the Cayley-Hamilton series with a thread per link (real
-// and imaginary parts), exchanging through shared memory. All three kernels
+// and imaginary parts), exchanging through shared memory. The kernels
 // are bound by integer multiply-add issue. A two-level smearing with its
 // adjoint at 16^4: 9.65 ms in fp64 arithmetic, 1.67 ms here (1.4 ms of it in
 // these kernels), at no larger an error (gradient 4.3e-16 against 4.8e-16).
@@ -33,8 +33,8 @@ __device__ __forceinline__ void fx_down_row(fx_acc& v) {
 
 // Ubar = exp(TA(C U^dag)) U, C = rho V stored when Cout is given
 // Blocks per SM, by 32^4 launches: gather 5.20 ms with four (168 registers),
-// 5.12 with five, 5.82 with six (spills); local adjoint 3.95 with four, 3.91
-// with five, 4.10 with six; forward 2.84 with seven, 2.93 with eight, 3.1 with
+// 5.12 with five, 5.82 with six (spills); local adjoint 3.90 with four, 3.71
+// with five, 3.97 with six; forward 2.84 with seven, 2.93 with eight, 3.1 with
 // five or six.
 #ifndef GF_FX_GATHER_MINB
 #define GF_FX_GATHER_MINB 5
