@@ -33,8 +33,8 @@ __device__ __forceinline__ void fx_down_row(fx_acc& v) {
 
 // Ubar = exp(TA(C U^dag)) U, C = rho V stored when Cout is given
 // Blocks per SM, by 32^4 launches: gather 5.20 ms with four (168 registers),
-// 5.12 with five, 5.82 with six (spills); local adjoint 3.90 with four, 3.71
-// with five, 3.97 with six; forward 2.84 with seven, 2.93 with eight, 3.1 with
+// 5.12 with five, 5.82 with six (spills); local adjoint 3.74 with four, 3.71
+// with five, 3.96 with six; forward 2.84 with seven, 2.93 with eight, 3.1 with
 // five or six.
 #ifndef GF_FX_GATHER_MINB
 #define GF_FX_GATHER_MINB 5
