@@ -737,8 +737,8 @@ static MDResult md_run(gf_ctx* ctx, gf_field* U, gf_field* P, const gf_md_params
     U32 = ctx->w_link32;
     link64_to_32(ctx, U32, U);
   }
-  const FxHold hold(ctx);
   if (keeps_fx(ctx, p)) Ufx = fx_links(ctx, U);  // null: no memory for it
+  const FxHold hold(ctx, Ufx);
   const gf_field* Ucopy = U32 ? U32 : Ufx;
   const gf_field* Upot = Ufx ? Ufx : U;  // the potential never takes the fp32 links
   MDResult r;
@@ -957,8 +957,8 @@ static void flow_steps(gf_ctx* ctx, gf_field* U, double eps, int nsteps, bool df
   const double c0 = 17.0 * eps / 36.0;
   if (nsteps == 0) return;
   // the fixed-point copy of U, W1, W2 in turn, written by their updates (null: no memory for it)
-  const FxHold hold(ctx);
   gf_field* F = fx_links(ctx, U);
+  const FxHold hold(ctx, F);
   for (int n = 0; n < nsteps; ++n) {
     flow_force(ctx, F ? F : U, G, c0, 0.0, df);                 // G = 17eps/36 F0
     exp_mom_links(ctx, W1, G, -9.0 / 17.0, U, df, F);           // W1 = exp(-eps/4 F0) U
@@ -1004,8 +1004,8 @@ extern "C" int gf_flow_loops(gf_ctx* ctx, gf_field* U, double eps, int nsteps, d
   const double c0 = 17.0 * eps / 36.0;
   const double c1 = -8.0 * eps / 9.0;
   const double c2 = -0.75 * eps;
-  const FxHold hold(ctx);
   gf_field* F = nsteps ? fx_links(ctx, U) : nullptr;  // of U, W1, W2 in turn
+  const FxHold hold(ctx, F);
   for (int n = 0; n < nsteps; ++n) {
     loops_force_coef(ctx, F ? F : U, G, c0 * c_plaq, c0 * c_rect, 0.0);  // G = 17eps/36 F0
     exp_mom_links(ctx, W1, G, -9.0 / 17.0, U, false, F);         // W1 = exp(-eps/4 F0) U

@@ -227,11 +227,17 @@ inline FxField fx_view(const gf_field* f) { return FxField{(const char*)f->ptr};
 // An allocation of the context that fails takes it back, but not while a
 // driver holds it or once a graph has captured it.
 gf_field* fx_links(gf_ctx* ctx, const gf_field* U);
+// `copy` null: the driver keeps none, and one left by an earlier call stays
+// reclaimable.
 struct FxHold {
   gf_ctx* ctx;
-  explicit FxHold(gf_ctx* c) : ctx(c) { ++ctx->fx_hold; }
+  FxHold(gf_ctx* c, const gf_field* copy) : ctx(copy ? c : nullptr) {
+    if (ctx) ++ctx->fx_hold;
+  }
   FxHold(const FxHold&) = delete;
-  ~FxHold() { --ctx->fx_hold; }
+  ~FxHold() {
+    if (ctx) --ctx->fx_hold;
+  }
 };
 // LINK64 / MAT64 or double-float pairs -> fixed point, and fixed point -> fp64
 void to_fx(gf_ctx* ctx, gf_field* dst, const gf_field* src);
