@@ -600,7 +600,7 @@ static gf_stout* ctx_stout(gf_ctx* ctx, const gf_md_params* p, int precision) {
 // The thin links for a forward pass of one of the context's stacks: a
 // fixed-point one reads the context's copy and needs none of its own.
 static const gf_field* stack_links(gf_ctx* ctx, const gf_stout* st, const gf_field* U) {
-  const gf_field* F = st->precision == GF_FP64 && U->kind == GF_LINK64 ? fx_links(ctx, U) : nullptr;
+  const gf_field* F = st->precision == GF_FP64 && U->kind == GF_LINK64 ? fx_links(ctx, U, true) : nullptr;
   return F ? F : U;
 }
 

@@ -131,13 +131,16 @@ __global__ void __launch_bounds__(GF_FX_THREADS * AXES, AXES > 1 ? 2 : GF_FX_MIN
   if (axis == 0) fx_update_mom(sh, se, P, mu, s0, V, -coef, keep);
 }
 
-gf_field* fx_links(gf_ctx* ctx, const gf_field* U) {
+gf_field* fx_links(gf_ctx* ctx, const gf_field* U, bool for_stack) {
   // the context's own stream is not given out, so only a caller's is captured
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (!ctx->own_stream) GF_CUDA(cudaStreamIsCapturing(ctx->stream, &capture));
   if (capture != cudaStreamCaptureStatusNone) {
-    // a graph can neither allocate the copy nor see it taken back
-    if (!ctx->w_linkfx) return nullptr;
+    // A graph may be replayed on any stream and beside any call, so a call that
+    // needs no state of the context captures none: the fp64 kernels read the
+    // links in place. The context's stacks are such state in any case, and
+    // nothing can be allocated here; their copy is kept from then on.
+    if (!for_stack || !ctx->w_linkfx) return nullptr;
     ctx->fx_graph = 1;
   }
   if (!ctx->w_linkfx) {

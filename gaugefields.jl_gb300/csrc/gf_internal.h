@@ -222,11 +222,12 @@ void plaquette_start_fx(gf_ctx* ctx, const gf_field* F, int slot);
 void plaquette_start(gf_ctx* ctx, const gf_field* U, int slot);
 inline FxField fx_view(const gf_field* f) { return FxField{(const char*)f->ptr}; }
 // the context's fixed-point copy of fp64 or double-float links, made anew; null
-// when there is no memory for it (or a graph is being captured and there is
-// none yet): the fp64 kernels, a fifth as fast, then read the links in place.
+// when there is no memory for it or a graph is being captured: the fp64
+// kernels, a fifth as fast, then read the links in place. for_stack: for one of
+// the context's stacks, which captured graphs use the copy with.
 // An allocation of the context that fails takes it back, but not while a
 // driver holds it or once a graph has captured it.
-gf_field* fx_links(gf_ctx* ctx, const gf_field* U);
+gf_field* fx_links(gf_ctx* ctx, const gf_field* U, bool for_stack = false);
 // `copy` null: the driver keeps none, and one left by an earlier call stays
 // reclaimable.
 struct FxHold {

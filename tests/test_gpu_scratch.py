@@ -47,3 +47,50 @@ def test_an_idle_copy_gives_way_to_a_trajectory_that_keeps_none(pkg):
     taken, want = trajectory(False)
     assert taken > COPY
     assert trajectory(True)[1] == want
+
+
+def launches(pkg):
+    import ctypes
+    from gaugefields_gb300 import _lib
+    n = ctypes.c_longlong()
+    _lib.check(_lib.load().gf_launch_count(ctypes.byref(n)))
+    return n.value
+
+
+def test_a_captured_force_touches_its_own_fields_only(pkg):
+    """A graph may be replayed on any stream beside the context's other calls,
+    so captured calls that need no state of the context use none: one launch
+    each, no conversion of the links into the context's copy before it. They
+    give the same to 1e-13."""
+    torch = pytest.importorskip("torch")
+    U = pkg.gauge_configuration((16, 16, 16, 16), start="hot", seed=5)
+    plain, loops = wilson(pkg, U), wilson(pkg, U)
+    pkg.push_(loops, -0.1, "rectangular")
+    F = [pkg.gauge_momenta(U) for _ in range(3)]
+    pkg.clear_U_(F[2])
+
+    def calls():
+        pkg.md_force_(F[0], plain, U)
+        pkg.md_force_(F[1], loops, U)
+        pkg.add_force_(F[2], U)
+
+    def forces():
+        return [f.to_host() for f in F]
+
+    calls()
+    want = forces()
+    for f in F:
+        pkg.gaussian_momenta_(f, seed=1)
+    pkg.clear_U_(F[2])
+    stream = torch.cuda.Stream()
+    U.ctx.set_stream(stream.cuda_stream)
+    U.ctx.torch_stream = stream
+    graph = torch.cuda.CUDAGraph()
+    before = launches(pkg)
+    with torch.cuda.graph(graph, stream=stream):
+        calls()
+    assert launches(pkg) - before == 3
+    graph.replay()
+    torch.cuda.synchronize()
+    for got, ref in zip(forces(), want):
+        assert np.abs(got - ref).max() <= 1e-13 * np.abs(ref).max()
