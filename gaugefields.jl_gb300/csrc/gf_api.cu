@@ -50,7 +50,15 @@ static void set_err(const gf_ctx* ctx, const std::string& m) {
   if (ctx) const_cast<gf_ctx*>(ctx)->err = m;
 }
 
-#define API_BEGIN try {
+// One call of a context at a time: calls share its scratch (the fixed-point copy
+// of the links, partial sums, staging, stacks) from their first launch to their
+// last, and a caller's threads may share the context.
+static std::unique_lock<std::recursive_mutex> lock_of(gf_ctx* ctx) {
+  return ctx ? std::unique_lock<std::recursive_mutex>(ctx->calls) : std::unique_lock<std::recursive_mutex>();
+}
+#define API_BEGIN(ctx)                      \
+  const auto one_call_ = lock_of(ctx);      \
+  try {
 #define API_END(ctx)                           \
   }                                            \
   catch (const gf_error& e) {                  \
@@ -85,7 +93,7 @@ static void need_ctx(const gf_ctx* ctx, const gf_field* f) {
 // ---------------------------------------------------------------------------
 extern "C" int gf_ctx_create(const int L[4], int device, gf_ctx** out) {
   gf_ctx* ctx = nullptr;
-  API_BEGIN
+  try {
   need(L != nullptr && out != nullptr, "gf_ctx_create: null argument");
   *out = nullptr;
   long long V = 1;
@@ -167,7 +175,7 @@ extern "C" int gf_ctx_destroy(gf_ctx* ctx) {
 }
 
 extern "C" int gf_ctx_set_stream(gf_ctx* ctx, void* cuda_stream) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx != nullptr, "gf_ctx_set_stream: null context");
   GF_CUDA(cudaStreamSynchronize(ctx->stream));
   if (ctx->own_stream) {
@@ -184,7 +192,7 @@ extern "C" int gf_ctx_set_stream(gf_ctx* ctx, void* cuda_stream) {
 }
 
 extern "C" int gf_ctx_synchronize(gf_ctx* ctx) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx != nullptr, "gf_ctx_synchronize: null context");
   GF_CUDA(cudaStreamSynchronize(ctx->stream));
   API_END(ctx)
@@ -196,7 +204,7 @@ extern "C" const char* gf_last_error(const gf_ctx* ctx) {
 }
 
 extern "C" int gf_ctx_volume(const gf_ctx* ctx, int64_t* out) {
-  API_BEGIN
+  try {
   need(ctx && out, "gf_ctx_volume: null argument");
   *out = ctx->geom.vol;
   API_END(ctx)
@@ -206,7 +214,7 @@ extern "C" int gf_ctx_volume(const gf_ctx* ctx, int64_t* out) {
 // fields
 // ---------------------------------------------------------------------------
 extern "C" int gf_field_alloc(gf_ctx* ctx, int kind, gf_field** out) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && out, "gf_field_alloc: null argument");
   need(kind >= GF_LINK64 && kind <= GF_MAT32, "gf_field_alloc: unknown kind");
   GF_CUDA(cudaSetDevice(ctx->device));
@@ -241,7 +249,7 @@ extern "C" int gf_field_device_ptr(const gf_field* f, void** ptr) {
 }
 
 extern "C" int gf_field_copy(gf_ctx* ctx, gf_field* dst, const gf_field* src) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && dst && src, "gf_field_copy: null argument");
   need_ctx(ctx, dst);
   need_ctx(ctx, src);
@@ -250,7 +258,7 @@ extern "C" int gf_field_copy(gf_ctx* ctx, gf_field* dst, const gf_field* src) {
 }
 
 extern "C" int gf_field_zero(gf_ctx* ctx, gf_field* f) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && f, "gf_field_zero: null argument");
   need_ctx(ctx, f);
   zero_field(ctx, f);
@@ -258,7 +266,7 @@ extern "C" int gf_field_zero(gf_ctx* ctx, gf_field* f) {
 }
 
 extern "C" int gf_field_axpy(gf_ctx* ctx, gf_field* y, double a, const gf_field* x) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && y && x, "gf_field_axpy: null argument");
   need_ctx(ctx, y);
   need_ctx(ctx, x);
@@ -274,28 +282,28 @@ extern "C" int gf_field_axpy(gf_ctx* ctx, gf_field* y, double a, const gf_field*
 // host transfer
 // ---------------------------------------------------------------------------
 extern "C" int gf_upload_links(gf_ctx* ctx, gf_field* U, const double* host) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U && host, "gf_upload_links: null argument");
   need_ctx(ctx, U);
   upload_links(ctx, U, host);
   API_END(ctx)
 }
 extern "C" int gf_download_links(gf_ctx* ctx, const gf_field* U, double* host) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U && host, "gf_download_links: null argument");
   need_ctx(ctx, U);
   download_links(ctx, U, host);
   API_END(ctx)
 }
 extern "C" int gf_upload_mom(gf_ctx* ctx, gf_field* P, const double* host) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && P && host, "gf_upload_mom: null argument");
   need_ctx(ctx, P);
   upload_mom(ctx, P, host);
   API_END(ctx)
 }
 extern "C" int gf_download_mom(gf_ctx* ctx, const gf_field* P, double* host) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && P && host, "gf_download_mom: null argument");
   need_ctx(ctx, P);
   download_mom(ctx, P, host);
@@ -306,21 +314,21 @@ extern "C" int gf_download_mom(gf_ctx* ctx, const gf_field* P, double* host) {
 // starts
 // ---------------------------------------------------------------------------
 extern "C" int gf_cold_start(gf_ctx* ctx, gf_field* U) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U, "gf_cold_start: null argument");
   need_ctx(ctx, U);
   cold_start(ctx, U);
   API_END(ctx)
 }
 extern "C" int gf_hot_start(gf_ctx* ctx, gf_field* U, uint64_t seed) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U, "gf_hot_start: null argument");
   need_ctx(ctx, U);
   hot_start(ctx, U, seed);
   API_END(ctx)
 }
 extern "C" int gf_gaussian_momenta(gf_ctx* ctx, gf_field* P, uint64_t seed, uint64_t sweep) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && P, "gf_gaussian_momenta: null argument");
   need_ctx(ctx, P);
   gaussian_momenta(ctx, P, seed, sweep);
@@ -328,7 +336,7 @@ extern "C" int gf_gaussian_momenta(gf_ctx* ctx, gf_field* P, uint64_t seed, uint
 }
 
 extern "C" int gf_mom_scale(gf_ctx* ctx, gf_field* P, double a) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && P, "gf_mom_scale: null argument");
   need_ctx(ctx, P);
   need_kind(P, GF_MOM64, "gf_mom_scale: P");
@@ -337,7 +345,7 @@ extern "C" int gf_mom_scale(gf_ctx* ctx, gf_field* P, double a) {
   API_END(ctx)
 }
 extern "C" int gf_reunitarize(gf_ctx* ctx, gf_field* U) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U, "gf_reunitarize: null argument");
   need_ctx(ctx, U);
   reunitarize_links(ctx, U);
@@ -348,14 +356,14 @@ extern "C" int gf_reunitarize(gf_ctx* ctx, gf_field* U) {
 // measurements
 // ---------------------------------------------------------------------------
 extern "C" int gf_plaquette(gf_ctx* ctx, const gf_field* U, double* out) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U && out, "gf_plaquette: null argument");
   need_ctx(ctx, U);
   *out = plaquette_sum(ctx, U);
   API_END(ctx)
 }
 extern "C" int gf_polyakov_loop(gf_ctx* ctx, const gf_field* U, double* out) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U && out, "gf_polyakov_loop: null argument");
   need_ctx(ctx, U);
   need_kind(U, GF_LINK64, "gf_polyakov_loop: U");
@@ -363,7 +371,7 @@ extern "C" int gf_polyakov_loop(gf_ctx* ctx, const gf_field* U, double* out) {
   API_END(ctx)
 }
 extern "C" int gf_action(gf_ctx* ctx, const gf_field* U, double beta, double* out) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U && out, "gf_action: null argument");
   need_ctx(ctx, U);
   need(std::isfinite(beta), "gf_action: beta must be finite");
@@ -371,7 +379,7 @@ extern "C" int gf_action(gf_ctx* ctx, const gf_field* U, double beta, double* ou
   API_END(ctx)
 }
 extern "C" int gf_rectangle(gf_ctx* ctx, const gf_field* U, double* out) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U && out, "gf_rectangle: null argument");
   need_ctx(ctx, U);
   need_kind(U, GF_LINK64, "gf_rectangle: U");
@@ -379,7 +387,7 @@ extern "C" int gf_rectangle(gf_ctx* ctx, const gf_field* U, double* out) {
   API_END(ctx)
 }
 extern "C" int gf_action_loops(gf_ctx* ctx, const gf_field* U, double c_plaq, double c_rect, double* out) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U && out, "gf_action_loops: null argument");
   need_ctx(ctx, U);
   need(std::isfinite(c_plaq) && std::isfinite(c_rect), "gf_action_loops: the coefficients must be finite");
@@ -390,7 +398,7 @@ extern "C" int gf_action_loops(gf_ctx* ctx, const gf_field* U, double c_plaq, do
   API_END(ctx)
 }
 extern "C" int gf_kinetic(gf_ctx* ctx, const gf_field* P, double* out) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && P && out, "gf_kinetic: null argument");
   need_ctx(ctx, P);
   need_kind(P, GF_MOM64, "gf_kinetic");
@@ -398,7 +406,7 @@ extern "C" int gf_kinetic(gf_ctx* ctx, const gf_field* P, double* out) {
   API_END(ctx)
 }
 extern "C" int gf_staple(gf_ctx* ctx, const gf_field* U, int mu, gf_field* V) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U && V, "gf_staple: null argument");
   need_ctx(ctx, U);
   need_ctx(ctx, V);
@@ -484,7 +492,7 @@ static gf_stout* stout_new(gf_ctx* ctx, int nlev, const double* rho, int precisi
 }
 
 extern "C" int gf_stout_create(gf_ctx* ctx, int nlev, const double* rho, int precision, int store, gf_stout** out) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && rho && out, "gf_stout_create: null argument");
   need(precision == GF_FP64 || precision == GF_MIXED || precision == GF_DFLOAT,
        "gf_stout_create: precision must be GF_FP64, GF_MIXED or GF_DFLOAT");
@@ -515,7 +523,7 @@ extern "C" int gf_stout_destroy(gf_stout* st) {
 }
 
 extern "C" int gf_stout_forward(gf_ctx* ctx, gf_stout* st, const gf_field* U, gf_field* Uout) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && st && U, "gf_stout_forward: null argument");
   need_ctx(ctx, U);
   need_ctx(ctx, Uout);
@@ -525,7 +533,7 @@ extern "C" int gf_stout_forward(gf_ctx* ctx, gf_stout* st, const gf_field* U, gf
 }
 
 extern "C" int gf_stout_backward(gf_ctx* ctx, gf_stout* st, const gf_field* dSdUbar, gf_field* dSdU) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && st && dSdUbar && dSdU, "gf_stout_backward: null argument");
   need_ctx(ctx, dSdUbar);
   need_ctx(ctx, dSdU);
@@ -535,7 +543,7 @@ extern "C" int gf_stout_backward(gf_ctx* ctx, gf_stout* st, const gf_field* dSdU
 
 extern "C" int gf_stout_param_derivatives(gf_ctx* ctx, gf_stout* st, const gf_field* U, const gf_field* dSdUbar,
                                           double* dSdrho) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && st && U && dSdUbar && dSdrho, "gf_stout_param_derivatives: null argument");
   need_ctx(ctx, U);
   need_ctx(ctx, dSdUbar);
@@ -547,7 +555,7 @@ extern "C" int gf_stout_param_derivatives(gf_ctx* ctx, gf_stout* st, const gf_fi
 
 extern "C" int gf_stout_mom_update(gf_ctx* ctx, gf_stout* st, gf_field* P, const gf_field* U, double eps,
                                    double beta) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && st && P && U, "gf_stout_mom_update: null argument");
   need_ctx(ctx, P);
   need_ctx(ctx, U);
@@ -794,7 +802,7 @@ static MDResult md_run(gf_ctx* ctx, gf_field* U, gf_field* P, const gf_md_params
 }
 
 extern "C" int gf_force(gf_ctx* ctx, const gf_field* U, double beta, gf_field* F) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U && F, "gf_force: null argument");
   need_ctx(ctx, U);
   need_ctx(ctx, F);
@@ -804,7 +812,7 @@ extern "C" int gf_force(gf_ctx* ctx, const gf_field* U, double beta, gf_field* F
 }
 
 extern "C" int gf_force_loops(gf_ctx* ctx, const gf_field* U, double c_plaq, double c_rect, gf_field* F) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U && F, "gf_force_loops: null argument");
   need_ctx(ctx, U);
   need_ctx(ctx, F);
@@ -815,7 +823,7 @@ extern "C" int gf_force_loops(gf_ctx* ctx, const gf_field* U, double c_plaq, dou
 }
 
 extern "C" int gf_mom_update(gf_ctx* ctx, gf_field* P, const gf_field* U, double eps, double beta) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U && P, "gf_mom_update: null argument");
   need_ctx(ctx, U);
   need_ctx(ctx, P);
@@ -826,7 +834,7 @@ extern "C" int gf_mom_update(gf_ctx* ctx, gf_field* P, const gf_field* U, double
 }
 
 extern "C" int gf_link_update(gf_ctx* ctx, gf_field* U, const gf_field* P, double eps, int reunit) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U && P, "gf_link_update: null argument");
   need_ctx(ctx, U);
   need_ctx(ctx, P);
@@ -837,7 +845,7 @@ extern "C" int gf_link_update(gf_ctx* ctx, gf_field* U, const gf_field* P, doubl
 
 extern "C" int gf_hamiltonian(gf_ctx* ctx, const gf_field* U, const gf_field* P, const gf_md_params* prm,
                               double* out) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U && P && out, "gf_hamiltonian: null argument");
   need_ctx(ctx, U);
   need_ctx(ctx, P);
@@ -849,7 +857,7 @@ extern "C" int gf_hamiltonian(gf_ctx* ctx, const gf_field* U, const gf_field* P,
 }
 
 extern "C" int gf_md_mom_update(gf_ctx* ctx, gf_field* P, const gf_field* U, double eps, const gf_md_params* prm) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U && P, "gf_md_mom_update: null argument");
   need_ctx(ctx, U);
   need_ctx(ctx, P);
@@ -868,7 +876,7 @@ extern "C" int gf_md_mom_update(gf_ctx* ctx, gf_field* P, const gf_field* U, dou
 }
 
 extern "C" int gf_md_link_update(gf_ctx* ctx, gf_field* U, const gf_field* P, double eps, const gf_md_params* prm) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U && P, "gf_md_link_update: null argument");
   need_ctx(ctx, U);
   need_ctx(ctx, P);
@@ -881,7 +889,7 @@ extern "C" int gf_md_link_update(gf_ctx* ctx, gf_field* U, const gf_field* P, do
 }
 
 extern "C" int gf_md_trajectory(gf_ctx* ctx, gf_field* U, gf_field* P, const gf_md_params* prm, double out[3]) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U && P && out, "gf_md_trajectory: null argument");
   need_ctx(ctx, U);
   need_ctx(ctx, P);
@@ -901,7 +909,7 @@ extern "C" int gf_md_trajectory(gf_ctx* ctx, gf_field* U, gf_field* P, const gf_
 
 extern "C" int gf_hmc_update(gf_ctx* ctx, gf_field* U, gf_field* P, const gf_md_params* prm, uint64_t seed,
                              uint64_t sweep, double unif, double out[4]) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U && P && out, "gf_hmc_update: null argument");
   need_ctx(ctx, U);
   need_ctx(ctx, P);
@@ -936,7 +944,7 @@ extern "C" int gf_hmc_update(gf_ctx* ctx, gf_field* U, gf_field* P, const gf_md_
 // the running combination: G = 17eps/36 F0 -> G - 8eps/9 F1 -> -G - 3eps/4 F2.
 // ---------------------------------------------------------------------------
 extern "C" int gf_flow_force(gf_ctx* ctx, const gf_field* U, gf_field* F, double factor) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U && F, "gf_flow_force: null argument");
   need_ctx(ctx, U);
   need_ctx(ctx, F);
@@ -974,7 +982,7 @@ extern "C" int gf_flow(gf_ctx* ctx, gf_field* U, double eps, int nsteps) {
 }
 
 extern "C" int gf_flow_precision(gf_ctx* ctx, gf_field* U, double eps, int nsteps, int precision) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U, "gf_flow: null argument");
   need_ctx(ctx, U);
   need_kind(U, GF_LINK64, "gf_flow: U");
@@ -988,7 +996,7 @@ extern "C" int gf_flow_precision(gf_ctx* ctx, gf_field* U, double eps, int nstep
 // The same RK3 steps with the force TA(U dS/dU) of the plaquette + rectangle
 // action (Gradientflow_general); (c_plaq, c_rect) = (1, 0) is the Wilson flow.
 extern "C" int gf_flow_loops(gf_ctx* ctx, gf_field* U, double eps, int nsteps, double c_plaq, double c_rect) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && U, "gf_flow_loops: null argument");
   need_ctx(ctx, U);
   need_kind(U, GF_LINK64, "gf_flow_loops: U");
@@ -1021,7 +1029,7 @@ extern "C" int gf_flow_loops(gf_ctx* ctx, gf_field* U, double eps, int nsteps, d
 // instrumentation
 // ---------------------------------------------------------------------------
 extern "C" int gf_prof_enable(gf_ctx* ctx, int on) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx != nullptr, "gf_prof_enable: null context");
   if (on && !ctx->prof_ev) {
     ctx->prof_ev = new cudaEvent_t[2 * GF_PROF_CAP];
@@ -1040,7 +1048,7 @@ extern "C" int gf_prof_enable(gf_ctx* ctx, int on) {
 }
 
 extern "C" int gf_prof_read(gf_ctx* ctx, int kernel_class, double* total_ms, long long* launches) {
-  API_BEGIN
+  API_BEGIN(ctx)
   need(ctx && total_ms && launches, "gf_prof_read: null argument");
   need(kernel_class >= 0 && kernel_class < GF_K_COUNT, "gf_prof_read: unknown kernel class");
   if (ctx->prof_on) prof_flush(ctx);

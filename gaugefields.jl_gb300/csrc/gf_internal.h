@@ -75,6 +75,7 @@ struct gf_field {
 };
 
 struct gf_ctx {
+  std::recursive_mutex calls;  // held by each C call on the context
   int device;
   int sm_count;  // streaming multiprocessors of the device (grid sizing)
   gf::Geom geom;

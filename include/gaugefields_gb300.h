@@ -94,11 +94,18 @@ typedef struct gf_md_params {
 /* ---- context ------------------------------------------------------------ */
 /* Replaces the lattice/PE bookkeeping of Gaugefields_4D_MPILattice
  * (src/4D/mpi_jacc/gaugefields_4D_MPILattice.jl:34-121). L = {NX,NY,NZ,NT};
- * NX must be even (even/odd site order); one CUDA device per context. */
+ * NX must be even (even/odd site order); one CUDA device per context.
+ * A context runs one call at a time: calls from several threads wait for one
+ * another (its scratch memory serves them all), those of different contexts do
+ * not. */
 int gf_ctx_create(const int L[4], int device, gf_ctx** out);
 int gf_ctx_destroy(gf_ctx* ctx);
 /* Run all work of the context on a caller-owned cudaStream_t (NULL restores
- * the context's own stream). */
+ * the context's own stream). Under capture on such a stream, forces, flows,
+ * link updates, copies and the calls on a gf_stout use the fields and the stack
+ * that they are given (and the flows the context's scratch); the smeared
+ * gf_md_mom_update uses the context's own stack. Replays of one that uses the
+ * context's state must be ordered with its other calls. */
 int gf_ctx_set_stream(gf_ctx* ctx, void* cuda_stream);
 int gf_ctx_synchronize(gf_ctx* ctx);
 const char* gf_last_error(const gf_ctx* ctx);

@@ -94,3 +94,37 @@ def test_a_captured_force_touches_its_own_fields_only(pkg):
     torch.cuda.synchronize()
     for got, ref in zip(forces(), want):
         assert np.abs(got - ref).max() <= 1e-13 * np.abs(ref).max()
+
+
+def test_threads_of_one_context_wait_for_one_another(pkg):
+    """Forces, plaquettes and smeared links of two configurations from two
+    threads that share a context: bitwise those of one thread."""
+    import threading
+    L = (8, 8, 8, 16)
+    U = pkg.gauge_configuration(L, start="hot", seed=5)
+    V = U.similar().from_host(pkg.gauge_configuration(L, start="hot", seed=6).to_host())
+    action, smearing = wilson(pkg, U), pkg.stout_smearing(U)
+    F = {id(W): pkg.gauge_momenta(U) for W in (U, V)}
+
+    def results(W):
+        plaq = pkg.calculate_Plaquette(W)
+        pkg.md_force_(F[id(W)], action, W)
+        return plaq, F[id(W)].to_host(), pkg.smear(W, smearing).to_host()
+
+    want = {id(W): results(W) for W in (U, V)}
+    wrong, errors = [], []
+
+    def work(W):
+        try:
+            for _ in range(200):
+                got = results(W)
+                wrong.extend(1 for a, b in zip(got, want[id(W)]) if not np.array_equal(a, b))
+        except Exception as e:  # reported below: a thread's own would be lost
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(W,)) for W in (U, V)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors and not wrong
