@@ -62,6 +62,7 @@ SIGNATURES = {
     "gf_ctx_destroy": [_P],
     "gf_ctx_set_stream": [_P, _P],
     "gf_ctx_synchronize": [_P],
+    "gf_ctx_trim": [_P],
     "gf_ctx_volume": [_P, ctypes.POINTER(ctypes.c_int64)],
     "gf_field_alloc": [_P, _I, ctypes.POINTER(_P)],
     "gf_field_free": [_P],

@@ -73,6 +73,10 @@ class _Context:
     def sync(self):
         call("gf_ctx_synchronize", self.h, ctx=self.h)
 
+    def trim(self):
+        """Gives back the device memory kept only to save allocations."""
+        call("gf_ctx_trim", self.h, ctx=self.h)
+
     def set_stream(self, stream_handle):
         call("gf_ctx_set_stream", self.h, ctypes.c_void_p(stream_handle), ctx=self.h)
 

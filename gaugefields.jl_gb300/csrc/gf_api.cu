@@ -130,6 +130,7 @@ extern "C" int gf_ctx_create(const int L[4], int device, gf_ctx** out) {
   // the fixed-point copy of the links that most calls make: small ones at
   // once, so that the first call on a small lattice does not wait for them
   if (field_bytes(ctx->geom, GF_LINKFX) <= ((size_t)32 << 20)) ctx->w_linkfx = field_new(ctx, GF_LINKFX);
+  ctx_enlist(ctx);
   *out = ctx;
   return GF_OK;
   }
@@ -149,6 +150,7 @@ extern "C" int gf_stout_destroy(gf_stout* st);
 
 extern "C" int gf_ctx_destroy(gf_ctx* ctx) {
   if (!ctx) return GF_OK;
+  ctx_delist(ctx);
   cudaSetDevice(ctx->device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   field_delete(ctx->w_link64);
@@ -188,6 +190,13 @@ extern "C" int gf_ctx_set_stream(gf_ctx* ctx, void* cuda_stream) {
     GF_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     ctx->own_stream = 1;
   }
+  API_END(ctx)
+}
+
+extern "C" int gf_ctx_trim(gf_ctx* ctx) {
+  API_BEGIN(ctx)
+  need(ctx != nullptr, "gf_ctx_trim: null context");
+  ctx_trim(ctx);
   API_END(ctx)
 }
 

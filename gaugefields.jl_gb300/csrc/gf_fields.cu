@@ -39,21 +39,45 @@ void pool_trim(gf_pool* pool, bool close) {
   for (auto& k : kept) cudaFree(k.second);
 }
 
-// cudaMalloc, once more after the pool, and then the fixed-point copy of the
-// links, have given back what they keep
+// the contexts alive, for memory that they can spare
+static std::mutex g_contexts_lock;
+static std::vector<gf_ctx*> g_contexts;
+void ctx_enlist(gf_ctx* ctx) {
+  std::lock_guard<std::mutex> hold(g_contexts_lock);
+  g_contexts.push_back(ctx);
+}
+void ctx_delist(gf_ctx* ctx) {
+  std::lock_guard<std::mutex> hold(g_contexts_lock);
+  g_contexts.erase(std::remove(g_contexts.begin(), g_contexts.end(), ctx), g_contexts.end());
+}
+
+void ctx_trim(gf_ctx* ctx) {
+  pool_trim(ctx->pool.get(), false);
+  if (ctx->w_linkfx && !ctx->fx_hold && !ctx->fx_graph) {
+    field_delete(ctx->w_linkfx);  // cudaFree waits for the kernels that read it
+    ctx->w_linkfx = nullptr;
+  }
+}
+
+// cudaMalloc, once more after the pool, then the fixed-point copy of the links
+// and then the other contexts on the device (those that no call holds) have
+// given back what they keep
 static void* device_alloc(gf_ctx* ctx, size_t bytes) {
   void* p = nullptr;
   cudaError_t e = cudaMalloc(&p, bytes);
-  if (e == cudaErrorMemoryAllocation && ctx->pool) {
+  for (int stage = 0; stage < 3 && e == cudaErrorMemoryAllocation; ++stage) {
     cudaGetLastError();
-    pool_trim(ctx->pool.get(), false);
-    e = cudaMalloc(&p, bytes);
-    if (e == cudaErrorMemoryAllocation && ctx->w_linkfx && !ctx->fx_hold && !ctx->fx_graph) {
-      cudaGetLastError();
-      field_delete(ctx->w_linkfx);  // cudaFree waits for the kernels that read it
-      ctx->w_linkfx = nullptr;
-      e = cudaMalloc(&p, bytes);
+    if (stage == 0) pool_trim(ctx->pool.get(), false);
+    else if (stage == 1) ctx_trim(ctx);
+    else {
+      std::lock_guard<std::mutex> hold(g_contexts_lock);
+      for (gf_ctx* c : g_contexts) {
+        if (c == ctx || c->device != ctx->device || !c->calls.try_lock()) continue;
+        ctx_trim(c);
+        c->calls.unlock();
+      }
     }
+    e = cudaMalloc(&p, bytes);
   }
   if (e != cudaSuccess) {
     cudaGetLastError();

@@ -54,8 +54,8 @@ void count_launch();
 // Buffers of stout stacks kept for the next stack of the context (a stack is
 // made per calc_smearedU call; at 16^4 its nine cudaMalloc / cudaFree pairs took
 // 1.0 of 2.6 ms). Reuse is ordered by the context's stream. At most GF_POOL_CAP
-// bytes are kept; they go back when an allocation fails and with the context,
-// and a stack that outlives its context frees its buffers itself. Only
+// bytes are kept; they go back when an allocation (of any context) fails, with
+// gf_ctx_trim and with the context, and a stack that outlives its context frees its buffers itself. Only
 // buffers whose address never leaves the library are pooled.
 #define GF_POOL_CAP ((size_t)1 << 30)
 struct gf_pool {
@@ -155,6 +155,12 @@ gf_field* field_new(gf_ctx* ctx, int kind);
 gf_field* field_pooled(gf_ctx* ctx, int kind);
 // frees what the pool keeps; close: later releases free at once
 void pool_trim(gf_pool* pool, bool close);
+// gives back what the context keeps and does not need: the pool's buffers and
+// an idle fixed-point copy of the links
+void ctx_trim(gf_ctx* ctx);
+// contexts that an allocation of another one may trim
+void ctx_enlist(gf_ctx* ctx);
+void ctx_delist(gf_ctx* ctx);
 // a non-owning field of `kind` over scratch block `which` at byte offset `off`
 gf_field* arena_view(gf_ctx* ctx, int which, size_t off, int kind);
 void field_delete(gf_field* f);
@@ -226,8 +232,8 @@ inline FxField fx_view(const gf_field* f) { return FxField{(const char*)f->ptr};
 // when there is no memory for it or a graph is being captured: the fp64
 // kernels, a fifth as fast, then read the links in place. for_stack: for one of
 // the context's stacks, which captured graphs use the copy with.
-// An allocation of the context that fails takes it back, but not while a
-// driver holds it or once a graph has captured it.
+// An allocation that fails, of this or another context, takes it back, but not
+// while a driver holds it or once a graph has captured it.
 gf_field* fx_links(gf_ctx* ctx, const gf_field* U, bool for_stack = false);
 // `copy` null: the driver keeps none, and one left by an earlier call stays
 // reclaimable.

@@ -108,6 +108,11 @@ int gf_ctx_destroy(gf_ctx* ctx);
  * context's state must be ordered with its other calls. */
 int gf_ctx_set_stream(gf_ctx* ctx, void* cuda_stream);
 int gf_ctx_synchronize(gf_ctx* ctx);
+/* Gives back the device memory that the context keeps between calls only to
+ * save allocations: a fixed-point copy of the links (148 bytes a link, made by
+ * the first force or sum) and up to 1 GiB of stack buffers. Failing allocations
+ * of this library do so by themselves; other users of the device cannot. */
+int gf_ctx_trim(gf_ctx* ctx);
 const char* gf_last_error(const gf_ctx* ctx);
 int gf_ctx_volume(const gf_ctx* ctx, int64_t* out);
 

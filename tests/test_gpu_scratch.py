@@ -128,3 +128,30 @@ def test_threads_of_one_context_wait_for_one_another(pkg):
     for t in threads:
         t.join()
     assert not errors and not wrong
+
+
+def test_kept_memory_is_given_back(pkg):
+    """What a context keeps between calls only to save allocations goes back on
+    request, and to an allocation of another context that would fail."""
+    torch = pytest.importorskip("torch")
+    A = pkg.gauge_configuration(L24, start="hot", seed=11)
+    B = pkg.gauge_configuration(L24, start="cold")
+    A.ctx.trim()
+    idle = free_bytes(torch)
+    plaq = pkg.calculate_Plaquette(A)
+    top = pkg.smear(A, pkg.stout_smearing(A))
+    del top
+    assert free_bytes(torch) < idle - COPY  # the copy, and buffers of the stack
+    A.ctx.trim()
+    assert free_bytes(torch) == idle
+    pkg.calculate_Plaquette(A)
+    size = 4 * 24 ** 4 * 144
+    filler = torch.empty(free_bytes(torch) - size // 2, dtype=torch.uint8, device="cuda")
+    try:
+        B2 = B.similar()
+        assert pkg.calculate_Plaquette(A) == pytest.approx(plaq, rel=1e-13)
+        del B2
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    assert pkg.calculate_Plaquette(A) == plaq
