@@ -129,7 +129,13 @@ extern "C" int gf_ctx_create(const int L[4], int device, gf_ctx** out) {
   ctx->h_hash = (unsigned long long*)(ctx->h_result + 4);
   // the fixed-point copy of the links that most calls make: small ones at
   // once, so that the first call on a small lattice does not wait for them
-  if (field_bytes(ctx->geom, GF_LINKFX) <= ((size_t)32 << 20)) ctx->w_linkfx = field_new(ctx, GF_LINKFX);
+  if (field_bytes(ctx->geom, GF_LINKFX) <= ((size_t)32 << 20)) {
+    try {
+      ctx->w_linkfx = field_new(ctx, GF_LINKFX);
+    } catch (const gf_error& e) {
+      if (e.code != GF_ENOMEM) throw;  // the calls do without
+    }
+  }
   ctx_enlist(ctx);
   *out = ctx;
   return GF_OK;

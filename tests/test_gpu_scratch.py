@@ -155,3 +155,28 @@ def test_kept_memory_is_given_back(pkg):
         del filler
         torch.cuda.empty_cache()
     assert pkg.calculate_Plaquette(A) == plaq
+
+
+def test_a_context_without_memory_for_its_copy(pkg):
+    """A new context on a device that is nearly full does without the copy that
+    small lattices get at once."""
+    torch = pytest.importorskip("torch")
+    L = (14, 14, 14, 14)
+    want = pkg.calculate_Plaquette(pkg.gauge_configuration(L, start="cold"))
+    torch.empty(1, device="cuda")
+    filler, keep = [], 12 << 20  # the copy takes 22.8 MB
+    while free_bytes(torch) > keep + (2 << 20):
+        n = (free_bytes(torch) - keep) >> 21 << 21
+        try:
+            filler.append(torch.empty(n, dtype=torch.uint8, device="cuda"))
+        except torch.cuda.OutOfMemoryError:
+            break
+    try:
+        assert free_bytes(torch) < 20 << 20
+        U = pkg.api._Context(L)
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    V = pkg.Gaugefields4D(U)
+    pkg._lib.call("gf_cold_start", U.h, V.field.h)
+    assert pkg.calculate_Plaquette(V) == want
