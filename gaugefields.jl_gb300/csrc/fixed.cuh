@@ -36,6 +36,11 @@ typedef unsigned long long u64;
 // exponent of a matrix holding a NaN or an infinity; sums of exponents keep
 // it recognisable (every regular exponent sum is far below GF_FX_BAD / 2)
 #define GF_FX_BAD (1 << 24)
+// "exponent" of a matrix whose slot holds its fp64 entries (fx_graded). A sum of
+// exponents with one among them is at least GF_FX_F64_SUM, any other (up to
+// seven GF_FX_BAD) below.
+#define GF_FX_F64 (1 << 27)
+#define GF_FX_F64_SUM (15 << 23)
 
 struct fx_row {  // operand: row of a left factor, a = Re, b = Im
   int ah[3], al[3], bh[3], bl[3];
@@ -423,9 +428,10 @@ GF_HD float fx_leading(double d, int emax) {
 // spectral norm, max_i sum_j |(M^dag M)_ij| in fp32 from the leading bits, is
 // at most 1 (1 + 2^-10). It is 1 for a unitary matrix. False for a matrix that
 // is not finite.
-GF_HD bool fx_exponent_of(const double* m /* 18, row-major, re im */, int& emax, int& up) {
+// small: entries below 2^-7 of that unit.
+GF_HD bool fx_exponent_of(const double* m /* 18, row-major, re im */, int& emax, int& up, int& small) {
   emax = 1;
-  up = 0;
+  up = small = 0;
 #pragma unroll
   for (int i = 0; i < 18; ++i) {
     const int e = fx_exponent_field(m[i]);
@@ -455,12 +461,64 @@ GF_HD bool fx_exponent_of(const double* m /* 18, row-major, re im */, int& emax,
   }
   // bound < 3 * 72 < 4^4
   up = (bound > 1.0009765625f) + (bound > 4.00390625f) + (bound > 16.015625f) + (bound > 64.0625f);
+  const float tiny = 0.0078125f * (float)(1 << up);
+  small = 0;
+#pragma unroll
+  for (int i = 0; i < 18; ++i) small += fabsf(f[i]) < tiny;
   return true;
 }
+GF_HD bool fx_has_f64(int e) { return e >= GF_FX_F64_SUM; }
+
+// One exponent per matrix gives every entry the same absolute error, 2^-61 of
+// the norm. That is below fp64's rounding of the matrix, but an entry below
+// 2^-7 of the norm had more digits of its own in fp64. Where the small entries
+// are a pattern that products keep, results live off those digits: links near
+// the identity (weak fields; 15 small entries), near the diagonal (12), real
+// ones (9), SU(2) subgroups (8), rows or columns of another size (6). A matrix
+// with such a pattern is "graded": its slot keeps fp64, and what it enters is
+// computed in fp64. Exact zeros lose nothing, so entries below 2^-7 must
+// include one that is not zero. A Haar-random link is graded with probability
+// 10^-10 (each of its 18 numbers is small with probability 0.015).
+// small: bit i for entry i below 2^-7 2^(unit - 1023); returns whether they form
+// a pattern (zeros included).
+GF_HD bool fx_small_pattern(unsigned small) {
+  unsigned n = small - ((small >> 1) & 0x55555555u);
+  n = (n & 0x33333333u) + ((n >> 2) & 0x33333333u);
+  n = (n + (n >> 4)) & 0x0F0F0F0Fu;
+  n = (n + (n >> 8) + (n >> 16)) & 0xFFu;
+  bool line = false;
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    line = line || (small & (0x3Fu << (6 * k))) == (0x3Fu << (6 * k)) ||
+           (small & (0x30C3u << (2 * k))) == (0x30C3u << (2 * k));
+  return n >= 8 || line;
+}
+GF_HD bool fx_is_small(double d, int unit) {
+  return ((int)(fx_bits(d) >> 32) & 0x7FFFFFFF) < (int)((unsigned)(unit - 7) << 20);
+}
+GF_HD bool fx_small_nonzero(double d, int unit) { return fx_is_small(d, unit) && (fx_bits(d) << 1) != 0; }
+#define GF_FX_PATTERN_MIN 6  // the fewest small entries of a pattern
+GF_HD bool fx_graded(const double* m, int unit) {
+  unsigned small = 0;
+  bool any = false;
+#pragma unroll
+  for (int i = 0; i < 18; ++i) {
+    small |= (unsigned)fx_is_small(m[i], unit) << i;
+    any = any || fx_small_nonzero(m[i], unit);
+  }
+  return any && fx_small_pattern(small);
+}
+// an entry of a slot that holds fp64
+GF_HD int4 fx_pack64(double re, double im) {
+  const u64 a = fx_bits(re), b = fx_bits(im);
+  return make_int4((int)(unsigned)a, (int)(unsigned)(a >> 32), (int)(unsigned)b, (int)(unsigned)(b >> 32));
+}
+GF_HD double fx_unpack64(int lo, int hi) { return fx_from_bits(((u64)(unsigned)hi << 32) | (unsigned)lo); }
+
 // One matrix to fixed point; returns its exponent.
 GF_HD int fx_from_f64(const double* m, int4 out[9]) {
-  int emax, up;
-  if (!fx_exponent_of(m, emax, up)) {
+  int emax, up, small;
+  if (!fx_exponent_of(m, emax, up, small)) {
 #pragma unroll
     for (int i = 0; i < 9; ++i) out[i] = make_int4(0, 0, 0, 0);
     return GF_FX_BAD;
@@ -471,6 +529,24 @@ GF_HD int fx_from_f64(const double* m, int4 out[9]) {
     fx_split<0>(fx_mantissa(m[2 * i + 1], emax, up), out[i].z, out[i].w);
   }
   return emax - 1023 + up;
+}
+
+// One matrix to what its slot holds: fixed point, or fp64 if it is graded.
+GF_HD int fx_encode(const double* m, int4 out[9]) {
+  int emax, up, small;
+  if (!fx_exponent_of(m, emax, up, small)) {
+#pragma unroll
+    for (int i = 0; i < 9; ++i) out[i] = make_int4(0, 0, 0, 0);
+    return GF_FX_BAD;
+  }
+  const bool f64 = small >= GF_FX_PATTERN_MIN && fx_graded(m, emax + up);
+#pragma unroll
+  for (int i = 0; i < 9; ++i) {
+    fx_split<0>(fx_mantissa(m[2 * i], emax, up), out[i].x, out[i].y);
+    fx_split<0>(fx_mantissa(m[2 * i + 1], emax, up), out[i].z, out[i].w);
+    if (f64) out[i] = fx_pack64(m[2 * i], m[2 * i + 1]);
+  }
+  return f64 ? GF_FX_F64 : emax - 1023 + up;
 }
 
 // real and imaginary parts of the f_j, side by side: f at [2 j + im]

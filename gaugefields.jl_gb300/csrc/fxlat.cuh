@@ -2,13 +2,18 @@
 // shared by all of them and staple chains by rows.
 //
 // A fixed-point link or matrix field is tiled by 32 sites: per direction and
-// tile, int4 [9][32] (re.h, re.l, im.h, im.l) and the exponents int [32]. The
+// tile, int4 [9][32] (re.h, re.l, im.h, im.l; or two doubles, for a matrix kept
+// in fp64) and the exponents int [32]. The
 // elements of a matrix are then at constant distances (one address per
 // matrix, immediate offsets for its nine loads) and coalesced over sites.
 //
 // Blocks are 96 threads = 32 links of one direction x 3 rows, thread
 // t = 3 link + row: the rows of a link sit in the same warp or the next one,
 // so a matrix element that all three read is one transaction.
+//
+// A kernel runs its fixed-point arithmetic on whatever the slots hold and sums
+// the exponents beside it; a sum that shows an fp64 matrix (fx_has_f64) means that
+// the link's result is formed anew in fp64 (fxrows64.cuh) before it is stored.
 #pragma once
 #include "fixed.cuh"
 
@@ -17,6 +22,12 @@ namespace gf {
 #ifndef GF_FX_MINB
 #define GF_FX_MINB 7
 #endif
+// Up to so many sites the blocks of a stencil fit on the GPU at five per SM, and
+// the kernels take the registers that leaves: 8^4 trajectory 681 us, with seven
+// 721; at 24^4, where the GPU is full, the force takes 736 us with seven and 753
+// with six.
+#define GF_FX_FEW_MAX 6144
+#define GF_FX_FEW_MINB 5
 #define GF_FX_LINKS 32
 #define GF_FX_TILE (9 * 512 + 128)
 #define GF_FX_THREADS (3 * GF_FX_LINKS)
@@ -140,10 +151,11 @@ __device__ __forceinline__ double fx_unit(double c, int E) {
 // P <- keep P + coef c(M), c the su(3) coefficients of TA(M) for the 32
 // matrices M of a block (raw, exponents se); thread t serves link t % 32 and,
 // by t / 32, the coefficients (0, 1, 2), (3, 4, 7) or (5, 6).
+// Links whose products hold an fp64 matrix are left out (fx64_update_mom).
 __device__ __forceinline__ void fx_update_mom(const FxRaw& sh, const int* se, double* __restrict__ P, int mu, int s0,
                                               int V, double coef, double keep) {
   const int link = threadIdx.x & 31, part = threadIdx.x >> 5, s = s0 + link;
-  if (s >= V) return;
+  if (s >= V || fx_has_f64(se[link])) return;
   const int i = part == 2 ? 1 : 0, j = part == 0 ? 1 : 2;
   const int ij = 2 * (3 * i + j), ji = 2 * (3 * j + i);
   const i64 d1 = sh.v[1][link], d2 = sh.v[9][link], d3 = sh.v[17][link];
@@ -422,20 +434,41 @@ __device__ __forceinline__ int fx_norm_shift(float n, int e) {
   return ((k4 + 1) >> 1) - 40;
 }
 
-// fp64 view of a fixed-point field (fp64 kernels)
+// fp64 view of a fixed-point field: element by element, and whole matrices (fp64
+// kernels)
+struct FxMat64 {
+  FxMat m;
+  int e;
+  __device__ __forceinline__ double2 operator()(int el) const {
+    const int4 v = m(el);
+    if (e == GF_FX_F64) return make_double2(fx_unpack64(v.x, v.y), fx_unpack64(v.z, v.w));
+    return make_double2(fx_to_f64(fx_join(v.x, v.y), e), fx_to_f64(fx_join(v.z, v.w), e));
+  }
+};
+__device__ __forceinline__ FxMat64 fx_mat64(const FxField& F, int mu, int s, int V) {
+  return FxMat64{fx_mat(F, mu, s, V), fx_exp(F, mu, s, V)};
+}
 struct LinkSrcFx64 {
   FxField F;
   __device__ __forceinline__ mat3<double> operator()(int mu, int s, int V) const {
     mat3<double> m;
-    const FxMat M = fx_mat(F, mu, s, V);
-    const int e = fx_exp(F, mu, s, V);
+    const FxMat64 M = fx_mat64(F, mu, s, V);
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
-      const int4 v = M(k);
-      m.e[k / 3][k % 3] = mk(fx_to_f64(fx_join(v.x, v.y), e), fx_to_f64(fx_join(v.z, v.w), e));
+      const double2 v = M(k);
+      m.e[k / 3][k % 3] = mk(v.x, v.y);
     }
     return m;
   }
 };
+// one matrix into a field, in the form that it takes (fx_encode)
+__device__ __forceinline__ void fx_store64(char* p, int mu, int s, int V, const double* m) {
+  int4 f[9];
+  const int e = fx_encode(m, f);
+  char* o = p + fx_offset(mu, s, V);
+#pragma unroll
+  for (int k = 0; k < 9; ++k) *reinterpret_cast<int4*>(o + 512 * k) = f[k];
+  *reinterpret_cast<int*>(o + 9 * 512 - 12 * (s & 31)) = e;
+}
 
 }  // namespace gf

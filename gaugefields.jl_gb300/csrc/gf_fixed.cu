@@ -2,6 +2,7 @@
 // conversions, the plaquette sum and the Wilson force.
 #include "gf_internal.h"
 #include <algorithm>
+#include "fxrows64.cuh"
 #include "stencil.cuh"
 
 namespace gf {
@@ -13,7 +14,7 @@ __device__ __forceinline__ double2 fx_complex64(float4 v) {
   return make_double2(df_to_double(dfl(v.x, v.y)), df_to_double(dfl(v.z, v.w)));
 }
 template <typename E>
-__global__ void __launch_bounds__(128) k_to_fx(const E* __restrict__ in, char* __restrict__ out, int V) {
+__global__ void __launch_bounds__(128, 5) k_to_fx(const E* __restrict__ in, char* __restrict__ out, int V) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x, mu = blockIdx.y;
   if (s >= V) return;
   const E* b = in + (size_t)mu * 9 * V + s;
@@ -24,12 +25,7 @@ __global__ void __launch_bounds__(128) k_to_fx(const E* __restrict__ in, char* _
     m[2 * k] = v.x;
     m[2 * k + 1] = v.y;
   }
-  int4 f[9];
-  const int e = fx_from_f64(m, f);
-  char* o = out + fx_offset(mu, s, V);
-#pragma unroll
-  for (int k = 0; k < 9; ++k) *reinterpret_cast<int4*>(o + 512 * k) = f[k];
-  *reinterpret_cast<int*>(o + 9 * 512 - 12 * (s & 31)) = e;
+  fx_store64(out, mu, s, V, m);
 }
 
 void to_fx(gf_ctx* ctx, gf_field* dst, const gf_field* src) {
@@ -61,8 +57,18 @@ void fx_to_f64_field(gf_ctx* ctx, gf_field* dst, const gf_field* src) {
 // Integer-issue-bound: 2M sites (32^3 x 64) 7.16 ms in fp64, 1.68 ms here with
 // the conversion (0.4 ms, bandwidth-bound); 8^4 89 -> 25.6 us, the launches of
 // the conversion and the sum and one wait.
+// Links with an fp64 slot: the same row in fp64.
+__device__ __noinline__ double plaquette_row64(const FxField U, int mu, int nu, int s, int xpm, int xpn, int r, int V) {
+  row64 a = mul64<false>(load_row64<false>(fx_mat64(U, mu, s, V), r), fx_mat64(U, nu, xpm, V));
+  a = mul64<true>(a, fx_mat64(U, mu, xpn, V));
+  const row64 b = load_row64<false>(fx_mat64(U, nu, s, V), r);
+  double v = 0.0;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) v = fma(a.re[k], b.re[k], fma(a.im[k], b.im[k], v));
+  return v;
+}
 __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_MINB)
-    k_plaquette_fx(FxField U, Geom g, int items, SumOut to) {
+    k_plaquette_fx(FxField U, const __grid_constant__ Geom g, int items, SumOut to) {
   const int t = threadIdx.x, V = g.vol;
   const int link = t / 3, r = t - 3 * link;
   double v = 0.0;
@@ -76,6 +82,10 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_MINB)
     const int xpm = eo_of_lex(g, st.lex + fx_up(g, st, mu), st.par ^ 1);
     const int xpn = eo_of_lex(g, st.lex + fx_up(g, st, nu), st.par ^ 1);
     const int e = fx_exp(U, mu, s, V) + fx_exp(U, nu, xpm, V) + fx_exp(U, mu, xpn, V) + fx_exp(U, nu, s, V);
+    if (fx_has_f64(e)) {
+      v += plaquette_row64(U, mu, nu, s, xpm, xpn, r, V);
+      continue;
+    }
     fx_acc a = fx_row_mul<false>(fx_load_row<false>(fx_mat(U, mu, s, V), r), fx_mat(U, nu, xpm, V));
     a = fx_row_mul<true>(fx_operand<0>(a), fx_mat(U, mu, xpn, V));
     const fx_row b = fx_load_row<false>(fx_mat(U, nu, s, V), r);
@@ -107,14 +117,28 @@ void plaquette_start_fx(gf_ctx* ctx, const gf_field* F, int slot) {
 // four cycles: 81 per row product, 13 products). 24^4, conversion included:
 // 4.71 ms in fp64 arithmetic, 0.70 ms here. Seven blocks per SM (80
 // registers) measured 0.70 ms, six 0.73, five 0.74, eight (spills) 0.72.
-template <int AXES>
-__global__ void __launch_bounds__(GF_FX_THREADS * AXES, AXES > 1 ? 2 : GF_FX_MINB)
-    k_force_fx(FxField U, double* __restrict__ P, Geom g, double coef, double keep) {
+// Links with an fp64 slot among their staples: force_rows64, in the block's
+// first 96 threads.
+__device__ __noinline__ void force_rows64(const FxField U, double* P, const Geom& g, int mu, int s0, double coef,
+                                          double keep, FxRaw& sh, const int* se) {
+  const int t = threadIdx.x, link = t / 3, r = t - 3 * link, V = g.vol;
+  __syncthreads();  // sh has been read
+  if (t < GF_FX_THREADS && fx_has_f64(se[link])) {
+    const int s = min(s0 + link, V - 1);
+    share64(sh64(sh, link), r, mul64<true>(staple_row64(U, g, site_of(g, s), s, mu, r), fx_mat64(U, mu, s, V)));
+  }
+  __syncthreads();
+  if (t < GF_FX_THREADS) update_mom64(sh64(sh, t & 31), se, P, mu, s0, V, coef, keep);
+}
+template <int AXES, int MINB>
+__global__ void __launch_bounds__(GF_FX_THREADS * AXES, MINB)
+    k_force_fx(FxField U, double* __restrict__ P, const __grid_constant__ Geom g, double coef, double keep) {
   __shared__ FxRaw sh;
   __shared__ FxAxes<AXES> ax;
   __shared__ int se[GF_FX_LINKS];
   const int axis = AXES > 1 ? threadIdx.x / GF_FX_THREADS : 0, t = threadIdx.x - axis * GF_FX_THREADS;
   const int mu = blockIdx.x & 3, V = g.vol, s0 = (blockIdx.x >> 2) * GF_FX_LINKS;
+  bool f64 = false;
   {
     const int link = t / 3, r = t - 3 * link;
     const int s = min(s0 + link, V - 1);
@@ -124,11 +148,14 @@ __global__ void __launch_bounds__(GF_FX_THREADS * AXES, AXES > 1 ? 2 : GF_FX_MIN
     if (axis == 0) {
       // |V| <= 6: three bits down to serve as an operand
       fx_share(sh, link, r, fx_row_mul<true>(fx_operand<3>(acc), fx_mat(U, mu, s, V)));
-      if (r == 0) se[link] = ea + 3 + fx_exp(U, mu, s, V);
+      const int e = ea + 3 + fx_exp(U, mu, s, V);
+      if (r == 0) se[link] = e;
+      f64 = fx_has_f64(e);
     }
   }
-  __syncthreads();
+  const bool any64 = __syncthreads_or(f64);
   if (axis == 0) fx_update_mom(sh, se, P, mu, s0, V, -coef, keep);
+  if (any64) force_rows64(U, P, g, mu, s0, -coef, keep, sh, se);
 }
 
 gf_field* fx_links(gf_ctx* ctx, const gf_field* U, bool for_stack) {
@@ -158,7 +185,8 @@ gf_field* fx_links(gf_ctx* ctx, const gf_field* U, bool for_stack) {
 void wilson_force_fx(gf_ctx* ctx, const gf_field* F, gf_field* P, double coef, double keep) {
   const int nb = 4 * blocks_for(ctx->geom.vol, GF_FX_LINKS);
   const int axes = ctx->geom.vol <= GF_FX_SPLIT_MAX ? 3 : 1;
-  auto kern = axes == 3 ? k_force_fx<3> : k_force_fx<1>;
+  auto kern = axes == 3 ? k_force_fx<3, 2>
+                        : (ctx->geom.vol <= GF_FX_FEW_MAX ? k_force_fx<1, GF_FX_FEW_MINB> : k_force_fx<1, GF_FX_MINB>);
   kern<<<nb, axes * GF_FX_THREADS, 0, ctx->stream>>>(fx_view(F), (double*)P->ptr, ctx->geom, coef, keep);
   GF_CHECK_LAUNCH();
 }

@@ -3,6 +3,7 @@
 // by integer multiply-add issue; the force on 65,520 sites: 5.95 ms in fp64
 // arithmetic, 0.65 ms here.
 #include "gf_internal.h"
+#include "fxrows64.cuh"
 #include "stencil.cuh"
 #include <algorithm>
 
@@ -83,10 +84,23 @@ __device__ __forceinline__ int fx_steps(const Geom& g, const Site& st, int mu, i
   return (n - c) * g.stride[mu];
 }
 
+// row r of a rectangle's product in fp64, times row r of U_nu(x)
+__device__ __noinline__ double rect_row64(const FxField U, int mu, int nu, int s, int xm, int xmn, int xnn, int xn,
+                                          int r, int V) {
+  row64 a = mul64<false>(load_row64<false>(fx_mat64(U, mu, s, V), r), fx_mat64(U, nu, xm, V));
+  a = mul64<false>(a, fx_mat64(U, nu, xmn, V));
+  a = mul64<true>(mul64<true>(a, fx_mat64(U, mu, xnn, V)), fx_mat64(U, nu, xn, V));
+  const row64 b = load_row64<false>(fx_mat64(U, nu, s, V), r);
+  double v = 0.0;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) v = fma(a.re[k], b.re[k], fma(a.im[k], b.im[k], v));
+  return v;
+}
+
 // Sum over sites and planes of Re tr of the 1x2 and 2x1 rectangles, one
 // partial per block; a work item is one plane of 32 sites.
 __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_MINB)
-    k_rect_sum_fx(FxField U, Geom g, int items, SumOut to) {
+    k_rect_sum_fx(FxField U, const __grid_constant__ Geom g, int items, SumOut to) {
   const int t = threadIdx.x, V = g.vol;
   const int link = t / 3, r = t - 3 * link;
   double v = 0.0;
@@ -110,6 +124,10 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_MINB)
     FxChain c{U, V, {}, fx_exp(U, mu, s, V) + fx_exp(U, nu, s, V)};
     c.mul<false>(fx_load_row<false>(fx_mat(U, mu, s, V), r), nu, xm).mul<false>(nu, xmn);
     c.mul<true>(mu, xnn).mul<true>(nu, xn);
+    if (fx_has_f64(c.e)) {
+      v += rect_row64(U, mu, nu, s, xm, xmn, xnn, xn, r, V);
+      continue;
+    }
     const fx_row b = fx_load_row<false>(fx_mat(U, nu, s, V), r);
     fx_sum d = fx_zero_sum();
 #pragma unroll
@@ -240,6 +258,59 @@ __device__ __forceinline__ fx_acc fx_loops_row(const FxField& U, const Geom& g, 
   return acc;
 }
 
+// the same row in fp64, in the chains of fx_loops_row
+__device__ __forceinline__ row64 loops_row64(const FxField& U, const Geom& g, const Site& st, int s, int mu, int r,
+                                             double cp, double cr) {
+  const int V = g.vol;
+  row64 acc = zero64(), far = zero64();
+  const int m1 = fx_steps(g, st, mu, 1), m2 = fx_steps(g, st, mu, 2), mm = fx_steps(g, st, mu, -1);
+  const int xm = eo_of_lex(g, st.lex + m1, st.par ^ 1), x2m = eo_of_lex(g, st.lex + m2, st.par);
+  const int xmm = eo_of_lex(g, st.lex + mm, st.par ^ 1);
+#pragma unroll 1
+  for (int k = 2; k < 8; ++k) {
+    const int nu = (mu + (k >> 1)) & 3;
+    const bool low = k & 1;
+    const int n1 = fx_steps(g, st, nu, low ? -1 : 1), n2 = fx_steps(g, st, nu, low ? -2 : 2);
+    const int xn = eo_of_lex(g, st.lex + n1, st.par ^ 1), x2n = eo_of_lex(g, st.lex + n2, st.par);
+    const int xmn = eo_of_lex(g, st.lex + m1 + n1, st.par), xmmn = eo_of_lex(g, st.lex + mm + n1, st.par);
+    const int xmnn = low ? eo_of_lex(g, st.lex + m1 + n2, st.par ^ 1) : xmn;
+    const int x2mn = low ? eo_of_lex(g, st.lex + m2 + n1, st.par ^ 1) : x2m;
+    const FxMat64 start = fx_mat64(U, nu, low ? xn : s, V);
+    const row64 first = low ? load_row64<true>(start, r) : load_row64<false>(start, r);
+    row64 t = mul64(first, fx_mat64(U, nu, low ? x2n : xn, V), low);  // (a), (b)
+    t = mul64(mul64<false>(t, fx_mat64(U, mu, x2n, V)), fx_mat64(U, nu, xmnn, V), !low);
+    // (e), (f)
+    const row64 te = mul64(load_row64<true>(fx_mat64(U, mu, xmm, V), r), fx_mat64(U, nu, low ? xmmn : xmm, V), low);
+    add64(t, mul64<false>(mul64<false>(te, fx_mat64(U, mu, xmmn, V)), fx_mat64(U, mu, xn, V)));
+    const row64 p = mul64<false>(first, fx_mat64(U, mu, xn, V));
+    add64(far, mul64(mul64<false>(p, fx_mat64(U, mu, xmn, V)), fx_mat64(U, nu, x2mn, V), !low));  // (c), (d)
+    row64 w = zero64();
+    add64(w, p, cp);
+    add64(w, t, cr);
+    add64(acc, mul64(w, fx_mat64(U, nu, low ? xmn : xm, V), !low));
+  }
+  add64(acc, mul64<true>(far, fx_mat64(U, mu, xm, V)), cr);
+  return acc;
+}
+template <bool DSDU>
+__device__ __noinline__ void loops_rows64(const FxField U, double* P, char* D, const Geom& g, int mu, int s0, double cp,
+                                          double cr, double keep, FxRaw& sh, const int* se) {
+  const int t = threadIdx.x, link = t / 3, r = t - 3 * link, V = g.vol;
+  __syncthreads();  // sh has been read
+  if (fx_has_f64(se[link])) {
+    const int s = min(s0 + link, V - 1);
+    row64 a = loops_row64(U, g, site_of(g, s), s, mu, r, cp, cr);
+    if (!DSDU) a = mul64<true>(a, fx_mat64(U, mu, s, V));
+    share64(sh64(sh, link), r, a);
+  }
+  __syncthreads();
+  if (!DSDU) {
+    update_mom64(sh64(sh, t & 31), se, P, mu, s0, V, -1.0, keep);
+  } else if (t < GF_FX_LINKS && s0 + t < V && fx_has_f64(se[t])) {
+    store_field64(sh64(sh, t), D, mu, s0 + t, V, true);
+  }
+}
+
 // P <- keep P + c(U (cp S + cr R)), or (DSDU) D = cp S + cr R. Four blocks per
 // SM (168 registers): 3.30 ms at 24^4, five 3.36, six 3.81.
 #ifndef GF_FX_LOOPS_MINB
@@ -247,8 +318,8 @@ __device__ __forceinline__ fx_acc fx_loops_row(const FxField& U, const Geom& g, 
 #endif
 template <bool DSDU>
 __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_LOOPS_MINB)
-    k_loops_fx(FxField U, double* __restrict__ P, char* __restrict__ D, Geom g, fx_scalar cp, fx_scalar cr,
-               double keep) {
+    k_loops_fx(FxField U, double* __restrict__ P, char* __restrict__ D, const __grid_constant__ Geom g, fx_scalar cp, fx_scalar cr, double cp64,
+               double cr64, double keep) {
   __shared__ union {
     FxRaw m;
     float n[3][GF_FX_LINKS];
@@ -261,21 +332,26 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_LOOPS_MINB)
   const Site st = site_of(g, s);
   int ea;
   fx_acc a = fx_loops_row(U, g, st, s, mu, r, cp, cr, ea, park[0] + t);
+  const int e = ea + 3 + fx_exp(U, mu, s, V);
+  const bool f64 = fx_has_f64(DSDU ? ea : e);
+  if (r == 0) se[link] = DSDU ? ea : e;
+  bool any64;
   if (DSDU) {
     sh.n[r][link] = fx_square(a);
-    __syncthreads();
-    if (sx >= V) return;
-    const int k = fx_norm_shift(sh.n[0][link] + sh.n[1][link] + sh.n[2][link], ea);
-    const size_t off = fx_offset(mu, s, V);
+    any64 = __syncthreads_or(f64);
+    if (sx < V && !f64) {
+      const int k = fx_norm_shift(sh.n[0][link] + sh.n[1][link] + sh.n[2][link], ea);
+      const size_t off = fx_offset(mu, s, V);
 #pragma unroll
-    for (int j = 0; j < 3; ++j) fx_store(D, off, 3 * j + r, fx_shift(a.re[j], k), -fx_shift(a.im[j], k));
-    if (r == 0) fx_store_exp(D, off, s, ea + k);
-    return;
+      for (int j = 0; j < 3; ++j) fx_store(D, off, 3 * j + r, fx_shift(a.re[j], k), -fx_shift(a.im[j], k));
+      if (r == 0) fx_store_exp(D, off, s, ea + k);
+    }
+  } else {
+    fx_share(sh.m, link, r, fx_row_mul<true>(fx_operand<3>(a), fx_mat(U, mu, s, V)));
+    any64 = __syncthreads_or(f64);
+    fx_update_mom(sh.m, se, P, mu, s0, V, -1.0, keep);
   }
-  fx_share(sh.m, link, r, fx_row_mul<true>(fx_operand<3>(a), fx_mat(U, mu, s, V)));
-  if (r == 0) se[link] = ea + 3 + fx_exp(U, mu, s, V);
-  __syncthreads();
-  fx_update_mom(sh.m, se, P, mu, s0, V, -1.0, keep);
+  if (any64) loops_rows64<DSDU>(U, P, D, g, mu, s0, cp64, cr64, keep, sh.m, se);
 }
 
 void loops_fx(gf_ctx* ctx, const gf_field* F, gf_field* P, gf_field* D, double cp, double cr, double keep) {
@@ -287,10 +363,11 @@ void loops_fx(gf_ctx* ctx, const gf_field* F, gf_field* P, gf_field* D, double c
   const int nb = 4 * blocks_for(ctx->geom.vol, GF_FX_LINKS);
   ProfScope prof(ctx, GF_K_RECT);
   if (D)
-    k_loops_fx<true><<<nb, GF_FX_THREADS, 0, ctx->stream>>>(fx_view(F), nullptr, (char*)D->ptr, ctx->geom, p, q, 0.0);
+    k_loops_fx<true><<<nb, GF_FX_THREADS, 0, ctx->stream>>>(fx_view(F), nullptr, (char*)D->ptr, ctx->geom, p, q, cp,
+                                                            cr, 0.0);
   else
-    k_loops_fx<false><<<nb, GF_FX_THREADS, 0, ctx->stream>>>(fx_view(F), (double*)P->ptr, nullptr, ctx->geom, p, q,
-                                                             keep);
+    k_loops_fx<false><<<nb, GF_FX_THREADS, 0, ctx->stream>>>(fx_view(F), (double*)P->ptr, nullptr, ctx->geom, p, q, cp,
+                                                             cr, keep);
   GF_CHECK_LAUNCH();
 }
 

@@ -5,6 +5,7 @@
 // 12-real shadow copy for the mixed-precision force path. One kernel for every
 // precision form: fp64 storage, fixed-point arithmetic of fp64 class.
 #include "gf_internal.h"
+#include "fxrows64.cuh"
 
 namespace gf {
 
@@ -150,19 +151,32 @@ __device__ __forceinline__ int fx_unitarise(fx_acc w[3]) {
   return 3;
 }
 
+// whether a link's update takes the fp64 path (update_link64)
+__device__ __forceinline__ bool fx_patterned(const double* m, int unit) {
+  unsigned small = 0;
+#pragma unroll
+  for (int i = 0; i < 18; ++i) small |= (unsigned)fx_is_small(m[i], unit) << i;
+  return fx_small_pattern(small);
+}
 // links of a matrix from fp64, the exponent from its Frobenius norm
-__device__ __forceinline__ int fx_from_f64_fast(const double* m, int4 out[9]) {
+__device__ __forceinline__ int fx_from_f64_fast(const double* m, int4 out[9], bool& patterned) {
   int emax = 1;
 #pragma unroll
   for (int i = 0; i < 18; ++i) emax = max(emax, fx_exponent_field(m[i]));
-  float n = 0.f;
+  float n = 0.f, f[18];
 #pragma unroll
   for (int i = 0; i < 18; ++i) {
-    const float f = fx_leading(m[i], emax);
-    n = fmaf(f, f, n);
+    f[i] = fx_leading(m[i], emax);
+    n = fmaf(f[i], f[i], n);
   }
   const int up = (n > 0.999f) + (n > 3.996f) + (n > 15.98f) + (n > 63.9f);
   const bool bad = emax == 0x7FF;
+  // entries below 2^-7 of the spectral norm, half the Frobenius norm's power of two
+  const float tiny = 0.00390625f * (float)(1 << up);
+  int small = 0;
+#pragma unroll
+  for (int i = 0; i < 18; ++i) small += fabsf(f[i]) < tiny;
+  patterned = small >= GF_FX_PATTERN_MIN && !bad && fx_patterned(m, emax + up - 1);
 #pragma unroll
   for (int i = 0; i < 9; ++i) {
     fx_split<0>(bad ? 0 : fx_mantissa(m[2 * i], emax, up), out[i].x, out[i].y);
@@ -171,9 +185,10 @@ __device__ __forceinline__ int fx_from_f64_fast(const double* m, int4 out[9]) {
   return bad ? GF_FX_BAD : emax - 1023 + up;
 }
 
-// an element of a unitary matrix, exponent 0
-__device__ __forceinline__ int4 fx_unitary_element(double2 v, bool ok) {
+// an element of a unitary matrix, exponent 0, or kept in fp64
+__device__ __forceinline__ int4 fx_unitary_element(double2 v, bool ok, bool f64) {
   int4 o;
+  if (f64) return fx_pack64(v.x, v.y);
   fx_split<0>(ok ? fx_mantissa(v.x, 1023, 0) : 0, o.x, o.y);
   fx_split<0>(ok ? fx_mantissa(v.y, 1023, 0) : 0, o.z, o.w);
   return o;
@@ -188,6 +203,52 @@ __device__ __forceinline__ fx_acc fx_shared_row(const FxRaw& m, int link, int r)
   return v;
 }
 
+// W = exp(i eps P) U of one link in fp64, where U is near the identity or has
+// another pattern of small entries (fx_small_pattern; exact zeros count, for
+// what the momentum puts in their place): stored like the others.
+template <bool REUNIT>
+__device__ __noinline__ void update_link64(const double2* Uin, double2* Uout, const double* __restrict__ P, int mu, int s,
+                                           int V, double eps, float4* sh32, char* fx) {
+  const double* p = P + (size_t)mu * 8 * V + s;
+  double c[8];
+#pragma unroll
+  for (int a = 0; a < 8; ++a) c[a] = 0.5 * eps * p[(size_t)a * V];
+  mat3<double> q;
+  const double d = c[7] * 0.57735026918962576451;
+  q.e[0][0] = mk(c[2] + d, 0.0);
+  q.e[1][1] = mk(d - c[2], 0.0);
+  q.e[2][2] = mk(-2.0 * d, 0.0);
+  q.e[0][1] = mk(c[0], -c[1]);
+  q.e[0][2] = mk(c[3], -c[4]);
+  q.e[1][2] = mk(c[5], -c[6]);
+  double n2 = 2.0 * (c[0] * c[0] + c[1] * c[1] + c[3] * c[3] + c[4] * c[4] + c[5] * c[5] + c[6] * c[6]);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    n2 += q.e[i][i].re * q.e[i][i].re;
+#pragma unroll
+    for (int j = 0; j < i; ++j) q.e[i][j] = conj(q.e[j][i]);
+  }
+  // |X|^2 <= (2/3) tr X^2: halved to |X| <= 1, and squared afterwards
+  int halvings = 0;
+  for (double x = n2 * (2.0 / 3.0); x > 1.0 && x <= 1.7976931348623157e308; x *= 0.25) ++halvings;
+  mat3<double> E = expiq(scale(scalbn(1.0, -halvings), q));
+#pragma unroll 1
+  for (int k = 0; k < halvings; ++k) E = mul_nn(E, E);
+  mat3<double> u;
+  const double2* b = Uin + (size_t)mu * 9 * V + s;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) u.e[k / 3][k % 3] = mk(b[(size_t)k * V].x, b[(size_t)k * V].y);
+  u = mul_nn(E, u);
+  if (REUNIT) reunitarize(u);
+  LinkFull<double>::store(Uout, mu, s, V, u);
+  if (sh32) {
+    mat3<float> h;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) h.e[k / 3][k % 3] = mk((float)u.e[k / 3][k % 3].re, (float)u.e[k / 3][k % 3].im);
+    Link12f::store(sh32, mu, s, V, h);
+  }
+  if (fx) fx_store64(fx, mu, s, V, &u.e[0][0].re);
+}
 // blocks per SM of the link update
 #ifndef GF_FX_UPDATE_MINB
 #define GF_FX_UPDATE_MINB 4
@@ -201,8 +262,8 @@ __device__ __forceinline__ fx_acc fx_shared_row(const FxRaw& m, int link, int r)
 // fp64 kernel's by 1.6e-16, the double-float one's by 6.2e-15.
 template <bool REUNIT>
 __global__ void __launch_bounds__(128, GF_FX_UPDATE_MINB)
-    k_link_update_fx(const double2* Uin, double2* Uout, const double* __restrict__ P, Geom g, fx_scalar eps,
-                     float4* __restrict__ sh32, char* __restrict__ fx) {
+    k_link_update_fx(const double2* Uin, double2* Uout, const double* __restrict__ P, const __grid_constant__ Geom g, fx_scalar eps,
+                     double eps64, float4* __restrict__ sh32, char* __restrict__ fx) {
   const int V = g.vol, mu = blockIdx.y, s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= V) return;
   constexpr int rows = REUNIT ? 2 : 3;  // re-unitarisation rebuilds row 3
@@ -226,7 +287,12 @@ __global__ void __launch_bounds__(128, GF_FX_UPDATE_MINB)
       m[2 * k] = v.x;
       m[2 * k + 1] = v.y;
     }
-    eu = fx_from_f64_fast(m, u);
+    bool patterned;
+    eu = fx_from_f64_fast(m, u, patterned);
+    if (patterned) {
+      update_link64<REUNIT>(Uin, Uout, P, mu, s, V, eps64, sh32, fx);
+      return;
+    }
   }
   if (e > GF_FX_BAD / 2) eu = GF_FX_BAD;
   fx_acc w[3];
@@ -274,20 +340,26 @@ __global__ void __launch_bounds__(128, GF_FX_UPDATE_MINB)
     // the fixed-point copy of what was stored, as k_to_fx makes it
     int4 el[9];
     const size_t off = fx_offset(mu, s, V);
+    double m[18];
+    int ef;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      m[2 * k] = v[k].x;
+      m[2 * k + 1] = v[k].y;
+    }
     if (REUNIT) {
       // a unitary matrix has exponent 0
+      int small = 0;
 #pragma unroll
-      for (int k = 0; k < 9; ++k) el[k] = fx_unitary_element(v[k], fine == 3);
-      fx_store_exp(fx, off, s, fine == 3 ? 0 : GF_FX_BAD);
+      for (int k = 0; k < 18; ++k) small += fx_is_small(m[k], 1023);
+      const bool f64 = small >= GF_FX_PATTERN_MIN && fine == 3 && fx_graded(m, 1023);
+      ef = f64 ? GF_FX_F64 : (fine == 3 ? 0 : GF_FX_BAD);
+#pragma unroll
+      for (int k = 0; k < 9; ++k) el[k] = fx_unitary_element(v[k], fine == 3, f64);
     } else {
-      double m[18];
-#pragma unroll
-      for (int k = 0; k < 9; ++k) {
-        m[2 * k] = v[k].x;
-        m[2 * k + 1] = v[k].y;
-      }
-      fx_store_exp(fx, off, s, fx_from_f64(m, el));
+      ef = fx_encode(m, el);
     }
+    *reinterpret_cast<int*>(fx + off + 9 * 512 - 12 * (s & 31)) = ef;
 #pragma unroll
     for (int k = 0; k < 9; ++k) *reinterpret_cast<int4*>(fx + off + 512 * k) = el[k];
   }
@@ -302,11 +374,13 @@ struct FxUpdateRows {
   FxOperand u;  // U, then (no re-unitarisation) the fp64 result
   int eu[GF_FX_LINKS];
   int fine[GF_FX_LINKS];
+  int patterned[GF_FX_LINKS];     // the link's update runs in fp64
+  unsigned small[3][GF_FX_LINKS];  // by rows: small entries of the result, bit 6 if one is not zero
 };
 template <bool REUNIT>
 __global__ void __launch_bounds__(GF_FX_THREADS, 4)
-    k_link_update_rows_fx(const double2* Uin, double2* Uout, const double* __restrict__ P, Geom g, fx_scalar eps,
-                          float4* __restrict__ sh32, char* __restrict__ fx) {
+    k_link_update_rows_fx(const double2* Uin, double2* Uout, const double* __restrict__ P, const __grid_constant__ Geom g, fx_scalar eps,
+                          double eps64, float4* __restrict__ sh32, char* __restrict__ fx) {
   __shared__ FxUpdateRows sh;
   const int V = g.vol, mu = blockIdx.y, link = threadIdx.x & 31, r = threadIdx.x >> 5;
   const int sx = blockIdx.x * GF_FX_LINKS + link, s = min(sx, V - 1);
@@ -338,7 +412,9 @@ __global__ void __launch_bounds__(GF_FX_THREADS, 4)
       m[2 * k + 1] = v.y;
     }
     int4 u[9];
-    sh.eu[link] = fx_from_f64_fast(m, u);
+    bool patterned;
+    sh.eu[link] = fx_from_f64_fast(m, u, patterned);
+    sh.patterned[link] = patterned;
 #pragma unroll
     for (int k = 0; k < 9; ++k) sh.u.v[k][link] = u[k];
   }
@@ -373,8 +449,20 @@ __global__ void __launch_bounds__(GF_FX_THREADS, 4)
   int4 el[3];
   int ef = fine == 3 ? 0 : GF_FX_BAD;
   if (fx && REUNIT) {
+    unsigned small = 0;
 #pragma unroll
-    for (int j = 0; j < 3; ++j) el[j] = fx_unitary_element(v[j], fine == 3);
+    for (int j = 0; j < 3; ++j) {
+      small |= (unsigned)fx_is_small(v[j].x, 1023) << (2 * j) | (unsigned)fx_is_small(v[j].y, 1023) << (2 * j + 1);
+      small |= (unsigned)(fx_small_nonzero(v[j].x, 1023) || fx_small_nonzero(v[j].y, 1023)) << 6;
+    }
+    sh.small[r][link] = small;
+    __syncthreads();
+    const unsigned a = sh.small[0][link], b = sh.small[1][link], c = sh.small[2][link];
+    const bool f64 =
+        fine == 3 && ((a | b | c) & 64) && fx_small_pattern((a & 63) | (b & 63) << 6 | (c & 63) << 12);
+    if (f64) ef = GF_FX_F64;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) el[j] = fx_unitary_element(v[j], fine == 3, f64);
   } else if (fx) {
     double2* x = reinterpret_cast<double2*>(sh.u.v) + link;
     __syncthreads();
@@ -387,16 +475,22 @@ __global__ void __launch_bounds__(GF_FX_THREADS, 4)
       m[2 * k] = x[k * GF_FX_LINKS].x;
       m[2 * k + 1] = x[k * GF_FX_LINKS].y;
     }
-    int emax, up;
-    const bool bad = !fx_exponent_of(m, emax, up);
-    ef = bad ? GF_FX_BAD : emax - 1023 + up;
+    int emax, up, small;
+    const bool bad = !fx_exponent_of(m, emax, up, small);
+    const bool f64 = !bad && small >= GF_FX_PATTERN_MIN && fx_graded(m, emax + up);
+    ef = bad ? GF_FX_BAD : (f64 ? GF_FX_F64 : emax - 1023 + up);
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       fx_split<0>(bad ? 0 : fx_mantissa(v[j].x, emax, up), el[j].x, el[j].y);
       fx_split<0>(bad ? 0 : fx_mantissa(v[j].y, emax, up), el[j].z, el[j].w);
+      if (f64) el[j] = fx_pack64(v[j].x, v[j].y);
     }
   }
   if (sx >= V) return;
+  if (sh.patterned[link]) {
+    if (r == 2) update_link64<REUNIT>(Uin, Uout, P, mu, s, V, eps64, sh32, fx);
+    return;
+  }
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
     const int k = 3 * r + j;
@@ -406,7 +500,7 @@ __global__ void __launch_bounds__(GF_FX_THREADS, 4)
           make_float2((float)v[j].x, (float)v[j].y);
     if (fx) *reinterpret_cast<int4*>(fx + off + 512 * k) = el[j];
   }
-  if (fx && r == 0) fx_store_exp(fx, off, s, ef);
+  if (fx && r == 0) *reinterpret_cast<int*>(fx + off + 9 * 512 - 12 * (s & 31)) = ef;
 }
 
 // The update writes the fixed-point copy itself: a launch and the copy's pass
@@ -437,7 +531,7 @@ static void update_links(gf_ctx* ctx, gf_field* W, const gf_field* P, double eps
   auto kern = rows ? (reunit ? k_link_update_rows_fx<true> : k_link_update_rows_fx<false>)
                    : (reunit ? k_link_update_fx<true> : k_link_update_fx<false>);
   kern<<<grid, threads, 0, ctx->stream>>>((const double2*)U->ptr, (double2*)W->ptr, (const double*)P->ptr, ctx->geom,
-                                      fx_scalar_of(eps), shadow32 ? (float4*)shadow32->ptr : nullptr,
+                                      fx_scalar_of(eps), eps, shadow32 ? (float4*)shadow32->ptr : nullptr,
                                       fx && fused ? (char*)fx->ptr : nullptr);
   GF_CHECK_LAUNCH();
   if (fx && !fused) to_fx(ctx, fx, W);
