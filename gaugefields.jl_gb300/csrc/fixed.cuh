@@ -233,11 +233,11 @@ GF_HD void fx_scale_row(fx_acc& v, const fx_scalar& c) {
 // imaginary parts, which two threads evaluate side by side. They are returned
 // in units of 2^(guard - 60), as are their derivatives in c1 and c0 (of q).
 // ---------------------------------------------------------------------------
-#define GF_FX_CH_TERMS 64
-#define GF_FX_CH_SCALES 5
+#define GF_FX_CH_TERMS 48
+#define GF_FX_CH_SCALES 3
 
 // 2^(s n) / n! in units of 2^(base - 60), rounded
-GF_HD constexpr int fx_kappa_base(int s) { return s == 0 ? 0 : (s == 1 ? 1 : (s == 2 ? 3 : (s == 3 ? 8 : 19))); }
+GF_HD constexpr int fx_kappa_base(int s) { return s == 0 ? 0 : (s == 1 ? 1 : 3); }
 struct fx_kappa {
   i64 k[GF_FX_CH_SCALES][GF_FX_CH_TERMS];
 };
@@ -298,19 +298,25 @@ struct fx_plan {
   int squares;  // squarings of the result, pow2 - series
   int guard;
   int terms;
+  bool beyond;  // with derivatives: |X| may exceed 4, which the series does not serve
 };
 // Terms: lam^n / n! < 2^-62 from n = terms - 4 on; the derivatives of the n-th
 // power's coefficients go as n lam^(n - 4), so they need the four more.
 // Without derivatives the series runs to |X| <= 2 and larger exponentials are
-// squared from it. With them it takes |X| <= 16 (larger ones are not summed to
-// the end) and the guard bits follow the largest coefficient, a derivative of
-// at most lam e^lam / 2 (1 / |q|)^4, half of it in each part.
+// squared from it. With them it serves |X| <= 4, the guard bits following the
+// largest coefficient, a derivative of at most lam e^lam / 2 (1 / |q|)^4, half of
+// it in each part: six bits at |X| = 4. (Sixteen would take 25 of the 60 bits:
+// exp(iX) was off by 5e-14 at |X| = 6 and 3e-8 at 16.) Larger X: the caller's.
 template <bool DERIV>
 GF_HD fx_plan fx_series(float lam) {
   fx_plan p;
   p.pow2 = 0;
   for (float x = lam; x > 1.f && p.pow2 < 60; x *= 0.5f) ++p.pow2;
-  if (DERIV && p.pow2 > GF_FX_CH_SCALES - 1) p.pow2 = GF_FX_CH_SCALES - 1;
+  p.beyond = DERIV && p.pow2 > GF_FX_CH_SCALES - 1;
+  if (p.beyond) {
+    p.pow2 = GF_FX_CH_SCALES - 1;
+    lam = 4.f;
+  }
   p.series = DERIV || p.pow2 < 1 ? p.pow2 : 1;
   p.squares = p.pow2 - p.series;
   for (int k = 0; k < p.squares; ++k) lam *= 0.5f;

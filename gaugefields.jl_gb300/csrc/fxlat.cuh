@@ -323,9 +323,9 @@ __device__ __forceinline__ int4 fx_herm_element(const fx_herm& q, int i, int j) 
 
 // Plan, operand and coefficients of exp(iX) for a block's links; thread per
 // link, im = 0 or 1. b: derivatives, df_j/dc1 at [2 j + im] and df_j/dc0 at
-// [6 + 2 j + im].
+// [6 + 2 j + im]. True if X is beyond the derivatives' series.
 template <bool DERIV>
-__device__ __forceinline__ void fx_exp_coefficients(FxExp& sh, i64 (*b)[GF_FX_LINKS], int link, int im, fx_herm q,
+__device__ __forceinline__ bool fx_exp_coefficients(FxExp& sh, i64 (*b)[GF_FX_LINKS], int link, int im, fx_herm q,
                                                     int e) {
   const fx_plan plan = fx_exp_plan<DERIV>(q, e);
   i64 c0, c1, f[3], b1[3], b2[3];
@@ -349,6 +349,7 @@ __device__ __forceinline__ void fx_exp_coefficients(FxExp& sh, i64 (*b)[GF_FX_LI
     const int most = __reduce_max_sync(0xffffffffu, plan.squares);
     if (link == 0) sh.most = most;
   }
+  return plan.beyond;
 }
 // X = -i TA(rho m) of the block's matrices m as entries and exponent
 __device__ __forceinline__ fx_herm fx_ta_herm(const FxExp& sh, int link, const fx_scalar rho, const fx_scalar rho3,

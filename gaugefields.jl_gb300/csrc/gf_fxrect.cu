@@ -318,8 +318,8 @@ __device__ __noinline__ void loops_rows64(const FxField U, double* P, char* D, c
 #endif
 template <bool DSDU>
 __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_LOOPS_MINB)
-    k_loops_fx(FxField U, double* __restrict__ P, char* __restrict__ D, const __grid_constant__ Geom g, fx_scalar cp, fx_scalar cr, double cp64,
-               double cr64, double keep) {
+    k_loops_fx(FxField U, double* __restrict__ P, char* __restrict__ D, const __grid_constant__ Geom g, fx_scalar cp,
+               fx_scalar cr, double cp64, double cr64, double keep) {
   __shared__ union {
     FxRaw m;
     float n[3][GF_FX_LINKS];

@@ -126,8 +126,8 @@ __device__ __noinline__ void fwd_rows64(const FxField U, char* Uout, char* Cout,
 
 template <int AXES, int MINB>
 __global__ void __launch_bounds__(GF_FX_THREADS * AXES, MINB)
-    k_stout_fwd_fx(FxField U, char* __restrict__ Uout, char* __restrict__ Cout, const __grid_constant__ Geom g, fx_scalar rho, fx_scalar rho3,
-                   double rho64) {
+    k_stout_fwd_fx(FxField U, char* __restrict__ Uout, char* __restrict__ Cout, const __grid_constant__ Geom g,
+                   fx_scalar rho, fx_scalar rho3, double rho64) {
   __shared__ FxExp sh;
   __shared__ FxAxes<AXES> ax;
   const int axis = AXES > 1 ? threadIdx.x / GF_FX_THREADS : 0, t = threadIdx.x - axis * GF_FX_THREADS;
@@ -232,7 +232,7 @@ struct FxLocal {
   FxOperand em;                // e^Q
   i64 b[12][GF_FX_LINKS];      // derivatives of the f_j, then trB_k at [2 k + im]
   int ey[GF_FX_LINKS];
-  int f64[GF_FX_LINKS];        // the link has an fp64 slot among its operands
+  int f64[GF_FX_LINKS];        // the link is formed in fp64: a slot among its operands, or a large X
   FxOperand db;                // TOP: halfbeta V of the smeared links
   FxOperand cm;                // recompute: C
 };
@@ -240,7 +240,8 @@ static size_t fx_local_bytes(bool top, bool recompute) {
   return offsetof(FxLocal, db) + (recompute ? 2 : (top ? 1 : 0)) * sizeof(FxOperand);
 }
 
-// The same in fp64 for the block's links that f64 marks.
+// The same in fp64 for the block's links that f64 marks; exp(Q) from Q halved to
+// |Q| <= 1, so that it serves any Q.
 template <bool TOP, bool RECOMPUTE>
 __device__ __noinline__ void local_rows64(const FxField U, const FxField F1, const FxField Cst, char* Zout, char* Dpout,
                                           const Geom& g, double rho, double halfbeta, int mu, int s0, FxLocal& sh) {
@@ -276,33 +277,61 @@ __device__ __noinline__ void local_rows64(const FxField U, const FxField F1, con
     lam = TOP ? mul64<true>(u, sh64(sh.db, link)) : mul64<false>(u, fx_mat64(F1, mu, s, V));
     share64(L, r, lam);
   }
-  if (t < GF_FX_LINKS && sh.f64[t]) {
-    int halvings;
-    mat3<double> q = ta_herm64(sh64(sh.x.m, t), 1.0, halvings);
-    q = scale(scalbn(1.0, halvings), q);
-    double c0, c1;
-    herm_invariants(q, c0, c1);
-    ch_coef<double> cc;
-    ch_coefficients<double, true>(c0, c1, cc);
+  if (t < GF_FX_LINKS) {
+    int halvings = 0;
+    if (sh.f64[t]) {
+      const mat3<double> q = ta_herm64(sh64(sh.x.m, t), 1.0, halvings);
+      double c0, c1;
+      herm_invariants(q, c0, c1);
+      ch_coef<double> cc;
+      ch_coefficients<double, true>(c0, c1, cc);
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      f[2 * j][t] = cc.f[j].re;
-      f[2 * j + 1][t] = cc.f[j].im;
-      b[2 * j][t] = cc.b1[j].re;
-      b[2 * j + 1][t] = cc.b1[j].im;
-      b[6 + 2 * j][t] = cc.b2[j].re;
-      b[7 + 2 * j][t] = cc.b2[j].im;
+      for (int j = 0; j < 3; ++j) {
+        f[2 * j][t] = cc.f[j].re;
+        f[2 * j + 1][t] = cc.f[j].im;
+        b[2 * j][t] = cc.b1[j].re;
+        b[2 * j + 1][t] = cc.b1[j].im;
+        b[6 + 2 * j][t] = cc.b2[j].re;
+        b[7 + 2 * j][t] = cc.b2[j].im;
+      }
+      share_herm64(sh64(sh.x.q, t), q);
     }
-    share_herm64(sh64(sh.x.q, t), q);
+    sh.x.sq[t] = halvings;
+    const int most = __reduce_max_sync(0xffffffffu, halvings);
+    if (t == 0) sh.x.most = most;
   }
   __syncthreads();
-  // W = Lambda Q, X = Q Lambda, Q^2, e^Q by rows; the traces' parts
-  row64 q = zero64(), q2 = zero64(), w = zero64();
+  row64 q = zero64(), q2 = zero64(), w = zero64(), e = zero64();
   if (mine) {
     q = load_row64<false>(Q, r);
     q2 = mul64<false>(q, Q);
+    e = exp_row64(f, link, r, q, q2);
+    share64(E, r, e);
+  }
+  // e^Q = F^n, n = 2^s, F = exp(Q / n): tr(Lambda de^Q) = tr(Lambda' dF) with
+  // Lambda' = sum_k F^k Lambda F^(n - 1 - k), which doubles its terms by
+  // Lambda' <- F Lambda' + Lambda' F, F <- F F
+  const int most = sh.x.most, halvings = sh.x.sq[link];
+#pragma unroll 1
+  for (int k = 0; k < most; ++k) {
+    const bool now = mine && k < halvings;
+    __syncthreads();
+    if (now) {
+      row64 l = mul64<false>(e, L);
+      add64(l, mul64<false>(lam, E));
+      lam = l;
+      e = mul64<false>(e, E);
+    }
+    __syncthreads();
+    if (now) {
+      share64(L, r, lam);
+      share64(E, r, e);
+    }
+  }
+  __syncthreads();
+  // Lambda Q, Q Lambda; the traces' parts (Lambda and Q the halved ones)
+  if (mine) {
     w = mul64<false>(lam, Q);
-    share64(E, r, exp_row64(f, link, r, q, q2));
     double re = 0.0, im = 0.0;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -335,14 +364,15 @@ __device__ __noinline__ void local_rows64(const FxField U, const FxField F1, con
     b[6 * k + 1][l] = im;
   }
   __syncthreads();
-  // Gamma
+  // Gamma, of the whole Q
   if (mine) {
-    row64 G = zero64();
+    row64 G = zero64(), h = zero64();
     cadd64(G, f[4][link], f[5][link], w);
     cadd64(G, f[2][link], f[3][link], lam);
     cadd64(G, b[0][link], b[1][link], q);
     cadd64(G, b[6][link], b[7][link], q2);
-    share64(M, r, G);
+    add64(h, G, scalbn(1.0, -halvings));
+    share64(M, r, h);
   }
   __syncthreads();
   // Y = TA(-i Gamma)
@@ -376,8 +406,9 @@ __device__ __noinline__ void local_rows64(const FxField U, const FxField F1, con
 
 template <bool TOP, bool RECOMPUTE>
 __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_LOCAL_MINB)
-    k_bwd_local_fx(FxField U, FxField F1, FxField Cst, char* __restrict__ Zout, char* __restrict__ Dpout, const __grid_constant__ Geom g,
-                   fx_scalar rho, fx_scalar one, fx_scalar one3, fx_scalar halfbeta, double rho64, double halfbeta64) {
+    k_bwd_local_fx(FxField U, FxField F1, FxField Cst, char* __restrict__ Zout, char* __restrict__ Dpout,
+                   const __grid_constant__ Geom g, fx_scalar rho, fx_scalar one, fx_scalar one3, fx_scalar halfbeta,
+                   double rho64, double halfbeta64) {
   extern __shared__ __align__(16) char smem[];
   FxLocal& sh = *reinterpret_cast<FxLocal*>(smem);
   const int t = threadIdx.x, mu = blockIdx.x & 3, V = g.vol;
@@ -411,9 +442,9 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_LOCAL_MINB)
   } else {
     ed = fx_exp(F1, mu, s, V);
   }
-  const bool f64 = fx_has_f64(ec + eu) || fx_has_f64(ed);
-  if (r == 0) sh.f64[link] = f64;
-  const bool any64 = __syncthreads_or(f64);
+  const bool slot64 = fx_has_f64(ec + eu) || fx_has_f64(ed);
+  if (r == 0) sh.f64[link] = slot64;
+  __syncthreads();
   // Lambda = U Dbar; the exponential of Q and its derivatives
   fx_acc lam;
   {
@@ -423,12 +454,14 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_LOCAL_MINB)
     fx_share<0>(sh.lam, link, r, lam);
   }
   const int el = eu + ed;
+  bool beyond = false;
   if (t < 64) {
     int e;
     const fx_herm q = fx_ta_herm(sh.x, t & 31, one, one3, e);
-    fx_exp_coefficients<true>(sh.x, sh.b, t & 31, t >> 5, q, e);
+    beyond = fx_exp_coefficients<true>(sh.x, sh.b, t & 31, t >> 5, q, e);
+    if (beyond) sh.f64[t & 31] = 1;
   }
-  __syncthreads();
+  const bool any64 = __syncthreads_or(beyond || slot64);
   // Lambda Q, Q Lambda, Q^2, e^Q by rows; partial traces
   fx_acc W, X, Q2;
   const fx_row qr = fx_load_row<false>(FxShMat{&sh.x.q, link}, r);
@@ -558,7 +591,7 @@ __global__ void __launch_bounds__(GF_FX_THREADS, GF_FX_LOCAL_MINB)
   else cr = fx_load_row<true>(fx_mat(Cst, mu, s, V), r);
   fx_add(dp, ed, fx_row_mul<true>(cr, Y), ec + ey);
   fx_down_row<1>(dp);
-  if (sx < V && !f64) {
+  if (sx < V && !sh.f64[link]) {
     fx_store_row(Zout, off, r, z);
     fx_store_row(Dpout, off, r, dp);
     if (r == 0) {
@@ -683,8 +716,8 @@ __device__ __noinline__ void gather_rows64(const FxField U, const FxField Z, con
 // 2: the thin-link momentum update P += coef c(U D) instead.
 template <int OUT, int AXES>
 __global__ void __launch_bounds__(GF_FX_THREADS * AXES, AXES > 1 ? 2 : GF_FX_GATHER_MINB)
-    k_bwd_gather_fx(FxField U, FxField Z, FxField Dp, char* __restrict__ Dout, double* __restrict__ P, const __grid_constant__ Geom g,
-                    fx_scalar rho, double rho64, double coef) {
+    k_bwd_gather_fx(FxField U, FxField Z, FxField Dp, char* __restrict__ Dout, double* __restrict__ P,
+                    const __grid_constant__ Geom g, fx_scalar rho, double rho64, double coef) {
   __shared__ union {
     FxOperand d;
     FxRaw m;

@@ -207,8 +207,8 @@ __device__ __forceinline__ fx_acc fx_shared_row(const FxRaw& m, int link, int r)
 // another pattern of small entries (fx_small_pattern; exact zeros count, for
 // what the momentum puts in their place): stored like the others.
 template <bool REUNIT>
-__device__ __noinline__ void update_link64(const double2* Uin, double2* Uout, const double* __restrict__ P, int mu, int s,
-                                           int V, double eps, float4* sh32, char* fx) {
+__device__ __noinline__ void update_link64(const double2* Uin, double2* Uout, const double* __restrict__ P, int mu,
+                                           int s, int V, double eps, float4* sh32, char* fx) {
   const double* p = P + (size_t)mu * 8 * V + s;
   double c[8];
 #pragma unroll
@@ -262,8 +262,8 @@ __device__ __noinline__ void update_link64(const double2* Uin, double2* Uout, co
 // fp64 kernel's by 1.6e-16, the double-float one's by 6.2e-15.
 template <bool REUNIT>
 __global__ void __launch_bounds__(128, GF_FX_UPDATE_MINB)
-    k_link_update_fx(const double2* Uin, double2* Uout, const double* __restrict__ P, const __grid_constant__ Geom g, fx_scalar eps,
-                     double eps64, float4* __restrict__ sh32, char* __restrict__ fx) {
+    k_link_update_fx(const double2* Uin, double2* Uout, const double* __restrict__ P, const __grid_constant__ Geom g,
+                     fx_scalar eps, double eps64, float4* __restrict__ sh32, char* __restrict__ fx) {
   const int V = g.vol, mu = blockIdx.y, s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= V) return;
   constexpr int rows = REUNIT ? 2 : 3;  // re-unitarisation rebuilds row 3
@@ -367,8 +367,9 @@ __global__ void __launch_bounds__(128, GF_FX_UPDATE_MINB)
 
 // The same with a warp per row of 32 links, for lattices that do not fill the
 // GPU with a thread per link: there the update takes as long as one thread's
-// instructions, some 6,000 of them (GF_FX_ROWS_MAX has the figures). Warps 0 and 1 form the real and imaginary parts of the series
-// while warp 2 brings U to fixed point. Same results as above.
+// instructions, some 6,000 of them (GF_FX_ROWS_MAX has the figures). Warps 0
+// and 1 form the real and imaginary parts of the series while warp 2 brings U to
+// fixed point. Same results as above.
 struct FxUpdateRows {
   FxExp x;      // x.m: the finished rows
   FxOperand u;  // U, then (no re-unitarisation) the fp64 result
@@ -379,8 +380,8 @@ struct FxUpdateRows {
 };
 template <bool REUNIT>
 __global__ void __launch_bounds__(GF_FX_THREADS, 4)
-    k_link_update_rows_fx(const double2* Uin, double2* Uout, const double* __restrict__ P, const __grid_constant__ Geom g, fx_scalar eps,
-                          double eps64, float4* __restrict__ sh32, char* __restrict__ fx) {
+    k_link_update_rows_fx(const double2* Uin, double2* Uout, const double* __restrict__ P, const __grid_constant__ Geom g,
+                          fx_scalar eps, double eps64, float4* __restrict__ sh32, char* __restrict__ fx) {
   __shared__ FxUpdateRows sh;
   const int V = g.vol, mu = blockIdx.y, link = threadIdx.x & 31, r = threadIdx.x >> 5;
   const int sx = blockIdx.x * GF_FX_LINKS + link, s = min(sx, V - 1);
