@@ -581,8 +581,8 @@ GF_HD void fx_ch_both(const i64* kappa, int down, int terms, i64 c0, i64 c1, i64
 }
 
 // R 2^(E - 60) as fp64, rounded once to nearest (ties up in magnitude; at
-// most half an ulp), by integer operations. Overflow gives an infinity, a
-// result below the normal range a zero, GF_FX_BAD a NaN.
+// most half an ulp, of the subnormal range too), by integer operations. Overflow
+// gives an infinity, GF_FX_BAD a NaN.
 GF_HD double fx_to_f64(i64 R, int E) {
   const u64 sign = R < 0 ? 1ull << 63 : 0ull;
   u64 a = R < 0 ? (u64)(-R) : (u64)R;
@@ -596,7 +596,11 @@ GF_HD double fx_to_f64(i64 R, int E) {
   a <<= lz;
   const u64 man = (a >> 11) + ((a >> 10) & 1);  // 2^52 <= man <= 2^53
   const int ex = 1023 + 3 - lz + E;              // value = (a / 2^63) 2^(63 - lz + E - 60)
-  if (ex <= 0) return fx_from_bits(sign);
+  if (ex <= 0) {  // below the normal range, in units of 2^-1074
+    const int d = 12 - ex;
+    if (d > 64) return fx_from_bits(sign);
+    return fx_from_bits(sign | ((d < 64 ? a >> d : 0) + ((a >> (d - 1)) & 1)));
+  }
   if (ex >= 0x7FF) return fx_from_bits(sign | 0x7FF0000000000000ull);
   return fx_from_bits(sign | (((u64)(ex - 1) << 52) + man));
 }

@@ -67,5 +67,15 @@ int main() {
     }
     std::printf("%s %d %d %d\n", names[kind], N, graded, wrong);
   }
+  // results around the smallest normal number: within half a unit of 2^-1074, or of fp64's rounding
+  int wrong = 0;
+  for (int t = 0; t < 200000; ++t) {
+    const i64 R = (i64)(g() >> (4 + t % 60)) * (t & 1 ? 1 : -1);
+    const int E = -1020 - (int)(g() % 70);
+    const long double x = ldexpl((long double)R, E - 60), y = fx_to_f64(R, E);
+    const long double unit = fmaxl(ldexpl(1.0L, -1074), fabsl(x) * ldexpl(1.0L, -52));
+    wrong += !(fabsl(x - y) <= 0.5L * unit);
+  }
+  std::printf("subnormal 200000 0 %d\n", wrong);
   return 0;
 }

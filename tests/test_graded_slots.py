@@ -36,3 +36,7 @@ def test_generic_matrices_and_exact_zeros_are_not(counted, kind):
     # embedded SU(2) matrix (8 numbers, each 1.2%) for one in ten
     assert graded <= {"gaussian": 1e-5, "exact_su2": 0.15}.get(kind, 0.0) * n
     assert wrong == 0
+
+
+def test_results_below_the_normal_range(counted):
+    assert counted["subnormal"][2] == 0
