@@ -23,8 +23,8 @@ namespace gf {
 #define GF_FX_MINB 7
 #endif
 // Up to so many sites the blocks of a stencil fit on the GPU at five per SM, and
-// the kernels take the registers that leaves: 8^4 trajectory 681 us, with seven
-// 721; at 24^4, where the GPU is full, the force takes 736 us with seven and 753
+// the kernels take the registers that leaves: 8^4 trajectory 684 us, with seven
+// 721; at 24^4, where the GPU is full, the force takes 711 us with seven and 753
 // with six.
 #define GF_FX_FEW_MAX 6144
 #define GF_FX_FEW_MINB 5
@@ -435,16 +435,23 @@ __device__ __forceinline__ int fx_norm_shift(float n, int e) {
   return ((k4 + 1) >> 1) - 40;
 }
 
+// an element of a slot as fp64. Out of line where it is not fp64 already: by
+// integer operations, for the fp64 pipe is what its callers wait for, and inlined
+// nine times a matrix they took registers from the fixed-point kernels around
+// (24^4 force 736 us, out of line 715).
+static __device__ __noinline__ double2 fx_convert64(int4 v, int e) {
+  return make_double2(fx_to_f64(fx_join(v.x, v.y), e), fx_to_f64(fx_join(v.z, v.w), e));
+}
+__device__ __forceinline__ double2 fx_element64(int4 v, int e) {
+  if (e == GF_FX_F64) return make_double2(fx_unpack64(v.x, v.y), fx_unpack64(v.z, v.w));
+  return fx_convert64(v, e);
+}
 // fp64 view of a fixed-point field: element by element, and whole matrices (fp64
 // kernels)
 struct FxMat64 {
   FxMat m;
   int e;
-  __device__ __forceinline__ double2 operator()(int el) const {
-    const int4 v = m(el);
-    if (e == GF_FX_F64) return make_double2(fx_unpack64(v.x, v.y), fx_unpack64(v.z, v.w));
-    return make_double2(fx_to_f64(fx_join(v.x, v.y), e), fx_to_f64(fx_join(v.z, v.w), e));
-  }
+  __device__ __forceinline__ double2 operator()(int el) const { return fx_element64(m(el), e); }
 };
 __device__ __forceinline__ FxMat64 fx_mat64(const FxField& F, int mu, int s, int V) {
   return FxMat64{fx_mat(F, mu, s, V), fx_exp(F, mu, s, V)};

@@ -5,11 +5,12 @@
 // thread 3 link + row forms its row for those links and sits out for the rest.
 // The rows stay within the registers that the calling kernels have. Fields that
 // are graded throughout are bound by the fp64 pipe: weak links at 24^4, force
-// 3.76 ms, plaquette + rectangle force 20.4, plaquette 0.92, two-level stout
-// force 49.4, link update 1.08, where kernels in fp64 altogether took 4.78, 30.4,
+// 3.57 ms, plaquette + rectangle force 18.7, plaquette 0.92, two-level stout
+// force 43.1, link update 1.08, where kernels in fp64 altogether took 4.78, 30.4,
 // 1.22, 46.3 and 0.95, and fixed point alone, with 10^-9 of the small parts
-// wrong, 0.74, 3.4, 0.29, 7.3 and 0.28. Generic links pay 2% to 4% for the test
-// and the call beside it (24^4 force 704 -> 736 us).
+// wrong, 0.74, 3.4, 0.29, 7.3 and 0.28. Generic links pay up to 2% for the test
+// and the call beside it (24^4 force 705 -> 711 us, 32^4 stout force 23.49 ->
+// 23.64 ms): a called function's registers count in its caller.
 #pragma once
 #include "fxlat.cuh"
 

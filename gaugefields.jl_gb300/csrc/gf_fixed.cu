@@ -41,7 +41,15 @@ void to_fx(gf_ctx* ctx, gf_field* dst, const gf_field* src) {
 __global__ void __launch_bounds__(128) k_fx_to_f64(FxField F, double2* __restrict__ out, int V) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x, mu = blockIdx.y;
   if (s >= V) return;
-  LinkFull<double>::store(out, mu, s, V, LinkSrcFx64{F}(mu, s, V));
+  const FxMat M = fx_mat(F, mu, s, V);
+  const int e = fx_exp(F, mu, s, V);
+  double2* b = out + (size_t)mu * 9 * V + s;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    const int4 v = M(k);
+    b[(size_t)k * V] = e == GF_FX_F64 ? make_double2(fx_unpack64(v.x, v.y), fx_unpack64(v.z, v.w))
+                                      : make_double2(fx_to_f64(fx_join(v.x, v.y), e), fx_to_f64(fx_join(v.z, v.w), e));
+  }
 }
 
 void fx_to_f64_field(gf_ctx* ctx, gf_field* dst, const gf_field* src) {
