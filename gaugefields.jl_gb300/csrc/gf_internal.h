@@ -268,11 +268,12 @@ void loops_fx(gf_ctx* ctx, const gf_field* F, gf_field* P, gf_field* D, double c
 
 // ---- link update (gf_update.cu) ----
 // U <- exp(i eps P) U, optional re-unitarisation, optional fp32 shadow copy.
-// df: double-float arithmetic on the fp32 pipes (the mixed form), else fp64.
+// One arithmetic for every form, fixed point or fp64 (gf_update.cu); df: the
+// kernel class that the launch is timed as (the mixed and double-float forms').
 // fx: also write the fixed-point copy of the updated links (a LINKFX field).
 void link_update(gf_ctx* ctx, gf_field* U, const gf_field* P, double eps, int reunit, gf_field* shadow32,
                  bool df = false, gf_field* fx = nullptr);
-// W = exp(i a P) U (fp64, or double-float arithmetic on the fp64 fields)
+// W = exp(i a P) U, the same
 void exp_mom_links(gf_ctx* ctx, gf_field* W, const gf_field* P, double a, const gf_field* U, bool df = false,
                    gf_field* fx = nullptr);
 void reunitarize_links(gf_ctx* ctx, gf_field* U);

@@ -990,22 +990,8 @@ GF_HD mat3<R> mul_nn_rows12(const mat3<R>& a, const mat3<R>& b) {
     }
   return r;
 }
-__device__ __forceinline__ mat3<dfl> mul_nn_rows12(const mat3<dfl>& a, const mat3<dfl>& b) {
-  return df_matmul<false, false, false, 2>(a, b, nullptr);
+__device__ __forceinline__ mat3<dfl> mul_nn(const mat3<dfl>& a, const mat3<dfl>& b) {
+  return df_matmul<false, false, false>(a, b, nullptr);
 }
-
-template <bool DA, bool DB>
-__device__ __forceinline__ mat3<dfl> df_mul(const mat3<dfl>& a, const mat3<dfl>& b) {
-  return df_matmul<DA, DB, false>(a, b, nullptr);
-}
-template <bool DA, bool DB>
-__device__ __forceinline__ void df_mac(mat3<dfl>& acc, const mat3<dfl>& a, const mat3<dfl>& b) {
-  acc = df_matmul<DA, DB, true>(a, b, &acc);
-}
-
-__device__ __forceinline__ mat3<dfl> mul_nn(const mat3<dfl>& a, const mat3<dfl>& b) { return df_mul<false, false>(a, b); }
-__device__ __forceinline__ mat3<dfl> mul_na(const mat3<dfl>& a, const mat3<dfl>& b) { return df_mul<false, true>(a, b); }
-__device__ __forceinline__ mat3<dfl> mul_an(const mat3<dfl>& a, const mat3<dfl>& b) { return df_mul<true, false>(a, b); }
-__device__ __forceinline__ mat3<dfl> mul_aa(const mat3<dfl>& a, const mat3<dfl>& b) { return df_mul<true, true>(a, b); }
 
 }  // namespace gf
