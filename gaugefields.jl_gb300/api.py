@@ -726,9 +726,8 @@ def md_hamiltonian(U, P, driver):
 
 
 def update_gaugefields_(U, P, step_size, driver):
-    """U_mu <- exp(step_size P_mu) U_mu (molecular_dynamics.jl:513-531), in
-    arithmetic of fp64 class in every form; the mixed form's writes its fp32
-    copy too."""
+    """U_mu <- exp(step_size P_mu) U_mu (molecular_dynamics.jl:513-531), the
+    same in every precision form: fp64 links, arithmetic of fp64 class."""
     if not math.isfinite(step_size):
         raise ValueError("the gauge-field step size must be finite; got %s" % step_size)
     p = driver.params()
