@@ -604,9 +604,11 @@ static void check_md(const gf_md_params* p) {
 // uses a forward-only double-float stack; the GF_DFLOAT form shares one full
 // stack between its force and its Hamiltonian.
 static gf_stout* ctx_stout(gf_ctx* ctx, const gf_md_params* p, int precision) {
+  const bool fwd_only = precision == GF_PREC_DF && p->precision == GF_MIXED;
+  // up to GF_FX_STACK_MAX sites the plain and the double-float form share one
+  if (!fwd_only && fx_stack(ctx, precision)) precision = GF_FP64;
   gf_stout** slot = precision == GF_FP64 ? &ctx->w_stout64
                     : (precision == GF_MIXED ? &ctx->w_stout32 : &ctx->w_stoutdf);
-  const bool fwd_only = precision == GF_PREC_DF && p->precision == GF_MIXED;
   int store = fwd_only ? 0 : (p->stout_recompute ? 0 : 1);
   bool same = *slot && (*slot)->nlev == p->nstout && (*slot)->store == store && (*slot)->fwd_only == (int)fwd_only;
   if (same)

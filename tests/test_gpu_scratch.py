@@ -180,3 +180,19 @@ def test_a_context_without_memory_for_its_copy(pkg):
     V = pkg.Gaugefields4D(U)
     pkg._lib.call("gf_cold_start", U.h, V.field.h)
     assert pkg.calculate_Plaquette(V) == want
+
+
+def test_plain_and_double_float_drivers_share_their_stack(pkg):
+    """The two forms' stacks are the same on lattices of this size: a driver of the
+    second form takes no memory that the first has not."""
+    torch = pytest.importorskip("torch")
+    U = pkg.gauge_configuration(L24, start="hot", seed=11)
+    net = pkg.CovNeuralnet(U)
+    pkg.push_(net, pkg.STOUT_Layer("plaquette", 0.1))
+    P, free, energy = pkg.gaussian_momenta(U, seed=3), [], []
+    for precision in ("fp64", "dfloat"):
+        drv = pkg.md_driver(U, wilson(pkg, U), steps=1, smearing=net, precision=precision)
+        energy.append(pkg.md_hamiltonian(U, P, drv))
+        pkg.update_momenta_(P, U, 0.0, drv)
+        free.append(free_bytes(torch))
+    assert free[0] == free[1] and energy[0] == energy[1]
