@@ -647,13 +647,21 @@ static void potential_start(gf_ctx* ctx, const gf_field* U, const gf_md_params* 
     stout_forward(ctx, st, stack_links(ctx, st, U), nullptr);
     links = stout_top(st);
     if (st->fwd_only) {
-      // the levels take the two scratch blocks in turn: the top's copy goes to the other one
-      gf_field* F = arena_view(ctx, p->nstout & 1, 0, GF_LINKFX);
-      to_fx(ctx, F, links);
-      plaquette_start(ctx, F, 0);
-      if (p->c_rect != 0.0) rectangle_start(ctx, F, 1);
-      field_delete(F);
-      return;
+      // the levels take the two scratch blocks in turn: the top's copy goes to
+      // the other one. Without room there the fp64 sums read the top in place.
+      gf_field* F = nullptr;
+      try {
+        F = arena_view(ctx, p->nstout & 1, 0, GF_LINKFX);
+      } catch (const gf_error& e) {
+        if (e.code != GF_ENOMEM) throw;
+      }
+      if (F) {
+        to_fx(ctx, F, links);
+        plaquette_start(ctx, F, 0);
+        if (p->c_rect != 0.0) rectangle_start(ctx, F, 1);
+        field_delete(F);
+        return;
+      }
     }
   }
   plaquette_start(ctx, links, 0);

@@ -110,12 +110,19 @@ gf_field* field_pooled(gf_ctx* ctx, int kind) {
 }
 
 gf_field* arena_view(gf_ctx* ctx, int which, size_t off, int kind) {
-  const size_t cap = std::max(field_bytes(ctx->geom, GF_LINK64), field_bytes(ctx->geom, GF_LINKFX));
+  const size_t bytes = field_bytes(ctx->geom, kind), link64 = field_bytes(ctx->geom, GF_LINK64);
   if (!ctx->arena[which]) {
-    ctx->arena[which] = device_alloc(ctx, cap);
+    // with room for a fixed-point field if there is memory for it
+    size_t cap = std::max(link64, field_bytes(ctx->geom, GF_LINKFX));
+    try {
+      ctx->arena[which] = device_alloc(ctx, cap);
+    } catch (const gf_error&) {
+      if (off + bytes > link64) throw;
+      ctx->arena[which] = device_alloc(ctx, cap = link64);
+    }
+    ctx->arena_bytes[which] = cap;
   }
-  const size_t bytes = field_bytes(ctx->geom, kind);
-  if (off + bytes > cap) throw gf_error(GF_EINVAL, "scratch view beyond its block");
+  if (off + bytes > ctx->arena_bytes[which]) throw gf_error(GF_ENOMEM, "scratch view beyond its block");
   return new gf_field{ctx, kind, (char*)ctx->arena[which] + off, bytes, 0, nullptr};
 }
 

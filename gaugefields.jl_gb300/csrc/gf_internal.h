@@ -95,12 +95,14 @@ struct gf_ctx {
   gf_field* w_linkfx;     // fixed-point copy of the links (fp64-class kernels)
   int fx_hold;            // drivers that keep w_linkfx across other calls (FxHold)
   int fx_graph;           // 1: a captured graph uses w_linkfx
-  // Two scratch blocks of one link field each (fp64 or fixed point), shared by
+  // Two scratch blocks of one link field each (fixed point, or fp64 if there is
+  // no memory for the 2.8% more), shared by
   // the mixed form's internal stacks: the Hamiltonian's double-float level
   // buffers, the fixed-point copy of their top for the loop sums, and the force
   // adjoint's Z, Dp, D[0], D[1] (fp32). They are never live together:
   // the potential runs before and after the MD steps, the adjoint within them.
   void* arena[2];
+  size_t arena_bytes[2];
   gf_stout* w_stout64;    // stout workspace, fp64
   gf_stout* w_stout32;    // stout workspace, fp32
   gf_stout* w_stoutdf;    // double-float stack: mixed-form Hamiltonian (forward only) or GF_DFLOAT

@@ -196,3 +196,32 @@ def test_plain_and_double_float_drivers_share_their_stack(pkg):
         pkg.update_momenta_(P, U, 0.0, drv)
         free.append(free_bytes(torch))
     assert free[0] == free[1] and energy[0] == energy[1]
+
+
+@pytest.mark.parametrize("blocks", [1.02, 1.5])
+def test_mixed_energy_in_one_scratch_block(pkg, blocks):
+    """The mixed form's smeared energy needs one scratch block of a link field for a
+    level of smearing; the fixed-point sums take a second, larger one if there is
+    memory, and the fp64 sums do without: the same to 1e-13."""
+    torch = pytest.importorskip("torch")
+    link64 = 4 * 24 ** 4 * 144
+
+    def energy(fill):
+        U = pkg.gauge_configuration(L24, start="hot", seed=11)
+        P = pkg.gaussian_momenta(U, seed=3)
+        net = pkg.CovNeuralnet(U)
+        pkg.push_(net, pkg.STOUT_Layer("plaquette", 0.1))
+        action = wilson(pkg, U)
+        pkg.push_(action, -0.1, "rectangular")
+        drv = pkg.md_driver(U, action, steps=1, smearing=net, precision="mixed")
+        filler = None
+        if fill:
+            filler = torch.empty(free_bytes(torch) - int(blocks * link64), dtype=torch.uint8, device="cuda")
+        try:
+            return pkg.md_hamiltonian(U, P, drv)
+        finally:
+            del filler
+            torch.cuda.empty_cache()
+
+    want = energy(False)
+    assert energy(True) == pytest.approx(want, rel=1e-13)
