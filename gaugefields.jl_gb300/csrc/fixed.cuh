@@ -233,7 +233,7 @@ GF_HD void fx_scale_row(fx_acc& v, const fx_scalar& c) {
 // imaginary parts, which two threads evaluate side by side. They are returned
 // in units of 2^(guard - 60), as are their derivatives in c1 and c0 (of q).
 // ---------------------------------------------------------------------------
-#define GF_FX_CH_TERMS 48
+#define GF_FX_CH_TERMS 64  // 48 would do; lanes of two scales read it 3% faster at this distance (link update, 16^4)
 #define GF_FX_CH_SCALES 3
 
 // 2^(s n) / n! in units of 2^(base - 60), rounded
@@ -521,14 +521,17 @@ GF_HD int4 fx_pack64(double re, double im) {
 }
 GF_HD double fx_unpack64(int lo, int hi) { return fx_from_bits(((u64)(unsigned)hi << 32) | (unsigned)lo); }
 
-// One matrix to fixed point; returns its exponent.
-GF_HD int fx_from_f64(const double* m, int4 out[9]) {
+// One matrix to fixed point; returns its exponent. few: it has small entries
+// enough to be graded.
+GF_HD int fx_from_f64(const double* m, int4 out[9], bool& few) {
   int emax, up, small;
+  few = false;
   if (!fx_exponent_of(m, emax, up, small)) {
 #pragma unroll
     for (int i = 0; i < 9; ++i) out[i] = make_int4(0, 0, 0, 0);
     return GF_FX_BAD;
   }
+  few = small >= GF_FX_PATTERN_MIN;
 #pragma unroll
   for (int i = 0; i < 9; ++i) {
     fx_split<0>(fx_mantissa(m[2 * i], emax, up), out[i].x, out[i].y);
@@ -536,23 +539,21 @@ GF_HD int fx_from_f64(const double* m, int4 out[9]) {
   }
   return emax - 1023 + up;
 }
+GF_HD int fx_from_f64(const double* m, int4 out[9]) {
+  bool few;
+  return fx_from_f64(m, out, few);
+}
 
 // One matrix to what its slot holds: fixed point, or fp64 if it is graded.
 GF_HD int fx_encode(const double* m, int4 out[9]) {
-  int emax, up, small;
-  if (!fx_exponent_of(m, emax, up, small)) {
+  bool few;
+  int e = fx_from_f64(m, out, few);
+  if (few && fx_graded(m, e + 1023)) {
+    e = GF_FX_F64;
 #pragma unroll
-    for (int i = 0; i < 9; ++i) out[i] = make_int4(0, 0, 0, 0);
-    return GF_FX_BAD;
+    for (int i = 0; i < 9; ++i) out[i] = fx_pack64(m[2 * i], m[2 * i + 1]);
   }
-  const bool f64 = small >= GF_FX_PATTERN_MIN && fx_graded(m, emax + up);
-#pragma unroll
-  for (int i = 0; i < 9; ++i) {
-    fx_split<0>(fx_mantissa(m[2 * i], emax, up), out[i].x, out[i].y);
-    fx_split<0>(fx_mantissa(m[2 * i + 1], emax, up), out[i].z, out[i].w);
-    if (f64) out[i] = fx_pack64(m[2 * i], m[2 * i + 1]);
-  }
-  return f64 ? GF_FX_F64 : emax - 1023 + up;
+  return e;
 }
 
 // real and imaginary parts of the f_j, side by side: f at [2 j + im]
@@ -580,29 +581,40 @@ GF_HD void fx_ch_both(const i64* kappa, int down, int terms, i64 c0, i64 c1, i64
   }
 }
 
-// R 2^(E - 60) as fp64, rounded once to nearest (ties up in magnitude; at
-// most half an ulp, of the subnormal range too), by integer operations. Overflow
-// gives an infinity, GF_FX_BAD a NaN.
-GF_HD double fx_to_f64(i64 R, int E) {
+// R 2^(E - 60) as fp64, rounded once to nearest (ties up in magnitude; at most
+// half an ulp), by integer operations, for E above GF_FX_NORMAL, where no result
+// but zero is below the normal range. Overflow gives an infinity, GF_FX_BAD a NaN.
+#define GF_FX_NORMAL (-960)
+GF_HD int fx_leading_zeros(u64 a) {
+#ifdef __CUDA_ARCH__
+  return __clzll((i64)a);
+#else
+  return __builtin_clzll(a);
+#endif
+}
+GF_HD double fx_to_normal(i64 R, int E) {
   const u64 sign = R < 0 ? 1ull << 63 : 0ull;
   u64 a = R < 0 ? (u64)(-R) : (u64)R;
   if (E > GF_FX_BAD / 2) return fx_from_bits(0x7FF8000000000000ull);
   if (a == 0) return 0.0;
-#ifdef __CUDA_ARCH__
-  const int lz = __clzll((i64)a);
-#else
-  const int lz = __builtin_clzll(a);
-#endif
+  const int lz = fx_leading_zeros(a);
   a <<= lz;
   const u64 man = (a >> 11) + ((a >> 10) & 1);  // 2^52 <= man <= 2^53
   const int ex = 1023 + 3 - lz + E;              // value = (a / 2^63) 2^(63 - lz + E - 60)
-  if (ex <= 0) {  // below the normal range, in units of 2^-1074
-    const int d = 12 - ex;
-    if (d > 64) return fx_from_bits(sign);
-    return fx_from_bits(sign | ((d < 64 ? a >> d : 0) + ((a >> (d - 1)) & 1)));
-  }
   if (ex >= 0x7FF) return fx_from_bits(sign | 0x7FF0000000000000ull);
   return fx_from_bits(sign | (((u64)(ex - 1) << 52) + man));
+}
+// the same for any E
+GF_HD double fx_to_f64(i64 R, int E) {
+  const u64 a = R < 0 ? (u64)(-R) : (u64)R;
+  if (E <= GF_FX_NORMAL && a != 0) {
+    const int lz = fx_leading_zeros(a), d = 12 - (1023 + 3 - lz + E);
+    if (d >= 12) {  // below the normal range: in units of 2^-1074
+      const u64 n = d > 64 ? 0 : (d < 64 ? (a << lz) >> d : 0) + (((a << lz) >> (d - 1)) & 1);
+      return fx_from_bits((R < 0 ? 1ull << 63 : 0ull) | n);
+    }
+  }
+  return fx_to_normal(R, E);
 }
 
 }  // namespace gf

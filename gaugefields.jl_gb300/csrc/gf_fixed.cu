@@ -9,12 +9,8 @@ namespace gf {
 
 // LINK64 / MAT64 (double2) or double-float pairs (float4) -> fixed point, one
 // link per thread; bandwidth-bound (24^4: 57 us for 387 MB).
-__device__ __forceinline__ double2 fx_complex64(double2 v) { return v; }
-__device__ __forceinline__ double2 fx_complex64(float4 v) {
-  return make_double2(df_to_double(dfl(v.x, v.y)), df_to_double(dfl(v.z, v.w)));
-}
 template <typename E>
-__global__ void __launch_bounds__(128, 5) k_to_fx(const E* __restrict__ in, char* __restrict__ out, int V) {
+__global__ void __launch_bounds__(128) k_to_fx(const E* __restrict__ in, char* __restrict__ out, int V) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x, mu = blockIdx.y;
   if (s >= V) return;
   const E* b = in + (size_t)mu * 9 * V + s;
@@ -25,7 +21,14 @@ __global__ void __launch_bounds__(128, 5) k_to_fx(const E* __restrict__ in, char
     m[2 * k] = v.x;
     m[2 * k + 1] = v.y;
   }
-  fx_store64(out, mu, s, V, m);
+  int4 f[9];
+  bool few;
+  const int e = fx_from_f64(m, f, few);
+  char* o = out + fx_offset(mu, s, V);
+#pragma unroll
+  for (int k = 0; k < 9; ++k) *reinterpret_cast<int4*>(o + 512 * k) = f[k];
+  *reinterpret_cast<int*>(o + 9 * 512 - 12 * (s & 31)) = e;
+  if (few) fx_regrade(in, out, mu, s, V, e);
 }
 
 void to_fx(gf_ctx* ctx, gf_field* dst, const gf_field* src) {

@@ -159,7 +159,19 @@ __device__ __forceinline__ bool fx_patterned(const double* m, int unit) {
   return fx_small_pattern(small);
 }
 // links of a matrix from fp64, the exponent from its Frobenius norm
-__device__ __forceinline__ int fx_from_f64_fast(const double* m, int4 out[9], bool& patterned) {
+// the same out of line, of a stored link
+__device__ __noinline__ bool fx_patterned(const double2* U, int mu, int s, int V, int unit) {
+  const double2* b = U + (size_t)mu * 9 * V + s;
+  unsigned small = 0;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    const double2 v = b[(size_t)k * V];
+    small |= (unsigned)fx_is_small(v.x, unit) << (2 * k) | (unsigned)fx_is_small(v.y, unit) << (2 * k + 1);
+  }
+  return fx_small_pattern(small);
+}
+// small: how many entries are below 2^-7 of the unit, unit: for fx_patterned
+__device__ __forceinline__ int fx_from_f64_fast(const double* m, int4 out[9], int& small, int& unit) {
   int emax = 1;
 #pragma unroll
   for (int i = 0; i < 18; ++i) emax = max(emax, fx_exponent_field(m[i]));
@@ -173,10 +185,11 @@ __device__ __forceinline__ int fx_from_f64_fast(const double* m, int4 out[9], bo
   const bool bad = emax == 0x7FF;
   // entries below 2^-7 of the spectral norm, half the Frobenius norm's power of two
   const float tiny = 0.00390625f * (float)(1 << up);
-  int small = 0;
+  small = 0;
 #pragma unroll
   for (int i = 0; i < 18; ++i) small += fabsf(f[i]) < tiny;
-  patterned = small >= GF_FX_PATTERN_MIN && !bad && fx_patterned(m, emax + up - 1);
+  if (bad) small = 0;
+  unit = emax + up - 1;
 #pragma unroll
   for (int i = 0; i < 9; ++i) {
     fx_split<0>(bad ? 0 : fx_mantissa(m[2 * i], emax, up), out[i].x, out[i].y);
@@ -209,6 +222,10 @@ __device__ __forceinline__ fx_acc fx_shared_row(const FxRaw& m, int link, int r)
 template <bool REUNIT>
 __device__ __noinline__ void update_link64(const double2* Uin, double2* Uout, const double* __restrict__ P, int mu,
                                            int s, int V, double eps, float4* sh32, char* fx) {
+  mat3<double> u;
+  const double2* b = Uin + (size_t)mu * 9 * V + s;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) u.e[k / 3][k % 3] = mk(b[(size_t)k * V].x, b[(size_t)k * V].y);
   const double* p = P + (size_t)mu * 8 * V + s;
   double c[8];
 #pragma unroll
@@ -234,10 +251,6 @@ __device__ __noinline__ void update_link64(const double2* Uin, double2* Uout, co
   mat3<double> E = expiq(scale(scalbn(1.0, -halvings), q));
 #pragma unroll 1
   for (int k = 0; k < halvings; ++k) E = mul_nn(E, E);
-  mat3<double> u;
-  const double2* b = Uin + (size_t)mu * 9 * V + s;
-#pragma unroll
-  for (int k = 0; k < 9; ++k) u.e[k / 3][k % 3] = mk(b[(size_t)k * V].x, b[(size_t)k * V].y);
   u = mul_nn(E, u);
   if (REUNIT) reunitarize(u);
   LinkFull<double>::store(Uout, mu, s, V, u);
@@ -277,7 +290,7 @@ __global__ void __launch_bounds__(128, GF_FX_UPDATE_MINB)
     fx_ch_both(c_fx_kappa.k[plan.series], plan.guard - fx_kappa_base(plan.series), plan.terms, c0, c1, f);
   }
   int4 u[9];
-  int eu;
+  int eu, small, unit;
   {
     const double2* b = Uin + (size_t)mu * 9 * V + s;
     double m[18];
@@ -287,12 +300,7 @@ __global__ void __launch_bounds__(128, GF_FX_UPDATE_MINB)
       m[2 * k] = v.x;
       m[2 * k + 1] = v.y;
     }
-    bool patterned;
-    eu = fx_from_f64_fast(m, u, patterned);
-    if (patterned) {
-      update_link64<REUNIT>(Uin, Uout, P, mu, s, V, eps64, sh32, fx);
-      return;
-    }
+    eu = fx_from_f64_fast(m, u, small, unit);
   }
   if (e > GF_FX_BAD / 2) eu = GF_FX_BAD;
   fx_acc w[3];
@@ -321,14 +329,25 @@ __global__ void __launch_bounds__(128, GF_FX_UPDATE_MINB)
     fine = eu > GF_FX_BAD / 2 ? 0 : fx_unitarise(w);
     eu = 0;
   }
+  // here, where least is alive across the calls
+  if (small >= GF_FX_PATTERN_MIN && fx_patterned(Uin, mu, s, V, unit)) {
+    update_link64<REUNIT>(Uin, Uout, P, mu, s, V, eps64, sh32, fx);
+    return;
+  }
   double2* o = Uout + (size_t)mu * 9 * V + s;
   double2 v[9];
+  const bool tiny = eu <= GF_FX_NORMAL;
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
-    const int ew = k / 3 < fine ? eu : GF_FX_BAD;
-    v[k] = make_double2(fx_to_f64(w[k / 3].re[k % 3], ew), fx_to_f64(w[k / 3].im[k % 3], ew));
-    o[(size_t)k * V] = v[k];
+    const int ew = k / 3 < fine ? (tiny ? eu + 1000 : eu) : GF_FX_BAD;
+    v[k] = make_double2(fx_to_normal(w[k / 3].re[k % 3], ew), fx_to_normal(w[k / 3].im[k % 3], ew));
   }
+  if (tiny) {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) v[k] = make_double2(v[k].x * 0x1p-1000, v[k].y * 0x1p-1000);
+  }
+#pragma unroll
+  for (int k = 0; k < 9; ++k) o[(size_t)k * V] = v[k];
   if (sh32) {
     float4* q4 = sh32 + (size_t)mu * 3 * V + s;
 #pragma unroll
@@ -340,28 +359,31 @@ __global__ void __launch_bounds__(128, GF_FX_UPDATE_MINB)
     // the fixed-point copy of what was stored, as k_to_fx makes it
     int4 el[9];
     const size_t off = fx_offset(mu, s, V);
-    double m[18];
+    bool few;
     int ef;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-      m[2 * k] = v[k].x;
-      m[2 * k + 1] = v[k].y;
-    }
     if (REUNIT) {
       // a unitary matrix has exponent 0
-      int small = 0;
+      int n = 0;
 #pragma unroll
-      for (int k = 0; k < 18; ++k) small += fx_is_small(m[k], 1023);
-      const bool f64 = small >= GF_FX_PATTERN_MIN && fine == 3 && fx_graded(m, 1023);
-      ef = f64 ? GF_FX_F64 : (fine == 3 ? 0 : GF_FX_BAD);
-#pragma unroll
-      for (int k = 0; k < 9; ++k) el[k] = fx_unitary_element(v[k], fine == 3, f64);
+      for (int k = 0; k < 9; ++k) {
+        el[k] = fx_unitary_element(v[k], fine == 3, false);
+        n += fx_is_small(v[k].x, 1023) + fx_is_small(v[k].y, 1023);
+      }
+      ef = fine == 3 ? 0 : GF_FX_BAD;
+      few = n >= GF_FX_PATTERN_MIN && fine == 3;
     } else {
-      ef = fx_encode(m, el);
+      double m[18];
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        m[2 * k] = v[k].x;
+        m[2 * k + 1] = v[k].y;
+      }
+      ef = fx_from_f64(m, el, few);
     }
-    *reinterpret_cast<int*>(fx + off + 9 * 512 - 12 * (s & 31)) = ef;
+    fx_store_exp(fx, off, s, ef);
 #pragma unroll
     for (int k = 0; k < 9; ++k) *reinterpret_cast<int4*>(fx + off + 512 * k) = el[k];
+    if (few) fx_regrade(Uout, fx, mu, s, V, ef);
   }
 }
 
@@ -413,9 +435,9 @@ __global__ void __launch_bounds__(GF_FX_THREADS, 4)
       m[2 * k + 1] = v.y;
     }
     int4 u[9];
-    bool patterned;
-    sh.eu[link] = fx_from_f64_fast(m, u, patterned);
-    sh.patterned[link] = patterned;
+    int small, unit;
+    sh.eu[link] = fx_from_f64_fast(m, u, small, unit);
+    sh.patterned[link] = small >= GF_FX_PATTERN_MIN && fx_patterned(m, unit);
 #pragma unroll
     for (int k = 0; k < 9; ++k) sh.u.v[k][link] = u[k];
   }
@@ -441,10 +463,12 @@ __global__ void __launch_bounds__(GF_FX_THREADS, 4)
     eu = 0;
   }
   double2 v[3];
+  const bool tiny = eu <= GF_FX_NORMAL;
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
-    const int ew = r < fine ? eu : GF_FX_BAD;
-    v[j] = make_double2(fx_to_f64(w.re[j], ew), fx_to_f64(w.im[j], ew));
+    const int ew = r < fine ? (tiny ? eu + 1000 : eu) : GF_FX_BAD;
+    v[j] = make_double2(fx_to_normal(w.re[j], ew), fx_to_normal(w.im[j], ew));
+    if (tiny) v[j] = make_double2(v[j].x * 0x1p-1000, v[j].y * 0x1p-1000);
   }
   const size_t off = fx_offset(mu, s, V);
   int4 el[3];
