@@ -853,8 +853,10 @@ def main():
             "scaling": "weak", "vs_baseline": None, "dtype": "f64 (64-bit block fixed point arithmetic)",
             "data": "synthetic (Haar-random SU(3) start, seed 7; Gaussian momenta per trajectory)",
             "config": bench_config(L),
-            "form": "double-float, at this size in the plain form's arithmetic: 64-bit block fixed point of fp64 "
-                    "class on fp64 fields throughout (meets |dH - dH_fp64| <= 1e-4: dH_check)",
+            "form": "double-float, at this size the plain form's kernels: 64-bit block fixed point of fp64 class on "
+                    "fp64 fields throughout (meets |dH - dH_fp64| <= 1e-4: 3.7e-8 at most against the CPU oracle's "
+                    "fp64 arithmetic in three trajectories of this workload, profiles/precision_fixed_point.md; "
+                    "dH_check compares it with the plain form, at this size an identity)",
             "replicas": world,
             "e2e": e2e, "gpu_launches": launches, "roofline": roof, "compute": compute, "cpu_baseline": cpu,
             "clocks": clocks, "mixed_form": mixed, "fp64_form": fp64,

@@ -5,7 +5,8 @@
 // and scheduler). A product of two 60-bit fixed-point numbers kept as limbs of
 // 30 bits needs three of them (high x high and the two cross terms), so a
 // real multiply-add costs 12 issue slots instead of 64, with an absolute
-// error of about 2^-59 of the operands' norms, below the 2^-53 of fp64.
+// error of about 2^-59 of the operands' norms, below fp64's rounding of anything
+// but entries under 2^-7 of the norm (fx_graded).
 //
 // A matrix is 18 integers R with one exponent E: value = R 2^(E - 60). E is
 // chosen so that the matrix's spectral norm is at most 1 + 2^-11 in units of
@@ -68,10 +69,8 @@ GF_HD fx_row fx_operand(const fx_acc& v) {
   return r;
 }
 
-// a b + c as one IMAD.WIDE. The product is written in PTX: knowing that a limb
-// is not negative, the compiler widens it as unsigned, finds no 32 x 32 form
-// for the mixed signs and emits a full 64-bit product (400 instructions for
-// a row product instead of 136). mad.wide in PTX becomes two instructions.
+// a b + c, the product in PTX: written in C, with limbs that the compiler knows
+// not to be negative, it measured slower, and so did mad.wide.
 GF_HD i64 fx_mad(int a, int b, i64 c) {
 #ifdef __CUDA_ARCH__
   i64 d;

@@ -126,8 +126,9 @@ void plaquette_start_fx(gf_ctx* ctx, const gf_field* F, int slot) {
 // by rows), and TA(M^dag) = -TA(M).
 // Bound by integer multiply-add issue (IMAD.WIDE holds the issue port for
 // four cycles: 81 per row product, 13 products). 24^4, conversion included:
-// 4.71 ms in fp64 arithmetic, 0.70 ms here. Seven blocks per SM (80
-// registers) measured 0.70 ms, six 0.73, five 0.74, eight (spills) 0.72.
+// 4.71 ms in fp64 arithmetic, 0.71 ms here. Seven blocks per SM (80
+// registers) measured 0.71 ms, six 0.75; before links could be graded 0.70,
+// 0.73, five 0.74, eight (spills) 0.72.
 // Links with an fp64 slot among their staples: force_rows64, in the block's
 // first 96 threads.
 __device__ __noinline__ void force_rows64(const FxField U, double* P, const Geom& g, int mu, int s0, double coef,

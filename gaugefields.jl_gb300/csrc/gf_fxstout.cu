@@ -4,8 +4,9 @@
 // two warps evaluate the Cayley-Hamilton series with a thread per link (real
 // and imaginary parts), exchanging through shared memory. The kernels
 // are bound by integer multiply-add issue. A two-level smearing with its
-// adjoint at 16^4: 9.65 ms in fp64 arithmetic, 1.67 ms here (1.4 ms of it in
-// these kernels), at no larger an error (gradient 4.3e-16 against 4.8e-16).
+// adjoint at 16^4: 9.65 ms in fp64 arithmetic, 1.69 ms here (1.4 ms of it in
+// these kernels), at no larger an error (gradient 4.3e-16 against 4.8e-16 of
+// the largest entry).
 #include "gf_internal.h"
 #include "fxrows64.cuh"
 #include <cstddef>

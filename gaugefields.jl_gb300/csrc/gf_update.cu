@@ -267,7 +267,7 @@ __device__ __noinline__ void update_link64(const double2* Uin, double2* Uout, co
 #define GF_FX_UPDATE_MINB 4
 #endif
 // W = exp(i eps P) U on fp64 links (Uin, Uout may be the same field). Bound by
-// integer issue: 48^4 4.51 ms, where the double-float kernel took 7.18 ms and
+// integer issue: 48^4 4.55 ms, where the double-float kernel took 7.18 ms and
 // the fp64 one 20 ms; four blocks per SM (128 registers) against 4.88 ms with
 // two or three, and 7.85 ms for a row of the link per thread, whose series and
 // row-after-row re-unitarisation leave warps waiting at barriers. Against

@@ -43,8 +43,10 @@ extern "C" {
 #define GF_MAT32 5  /* general 3x3 complex per link, fp32 */
 
 /* precision of the force / stout path */
-#define GF_FP64 0  /* plain form: fp64 fields, arithmetic of fp64 class (errors
-                       no larger than fp64's, in 64-bit block fixed point) */
+#define GF_FP64 0  /* plain form: fp64 fields, arithmetic of fp64 class: 64-bit
+                       block fixed point, errors no larger than fp64's relative
+                       to a matrix's norm, and fp64 for matrices whose small
+                       entries form a pattern (weak fields) */
 #define GF_MIXED 1 /* fp32 force and stout (12-real links), fp64 H / updates */
 #define GF_DFLOAT 2 /* as GF_FP64, but the stout stacks of lattices of more
                        than 2^21 sites in double-float arithmetic (fp32 pairs,
