@@ -483,7 +483,8 @@ GF_HD bool fx_has_f64(int e) { return e >= GF_FX_F64_SUM; }
 // with such a pattern is "graded": its slot keeps fp64, and what it enters is
 // computed in fp64. Exact zeros lose nothing, so entries below 2^-7 must
 // include one that is not zero. A Haar-random link is graded with probability
-// 10^-10 (each of its 18 numbers is small with probability 0.015).
+// 8 10^-8 (8 of 10^8 drawn; an entry close to the unit circle makes the rest of
+// its row and column small): one in three 32^4 configurations.
 // small: bit i for entry i below 2^-7 2^(unit - 1023); returns whether they form
 // a pattern (zeros included).
 GF_HD bool fx_small_pattern(unsigned small) {

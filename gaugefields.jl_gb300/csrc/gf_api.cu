@@ -53,12 +53,10 @@ static void set_err(const gf_ctx* ctx, const std::string& m) {
 // One call of a context at a time: calls share its scratch (the fixed-point copy
 // of the links, partial sums, staging, stacks) from their first launch to their
 // last, and a caller's threads may share the context.
-static std::unique_lock<std::recursive_mutex> lock_of(gf_ctx* ctx) {
-  return ctx ? std::unique_lock<std::recursive_mutex>(ctx->calls) : std::unique_lock<std::recursive_mutex>();
-}
-#define API_BEGIN(ctx)                      \
-  const auto one_call_ = lock_of(ctx);      \
-  try {
+#define API_BEGIN(ctx)                                                 \
+  std::unique_lock<std::recursive_mutex> one_call_;                    \
+  try {                                                                \
+    if (ctx) one_call_ = std::unique_lock<std::recursive_mutex>((ctx)->calls);
 #define API_END(ctx)                           \
   }                                            \
   catch (const gf_error& e) {                  \
