@@ -203,7 +203,10 @@ GF_HD i64 fx_rsqrt(i64 m, float y0) {
   return y;
 }
 
-// A kernel parameter c = (h 2^30 + l) 2^(e - 60), |h 2^30 + l| < 2^60
+// A kernel parameter c = (h 2^30 + l) 2^(e - 60), |h 2^30 + l| < 2^60. Zero has the
+// exponent GF_FX_ZERO, below any other, so that a sum with something that it
+// scales is not aligned to what it scales.
+#define GF_FX_ZERO (-(1 << 18))
 struct fx_scalar {
   int h, l, e;
 };
@@ -213,7 +216,7 @@ inline fx_scalar fx_scalar_of(double c) {
   if (!(m == m) || m - m != 0.0) return fx_scalar{0, 0, GF_FX_BAD};
   fx_scalar s;
   fx_split<0>((i64)ldexp(m, 60), s.h, s.l);
-  s.e = m == 0.0 ? 0 : e;
+  s.e = m == 0.0 ? GF_FX_ZERO : e;
   return s;
 }
 GF_HD fx_num fx_num_of(const fx_scalar& s) { return fx_num{s.h, s.l}; }

@@ -60,6 +60,39 @@ def test_forces_to_each_links_own_size(pkg, oracle, L, coefficients):
     assert (np.abs(F.to_host() - ref).max(axis=-1) <= 1e-13 * size).all()
 
 
+@pytest.mark.parametrize("coefficients", [(0.0, 1.0), (1e-8, 1.0), (1.0, 1e-8)])
+@pytest.mark.parametrize("L", SIZES)
+def test_a_small_coefficient_leaves_the_other_term_its_digits(pkg, oracle, L, coefficients):
+    """Factors of e^-20 .. e^20: plaquette staples that dwarf the rectangle ones,
+    but for their coefficient."""
+    Uh, n = scaled(oracle, L, 20)
+    U = pkg.gauge_configuration(L, start="cold").from_host(Uh)
+    action = pkg.GaugeAction(U)
+    for c, loop in zip(coefficients, ("plaquette", "rectangular")):
+        pkg.push_(action, c, loop)
+    F = pkg.gauge_momenta(U)
+    pkg.md_force_(F, action, U)
+    ref = oracle.force_loops(list(L), Uh, *coefficients)
+    size = sum(abs(c) * loops_through(L, n, s) for c, s in zip(coefficients, (1, 2)))
+    assert (np.abs(F.to_host() - ref).max(axis=-1) <= 1e-13 * size).all()
+
+
+@pytest.mark.parametrize("L", SIZES)
+def test_the_adjoint_of_no_smearing_is_the_derivative_itself(pkg, oracle, L):
+    """rho = 0 on links off the group by e^-5 .. e^5: what rho multiplies is up to
+    e^10 times larger."""
+    Uh, _ = scaled(oracle, L, 5)
+    U = pkg.gauge_configuration(L, start="cold").from_host(Uh)
+    net = pkg.CovNeuralnet(U)
+    pkg.push_(net, pkg.STOUT_Layer("plaquette", 0.0))
+    rng = np.random.RandomState(2)
+    d = rng.normal(size=Uh.shape) + 1j * rng.normal(size=Uh.shape)
+    D = pkg.Gaugefields4D(U.ctx, pkg._lib.GF_MAT64).from_host(d)
+    _, history, _ = pkg.calc_smearedU(U, net)
+    got = pkg.back_prop(D, net, history, U).to_host()
+    assert np.abs(got - d).max() <= 1e-15 * np.abs(d).max()
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("reunit", [False, True])
 @pytest.mark.parametrize("kind", ["unitary", "scaled", "weak"])
