@@ -293,6 +293,9 @@ GF_HD void fx_invariants(const fx_herm& q, i64& c0, i64& c1) {
   c0 = fx_get(det) + 2 * fx_get(r);
 }
 
+// Beyond |X| = 2^53 the phases of exp(iX) are lost in the rounding of X, in any
+// arithmetic of this size: the result is a NaN.
+#define GF_FX_MAX_POW2 53
 // How to sum the series for a norm bound lam of X (real).
 struct fx_plan {
   int pow2;     // q = X / 2^pow2

@@ -143,6 +143,16 @@ __device__ __forceinline__ void store_field64(const Sh64& m, char* p, int mu, in
   fx_store64(p, mu, s, V, e);
 }
 
+// halvings that bring |X| to 1, from |X|^2 <= (2/3) tr X^2; at most one more than
+// leave the phases of exp(iX) any digit, and none for what is not finite
+__device__ __forceinline__ int halvings64(double trx2) {
+  int n = 0;
+  for (double x = trx2 * (2.0 / 3.0); x > 1.0 && n <= GF_FX_MAX_POW2 && x <= 1.7976931348623157e308; x *= 0.25) ++n;
+  return n;
+}
+__device__ __forceinline__ double halve64(int n) {
+  return n > GF_FX_MAX_POW2 ? __longlong_as_double(0x7FF8000000000000ll) : scalbn(1.0, -n);
+}
 // X = -i TA(rho m) of a matrix, Hermitian, and the halvings that bring |X| to 1
 __device__ __forceinline__ mat3<double> ta_herm64(const Sh64& m, double rho, int& halvings) {
   mat3<double> q;
@@ -160,11 +170,8 @@ __device__ __forceinline__ mat3<double> ta_herm64(const Sh64& m, double rho, int
       n2 += 2.0 * (q.e[i][j].re * q.e[i][j].re + q.e[i][j].im * q.e[i][j].im);
     }
   }
-  halvings = 0;
-  // |X|^2 <= (2/3) tr X^2; none for what is not finite
-  for (double x = n2 * (2.0 / 3.0); x > 1.0 && x <= 1.7976931348623157e308; x *= 0.25) ++halvings;
-  const double h = scalbn(1.0, -halvings);
-  return scale(h, q);
+  halvings = halvings64(n2);
+  return scale(halve64(halvings), q);
 }
 
 }  // namespace gf

@@ -156,13 +156,13 @@ __global__ void __launch_bounds__(GF_FX_THREADS * AXES, MINB)
     }
   }
   const bool any64 = __syncthreads_or(f64);
-  const int E0 = sh.e[link];
   if (threadIdx.x < 64) {
     int e;
     const fx_herm q = fx_ta_herm(sh, t & 31, rho, rho3, e);
     fx_exp_coefficients<false>(sh, nullptr, t & 31, t >> 5, q, e);
   }
   __syncthreads();
+  const int E0 = sh.s[link] > GF_FX_MAX_POW2 ? GF_FX_BAD : sh.e[link];
   if (AXES > 1 && axis > 0) {
     // the other axes' threads only keep step with the squarings' barriers
     for (int k = 0; k < 2 * sh.most; ++k) __syncthreads();

@@ -245,10 +245,9 @@ __device__ __noinline__ void update_link64(const double2* Uin, double2* Uout, co
 #pragma unroll
     for (int j = 0; j < i; ++j) q.e[i][j] = conj(q.e[j][i]);
   }
-  // |X|^2 <= (2/3) tr X^2: halved to |X| <= 1, and squared afterwards
-  int halvings = 0;
-  for (double x = n2 * (2.0 / 3.0); x > 1.0 && x <= 1.7976931348623157e308; x *= 0.25) ++halvings;
-  mat3<double> E = expiq(scale(scalbn(1.0, -halvings), q));
+  // halved to |X| <= 1, and squared afterwards
+  const int halvings = halvings64(n2);
+  mat3<double> E = expiq(scale(halve64(halvings), q));
 #pragma unroll 1
   for (int k = 0; k < halvings; ++k) E = mul_nn(E, E);
   u = mul_nn(E, u);
@@ -302,7 +301,7 @@ __global__ void __launch_bounds__(128, GF_FX_UPDATE_MINB)
     }
     eu = fx_from_f64_fast(m, u, small, unit);
   }
-  if (e > GF_FX_BAD / 2) eu = GF_FX_BAD;
+  if (e > GF_FX_BAD / 2 || plan.pow2 > GF_FX_MAX_POW2) eu = GF_FX_BAD;
   fx_acc w[3];
   const FxHermMat qm{q};
   if (plan.squares == 0) {
@@ -419,7 +418,7 @@ __global__ void __launch_bounds__(GF_FX_THREADS, 4)
     if (r == 0) {
 #pragma unroll
       for (int el = 0; el < 9; ++el) sh.x.q.v[el][link] = fx_herm_element(q, el / 3, el % 3);
-      sh.x.e[link] = e;
+      sh.x.e[link] = plan.pow2 > GF_FX_MAX_POW2 ? GF_FX_BAD : e;
       sh.x.g[link] = plan.guard;
       sh.x.sq[link] = plan.squares;
       const int most = __reduce_max_sync(0xffffffffu, plan.squares);

@@ -108,3 +108,29 @@ def test_a_force_far_off_the_group(pkg, oracle):
     P = pkg.update_momenta_(pkg.gauge_momenta(U), U, 1.0, pkg.md_driver(U, action, steps=1, smearing=net))
     assert 20 < x < 80
     assert np.abs(P.to_host() - want).max() <= 1e-13 * x * np.abs(want).max()
+
+
+def test_exponents_without_digits_give_no_number(pkg):
+    """|X| beyond 2^53: the phases are lost in the rounding of X. Smeared links,
+    gradients and updated links are NaN and not some unitary matrix."""
+    for rho, links in ((1e20, "hot"), (1e20, "weak")):
+        U = pkg.gauge_configuration(L, start="hot", seed=4)
+        if links == "weak":
+            x = U.to_host()
+            U.from_host(np.eye(3) + 1e-3 * (x - dag(x)))
+        net = pkg.CovNeuralnet(U)
+        pkg.push_(net, pkg.STOUT_Layer("plaquette", rho))
+        top, history, _ = pkg.calc_smearedU(U, net)
+        D = pkg.Gaugefields4D(U.ctx, pkg._lib.GF_MAT64).from_host(U.to_host())
+        assert np.isnan(top.to_host()).all()
+        assert np.isnan(pkg.back_prop(D, net, history, U).to_host()).any(axis=(-1, -2)).all()
+    for size in (L, (14, 8, 8, 8)):
+        for start in ("hot", "cold"):
+            U = pkg.gauge_configuration(size, start=start, seed=4)
+            action = pkg.GaugeAction(U)
+            pkg.push_(action, 3.0, "plaquette")
+            for reunit in (False, True):
+                W = U.similar().from_host(U.to_host())
+                pkg.update_gaugefields_(W, pkg.gaussian_momenta(U, seed=1), 1e20,
+                                        pkg.md_driver(U, action, steps=1, reunitarize=reunit))
+                assert np.isnan(W.to_host()).all()
